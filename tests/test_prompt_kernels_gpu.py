@@ -1,0 +1,71 @@
+"""Kernels that take many tokens of a prompt side by side, at the sizes where their tiles and chunks begin and end, against
+the 64-bit run of ``fake_ops.FakeOps`` (the operations token by token) and against their own answers for the same rows in
+other batches."""
+
+from __future__ import annotations
+
+import types
+
+import pytest
+import torch
+
+from fake_ops import FakeOps
+from mini_llm_runtime_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+DEVICE = "cuda:0"
+FAKE = FakeOps()
+UNIT = 2.0 ** -24          # relative rounding of one 32-bit operation
+
+
+def cuda():
+    return ops.current()
+
+
+def generator(seed):
+    return torch.Generator().manual_seed(seed)
+
+
+def rnd(seed, *shape, std=1.0):
+    return torch.randn(shape, generator=generator(seed)) * std
+
+
+def spaced(tensor, extra=4):
+    """The same rows as a column range of a wider product."""
+    wide = torch.full((tensor.shape[0], tensor.shape[1] + 2 * extra), float("nan"))
+    wide[:, extra:extra + tensor.shape[1]] = tensor
+    return wide.to(DEVICE)[:, extra:extra + tensor.shape[1]]
+
+
+def segments(lengths, slots, order=None):
+    """A ragged batch; ``order`` lists the requests in the order of their rows (as listed by default)."""
+    starts, at = [0] * len(lengths), 0
+    for index in order or range(len(lengths)):
+        starts[index] = at
+        at += lengths[index]
+    dev = lambda values: torch.tensor(values, dtype=torch.int32, device=DEVICE)      # noqa: E731
+    return types.SimpleNamespace(
+        seg_q_start=dev(starts), seg_q_len=dev(lengths), seg_slot=dev(slots), num_segments=len(lengths), max_q_len=max(lengths),
+        segments=[types.SimpleNamespace(row_start=a, length=n, slot=s) for a, n, s in zip(starts, lengths, slots)])
+
+
+def close(got, want, bound, what):
+    """Relative error in the 2-norm, of the whole and of the worst row."""
+    got, want = got.double().cpu().flatten(1), want.double().flatten(1)
+    assert torch.isfinite(got).all(), what
+    error = (got - want).norm(dim=1) / want.norm(dim=1).clamp_min(1e-3 * want.norm() / want.shape[0] ** 0.5)
+    assert float(error.max()) <= bound, f"{what}: {float(error.max()):.2e}, allowed {bound:.2e}"
+
+
+@pytest.mark.parametrize("n,k", [(130, 1023), (70, 2052), (33, 4101), (16400, 72)])
+def test_products_of_the_32_bit_path_do_not_depend_on_the_rows_beside(n, k):
+    """Row counts on both sides of every tile's edge; the sums' order is the same in every tile, so equal rows get equal bits."""
+    x, w, bias = rnd(1, 1100, k), rnd(2, n, k, std=0.2), rnd(3, n)
+    xd, wd, bd = x.to(DEVICE), w.to(DEVICE), bias.to(DEVICE)
+    whole = cuda().linear(xd, wd, bd)
+    # k products and sums, each rounded once: the error of an output is below k * UNIT times the sum of magnitudes
+    magnitude = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    assert bool(((whole.double().cpu() - (x.double() @ w.double().T + bias.double())).abs() <= k * UNIT * magnitude).all())
+    for rows in (1, 4, 16, 17, 32, 33, 63, 64, 65, 200):
+        assert torch.equal(cuda().linear(xd[5:5 + rows].contiguous(), wd, bd), whole[5:5 + rows]), rows
