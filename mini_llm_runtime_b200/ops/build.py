@@ -43,6 +43,7 @@ LIBRARIES: dict[str, tuple[str, ...]] = {
     "gemm_skinny": (),
     "attention_tcgen05": (),
     "sequence_mix": (),
+    "gated_chunks": (),
     "attention_diff": (),
     "attention_diff_mma": (),
     "stream32": (),

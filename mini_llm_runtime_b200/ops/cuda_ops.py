@@ -857,6 +857,11 @@ class CudaOps:
             raise KernelError(f"{name} must be a float32 CUDA view [{rows}, {width}] with unit column stride")
         return _ptr(tensor), ctypes.c_longlong(tensor.stride(0))
 
+    use_gated_chunks = True
+    # Longest portion of a step from which chunks pay.  Measured in us, walked by one CTA per head part / in chunks: 128 rows
+    # 37 / 41 (14 heads of 64), 44 / 42 (32 of 64), 44 / 55 (7 and 16 of 128); 512 rows 129 / 42, 135 / 46, 157 / 70.
+    GATED_CHUNK_ROWS = 192
+
     def _recurrence(self, mode, r, b, v, raw, gate, bias, aux, weight, eps, state, ctx, heads, dim, vdim, out_dtype):
         rows = r.shape[0]
         for name, vector, size in (("bias", bias, heads * dim), ("aux", aux, heads * dim),
@@ -869,14 +874,26 @@ class CudaOps:
             raise KernelError(f"state has shape {tuple(state.shape)}, expected [slots, {heads}, {dim}, {vdim}]")
         null = (ctypes.c_void_p(0), ctypes.c_longlong(0))
         out = torch.empty((rows, heads * vdim), dtype=out_dtype, device=r.device)
+        views = (*self._view(r, "r", rows, heads * dim), *(null if b is None else self._view(b, "b", rows, heads * dim)),
+                 *self._view(v, "v", rows, heads * vdim), *self._view(raw, "raw", rows, heads * dim),
+                 *(null if gate is None else self._view(gate, "gate", rows, heads * vdim)))
+        if (self.use_gated_chunks and ctx.max_q_len >= self.GATED_CHUNK_ROWS and dim == vdim and dim in (64, 128)
+                and all(t is None or (t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0) for t in (r, b, v, raw, gate))
+                and weight.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0):
+            # long segments: chunks of tokens side by side
+            lib = build.load_library("gated_chunks")
+            lib.mlr_gated_chunk_scratch.restype = ctypes.c_longlong
+            scratch = torch.empty(lib.mlr_gated_chunk_scratch(rows, heads, dim, vdim), dtype=torch.float32, device=r.device)
+            _check(lib.mlr_gated_recurrence_chunks(
+                mode, *views, _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out), _ptr(scratch),
+                _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len),
+                heads, dim, vdim, _code(out_dtype), _stream()), "gated_recurrence_chunks")
+            return out
         # steps with long segments, and heads too large for one CTA, spread a head's value channels
         # over CTAs and finish in a second kernel, which reads the un-normalised rows from here
         scratch = torch.empty((rows, heads * vdim), dtype=torch.float32, device=r.device) if vdim > 32 else None
         _check(build.load_library("sequence_mix").mlr_gated_recurrence(
-            mode, *self._view(r, "r", rows, heads * dim), *(null if b is None else self._view(b, "b", rows, heads * dim)),
-            *self._view(v, "v", rows, heads * vdim), *self._view(raw, "raw", rows, heads * dim),
-            *(null if gate is None else self._view(gate, "gate", rows, heads * vdim)),
-            _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out), _ptr(scratch),
+            mode, *views, _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out), _ptr(scratch),
             _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len),
             heads, dim, vdim, _code(out_dtype), _stream()),
             "gated_recurrence")

@@ -58,6 +58,42 @@ def close(got, want, bound, what):
     assert float(error.max()) <= bound, f"{what}: {float(error.max()):.2e}, allowed {bound:.2e}"
 
 
+CHUNKED = [([1, 64, 65, 200], [3, 0, 2, 1], None), ([193, 128, 63, 1, 127], [4, 1, 0, 2, 3], [3, 1, 4, 0, 2]), ([321], [0], None)]
+
+
+@pytest.mark.parametrize("mode", ["bonus", "forget"])
+@pytest.mark.parametrize("heads,dim", [(3, 64), (2, 128)])
+@pytest.mark.parametrize("lengths,slots,order", CHUNKED)
+def test_gated_recurrences_in_chunks(mode, heads, dim, lengths, slots, order):
+    """Segments around the borders of chunks of 64 tokens, rows of requests in any order, decays of zero and one."""
+    ctx, rows, n = segments(lengths, slots, order), sum(lengths), heads * dim
+    r, k, v, gate = (rnd(i, rows, n, std=0.7) for i in range(4))
+    raw, bias, weight = rnd(5, rows, n, std=0.5), rnd(6, n) * 2 - 2, 1 + rnd(7, n, std=0.1)
+    raw[rows // 3, : n // 2], raw[rows // 2, n // 2:] = 60.0, -60.0        # decays of 0 and of 1 (lower bound and 1)
+    aux = torch.rand(n, generator=generator(8)) if mode == "forget" else rnd(8, n, std=0.3)
+    state = rnd(9, len(lengths), heads, dim, dim, std=0.5)
+    want_state, got_state = state.double(), state.to(DEVICE)
+    # a row's result is a sum over the channels of products that went through up to CHUNK decays; 64 roundings each way, and
+    # the norm's and gate's own, stay below 200 roundings in the 2-norm of a row
+    bound = 200 * UNIT
+    for dtype in (torch.float32, torch.bfloat16):
+        got_state.copy_(state)
+        if mode == "bonus":
+            want_state = state.double()
+            want = FAKE.bonus_recurrence(*(t.double() for t in (r, k, v, raw, gate, bias, aux, weight)), 1e-6, want_state, ctx,
+                                         heads, dim, torch.float32)
+            got = cuda().bonus_recurrence(*(spaced(t) for t in (r, k, v, raw, gate)), *(t.to(DEVICE) for t in (bias, aux, weight)),
+                                          1e-6, got_state, ctx, heads, dim, dtype)
+        else:
+            want_state = state.double()
+            want = FAKE.forget_gate_recurrence(*(t.double() for t in (r, raw, v, bias, aux, weight[:dim])), 1e-6, want_state, ctx,
+                                               heads, dim, dim, torch.float32)
+            got = cuda().forget_gate_recurrence(*(spaced(t) for t in (r, raw, v)), bias.to(DEVICE), aux.to(DEVICE),
+                                                weight[:dim].contiguous().to(DEVICE), 1e-6, got_state, ctx, heads, dim, dim, dtype)
+        close(got, want, bound if dtype == torch.float32 else 2.0 ** -8, f"{mode} {dtype}")
+        close(got_state.flatten(0, 1), want_state.flatten(0, 1), bound, f"{mode} state")
+
+
 @pytest.mark.parametrize("n,k", [(130, 1023), (70, 2052), (33, 4101), (16400, 72)])
 def test_products_of_the_32_bit_path_do_not_depend_on_the_rows_beside(n, k):
     """Row counts on both sides of every tile's edge; the sums' order is the same in every tile, so equal rows get equal bits."""
