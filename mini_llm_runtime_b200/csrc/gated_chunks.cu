@@ -16,11 +16,10 @@
 // 64): bound by the latency of that chain.  Walked in chunks it is bound by instructions issued: three operations per state
 // entry and token in the walk, one in finish.  2,048 tokens of one request, B200: 761 -> 63 us (14 heads of 64), 768 -> 114
 // (32 of 64), 608 -> 88 (7 of 128), 709 -> 158 (16 of 128).
+#include "chunk_places.cuh"
 #include "copy_async.cuh"
 
 namespace mlr {
-
-constexpr int CHUNK = 64;
 
 struct ChunkArgs {
   const float *r, *b, *v, *raw, *gate;           // row-major views, one row per token; rows of whole 16-byte pieces
@@ -36,11 +35,6 @@ struct ChunkArgs {
   int heads, weight_per_head;
 };
 
-// Where a chunk that starts at `row` keeps its state: one place per aligned run of CHUNK rows for a segment's first
-// chunk and one for another chunk.  Among segments of several chunks (the only ones with places) no two chunks share one: a
-// second first chunk in the run would start more than CHUNK rows after the first, and so would a second later chunk.
-__device__ __forceinline__ size_t chunk_place(int row, bool first) { return 2 * (size_t)(row / CHUNK) + (first ? 1 : 0); }
-
 // Thread (lane, warp) walks key channels [16 * slice, +16) of C neighbouring value channels; T tokens at a time are
 // staged (16-byte asynchronous copies, the next T under the walk over these) and transformed in place.
 template <int MODE, int DIM, int VDIM>
@@ -52,24 +46,6 @@ struct WalkShape {
   static constexpr int STAGE = T * (3 * DIM + VDIM);     // r, a, b, v of T tokens
   static constexpr size_t SHARED = sizeof(float) * (2 * (size_t)STAGE + (size_t)SLICES * T * VDIM + T);
 };
-
-template <int C>
-__device__ __forceinline__ void load_columns(float (&v)[C], const float* src) {
-  if constexpr (C == 2) {
-    const float2 q = *reinterpret_cast<const float2*>(src);
-    v[0] = q.x, v[1] = q.y;
-  } else {
-    const float4 q = *reinterpret_cast<const float4*>(src);
-    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-  }
-}
-template <int C>
-__device__ __forceinline__ void store_columns(float* dst, const float (&v)[C]) {
-  if constexpr (C == 2)
-    *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
-  else
-    *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-}
 
 template <int MODE, int DIM, int VDIM>
 __global__ void __launch_bounds__(WalkShape<MODE, DIM, VDIM>::THREADS)
@@ -386,10 +362,10 @@ using namespace mlr;
 
 MLR_DEFINE_PDL_SWITCH
 
-// float32 scratch of a step, in numbers: the walk's outputs, its reads, and for up to 2 * (rows / CHUNK + 1) chunks their end
-// states and decay products.
+// float32 scratch of a step, in numbers: the walk's outputs, its reads, and per chunk place an end
+// state and decay products.
 MLR_EXPORT long long mlr_gated_chunk_scratch(int rows, int heads, int dim, int vdim) {
-  return (long long)heads * ((long long)rows * (dim + vdim) + 2ll * (rows / CHUNK + 1) * dim * (vdim + 1));
+  return (long long)heads * ((long long)rows * (dim + vdim) + chunk_places(rows) * dim * (vdim + 1));
 }
 
 // As mlr_gated_recurrence, for square heads of 64 or 128 and inputs (state, weights, output and scratch too) whose rows begin
@@ -415,7 +391,7 @@ MLR_EXPORT int mlr_gated_recurrence_chunks(int mode, const float* r, long long r
   args.outputs = scratch;
   args.reads = args.outputs + (size_t)rows * heads * vdim;
   args.ends = args.reads + (size_t)rows * heads * dim;
-  args.decays = args.ends + (size_t)2 * (rows / CHUNK + 1) * heads * dim * vdim;
+  args.decays = args.ends + (size_t)chunk_places(rows) * heads * dim * vdim;
   args.seg_q_start = seg_q_start; args.seg_q_len = seg_q_len; args.seg_slot = seg_slot;
   args.heads = heads; args.weight_per_head = mode == 0 ? 1 : 0;
   if (mode == 0) return launch_chunks<0>(args, out, segments, max_q_len, dim, vdim, out_dtype, stream);

@@ -54,6 +54,7 @@ LIBRARIES: dict[str, tuple[str, ...]] = {
     "attention_sigmoid": (),
     "attention_sigmoid_mma": (),
     "state_space": (),
+    "state_space_chunks": (),
     "delta_rule": (),
     "attention_shaped_mma": (),
     "matrix_memory": (),

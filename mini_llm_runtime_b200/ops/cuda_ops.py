@@ -1895,6 +1895,11 @@ class CudaOps:
             int(activation == "silu"), _stream()), "causal_conv")
         return out
 
+    use_state_space_chunks = True
+    # Longest portion of a step from which chunks pay.  Measured in us, token by token / in chunks: 128 rows 30 / 31 (14 heads,
+    # states of 64), 42 / 50 (32 heads, states of 128); 512 rows 108 / 31, 161 / 64.
+    STATE_SPACE_CHUNK_ROWS = 192
+
     def state_space_scan(self, x, B, C, dt_raw, dt_bias, A_log, D, state, ctx, heads: int, vdim: int, n: int,
                          groups: int) -> torch.Tensor:
         """Per request and head h (group g = h // (heads / groups)), token by token: dt = softplus(dt_raw +
@@ -1910,9 +1915,21 @@ class CudaOps:
         if tuple(state.shape[1:]) != (heads, vdim, n):
             raise KernelError(f"state has shape {tuple(state.shape)}, expected [slots, {heads}, {vdim}, {n}]")
         y = torch.empty((rows, heads * vdim), dtype=torch.float32, device=x.device)
+        views = (*self._view(x, "x", rows, heads * vdim), *self._view(B, "B", rows, groups * n),
+                 *self._view(C, "C", rows, groups * n), *self._view(dt_raw, "dt_raw", rows, heads))
+        if (self.use_state_space_chunks and ctx.max_q_len >= self.STATE_SPACE_CHUNK_ROWS and vdim == 64 and n in (64, 128)
+                and all(t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0 for t in (x, B, C)) and state.data_ptr() % 16 == 0):
+            # long segments: chunks of tokens side by side
+            lib = build.load_library("state_space_chunks")
+            lib.mlr_state_space_chunk_scratch.restype = ctypes.c_longlong
+            scratch = torch.empty(lib.mlr_state_space_chunk_scratch(rows, heads, n, groups), dtype=torch.float32, device=x.device)
+            _check(lib.mlr_state_space_chunks(
+                *views, _ptr(dt_bias), _ptr(A_log), _ptr(D), _ptr(state), _ptr(y), _ptr(scratch), _ptr(ctx.seg_q_start),
+                _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), heads, vdim, n, groups,
+                _stream()), "state_space_chunks")
+            return y
         _check(build.load_library("state_space").mlr_state_space_scan(
-            *self._view(x, "x", rows, heads * vdim), *self._view(B, "B", rows, groups * n),
-            *self._view(C, "C", rows, groups * n), *self._view(dt_raw, "dt_raw", rows, heads), _ptr(dt_bias), _ptr(A_log),
+            *views, _ptr(dt_bias), _ptr(A_log),
             _ptr(D), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot),
             ctx.num_segments, heads, vdim, n, groups, _stream()), "state_space_scan")
         return y

@@ -105,3 +105,21 @@ def test_products_of_the_32_bit_path_do_not_depend_on_the_rows_beside(n, k):
     assert bool(((whole.double().cpu() - (x.double() @ w.double().T + bias.double())).abs() <= k * UNIT * magnitude).all())
     for rows in (1, 4, 16, 17, 32, 33, 63, 64, 65, 200):
         assert torch.equal(cuda().linear(xd[5:5 + rows].contiguous(), wd, bd), whole[5:5 + rows]), rows
+
+
+@pytest.mark.parametrize("heads,n,groups", [(4, 64, 1), (6, 128, 2)])
+@pytest.mark.parametrize("lengths,slots,order", CHUNKED)
+def test_state_space_in_chunks(heads, n, groups, lengths, slots, order):
+    """Segments around the borders of chunks; decays from zero to one, among them tokens that neither keep nor forget."""
+    ctx, rows, inner = segments(lengths, slots, order), sum(lengths), heads * 64
+    x, B, C, dt = rnd(1, rows, inner), rnd(2, rows, groups * n), rnd(3, rows, groups * n), rnd(4, rows, heads, std=2.0)
+    dt[rows // 3], dt[rows // 2] = 90.0, -90.0
+    dt_bias, a_log, skip = rnd(5, heads), rnd(6, heads), rnd(7, heads)
+    state = rnd(8, len(lengths), heads, 64, n, std=0.5)
+    want_state, got_state = state.double(), state.to(DEVICE)
+    want = FAKE.state_space_scan(*(t.double() for t in (x, B, C, dt, dt_bias, a_log, skip)), want_state, ctx, heads, 64, n, groups)
+    got = cuda().state_space_scan(*(spaced(t) for t in (x, B, C, dt)), *(t.to(DEVICE) for t in (dt_bias, a_log, skip)), got_state,
+                                  ctx, heads, 64, n, groups)
+    # sums of up to n + CHUNK products of numbers that went through up to CHUNK decays each
+    close(got, want, 200 * UNIT, "state-space outputs")
+    close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "state-space state")
