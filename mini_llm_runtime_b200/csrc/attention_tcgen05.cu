@@ -52,19 +52,28 @@ constexpr uint32_t FA_TMEM_O = 2 * FA_KEYS;
 constexpr int FA_P_BYTES = FA_ROWS * FA_KEYS * 2;          // one tile of probabilities
 constexpr float FA_LAZY = 8.f;      // the base exponent follows the running max in steps of more than this
 
-// Sizes that depend on the head size.  With 128 the shared memory of two resident CTAs only fits
-// with a two-stage ring and one buffer of probabilities.
-template <int D>
+// Sizes that depend on the head sizes (D of queries and keys, DV of values).  With 128 the shared memory of two
+// resident CTAs only fits with a two-stage ring and one buffer of probabilities.
+template <int D, int DV>
 struct FaShape {
-  static constexpr int HALVES = D / 64;                      // 64-wide (128-byte) column blocks of a row
-  static constexpr int STAGES = D == 64 ? 4 : 2;
+  static constexpr int HALVES = D / 64, V_HALVES = DV / 64;  // 64-wide (128-byte) column blocks of a row
+  static constexpr int STAGES = D + DV == 128 ? 4 : D + DV == 192 ? 3 : 2;
   static constexpr int P_BUFFERS = 1;
   static constexpr int Q_BYTES = FA_ROWS * D * 2;
   static constexpr int Q_HALF_BYTES = FA_ROWS * 128;
-  static constexpr int KV_TILE_BYTES = FA_KEYS * D * 2;      // one K or V tile
+  static constexpr int K_TILE_BYTES = FA_KEYS * D * 2, V_TILE_BYTES = FA_KEYS * DV * 2;
+  static constexpr int STAGE_BYTES = K_TILE_BYTES + V_TILE_BYTES;      // a K tile, then a V tile
   static constexpr int KV_HALF_BYTES = FA_KEYS * 128;
-  static constexpr int DATA_BYTES = Q_BYTES + P_BUFFERS * FA_P_BYTES + STAGES * 2 * KV_TILE_BYTES;
+  static constexpr int DATA_BYTES = Q_BYTES + P_BUFFERS * FA_P_BYTES + STAGES * STAGE_BYTES;
 };
+
+// What a launch computes: softmax attention, the same with shaped scores, or the two maps of a differential attention
+// (a map is a head of its own here: head = 2 * head + map; keys hold the maps side by side; the normalised rows
+// leave as float32, and the first `keep` positions stay visible beside the window).  The maps' walk over the keys is
+// the softmax threads' like any head's; on mma.sync it was bound by fragment loads, one query tile's K and V fetched per
+// (head, map), and by a combination of 32 CTAs: 2,048 rows, window 1,024, 7 heads of 2 x 64 with values of 128: 290 -> 55 us,
+// 16 heads: 595 -> 72 us (0.027 -> 0.22 of 1,590 TFLOP/s for the latter).
+enum FaMode { FA_PLAIN, FA_SHAPED, FA_MAPS };
 
 // Barriers and the few words the warps share; behind the tiles in dynamic shared memory.
 struct FaControl {
@@ -160,6 +169,7 @@ struct FaScore {
   const float *slopes, *sinks;      // [heads] or null
   const bf16* gate;                 // rows of heads * D, or null
   long long gate_stride;
+  int keep;                         // maps only: positions that are always visible
 };
 
 // A row's 64 raw scores to shaped ones.  tanh as an odd polynomial in the raw score (its Taylor series): up to
@@ -254,10 +264,10 @@ __device__ __forceinline__ void fa_store32(bf16* dst, const float* v, float fact
   }
 }
 
-template <int D, bool SHAPED>
+template <int D, int DV, int MODE>
 __global__ void __launch_bounds__(FA_THREADS, 2)      // two CTAs per SM: at most 204 registers
 prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
-                                 const __grid_constant__ CUtensorMap v_map, bf16* __restrict__ out,
+                                 const __grid_constant__ CUtensorMap v_map, void* __restrict__ out,
                                  const int* __restrict__ tile_seg, const int* __restrict__ tile_row0,
                                  const int* __restrict__ seg_q_start, const int* __restrict__ seg_q_len,
                                  const int* __restrict__ seg_pos0, const int* __restrict__ block_table, const int* __restrict__ seg_slot,
@@ -265,8 +275,9 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
                                  int page_shift, int window, float scale_log2, int* queue, int* error_word,
                                  int max_parts, int tiles_per_unit, float* __restrict__ scratch,
                                  int* __restrict__ counters, int shared_bytes, const FaScore score) {
-  using Shape = FaShape<D>;
+  using Shape = FaShape<D, DV>;
   constexpr int STAGES = Shape::STAGES;
+  constexpr bool SHAPED = MODE == FA_SHAPED, MAPS = MODE == FA_MAPS;
   extern __shared__ uint8_t fa_shared_raw[];
   uint8_t* aligned = (uint8_t*)(((uintptr_t)fa_shared_raw + 1023) & ~(uintptr_t)1023);
   if (aligned + Shape::DATA_BYTES + FA_CONTROL_BYTES > fa_shared_raw + shared_bytes) {
@@ -277,7 +288,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   uint8_t* q_tile = aligned;                                                         // [halves][128][64]
   uint8_t* p_tiles = aligned + Shape::Q_BYTES;                                       // P_BUFFERS x [128][64]
   uint8_t* kv_ring = p_tiles + Shape::P_BUFFERS * FA_P_BYTES;                        // STAGES x (K, V), each [halves][64][64]
-  FaControl& ctl = *reinterpret_cast<FaControl*>(kv_ring + STAGES * 2 * Shape::KV_TILE_BYTES);
+  FaControl& ctl = *reinterpret_cast<FaControl*>(kv_ring + STAGES * Shape::STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -318,7 +329,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
     if (unit >= total_units) break;
     const int part = unit / total_items, item = unit - part * total_items;
     const int tile = item / heads, head = item - tile * heads;
-    const int kv_head = head / (heads / kv_heads);
+    const int kv_head = head / (heads / kv_heads), key_column = MAPS ? (head & 1) * D : 0;
     const int seg = tile_seg[tile], row0 = tile_row0[tile];
     const int q_start = seg_q_start[seg], q_len = seg_q_len[seg], pos0 = seg_pos0[seg];
     const int rows = min(FA_ROWS, q_len - row0);
@@ -332,15 +343,23 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
     const int lowest = lowest_of(first_pos);
     // An item with many key tiles is cut into parts of equal length; each part is a unit of its
     // own (its state goes to scratch memory, the part that finishes last merges them in part order).
-    const int item_begin = lowest / FA_KEYS, item_tiles = last_pos / FA_KEYS - item_begin + 1;
+    // The key tiles of an item: those of its window, behind those that only hold kept positions.
+    const int item_begin = lowest / FA_KEYS;
+    const int kept_tiles = MAPS ? min((score.keep + FA_KEYS - 1) / FA_KEYS, item_begin) : 0;
+    const int item_tiles = kept_tiles + last_pos / FA_KEYS - item_begin + 1;
     const int parts = min(max_parts, (item_tiles + tiles_per_unit - 1) / tiles_per_unit);
     if (part >= parts) {
       __syncthreads();              // ctl.item is rewritten by the next draw
       continue;
     }
     const int per_part = (item_tiles + parts - 1) / parts;
-    const int tile_begin = item_begin + part * per_part;
+    const int tile_begin = (MAPS ? 0 : item_begin) + part * per_part;
     const int tiles = min(per_part, item_tiles - part * per_part);
+    auto first_key = [&](int j) {      // of the part's j-th key tile
+      const int at = tile_begin + j;
+      return (!MAPS || at < kept_tiles ? at : at - kept_tiles + item_begin) * FA_KEYS;
+    };
+    auto visible_to_item = [&](int key) { return key <= last_pos && (key >= lowest || (MAPS && key < score.keep)); };
 
     if (warp == 5) {
       // ------------------------------------------------------------ loads
@@ -351,8 +370,8 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       // reads, waits and the issue of up to 16 bulk copies per key tile took the MMA warp longer
       // than the softmax takes, when it did both.)
       auto lookup = [&](int j) -> int {                     // the page, or -1
-        if (j >= tiles || lane >= boxes * Shape::HALVES) return -1;
-        const int logical = ((tile_begin + j) * FA_KEYS + (lane % boxes) * box_rows) >> page_shift;
+        if (j >= tiles || lane >= boxes * (Shape::HALVES > Shape::V_HALVES ? Shape::HALVES : Shape::V_HALVES)) return -1;
+        const int logical = (first_key(j) + (lane % boxes) * box_rows) >> page_shift;
         return logical < table_width ? table[logical] : -1;
       };
       auto load_tile = [&](int j, int page, bool values) {
@@ -363,16 +382,16 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         if (use > 0) fa_wait(values ? &ctl.pv_done[stage] : &ctl.qk_done[stage], (use - 1) & 1u, error_word, 0x61, gave_up);
         gave_up = __any_sync(0xffffffffu, gave_up);
         if (gave_up) return;
-        if (lane == 0) mbar_expect_tx(full, (uint32_t)Shape::KV_TILE_BYTES);
+        if (lane == 0) mbar_expect_tx(full, (uint32_t)(values ? Shape::V_TILE_BYTES : Shape::K_TILE_BYTES));
         __syncwarp();
-        if (lane < boxes * Shape::HALVES) {
+        if (lane < boxes * (values ? Shape::V_HALVES : Shape::HALVES)) {
           const int box = lane % boxes, half = lane / boxes;
-          int offset = ((tile_begin + j) * FA_KEYS + box * box_rows) & (page_size - 1);
+          int offset = (first_key(j) + box * box_rows) & (page_size - 1);
           if (page < 0) { page = 0; offset = 0; }
           const int y = (page * kv_heads + kv_head) * page_size + offset;
-          uint8_t* dst = kv_ring + (size_t)stage * 2 * Shape::KV_TILE_BYTES + (values ? Shape::KV_TILE_BYTES : 0)
+          uint8_t* dst = kv_ring + (size_t)stage * Shape::STAGE_BYTES + (values ? Shape::K_TILE_BYTES : 0)
                          + half * Shape::KV_HALF_BYTES + box * box_rows * 128;
-          tma_load_2d(values ? &v_map : &k_map, full, dst, half * 64, y);
+          tma_load_2d(values ? &v_map : &k_map, full, dst, (values ? 0 : key_column) + half * 64, y);
         }
       };
       if (lane == 0) {
@@ -408,11 +427,11 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
     } else if (warp == 4) {
       // ------------------------------------------------------------ MMAs
       constexpr uint32_t idesc_qk = fa_idesc(FA_ROWS, FA_KEYS, false);
-      constexpr uint32_t idesc_pv = fa_idesc(FA_ROWS, D, true);
+      constexpr uint32_t idesc_pv = fa_idesc(FA_ROWS, DV, true);
       const uint32_t q_addr = smem_u32(q_tile), p_addr0 = smem_u32(p_tiles);
       // descriptors differ from tile to tile in their address field only (bytes / 16 in the low bits)
       const uint64_t q_desc = fa_desc_k_major(q_addr), kv_desc = fa_desc_k_major(smem_u32(kv_ring));
-      const uint64_t v_desc = fa_desc_mn_major(smem_u32(kv_ring) + Shape::KV_TILE_BYTES, Shape::KV_HALF_BYTES);
+      const uint64_t v_desc = fa_desc_mn_major(smem_u32(kv_ring) + Shape::K_TILE_BYTES, Shape::KV_HALF_BYTES);
       const uint64_t p_desc = fa_desc_k_major(p_addr0);
       auto issue_qk = [&](int j) {
         const unsigned t = tiles_before + (unsigned)j;
@@ -424,7 +443,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         gave_up = __any_sync(0xffffffffu, gave_up);
         fa_fence_after();
         if (lane == 0 && !gave_up) {
-          const uint64_t k_desc = kv_desc + (uint64_t)((stage * 2 * Shape::KV_TILE_BYTES) >> 4);
+          const uint64_t k_desc = kv_desc + (uint64_t)((stage * Shape::STAGE_BYTES) >> 4);
 #pragma unroll
           for (int k = 0; k < D / 16; ++k)
             fa_mma(tmem_base + buffer * FA_KEYS, q_desc + (uint64_t)(((k >> 2) * Shape::Q_HALF_BYTES + (k & 3) * 32) >> 4),
@@ -448,7 +467,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         gave_up = __any_sync(0xffffffffu, gave_up);
         fa_fence_after();
         if (lane == 0 && !gave_up) {
-          const uint64_t v_tile = v_desc + (uint64_t)((stage * 2 * Shape::KV_TILE_BYTES) >> 4);
+          const uint64_t v_tile = v_desc + (uint64_t)((stage * Shape::STAGE_BYTES) >> 4);
           const uint64_t p_tile = p_desc + (uint64_t)(((Shape::P_BUFFERS == 2 ? (t & 1u) : 0u) * FA_P_BYTES) >> 4);
 #pragma unroll
           for (int k = 0; k < FA_KEYS / 16; ++k)       // the output row accumulates over all key tiles of the unit
@@ -485,7 +504,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       for (int j = 0; j < tiles; ++j) {
         const unsigned t = tiles_before + (unsigned)j;
         const int buffer = t & 1, stage = t % STAGES;
-        const int key0 = (tile_begin + j) * FA_KEYS;
+        const int key0 = first_key(j);
         fa_wait(&ctl.qk_done[stage], (t / STAGES) & 1u, error_word, 0x66, gave_up);
         fa_fence_after();
         float s[FA_KEYS];
@@ -499,7 +518,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
 #pragma unroll
           for (int c = 0; c < FA_KEYS; ++c) {
             const int key = key0 + c;
-            if (!(key >= limit_lo && key <= limit_hi)) s[c] = -INFINITY;
+            if (!((key >= limit_lo || (MAPS && key < score.keep)) && key <= limit_hi)) s[c] = -INFINITY;
           }
         }
         // four interleaved chains of three-input max (one chain of dependent operations would cost
@@ -549,7 +568,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         if (rescale) {
           const float2 alpha2 = make_float2(alpha, alpha);
 #pragma unroll
-          for (int c = 0; c < D; c += 32) {
+          for (int c = 0; c < DV; c += 32) {
             float o[32];
             fa_tmem_load16(lane_base + FA_TMEM_O + c, reinterpret_cast<uint32_t*>(o));
             fa_tmem_load16(lane_base + FA_TMEM_O + c + 16, reinterpret_cast<uint32_t*>(o) + 16);
@@ -569,11 +588,11 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         if (key0 < lowest || key0 + FA_KEYS - 1 > last_pos) {
           // ragged tile: V rows of keys outside the range become zeros (this thread takes its share of rows)
           fa_wait(&ctl.v_full[stage], (t / STAGES) & 1u, error_word, 0x68, gave_up);
-          uint8_t* v_tile = kv_ring + (size_t)stage * 2 * Shape::KV_TILE_BYTES + Shape::KV_TILE_BYTES;
-          for (int idx = threadIdx.x; idx < FA_KEYS * 8 * Shape::HALVES; idx += FA_SOFTMAX_THREADS) {
+          uint8_t* v_tile = kv_ring + (size_t)stage * Shape::STAGE_BYTES + Shape::K_TILE_BYTES;
+          for (int idx = threadIdx.x; idx < FA_KEYS * 8 * Shape::V_HALVES; idx += FA_SOFTMAX_THREADS) {
             const int half = idx / (FA_KEYS * 8), within = idx - half * (FA_KEYS * 8);
             const int row = within >> 3;
-            if (key0 + row < lowest || key0 + row > last_pos)
+            if (!visible_to_item(key0 + row))
               *reinterpret_cast<uint4*>(v_tile + half * Shape::KV_HALF_BYTES + row * 128 + (within & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
           }
         }
@@ -601,7 +620,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         const unsigned t = tiles_before + (unsigned)tiles - 1;
         fa_wait(&ctl.pv_done[t % STAGES], (t / STAGES) & 1u, error_word, 0x69, gave_up);
         fa_fence_after();
-        constexpr int STATE = D + 2;
+        constexpr int STATE = DV + 2;
         // a part's state of row r: base exponent, sum, unnormalised output; laid out [value][row]
         // so that the 128 threads write and read neighbouring addresses
         float* states = scratch + (size_t)item * max_parts * STATE * FA_ROWS + r;
@@ -615,16 +634,26 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         const float inv = finish_factor(m_base, l);
         const bf16* gate = SHAPED && score.gate != nullptr && r < rows
                                ? score.gate + (size_t)(q_start + row0 + r) * score.gate_stride + (size_t)head * D : nullptr;
-        bf16* dst = out + ((size_t)(q_start + row0 + r) * heads + head) * D;
+        const size_t at = ((size_t)(q_start + row0 + r) * heads + head) * DV;
+        auto store32 = [&](int c, const float* o, float factor) {
+          if constexpr (MAPS) {
+            float4* dst = reinterpret_cast<float4*>((float*)out + at + c);
 #pragma unroll
-        for (int c = 0; c < D; c += 32) {
+            for (int e = 0; e < 8; ++e)
+              dst[e] = make_float4(o[4 * e] * factor, o[4 * e + 1] * factor, o[4 * e + 2] * factor, o[4 * e + 3] * factor);
+          } else {
+            fa_store32((bf16*)out + at + c, o, factor);
+          }
+        };
+#pragma unroll
+        for (int c = 0; c < DV; c += 32) {
           float o[32];
           fa_tmem_load16(lane_base + FA_TMEM_O + c, reinterpret_cast<uint32_t*>(o));
           fa_tmem_load16(lane_base + FA_TMEM_O + c + 16, reinterpret_cast<uint32_t*>(o) + 16);
           fa_tmem_wait_ld();
           if (parts == 1) {
             if (SHAPED && gate != nullptr) fa_gate32(o, gate + c);
-            if (r < rows) fa_store32(dst + c, o, inv);
+            if (r < rows) store32(c, o, inv);
           } else {
 #pragma unroll
             for (int d = 0; d < 32; ++d) mine[(2 + c + d) * FA_ROWS] = o[d];
@@ -656,7 +685,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
               }
               const float inv_all = finish_factor(m_all, l_all);
 #pragma unroll
-              for (int c = 0; c < D; c += 32) {
+              for (int c = 0; c < DV; c += 32) {
                 float o[32];
 #pragma unroll
                 for (int d = 0; d < 32; ++d) o[d] = 0.f;
@@ -669,7 +698,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
                   }
                 }
                 if (SHAPED && gate != nullptr) fa_gate32(o, gate + c);
-                fa_store32(dst + c, o, inv_all);
+                store32(c, o, inv_all);
               }
             }
             if (threadIdx.x == 0) counters[item] = 0;       // ready for the next launch
@@ -714,7 +743,7 @@ static const int units_per_cta = 1;
 
 namespace mlr {
 
-template <int D, bool SHAPED = false>
+template <int D, int DV = D, int MODE = FA_PLAIN>
 static int fa_launch(const void* q, const void* k_pool, const void* v_pool, void* out, const int* tile_seg,
                      const int* tile_row0, const int* seg_q_start, const int* seg_q_len, const int* seg_pos0,
                      const int* block_table, const int* seg_slot, int table_width, int tiles, int q_rows, int heads,
@@ -722,20 +751,20 @@ static int fa_launch(const void* q, const void* k_pool, const void* v_pool, void
                      int max_kv_len, int* queue, int* error_word, void* scratch, long long scratch_bytes,
                      int* counters, int counters_len, cudaStream_t stream, long long q_stride = 0,
                      const FaScore& score = FaScore{}) {
-  using Shape = FaShape<D>;
+  using Shape = FaShape<D, DV>;
   const int box_rows = page_size >= FA_KEYS ? FA_KEYS : page_size;
   CUtensorMap q_map, k_map, v_map;
   if (!cached_tile_map(&q_map, q, q_rows, q_stride > 0 ? q_stride : (long long)heads * D, FA_ROWS) ||
-      !cached_tile_map(&k_map, k_pool, pool_rows, D, box_rows) ||
-      !cached_tile_map(&v_map, v_pool, pool_rows, D, box_rows))
+      !cached_tile_map(&k_map, k_pool, pool_rows, MODE == FA_MAPS ? 2 * D : D, box_rows) ||
+      !cached_tile_map(&v_map, v_pool, pool_rows, DV, box_rows))
     return MLR_BAD_SIZE;
   // With head_dim 128 two CTAs fit an SM only without the spare kilobyte for aligning the tiles:
   // dynamic shared memory then has to start on a 1024-byte boundary, which it does when the kernel
   // has no static shared memory; the kernel checks and reports through the error word if not.
-  const size_t shared = (D == 64 ? 1024 : 0) + (size_t)Shape::DATA_BYTES + FA_CONTROL_BYTES;
+  const size_t shared = (D + DV < 256 ? 1024 : 0) + (size_t)Shape::DATA_BYTES + FA_CONTROL_BYTES;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(prefill_attention_tcgen05_kernel<D, SHAPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    cudaError_t err = cudaFuncSetAttribute(prefill_attention_tcgen05_kernel<D, DV, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
@@ -751,16 +780,16 @@ static int fa_launch(const void* q, const void* k_pool, const void* v_pool, void
   if (tiles_per_unit < 4) tiles_per_unit = 4;
   int max_parts = (max_key_tiles + tiles_per_unit - 1) / tiles_per_unit;
   if (max_parts > 8) max_parts = 8;
-  const long long need = items * max_parts * FA_ROWS * (D + 2) * (long long)sizeof(float);
+  const long long need = items * max_parts * FA_ROWS * (DV + 2) * (long long)sizeof(float);
   if (max_parts > 1 && (scratch == nullptr || counters == nullptr || need > scratch_bytes || items > counters_len)) {
     max_parts = 1;
     tiles_per_unit = 1 << 30;
   }
   const long long units = items * max_parts;
   const int ctas = (int)(units < resident ? units : resident);
-  launch_kernel(prefill_attention_tcgen05_kernel<D, SHAPED>, dim3(ctas), dim3(FA_THREADS), shared, stream, q_map, k_map, v_map,
-                (bf16*)out, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot, table_width, tiles, heads,
-                kv_heads, page_size, page_shift, window, SHAPED && score.bent ? 1.f : scale * 1.4426950408889634f, queue, error_word, max_parts,
+  launch_kernel(prefill_attention_tcgen05_kernel<D, DV, MODE>, dim3(ctas), dim3(FA_THREADS), shared, stream, q_map, k_map, v_map,
+                out, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot, table_width, tiles, heads,
+                kv_heads, page_size, page_shift, window, MODE == FA_SHAPED && score.bent ? 1.f : scale * 1.4426950408889634f, queue, error_word, max_parts,
                 tiles_per_unit, (float*)scratch, counters, (int)shared, score);
   return launch_status();
 }
@@ -827,7 +856,7 @@ MLR_EXPORT int mlr_attention_shaped_prefill_tcgen05(
   const long long pool_rows = (long long)pool_pages * kv_heads * page_size;
   if (pool_rows >= (1ll << 31)) return MLR_TOO_LARGE;
   const float log2e = 1.4426950408889634f;
-  FaScore score;
+  FaScore score = {};
   score.capped = softcap > 0.f;
   score.bent = score.capped || slopes != nullptr || !(scale > 0.f);
   score.in_scale = score.capped ? scale / softcap : scale * log2e;
@@ -838,12 +867,91 @@ MLR_EXPORT int mlr_attention_shaped_prefill_tcgen05(
   score.gate = (const bf16*)gate;
   score.gate_stride = gate_stride;
   if (head_dim == 64)
-    return fa_launch<64, true>(q, k_pool, v_pool, out, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot,
+    return fa_launch<64, 64, FA_SHAPED>(q, k_pool, v_pool, out, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot,
                                table_width, tiles, q_rows, heads, kv_heads, page_size, page_shift, pool_rows, window, scale,
                                max_kv_len, queue, error_word, scratch, scratch_bytes, counters, counters_len, stream, q_stride,
                                score);
-  return fa_launch<128, true>(q, k_pool, v_pool, out, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot,
+  return fa_launch<128, 128, FA_SHAPED>(q, k_pool, v_pool, out, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot,
                               table_width, tiles, q_rows, heads, kv_heads, page_size, page_shift, pool_rows, window, scale,
                               max_kv_len, queue, error_word, scratch, scratch_bytes, counters, counters_len, stream, q_stride,
                               score);
+}
+
+namespace mlr {
+
+template <int KEY_SIZE, int VALUE_SIZE>
+struct FaSizes {
+  static constexpr int D = KEY_SIZE, DV = VALUE_SIZE;
+};
+
+// o = a1 - lambda * a2, o / rms(o) * out_scale, a warp per row.  grid: (tiles, FA_ROWS / 4)
+__global__ void __launch_bounds__(128)
+combine_maps_kernel(const float* maps, bf16* __restrict__ out, const int* __restrict__ tile_seg, const int* __restrict__ tile_row0,
+                    const int* __restrict__ seg_q_start, const int* __restrict__ seg_q_len, int heads, int vdim, float lambda,
+                    float eps, float out_scale) {
+  pdl_trigger();
+  pdl_wait();
+  const int tile = blockIdx.x, seg = tile_seg[tile], r = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (tile_row0[tile] + r >= seg_q_len[seg]) return;
+  const size_t row = (size_t)(seg_q_start[seg] + tile_row0[tile] + r);
+#pragma unroll 4
+  for (int head = 0; head < heads; ++head) {
+    const float* a1 = maps + (row * heads + head) * 2 * vdim + lane * 2;
+    float2 o[2];
+    float sq = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h * 64 >= vdim) break;
+      const float2 x = __ldcg(reinterpret_cast<const float2*>(a1 + h * 64)), y = __ldcg(reinterpret_cast<const float2*>(a1 + vdim + h * 64));
+      o[h] = make_float2(x.x - lambda * y.x, x.y - lambda * y.y);
+      sq = fmaf(o[h].x, o[h].x, fmaf(o[h].y, o[h].y, sq));
+    }
+    const float factor = out_scale / sqrtf(warp_sum(sq) / (float)vdim + eps);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h * 64 >= vdim) break;
+      *reinterpret_cast<__nv_bfloat162*>(out + (row * heads + head) * vdim + h * 64 + lane * 2) =
+          __floats2bfloat162_rn(o[h].x * factor, o[h].y * factor);
+    }
+  }
+}
+
+}  // namespace mlr
+
+// Differential attention of prompt portions: both maps of a head as attentions of their own, then their combination.  q:
+// bfloat16 [rows, heads, 2, dim]; k_pool [pages, kv_heads, page_size, 2 * dim], v_pool [.., vdim]; maps: float32 scratch [rows,
+// heads, 2, vdim]; out: bfloat16 [rows, heads, vdim]; dim and vdim 64 or 128; scale > 0; the rest as above.
+MLR_EXPORT int mlr_attention_diff_prefill_tcgen05(
+    const void* q, const void* k_pool, const void* v_pool, float* maps, void* out, const int* tile_seg, const int* tile_row0,
+    const int* seg_q_start, const int* seg_q_len, const int* seg_pos0, const int* block_table, const int* seg_slot, int table_width,
+    int tiles, int q_rows, int heads, int kv_heads, int dim, int vdim, int page_size, int pool_pages, int window, int keep_first,
+    float scale, float lambda, float eps, float out_scale, int max_kv_len, int* queue, int* error_word, void* scratch,
+    long long scratch_bytes, int* counters, int counters_len, cudaStream_t stream) {
+  if (tiles == 0) return MLR_OK;
+  if (tiles < 0 || q_rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || page_size <= 0 || window < 0 ||
+      keep_first < 0 || table_width <= 0 || pool_pages <= 0 || maps == nullptr || queue == nullptr || error_word == nullptr ||
+      !(scale > 0.f))
+    return MLR_BAD_SIZE;
+  if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128)) return MLR_BAD_SIZE;
+  if ((long long)tiles * heads >= (1ll << 29)) return MLR_TOO_LARGE;
+  const int page_shift = fa_shift_of(page_size);
+  if (page_shift < 3) return MLR_BAD_SIZE;
+  if (((uintptr_t)k_pool & 15) || ((uintptr_t)v_pool & 15) || ((uintptr_t)q & 15)) return MLR_BAD_ALIGNMENT;
+  const long long pool_rows = (long long)pool_pages * kv_heads * page_size;
+  if (pool_rows >= (1ll << 31)) return MLR_TOO_LARGE;
+  FaScore score = {};
+  score.keep = keep_first;
+  auto launch = [&](auto shape) -> int {
+    constexpr int D = decltype(shape)::D, DV = decltype(shape)::DV;
+    return fa_launch<D, DV, FA_MAPS>(q, k_pool, v_pool, maps, tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table,
+                                     seg_slot, table_width, tiles, q_rows, 2 * heads, kv_heads, page_size, page_shift, pool_rows,
+                                     window, scale, max_kv_len, queue, error_word, scratch, scratch_bytes, counters, counters_len,
+                                     stream, 0, score);
+  };
+  const int status = dim == 64 ? (vdim == 64 ? launch(FaSizes<64, 64>()) : launch(FaSizes<64, 128>()))
+                               : (vdim == 64 ? launch(FaSizes<128, 64>()) : launch(FaSizes<128, 128>()));
+  if (status != MLR_OK) return status;
+  launch_kernel(combine_maps_kernel, dim3(tiles, FA_ROWS / 4), dim3(128), 0, stream, (const float*)maps, (bf16*)out, tile_seg,
+                tile_row0, seg_q_start, seg_q_len, heads, vdim, lambda, eps, out_scale);
+  return launch_status();
 }

@@ -1011,6 +1011,28 @@ class CudaOps:
                 and (self.use_diff_decode_kernel or batch.num_decode == 0)):
             # prompt portions on the tensor cores: each map as an attention of its own, then the combination
             maps = torch.empty((q.shape[0], 2 * heads * vdim), dtype=torch.float32, device=q.device)
+            page_size = k_pool.shape[2]
+            # Measured in us, 7 heads of 2 x 64 with values of 128, mma.sync / tcgen05: 2,048 rows 291 / 57, 128 rows 127 / 24,
+            # 17 rows 38 / 25, 5 rows 33 / 28, 2 rows 21 / 25 (both wait for the host there).
+            if (self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and batch.max_q_len >= 4 and page_size >= 8
+                    and page_size & (page_size - 1) == 0 and scale > 0 and k_pool.data_ptr() % 16 == 0
+                    and v_pool.data_ptr() % 16 == 0):
+                space = self._workspace(q.device)
+                longest = int(batch.max_kv_len)
+                if window:
+                    # no item of 128 rows walks more key tiles than its rows' windows and the kept positions touch
+                    longest = min(longest, int(window) + int(keep_first) + 256)
+                _check(build.load_library("attention_tcgen05").mlr_attention_diff_prefill_tcgen05(
+                    _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(maps), _ptr(out), _ptr(batch.plan["big_tile_seg"]),
+                    _ptr(batch.plan["big_tile_row0"]), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_pos0),
+                    _ptr(batch.block_table), _ptr(batch.seg_slot), batch.block_table.shape[1], batch.counts["big"], q.shape[0],
+                    heads, kv_heads, dim, vdim, page_size, k_pool.shape[0], int(window or 0), int(keep_first),
+                    ctypes.c_float(scale), ctypes.c_float(lam), ctypes.c_float(eps), ctypes.c_float(out_scale), longest,
+                    _ptr(space["prefill_queue"]), _ptr(space["error_word"]),
+                    _ptr(space["prefill_scratch"] if self.split_prefill_items else None),
+                    ctypes.c_longlong(space["prefill_scratch"].numel()), _ptr(space["prefill_counters"]),
+                    space["prefill_counters"].numel(), _stream()), "differential attention (tcgen05)")
+                return out
             _check(build.load_library("attention_diff_mma").mlr_attention_diff_mma(
                 _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(maps), _ptr(out), _ptr(batch.plan["wide_tile_seg"]),
                 _ptr(batch.plan["wide_tile_row0"]), _ptr(batch.seg_q_start), _ptr(batch.seg_q_len),

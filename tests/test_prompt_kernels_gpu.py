@@ -11,6 +11,7 @@ import torch
 
 from fake_ops import FakeOps
 from mini_llm_runtime_b200 import ops
+from mini_llm_runtime_b200.ops import AttentionBatch
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +124,52 @@ def test_state_space_in_chunks(heads, n, groups, lengths, slots, order):
     # sums of up to n + CHUNK products of numbers that went through up to CHUNK decays each
     close(got, want, 200 * UNIT, "state-space outputs")
     close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "state-space state")
+
+
+def paged(lengths, before, visible, page_size, pools, seed):
+    """Pools [pages, heads, page_size, entries] and the batch, on the CPU and on the device.  Page 0 belongs to nobody; it and every
+    place that no row of its request sees (``visible(position, key)``) hold NaN, and pages without a visible key are given back."""
+    need = [-(-(n + b) // page_size) for n, b in zip(lengths, before)]
+    order = torch.randperm(sum(need), generator=generator(seed)) + 1
+    table = torch.full((len(lengths), max(need)), -1, dtype=torch.int32)
+    tensors = [torch.full((sum(need) + 1, heads, page_size, entries), float("nan"), dtype=torch.bfloat16) for heads, entries, _ in pools]
+    at = 0
+    for index, (n, b) in enumerate(zip(lengths, before)):
+        for logical in range(need[index]):
+            page = int(order[at])
+            at += 1
+            offsets = [o for o in range(page_size) if any(visible(p, logical * page_size + o) for p in range(b, b + n))]
+            if offsets:
+                table[index, logical] = page
+                for k, (tensor, (heads, entries, std)) in enumerate(zip(tensors, pools)):
+                    tensor[page, :, offsets] = rnd(seed + 100 * page + k, heads, len(offsets), entries, std=std).to(torch.bfloat16)
+    starts = torch.tensor([sum(lengths[:i]) for i in range(len(lengths))], dtype=torch.int32)
+    arrays, counts = cuda().plan_attention(lengths, before)
+    cpu = dict(seg_q_start=starts, seg_q_len=torch.tensor(lengths, dtype=torch.int32), seg_pos0=torch.tensor(before, dtype=torch.int32),
+               seg_slot=torch.arange(len(lengths), dtype=torch.int32), block_table=table)
+    rest = dict(num_segments=len(lengths), max_q_len=max(lengths), max_kv_len=max(n + b for n, b in zip(lengths, before)), counts=counts)
+    batch = AttentionBatch(**{k: v.to(DEVICE) for k, v in cpu.items()}, **rest,
+                           plan={k: torch.from_numpy(v).to(DEVICE) for k, v in arrays.items()})
+    return tensors, types.SimpleNamespace(**cpu, **rest), batch
+
+
+# Probabilities, keys and values in bfloat16 (8 bits each), sums in 32: of the rounding errors only those of the probabilities and of
+# the result are not the oracle's too, 2^-9 each at most and independent from key to key.
+ATTENTION_BOUND = 2.0 ** -7
+
+
+@pytest.mark.parametrize("dim,vdim,page_size", [(64, 128, 16), (128, 64, 8), (64, 64, 64), (128, 128, 32)])
+@pytest.mark.parametrize("window,keep", [(70, 5), (0, 0), (129, 70)])
+def test_differential_attention_of_prompts(dim, vdim, page_size, window, keep):
+    """Portions around the 128 rows of an item, tiles of 64 keys around the kept positions and the window."""
+    heads, kv_heads, lengths, before = 4, 2, [129, 5, 66, 4, 64], [0, 300, 100, 50, 64]
+    seen = lambda p, j: j <= p and (not window or p - j < window or j < keep)      # noqa: E731
+    pools, cpu, batch = paged(lengths, before, seen, page_size, [(kv_heads, 2 * dim, 1.0), (kv_heads, vdim, 0.7)], 3)
+    q = rnd(5, sum(lengths), 2 * heads * dim).to(torch.bfloat16)
+    args = (heads, kv_heads, dim, vdim, dim ** -0.5, window, keep, 0.4, 1e-6, 0.5)
+    want = FAKE.differential_attention(q.float(), *(t.float() for t in pools), cpu, *args)
+    got = cuda().differential_attention(q.to(DEVICE), *(t.to(DEVICE) for t in pools), batch, *args)
+    torch.cuda.synchronize()
+    cuda().raise_if_device_error()
+    # the difference of two maps, brought to unit size: its share of their errors grows by what the difference lost
+    close(got, want, 2 * ATTENTION_BOUND, "differential attention")
