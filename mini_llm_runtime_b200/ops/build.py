@@ -49,6 +49,7 @@ LIBRARIES: dict[str, tuple[str, ...]] = {
     "stream32": (),
     "attention_latent": (),
     "attention_latent_mma": (),
+    "attention_latent_tcgen05": (),
     "attention_rotated": (),
     "routed_experts": (),
     "attention_sigmoid": (),

@@ -1289,7 +1289,19 @@ class CudaOps:
                 _ptr(batch.seg_pos0), _ptr(batch.block_table), _ptr(batch.seg_slot), batch.block_table.shape[1], *tail),
                 "latent attention (decode)")
             tiles -= batch.num_decode       # the one-row segments' tiles are the last of the list
-        if tiles > 0 and on_tensor_cores:
+        page_size = pool.shape[2]
+        if (tiles > 0 and on_tensor_cores and self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and page_size >= 8
+                and page_size & (page_size - 1) == 0 and scale > 0 and q.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0
+                and (self.use_latent_decode_kernel or batch.num_decode == 0) and self._latent_tcgen05_fits(heads, rank, rot)):
+            # prompt portions with both products on tcgen05
+            space = self._workspace(q.device)
+            _check(build.load_library("attention_latent_tcgen05").mlr_latent_attention_prefill_tcgen05(
+                _ptr(q), _ptr(pool), _ptr(out), _ptr(batch.plan["big_tile_seg"]), _ptr(batch.plan["big_tile_row0"]),
+                _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_pos0), _ptr(batch.block_table), _ptr(batch.seg_slot),
+                batch.block_table.shape[1], batch.counts["big"], q.shape[0], heads, rank, rot, page_size, pool.shape[0],
+                int(window or 0), ctypes.c_float(scale), _ptr(sink), _ptr(space["prefill_queue"]), _ptr(space["error_word"]),
+                _stream()), "latent attention (tcgen05)")
+        elif tiles > 0 and on_tensor_cores:
             # prompt portions on the tensor cores
             _check(build.load_library("attention_latent_mma").mlr_latent_attention_mma(
                 _ptr(q), _ptr(pool), _ptr(out), _ptr(batch.plan["tile_seg"]), _ptr(batch.plan["tile_row0"]),
@@ -1302,6 +1314,13 @@ class CudaOps:
                 _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_pos0), _ptr(batch.block_table),
                 _ptr(batch.seg_slot), batch.block_table.shape[1], tiles, *tail), "latent attention")
         return out
+
+    def _latent_tcgen05_fits(self, heads: int, rank: int, rot: int) -> bool:
+        cache = self.__dict__.setdefault("_latent_wide_fits", {})
+        if (heads, rank, rot) not in cache:
+            cache[(heads, rank, rot)] = bool(build.load_library("attention_latent_tcgen05").mlr_latent_attention_tcgen05_fits(
+                heads, rank, rot))
+        return cache[(heads, rank, rot)]
 
     def _latent_mma_fits(self, rank: int, rot: int) -> bool:
         cache = self.__dict__.setdefault("_latent_fits", {})

@@ -173,3 +173,21 @@ def test_differential_attention_of_prompts(dim, vdim, page_size, window, keep):
     cuda().raise_if_device_error()
     # the difference of two maps, brought to unit size: its share of their errors grows by what the difference lost
     close(got, want, 2 * ATTENTION_BOUND, "differential attention")
+
+
+@pytest.mark.parametrize("heads,rank,rot,page_size", [(16, 512, 64, 16), (14, 256, 32, 16), (5, 384, 32, 64), (128, 64, 16, 8), (3, 48, 16, 32)])
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_latent_attention_of_prompts(heads, rank, rot, page_size, window, sinks):
+    """Portions around the tokens of an item (128 / heads) and around tiles of 32 and 64 keys; latents in one piece and in halves."""
+    lengths, before = [130, 2, 33, 9], [0, 300, 95, 31]
+    seen = lambda p, j: j <= p and (not window or p - j < window)      # noqa: E731
+    (pool,), cpu, batch = paged(lengths, before, seen, page_size, [(1, rank + rot, 1.0)], 7)
+    q = rnd(6, sum(lengths), heads * (rank + rot), std=0.5).to(torch.bfloat16)
+    sink = rnd(8, heads) if sinks else None
+    args = (heads, rank, rot, 2.0 * (rank + rot) ** -0.5, window)
+    want = FAKE.latent_attention(q.float(), pool.float(), cpu, *args, sink)
+    got = cuda().latent_attention(q.to(DEVICE), pool.to(DEVICE), batch, *args, None if sink is None else sink.to(DEVICE))
+    torch.cuda.synchronize()
+    cuda().raise_if_device_error()
+    close(got, want, ATTENTION_BOUND, "latent attention")
