@@ -8,13 +8,15 @@
 //
 // What bounds the layout is room.  A row's output of 512 columns of 32 bits is all of an SM's tensor memory, so latents of more
 // than 256 numbers are cut in two halves of value columns, units of their own that both form the scores (1.5 times the work of one
-// pass).  Queries of 128 x 576 and one tile of 64 keys would fill the shared memory; with the first 256 columns of the queries in
-// tensor memory (A operands may lie there), beside the output's 256, two buffers of scores and two of probabilities (also A
-// operands), four stages of 32 keys fit, and the scores' MMAs of those columns read no A from shared memory, which bounds the others:
-// 128 rows x 16 columns per 32 keys.  Latents of up to 256 numbers (up to 320 with the turned part): queries in shared memory,
-// three stages of 64 keys.
+// pass).  Queries of 128 x 576 and one tile of 64 keys would fill the shared memory; with the first 384 columns of the queries in
+// tensor memory (A operands may lie there), beside the output's 256 and two buffers of scores, whose places the probabilities
+// (also an A operand) take over, four stages of 32 keys fit.  Latents of up to 256 numbers (up to 320 with the turned part): queries
+// in shared memory, three stages of 64 keys.
 //
-// Measured (B200, 16 heads, 512 + 64): MEASURED
+// Measured (B200; mma.sync kernel before, this one with MMAs issued behind a test of the lane, by an elected lane): 1,024 rows behind
+// 1,024 cached ones, 16 heads of 512 + 64: 509, 188, 112 us; 14 heads of 256 + 32: 350, 52, 47 us; 2,048 rows: 581, 250, 160 and 400, 56,
+// 51 us.  A tile of 32 keys then takes 1,600 cycles: 1,100 for the issue of its 36 score MMAs, one per 31 cycles, which is also what
+// reading 128 rows of A takes; the softmax of a tile 900.
 #include "tcgen05.cuh"
 
 namespace mlr {
@@ -23,22 +25,22 @@ constexpr int LA_ROWS = 128;
 constexpr int LA_THREADS = 192;
 constexpr int LA_VALUES = 256;       // value columns of a unit at most
 constexpr uint32_t LA_TMEM_COLS = 512;
-constexpr int LA_Q_BLOCKS = 5;       // 64-wide column blocks of the queries in shared memory
 
 // KEYS per tile, STAGES of tiles, Q_TMEM: query columns in tensor memory.
 template <int KEYS_, int STAGES_, int Q_TMEM_, int BLOCKS_>
 struct LaShape {
   static constexpr int KEYS = KEYS_, STAGES = STAGES_, Q_TMEM = Q_TMEM_;
   static constexpr int BLOCKS = BLOCKS_;                                  // 64-wide column blocks of a key row at most
+  static constexpr int Q_BLOCKS = BLOCKS - Q_TMEM / 64;                   // of them of the queries in shared memory
   static constexpr int Q_BLOCK_BYTES = LA_ROWS * 128, K_BLOCK_BYTES = KEYS * 128;
   static constexpr int STAGE_BYTES = BLOCKS * K_BLOCK_BYTES;
-  static constexpr int DATA_BYTES = LA_Q_BLOCKS * Q_BLOCK_BYTES + STAGES * STAGE_BYTES;
-  // tensor memory: output | scores x 2 | probabilities x 2 | queries
-  static constexpr uint32_t S_AT = LA_VALUES, P_AT = S_AT + 2 * KEYS, Q_AT = P_AT + KEYS;
+  static constexpr int DATA_BYTES = Q_BLOCKS * Q_BLOCK_BYTES + STAGES * STAGE_BYTES;
+  // tensor memory: output | scores x 2 | queries.  A row's probabilities take the place of its scores once those are in registers.
+  static constexpr uint32_t S_AT = LA_VALUES, Q_AT = S_AT + 2 * KEYS;
   static_assert(Q_AT + Q_TMEM / 2 <= LA_TMEM_COLS, "tensor memory");
 };
 typedef LaShape<64, 3, 0, 5> LaNarrow;      // rank <= 256, width <= 320
-typedef LaShape<32, 4, 256, 9> LaWide;      // rank <= 512, width <= 576
+typedef LaShape<32, 4, 384, 9> LaWide;      // rank <= 512, width <= 576
 
 struct LaControl {
   uint64_t q_full, q_stored, k_full[4], s_done[4], pv_done[4], p_ready;
@@ -71,9 +73,9 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
     if (threadIdx.x == 0) atomicCAS(a.error_word, 0, 0x7f);
     return;
   }
-  uint8_t* ring = q_tile + LA_Q_BLOCKS * Shape::Q_BLOCK_BYTES;                              // STAGES x [blocks][KEYS][64]
+  uint8_t* ring = q_tile + Shape::Q_BLOCKS * Shape::Q_BLOCK_BYTES;                              // STAGES x [blocks][KEYS][64]
   LaControl& ctl = *reinterpret_cast<LaControl*>(ring + STAGES * Shape::STAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(&ctl.q_full, 1);
     mbar_init(&ctl.q_stored, 4);
@@ -95,7 +97,7 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
   pdl_trigger();
   __syncthreads();
   fa_fence_after();
-  const uint32_t tmem_base = ctl.tmem_holder;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl.tmem_holder, 0);
   pdl_wait();
 
   const int heads = a.heads;
@@ -104,7 +106,7 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
   const int boxes = a.page_size >= KEYS ? 1 : KEYS >> a.page_shift;
   const int box_rows = a.page_size >= KEYS ? KEYS : a.page_size;
   const int k_blocks = (a.width + 63) / 64, k_steps = a.width / 16;
-  const int q_blocks = k_blocks - Shape::Q_TMEM / 64;
+  const int q_blocks = max(0, k_blocks - Shape::Q_TMEM / 64);
   unsigned tiles_before = 0, units_before = 0;
   bool gave_up = false;
 
@@ -132,7 +134,8 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
     if (warp == 5) {
       // ------------------------------------------------------------ loads: the stage of tile j - STAGES is free once its P V is done
       if (lane == 0) {
-        mbar_expect_tx(&ctl.q_full, q_blocks * Shape::Q_BLOCK_BYTES);
+        if (q_blocks > 0) mbar_expect_tx(&ctl.q_full, q_blocks * Shape::Q_BLOCK_BYTES);
+        else mbar_arrive(&ctl.q_full);
         for (int b = 0; b < q_blocks; ++b)
           tma_load_2d(&q_map, &ctl.q_full, q_tile + b * Shape::Q_BLOCK_BYTES, Shape::Q_TMEM + b * 64, q_row);
       }
@@ -171,12 +174,12 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
       const uint64_t q_desc = fa_desc_k_major(smem_u32(q_tile)), k_desc = fa_desc_k_major(smem_u32(ring));
       const uint64_t v_desc = fa_desc_mn_major(smem_u32(ring) + (value0 / 64) * Shape::K_BLOCK_BYTES, Shape::K_BLOCK_BYTES);
       auto issue_scores = [&](int j) {
-        const unsigned t = tiles_before + (unsigned)j;
+        const unsigned t = __shfl_sync(0xffffffffu, tiles_before + (unsigned)j, 0);
         const int stage = t % STAGES;
         fa_wait(&ctl.k_full[stage], (t / STAGES) & 1u, a.error_word, 0x72, gave_up);
         gave_up = __any_sync(0xffffffffu, gave_up);
         fa_fence_after();
-        if (lane == 0 && !gave_up) {
+        if (!gave_up && elect_one()) {
           const uint64_t keys = k_desc + (uint64_t)((stage * Shape::STAGE_BYTES) >> 4);
           const uint32_t d = tmem_base + Shape::S_AT + (t & 1u) * KEYS;
           // unrolled over the most column blocks there can be, so that a product costs its descriptors' additions and no more: one
@@ -209,9 +212,9 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
         fa_wait(&ctl.p_ready, t & 1u, a.error_word, 0x75, gave_up);
         gave_up = __any_sync(0xffffffffu, gave_up);
         fa_fence_after();
-        if (lane == 0 && !gave_up) {
+        if (!gave_up && elect_one()) {
           const uint64_t values = v_desc + (uint64_t)((stage * Shape::STAGE_BYTES) >> 4);
-          const uint32_t p = tmem_base + Shape::P_AT + (t & 1u) * (KEYS / 2);
+          const uint32_t p = tmem_base + Shape::S_AT + (t & 1u) * KEYS;
 #pragma unroll
           for (int k = 0; k < KEYS / 16; ++k)
             fa_mma_tmem(tmem_base, p + k * 8, values + (uint64_t)((k * 2048) >> 4), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
@@ -230,7 +233,7 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
           uint32_t v[16];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const uint4 piece = r < rows ? __ldcg(src + c / 4 + e) : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 piece = r < rows && 2 * c + 8 * e < a.width ? __ldcg(src + c / 4 + e) : make_uint4(0u, 0u, 0u, 0u);
             v[4 * e] = piece.x, v[4 * e + 1] = piece.y, v[4 * e + 2] = piece.z, v[4 * e + 3] = piece.w;
           }
           fa_tmem_store16(lane_base + Shape::Q_AT + c, v);
@@ -318,7 +321,7 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const _
           }
         }
 #pragma unroll
-        for (int c = 0; c < KEYS / 2; c += 16) fa_tmem_store16(lane_base + Shape::P_AT + (t & 1u) * (KEYS / 2) + c, p + c);
+        for (int c = 0; c < KEYS / 2; c += 16) fa_tmem_store16(lane_base + Shape::S_AT + (t & 1u) * KEYS + c, p + c);
         fa_tmem_wait_st();
         if (key0 < lowest || key0 + KEYS - 1 > last_pos) {
           // ragged tile, its scores are formed: rows of keys outside the range become zeros for the second product

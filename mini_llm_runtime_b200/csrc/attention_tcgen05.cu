@@ -217,7 +217,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   uint8_t* kv_ring = p_tiles + Shape::P_BUFFERS * FA_P_BYTES;                        // STAGES x (K, V), each [halves][64][64]
   FaControl& ctl = *reinterpret_cast<FaControl*>(kv_ring + STAGES * Shape::STAGE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(&ctl.q_full, 1);
     for (int s = 0; s < STAGES; ++s) {
@@ -238,7 +238,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   pdl_trigger();
   __syncthreads();
   fa_fence_after();
-  const uint32_t tmem_base = ctl.tmem_holder;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl.tmem_holder, 0);
   pdl_wait();                       // before the first draw from the queue, the first read of q and the first write
 
   const int total_items = num_tiles * heads;
@@ -361,7 +361,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       const uint64_t v_desc = fa_desc_mn_major(smem_u32(kv_ring) + Shape::K_TILE_BYTES, Shape::KV_HALF_BYTES);
       const uint64_t p_desc = fa_desc_k_major(p_addr0);
       auto issue_qk = [&](int j) {
-        const unsigned t = tiles_before + (unsigned)j;
+        const unsigned t = __shfl_sync(0xffffffffu, tiles_before + (unsigned)j, 0);
         const int stage = t % STAGES, buffer = t & 1;
         fa_wait(&ctl.k_full[stage], (t / STAGES) & 1u, error_word, 0x62, gave_up);
         // The score buffer is free: scores go out two tiles ahead, after the probabilities of tile
@@ -369,7 +369,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         // (the same buffer); a unit's first two tiles follow the previous unit's end.
         gave_up = __any_sync(0xffffffffu, gave_up);
         fa_fence_after();
-        if (lane == 0 && !gave_up) {
+        if (!gave_up && elect_one()) {
           const uint64_t k_desc = kv_desc + (uint64_t)((stage * Shape::STAGE_BYTES) >> 4);
 #pragma unroll
           for (int k = 0; k < D / 16; ++k)
@@ -387,13 +387,13 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       issue_qk(0);
       if (tiles > 1) issue_qk(1);
       for (int j = 0; j < tiles; ++j) {
-        const unsigned t = tiles_before + (unsigned)j;
+        const unsigned t = __shfl_sync(0xffffffffu, tiles_before + (unsigned)j, 0);
         const int stage = t % STAGES;
         fa_wait(&ctl.p_ready, t & 1u, error_word, 0x65, gave_up);
         fa_wait(&ctl.v_full[stage], (t / STAGES) & 1u, error_word, 0x6a, gave_up);
         gave_up = __any_sync(0xffffffffu, gave_up);
         fa_fence_after();
-        if (lane == 0 && !gave_up) {
+        if (!gave_up && elect_one()) {
           const uint64_t v_tile = v_desc + (uint64_t)((stage * Shape::STAGE_BYTES) >> 4);
           const uint64_t p_tile = p_desc + (uint64_t)(((Shape::P_BUFFERS == 2 ? (t & 1u) : 0u) * FA_P_BYTES) >> 4);
 #pragma unroll

@@ -304,6 +304,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const GemmParams p) {
   constexpr int HALVES = BM / TILE_ROWS;
+  // How MMAs are issued.  Behind a test of the lane's number the compiler moves every operand of every MMA into uniform registers by
+  // itself, 73 cycles per MMA where the MMAs of a 128 x 128 block of 64 k need 32 each; with an elected lane of a warp whose
+  // control flow is uniform it keeps them there (ELECT), all the more so where the warp's number and the tensor memory's address
+  // are uniform too (UNIFORM).  [M, N, K] = [2048, 896, 4864]: 30.7 us by lane, 26.7 elected, 25.3 uniform too; [512, 4608, 3584]: 24.5,
+  // 21.5, 19.6.  With the gate in the epilogue uniform operands cost registers there ([2048, 9728, 896] 41.5 -> 57.6), and the
+  // pair form, whose MMAs are twice as long, gains nothing from election (41.5 -> 42.7).
+  constexpr bool UNIFORM = !SWIGLU, ELECT = !(SWIGLU && PAIR);
   constexpr uint32_t HALF_BYTES = TILE_ROWS * TILE_K * 2;
   constexpr uint32_t A_BYTES = BM * TILE_K * 2;
   constexpr int B_ROWS = PAIR ? BN / 2 : BN;               // rows of the BN-row operand this CTA loads
@@ -320,7 +327,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __shared__ uint32_t tmem_holder;
   __shared__ int is_last_cta, epilogue_failed;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = UNIFORM ? __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0) : threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages;
   // grouped form: the grid is (column tiles, row tiles), so that the CTAs that share a row tile's
   // activations run together; every weight tile of a group is read by one CTA per row tile anyway
@@ -368,8 +375,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __syncthreads();
   if (PAIR) cluster_sync_all();        // the other CTA's barriers exist before anything is sent to them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_holder;
+  const uint32_t tmem_base = UNIFORM ? __shfl_sync(0xffffffffu, tmem_holder, 0) : tmem_holder;
 
+  const bool issuer = UNIFORM ? warp == 1 && pair_rank == 0
+                    : ELECT ? __shfl_sync(0xffffffffu, warp == 1 && pair_rank == 0 ? 1 : 0, 0) != 0      // the same in the whole warp
+                            : warp == 1 && lane == 0 && pair_rank == 0;
   pdl_trigger();
   if (warp == 0 && lane == 0) {
     // ---------------- producer
@@ -416,32 +426,41 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       load_b(s, k);
       if (++s == stages) { s = 0; ++round; }
     }
-  } else if (warp == 1 && lane == 0 && pair_rank == 0) {
-    // ---------------- MMA issuer (of a pair: the even CTA's, for both)
+  } else if (issuer) {
+    // ---------------- MMA issuer (of a pair: the even CTA's, for both); with ELECT the whole warp walks the k blocks
     constexpr uint32_t idesc = instruction_descriptor(PAIR ? 2 * TILE_ROWS : TILE_ROWS, BN);
+    const uint32_t tiles_addr = ELECT ? __shfl_sync(0xffffffffu, smem_u32(tiles), 0) : smem_u32(tiles);
+    const uint32_t tmem_d = ELECT && !UNIFORM ? __shfl_sync(0xffffffffu, tmem_base, 0) : tmem_base;
     int s = 0, round = 0;
     for (int i = 0; i < num_kb; ++i) {
-      if (!mbar_wait(&full_bar[s], round & 1, p.error_word, 2)) break;
+      const bool there = mbar_wait(&full_bar[s], round & 1, p.error_word, 2);
+      if (ELECT ? !__all_sync(0xffffffffu, there) : !there) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_addr = smem_u32(tiles + (size_t)s * STAGE_BYTES);
+      const uint32_t a_addr = tiles_addr + (uint32_t)s * STAGE_BYTES;
       const uint32_t b_addr = a_addr + A_BYTES;
+      if (!ELECT || elect_one()) {
 #pragma unroll
-      for (int k = 0; k < TILE_K / MMA_K; ++k) {
-        if (PAIR) {
-          umma_pair(tmem_base, smem_descriptor(a_addr + k * MMA_K * 2), smem_descriptor(b_addr + k * MMA_K * 2), idesc,
-                    (i > 0 || k > 0) ? 1u : 0u);
-        } else {
+        for (int k = 0; k < TILE_K / MMA_K; ++k) {
+          if (PAIR) {
+            umma_pair(tmem_d, smem_descriptor(a_addr + k * MMA_K * 2), smem_descriptor(b_addr + k * MMA_K * 2), idesc,
+                      (i > 0 || k > 0) ? 1u : 0u);
+          } else {
 #pragma unroll
-          for (int half = 0; half < HALVES; ++half)
-            umma(tmem_base + half * BN, smem_descriptor(a_addr + half * HALF_BYTES + k * MMA_K * 2),
-                 smem_descriptor(b_addr + k * MMA_K * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+            for (int half = 0; half < HALVES; ++half)
+              umma(tmem_d + half * BN, smem_descriptor(a_addr + half * HALF_BYTES + k * MMA_K * 2),
+                   smem_descriptor(b_addr + k * MMA_K * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          }
         }
+        if (PAIR) umma_commit_pair(&empty_bar[s]); else umma_commit(&empty_bar[s]);
       }
-      if (PAIR) umma_commit_pair(&empty_bar[s]); else umma_commit(&empty_bar[s]);
+      if (ELECT) __syncwarp();
       if (++s == stages) { s = 0; ++round; }
     }
     // arrives once every MMA issued above has finished (in a pair: on both CTAs' barriers)
-    if (PAIR) umma_commit_pair(&accumulator_bar); else umma_commit(&accumulator_bar);
+    if (!ELECT || elect_one()) {
+      if (PAIR) umma_commit_pair(&accumulator_bar); else umma_commit(&accumulator_bar);
+    }
+    if (ELECT) __syncwarp();
   } else if (warp >= 2) {
     // ---------------- epilogue: thread <-> TMEM lane <-> tile row
     const int quarter = warp & 3;
