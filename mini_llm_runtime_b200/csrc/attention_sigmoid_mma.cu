@@ -4,7 +4,7 @@
 //   w_g(i, j) = sigmoid(q_g(i) . k_c(g)(j) * scale - r1_g ln(1 + r2_g (i - j)) + pb_g)
 //   w'_h(i, j) = sum_g talk[h, g] w_g(i, j)          (talk null: w' = w)
 //   out_h(i) = sum_j w'_h(i, j) v_c(h)(j)
-// One CTA of eight warps takes the 16 rows of one work-list entry with ALL heads (the mixing needs every
+// One CTA takes the 16 rows of one work-list entry with ALL heads (the mixing needs every
 // head's weight of a (row, key) pair in one place) and walks the keys in tiles of 32 aligned to absolute
 // positions, possibly one of several CTAs that share a row's keys in chunks (their sums are added up, in
 // chunk order, by a second kernel).  Per key tile: each warp forms the scores of its heads (Q K^T), turns
@@ -13,16 +13,20 @@
 // the values (W' V) into accumulators that stay in its registers over all key tiles.  The key tile of the
 // next step is fetched (cp.async) while the weights are mixed and multiplied, the value tile while the
 // next scores are formed.
-// Sizes: key size and value size 64 or 128, at most 16 heads (two per warp).
+// Sizes: key size and value size 64 or 128, at most 16 heads.
+//
+// Bound by instructions and the barriers between the phases (1.9 of 4 instructions per cycle and SM, tensor pipe 16 %).  Measured (B200),
+// before / after sixteen warps per SM, the mixing with a weight read once per share of the heads, and a logarithm per distance
+// instead of one per pair: portions of 1,450, 401 and 197 rows 276 / 175 us (16 heads of 128), 152 / 110 us (14 of 64); eight decoded
+// rows at 2,048 keys 46 / 30 us and 47 / 35 us.
 #include "mma_attention.cuh"
 
 namespace mlr {
 
-constexpr int SM_THREADS = 256;
-constexpr int SM_WARPS = SM_THREADS / 32;
 constexpr int SM_KEYS = 32;
 constexpr int SM_ROWS = 16;
-constexpr int SM_HEADS_PER_WARP = 2;
+constexpr int SM_HEADS = 16;        // at most
+constexpr int SM_BIAS = 48;         // distances that occur between the rows and keys of a tile (47), per head
 constexpr int SM_WSTRIDE = 40;      // entries between the rows of a weight matrix in shared memory (32 keys + padding)
 
 struct SigmoidMmaArgs {
@@ -33,12 +37,20 @@ struct SigmoidMmaArgs {
 };
 
 // grid: (work-list entries, key chunks)
-// Heads of 64 and 64 leave room for two blocks per SM (128 registers a thread: 64 of them output sums),
-// so that one block's barriers and dependent instructions pass under the other's work.
+// Sixteen warps per SM either way: heads of 64 and 64 as two blocks of eight warps with two heads each, larger heads, whose block fills
+// the shared memory, as one block of sixteen warps with a head each (with eight warps a barrier left the SM idle, 64 of a
+// thread's 128 registers are output sums).
 template <int D, int V>
-__global__ void __launch_bounds__(SM_THREADS, (D <= 64 && V <= 64) ? 2 : 1)
+struct SigmoidShape {
+  static constexpr int WARPS = D <= 64 && V <= 64 ? 8 : 16, THREADS = WARPS * 32, HEADS_PER_WARP = SM_HEADS / WARPS;
+};
+
+template <int D, int V>
+__global__ void __launch_bounds__(SigmoidShape<D, V>::THREADS, (D <= 64 && V <= 64) ? 2 : 1)
 attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_pool, bf16* out, float* partial,
                              SigmoidMmaArgs a) {
+  constexpr int SM_WARPS = SigmoidShape<D, V>::WARPS, SM_THREADS = SigmoidShape<D, V>::THREADS;
+  constexpr int SM_HEADS_PER_WARP = SigmoidShape<D, V>::HEADS_PER_WARP;
   pdl_trigger();
   extern __shared__ __align__(128) unsigned char shared_bytes[];
   const int H = a.heads, G = a.kv_heads, per_kv = H / G;
@@ -46,13 +58,18 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
   bf16* k_tiles = q_tiles + (size_t)H * SM_ROWS * D;                       // [G][32][D], swizzled per head
   bf16* v_tiles = k_tiles + (size_t)G * SM_KEYS * D;                       // [G][32][V]
   bf16* w_mix = v_tiles + (size_t)G * SM_KEYS * V;                         // [H][16][SM_WSTRIDE]
-  float* w_raw = reinterpret_cast<float*>(w_mix + (size_t)H * SM_ROWS * SM_WSTRIDE);      // [H][16][SM_WSTRIDE]
-  float* talk = w_raw + (size_t)H * SM_ROWS * SM_WSTRIDE;                  // [H][H]
-  int* key_row = reinterpret_cast<int*>(talk + H * H);                     // [2][32]: the cached row of every key of this and the next tile
+  const int HP = (H + 3) & ~3;                                             // heads in whole groups of four
+  float* w_raw = reinterpret_cast<float*>(w_mix + (size_t)H * SM_ROWS * SM_WSTRIDE);      // [HP][16][SM_WSTRIDE]
+  float* talk = w_raw + (size_t)HP * SM_ROWS * SM_WSTRIDE;                 // [SM_HEADS][SM_HEADS], zeros around [H][H]
+  float* bias = talk + SM_HEADS * SM_HEADS;                                // [SM_HEADS][SM_BIAS]: pb - r1 ln(1 + r2 distance)
+  int* key_row = reinterpret_cast<int*>(bias + SM_HEADS * SM_BIAS);        // [2][32]: the cached row of every key of this and the next tile
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-  if (a.talk != nullptr)
-    for (int i = threadIdx.x; i < H * H; i += SM_THREADS) talk[i] = a.talk[i];
+  if (a.talk != nullptr) {
+    for (int i = threadIdx.x; i < SM_HEADS * SM_HEADS; i += SM_THREADS)
+      talk[i] = i / SM_HEADS < H && i % SM_HEADS < H ? a.talk[i / SM_HEADS * H + i % SM_HEADS] : 0.f;
+    for (int i = threadIdx.x; i < (HP - H) * SM_ROWS * SM_WSTRIDE; i += SM_THREADS) w_raw[(size_t)H * SM_ROWS * SM_WSTRIDE + i] = 0.f;
+  }
   pdl_wait();
   const int seg = a.tile_seg[blockIdx.x];
   const int row0 = a.tile_row0[blockIdx.x];
@@ -134,6 +151,16 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
         warp_qk<D, SM_KEYS / 8, false, SM_KEYS>(s, q_frag, k_tiles + (size_t)(h / per_kv) * SM_KEYS * D, 0, lane);
         const float r1 = a.r1 != nullptr ? a.r1[h] : 0.f, r2 = a.r1 != nullptr ? a.r2[h] : 0.f;
         const float pb = a.pb != nullptr ? a.pb[h] : 0.f;
+        // the bias of the 47 distances between these rows and keys, entry row - key + 31 (distances below zero are not seen); the
+        // logarithm, like the exponential and the division below, is the hardware's approximate one (errors of a few units in the
+        // last place of a float32, far inside the bfloat16 rounding of the weight that follows)
+        float* head_bias = bias + h * SM_BIAS;
+#pragma unroll
+        for (int i = lane; i < SM_BIAS; i += 32) {
+          const int distance = first_pos - k0 + i - (SM_KEYS - 1);
+          head_bias[i] = a.r1 != nullptr && distance > 0 ? fmaf(-r1, __logf(fmaf(r2, (float)distance, 1.f)), pb) : pb;
+        }
+        __syncwarp();
         float* w = w_raw + (size_t)h * SM_ROWS * SM_WSTRIDE;
 #pragma unroll
         for (int j = 0; j < SM_KEYS / 8; ++j) {
@@ -147,10 +174,7 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
               const int distance = first_pos + row - (k0 + key);
               float weight = 0.f;
               if (distance >= 0 && row < rows) {
-                // the hardware's approximate logarithm, exponential and division (errors of a few units in
-                // the last place of a float32, far inside the bfloat16 rounding of the weight that follows)
-                float z = fmaf(s[j][2 * i + e], a.scale, pb);
-                if (a.r1 != nullptr) z -= r1 * __logf(fmaf(r2, (float)distance, 1.f));
+                const float z = fmaf(s[j][2 * i + e], a.scale, head_bias[row - key + SM_KEYS - 1]);
                 weight = __fdividef(1.f, 1.f + __expf(fminf(-z, 80.f)));
               }
               pair[e] = weight;
@@ -163,23 +187,39 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
     __syncthreads();
     if (more) fetch(false, parity ^ 1); else cp_async_commit();
     // ---- the weights mixed across the heads, rounded to bfloat16 for the second product
-    for (int idx = threadIdx.x; idx < H * SM_ROWS * (SM_KEYS / 2); idx += SM_THREADS) {
-      const int j = (idx % (SM_KEYS / 2)) * 2, r = (idx / (SM_KEYS / 2)) % SM_ROWS, h = idx / ((SM_KEYS / 2) * SM_ROWS);
-      float lo, hi;
+    // a thread takes two keys of a row for a share of the heads, so that every weight is read once per share
+    {
+      constexpr int PAIRS = SM_ROWS * SM_KEYS / 2, SHARE = SM_HEADS / (SM_THREADS / PAIRS);
+      const int j = (threadIdx.x % (SM_KEYS / 2)) * 2, r = (threadIdx.x / (SM_KEYS / 2)) % SM_ROWS, h0 = threadIdx.x / PAIRS * SHARE;
+      const float* weights = w_raw + r * SM_WSTRIDE + j;
+      bf16* mixed = w_mix + (size_t)r * SM_WSTRIDE + j;
       if (a.talk != nullptr) {
-        lo = hi = 0.f;
-        for (int g = 0; g < H; ++g) {
-          const float2 w = *reinterpret_cast<const float2*>(w_raw + ((size_t)g * SM_ROWS + r) * SM_WSTRIDE + j);
-          const float t = talk[h * H + g];
-          lo = fmaf(t, w.x, lo);
-          hi = fmaf(t, w.y, hi);
+        float2 sum[SHARE] = {};
+        for (int g = 0; g < HP; g += 4) {
+          float2 w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[e] = *reinterpret_cast<const float2*>(weights + (size_t)(g + e) * SM_ROWS * SM_WSTRIDE);
+#pragma unroll
+          for (int h = 0; h < SHARE; ++h) {
+            const float4 t = *reinterpret_cast<const float4*>(talk + (h0 + h) * SM_HEADS + g);
+            sum[h].x = fmaf(t.x, w[0].x, sum[h].x); sum[h].y = fmaf(t.x, w[0].y, sum[h].y);
+            sum[h].x = fmaf(t.y, w[1].x, sum[h].x); sum[h].y = fmaf(t.y, w[1].y, sum[h].y);
+            sum[h].x = fmaf(t.z, w[2].x, sum[h].x); sum[h].y = fmaf(t.z, w[2].y, sum[h].y);
+            sum[h].x = fmaf(t.w, w[3].x, sum[h].x); sum[h].y = fmaf(t.w, w[3].y, sum[h].y);
+          }
         }
+#pragma unroll
+        for (int h = 0; h < SHARE; ++h)
+          if (h0 + h < H)
+            *reinterpret_cast<uint32_t*>(mixed + (size_t)(h0 + h) * SM_ROWS * SM_WSTRIDE) = pack_bf16(sum[h].x, sum[h].y);
       } else {
-        const float2 w = *reinterpret_cast<const float2*>(w_raw + ((size_t)h * SM_ROWS + r) * SM_WSTRIDE + j);
-        lo = w.x;
-        hi = w.y;
+#pragma unroll
+        for (int h = 0; h < SHARE; ++h)
+          if (h0 + h < H) {
+            const float2 w = *reinterpret_cast<const float2*>(weights + (size_t)(h0 + h) * SM_ROWS * SM_WSTRIDE);
+            *reinterpret_cast<uint32_t*>(mixed + (size_t)(h0 + h) * SM_ROWS * SM_WSTRIDE) = pack_bf16(w.x, w.y);
+          }
       }
-      *reinterpret_cast<uint32_t*>(w_mix + ((size_t)h * SM_ROWS + r) * SM_WSTRIDE + j) = pack_bf16(lo, hi);
     }
     cp_async_wait<1>();      // this tile's values (the next keys may still be on their way)
     __syncthreads();
@@ -249,7 +289,7 @@ add_chunks_bf16_kernel(const float* partial, bf16* __restrict__ out, long long c
 static size_t sigmoid_mma_shared(int heads, int kv_heads, int dim, int vdim) {
   return sizeof(bf16) * ((size_t)heads * SM_ROWS * dim + (size_t)kv_heads * SM_KEYS * (dim + vdim) +
                          (size_t)heads * SM_ROWS * SM_WSTRIDE) +
-         sizeof(float) * ((size_t)heads * SM_ROWS * SM_WSTRIDE + (size_t)heads * heads) + sizeof(int) * 2 * SM_KEYS;
+         sizeof(float) * ((size_t)((heads + 3) & ~3) * SM_ROWS * SM_WSTRIDE + SM_HEADS * (SM_HEADS + SM_BIAS)) + sizeof(int) * 2 * SM_KEYS;
 }
 
 }  // namespace mlr
@@ -260,7 +300,7 @@ MLR_DEFINE_PDL_SWITCH
 
 // 1 if the tensor-core kernel takes these sizes, else 0.
 MLR_EXPORT int mlr_attention_sigmoid_mma_fits(int heads, int kv_heads, int dim, int vdim) {
-  if (heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || heads > SM_WARPS * SM_HEADS_PER_WARP) return 0;
+  if (heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || heads > SM_HEADS) return 0;
   if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128)) return 0;
   return sigmoid_mma_shared(heads, kv_heads, dim, vdim) <= 220 * 1024 ? 1 : 0;
 }
@@ -286,10 +326,10 @@ MLR_EXPORT int mlr_attention_sigmoid_mma(const void* q, const void* k_pool, cons
   SigmoidMmaArgs a{tile_seg, tile_row0, seg_q_start, seg_q_len, seg_pos0, block_table, seg_slot, r1, r2, pb, talk,
                    table_width, heads, kv_heads, page_size, chunk_keys, total_rows, scale};
   const size_t shared = sigmoid_mma_shared(heads, kv_heads, dim, vdim);
-  auto launch = [&](auto kernel) -> int {
+  auto launch = [&](auto kernel, int threads) -> int {
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     if (err != cudaSuccess) return (int)err;
-    launch_kernel(kernel, dim3(tiles, chunks), dim3(SM_THREADS), shared, stream, (const bf16*)q, (const bf16*)k_pool,
+    launch_kernel(kernel, dim3(tiles, chunks), dim3(threads), shared, stream, (const bf16*)q, (const bf16*)k_pool,
                   (const bf16*)v_pool, (bf16*)out, partial, a);
     int status = launch_status();
     if (status != MLR_OK || chunks == 1) return status;
@@ -298,8 +338,8 @@ MLR_EXPORT int mlr_attention_sigmoid_mma(const void* q, const void* k_pool, cons
                   (const float*)partial, (bf16*)out, count, chunks);
     return launch_status();
   };
-  if (dim == 64 && vdim == 64) return launch(attention_sigmoid_mma_kernel<64, 64>);
-  if (dim == 64 && vdim == 128) return launch(attention_sigmoid_mma_kernel<64, 128>);
-  if (dim == 128 && vdim == 64) return launch(attention_sigmoid_mma_kernel<128, 64>);
-  return launch(attention_sigmoid_mma_kernel<128, 128>);
+  if (dim == 64 && vdim == 64) return launch(attention_sigmoid_mma_kernel<64, 64>, SigmoidShape<64, 64>::THREADS);
+  if (dim == 64 && vdim == 128) return launch(attention_sigmoid_mma_kernel<64, 128>, SigmoidShape<64, 128>::THREADS);
+  if (dim == 128 && vdim == 64) return launch(attention_sigmoid_mma_kernel<128, 64>, SigmoidShape<128, 64>::THREADS);
+  return launch(attention_sigmoid_mma_kernel<128, 128>, SigmoidShape<128, 128>::THREADS);
 }

@@ -1586,7 +1586,7 @@ class CudaOps:
 
     SIGMOID_CHUNK_KEYS = 64       # keys one CTA of the sigmoid attention takes of a row, at least, when rows are few
     SIGMOID_MMA_CHUNK_KEYS = 128  # the same for the tensor-core kernel
-    SIGMOID_MMA_LONGEST = 512     # keys one CTA of the tensor-core kernel takes of a row, at most
+    SIGMOID_MMA_LONGEST = 384     # keys one CTA of the tensor-core kernel takes of a row, at most
     use_mma_sigmoid = True        # bfloat16 with key and value sizes of 64 or 128: the two products on the tensor cores
 
     def sigmoid_attention(self, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, batch: AttentionBatch,

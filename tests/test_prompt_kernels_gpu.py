@@ -191,3 +191,19 @@ def test_latent_attention_of_prompts(heads, rank, rot, page_size, window, sinks)
     torch.cuda.synchronize()
     cuda().raise_if_device_error()
     close(got, want, ATTENTION_BOUND, "latent attention")
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(16, 4, 128, 128), (14, 2, 64, 64), (3, 1, 64, 128), (6, 6, 128, 64)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, mixed):
+    """Head counts that fill no group of four, rows around the 16 of an entry, keys around tiles of 32 and a cut into chunks."""
+    lengths, before = [33, 5, 17], [0, 402, 95]
+    (k_pool, v_pool), cpu, batch = paged(lengths, before, lambda p, j: j <= p, 16, [(kv_heads, dim, 1.0), (kv_heads, vdim, 0.5)], 9)
+    q = rnd(6, sum(lengths), heads * dim).to(torch.bfloat16)
+    vectors = dict(distance=(torch.rand(heads, generator=generator(1)), torch.rand(heads, generator=generator(2))), score_bias=rnd(3, heads, std=0.3),
+                   head_mix=torch.eye(heads) + rnd(4, heads, heads, std=0.1)) if mixed else {}
+    args = (heads, kv_heads, dim, vdim, dim ** -0.5)
+    want = FAKE.sigmoid_attention(q.float(), k_pool.float(), v_pool.float(), cpu, *args, **vectors)
+    there = {k: tuple(t.to(DEVICE) for t in v) if isinstance(v, tuple) else v.to(DEVICE) for k, v in vectors.items()}
+    got = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, **there)
+    close(got, want, ATTENTION_BOUND, "sigmoid attention")
