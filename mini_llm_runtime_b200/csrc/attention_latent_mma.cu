@@ -284,9 +284,9 @@ latent_mma_kernel(const bf16* q, const bf16* pool, float* __restrict__ out, cons
 }
 
 // Chunks of a decoded row merged: one CTA per (item, head).  Warp 0 turns the chunks' maxima and
-// denominators into one factor per chunk; then every thread sums its four columns over the chunks in
-// chunk order, eight chunks' loads in flight at a time.
-__global__ void __launch_bounds__(128)
+// denominators into one factor per chunk; then every thread sums two columns over the chunks in
+// chunk order, sixteen chunks' loads in flight at a time.
+__global__ void __launch_bounds__(256)
 latent_merge_kernel(const float* partial, float* __restrict__ out, const int* __restrict__ decode_seg,
                     const int* __restrict__ seg_q_start, const float* __restrict__ sink, int items, int chunks, int heads,
                     int rank) {
@@ -310,13 +310,19 @@ latent_merge_kernel(const float* partial, float* __restrict__ out, const int* __
   }
   __syncthreads();
   float* dst = out + ((size_t)seg_q_start[seg] * heads + head) * rank;
-  for (int d = threadIdx.x * 2; d < rank; d += 256) {       // rank + 2 is even: pairs of columns are 8-byte aligned
+  for (int d = threadIdx.x * 2; d < rank; d += blockDim.x * 2) {       // rank + 2 is even: pairs of columns are 8-byte aligned
     float2 sum = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int c = 0; c < chunks; ++c) {
-      const float2 v = __ldcg(reinterpret_cast<const float2*>(mine + c * step + d));
-      sum.x = fmaf(v.x, factor[c], sum.x);
-      sum.y = fmaf(v.y, factor[c], sum.y);
+    for (int c0 = 0; c0 < chunks; c0 += 16) {
+      float2 v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (c0 + i < chunks) v[i] = __ldcg(reinterpret_cast<const float2*>(mine + (c0 + i) * step + d));
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (c0 + i < chunks) {
+          sum.x = fmaf(v[i].x, factor[c0 + i], sum.x);
+          sum.y = fmaf(v[i].y, factor[c0 + i], sum.y);
+        }
     }
     *reinterpret_cast<float2*>(dst + d) = sum;
   }
@@ -541,6 +547,20 @@ MLR_EXPORT int mlr_latent_attention_mma(const void* q, const void* pool, float* 
   return latent_mma_launch<2, false>(q, pool, out, tile_seg, tile_row0, dim3(tiles, (heads + 1) / 2), args, stream);
 }
 
+// A decoded row's CTAs are few and wait for memory: as many key tiles on their way as fit (up to three beside the one at work).
+static int latent_decode_stages(int heads, int width) {
+  int stages = 2;
+  while (stages < 4 && latent_mma_shared(heads <= LM_TOKENS ? 1 : 2, width, stages + 1) <= 160 * 1024) ++stages;
+  return stages;
+}
+
+// CTAs of a decode call that share an SM, by their shared memory.
+MLR_EXPORT int mlr_latent_attention_mma_decode_per_sm(int heads, int rank, int rot) {
+  const size_t shared = latent_mma_shared(heads <= LM_TOKENS ? 1 : 2, rank + rot, latent_decode_stages(heads, rank + rot));
+  const int together = (int)(227 * 1024 / (shared + 1024));
+  return together < 1 ? 1 : together > 2 ? 2 : together;
+}
+
 // Floats of scratch a decode call with `chunks` key chunks needs (0 for one chunk).
 MLR_EXPORT long long mlr_latent_attention_mma_decode_scratch(int count, int chunks, int heads, int rank) {
   return chunks <= 1 ? 0 : (long long)count * chunks * heads * (rank + 2);
@@ -563,14 +583,13 @@ MLR_EXPORT int mlr_latent_attention_mma_decode(const void* q, const void* pool, 
   args.decode_seg = decode_seg;
   args.partial = partial;
   const int blocks16 = (heads + LM_TOKENS - 1) / LM_TOKENS;
-  // a decoded row's CTAs are few and wait for memory: as many key tiles on their way as fit (up to three)
-  while (args.stages < 4 && latent_mma_shared(blocks16 == 1 ? 1 : 2, rank + rot, args.stages + 1) <= 160 * 1024) ++args.stages;
+  args.stages = latent_decode_stages(heads, rank + rot);
   if (blocks16 == 1)
     status = latent_mma_launch<1, true>(q, pool, out, nullptr, nullptr, dim3(count, 1, chunks), args, stream);
   else
     status = latent_mma_launch<2, true>(q, pool, out, nullptr, nullptr, dim3(count, (blocks16 + 1) / 2, chunks), args, stream);
   if (status != MLR_OK || chunks == 1) return status;
-  launch_kernel(latent_merge_kernel, dim3((unsigned)(count * heads)), dim3(128), 0, stream, (const float*)partial, out,
+  launch_kernel(latent_merge_kernel, dim3((unsigned)(count * heads)), dim3(rank > 256 ? 256 : 128), 0, stream, (const float*)partial, out,
                 decode_seg, seg_q_start, sink, count, chunks, heads, rank);
   return launch_status();
 }

@@ -392,40 +392,83 @@ expert_down_kernel(const T* hidden, const int* chosen, const float* weights, con
 __global__ void __launch_bounds__(1024)
 sort_pairs_kernel(const int* chosen, const float* weights, int* place, int* token_of, float* sorted_weights, int* tiles,
                   int pairs, int top, int experts, int tile_rows, int max_tiles) {
+  // Bound by round trips: a thread asks for eight of its choices at once (one at a time between the atomics, 12,288 pairs took 19 to
+  // 23 us, most of it waiting; 13 now), and a warp lays the experts' runs and tiles out by prefix sums.
+  constexpr int BATCH = 8;
   pdl_trigger();
-  extern __shared__ int counts[];        // [experts] counts, [experts + 1] starts, [experts] cursors
-  int* starts = counts + experts;
-  int* cursor = starts + experts + 1;
+  extern __shared__ int counts[];        // [experts] counts, [experts] cursors
+  int* cursor = counts + experts;
+  __shared__ int used_tiles;
   for (int e = threadIdx.x; e < experts; e += blockDim.x) counts[e] = 0;
   pdl_wait();
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&counts[chosen[p]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0, tile = 0;
-    for (int e = 0; e < experts; ++e) {
-      starts[e] = at;
-      cursor[e] = at;
-      for (int r = 0; r < counts[e] && tile < max_tiles; r += tile_rows, ++tile) {
-        tiles[3 * tile] = e;
-        tiles[3 * tile + 1] = at + r;
-        tiles[3 * tile + 2] = at + counts[e];
-      }
-      at += counts[e];
-    }
-    starts[experts] = at;
-    for (; tile < max_tiles; ++tile) {
-      tiles[3 * tile] = -1;
-      tiles[3 * tile + 1] = 0;
-      tiles[3 * tile + 2] = 0;
-    }
+  int first[BATCH];      // the thread's first choices, kept for the second pass
+#pragma unroll
+  for (int i = 0; i < BATCH; ++i) {
+    const int p = threadIdx.x + i * blockDim.x;
+    first[i] = p < pairs ? __ldcg(chosen + p) : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < BATCH; ++i)
+    if (first[i] >= 0) atomicAdd(&counts[first[i]], 1);
+  for (int p0 = threadIdx.x + BATCH * blockDim.x; p0 < pairs; p0 += BATCH * blockDim.x) {
+    int more[BATCH];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) more[i] = p0 + i * (int)blockDim.x < pairs ? __ldcg(chosen + p0 + i * blockDim.x) : -1;
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i)
+      if (more[i] >= 0) atomicAdd(&counts[more[i]], 1);
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int at = atomicAdd(&cursor[chosen[p]], 1);
+  if (threadIdx.x < 32) {
+    int at = 0, tile = 0;      // places and tiles of the experts before
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + threadIdx.x, count = e < experts ? counts[e] : 0, own = (count + tile_rows - 1) / tile_rows;
+      int places = count, tiles_to = own;      // inclusive prefix sums
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, places, offset), y = __shfl_up_sync(0xffffffffu, tiles_to, offset);
+        if ((int)threadIdx.x >= offset) {
+          places += x;
+          tiles_to += y;
+        }
+      }
+      const int start = at + places - count;
+      if (e < experts) cursor[e] = start;
+      for (int i = 0; i < own; ++i) {
+        const int index = tile + tiles_to - own + i;
+        if (index >= max_tiles) break;
+        tiles[3 * index] = e;
+        tiles[3 * index + 1] = start + i * tile_rows;
+        tiles[3 * index + 2] = start + count;
+      }
+      at += __shfl_sync(0xffffffffu, places, 31);
+      tile += __shfl_sync(0xffffffffu, tiles_to, 31);
+    }
+    if (threadIdx.x == 0) used_tiles = min(tile, max_tiles);
+  }
+  __syncthreads();
+  for (int index = used_tiles + threadIdx.x; index < max_tiles; index += blockDim.x) {
+    tiles[3 * index] = -1;
+    tiles[3 * index + 1] = 0;
+    tiles[3 * index + 2] = 0;
+  }
+  auto put = [&](int p, int expert) {
+    const int at = atomicAdd(&cursor[expert], 1);
     place[p] = at;
     token_of[at] = p / top;
     if (sorted_weights != nullptr) sorted_weights[at] = __ldcg(weights + p);
+  };
+#pragma unroll
+  for (int i = 0; i < BATCH; ++i)
+    if (first[i] >= 0) put(threadIdx.x + i * blockDim.x, first[i]);
+  for (int p0 = threadIdx.x + BATCH * blockDim.x; p0 < pairs; p0 += BATCH * blockDim.x) {
+    int more[BATCH];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) more[i] = p0 + i * (int)blockDim.x < pairs ? __ldcg(chosen + p0 + i * blockDim.x) : -1;
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i)
+      if (more[i] >= 0) put(p0 + i * blockDim.x, more[i]);
   }
 }
 
@@ -447,9 +490,38 @@ gather_rows_by_kernel(const T* x, const int* token_of, T* out, int width_bytes) 
 
 __global__ void __launch_bounds__(256)
 combine_pairs_kernel(const float* y, const int* place, const float* weights, float* out, int N, int top) {
+  // Bound by reading y once.  Pieces of four columns, four pairs asked for together (number by number behind a place and a weight of
+  // its own each: 37 us for 2,048 rows of 2,048 with six pairs, 29 now).
+  constexpr int BATCH = 4;
   pdl_trigger();
   pdl_wait();
   const int row = blockIdx.x;
+  if (N % 4 == 0) {      // y and out come from the allocator, 16-byte aligned
+    for (int n = threadIdx.x * 4; n < N; n += blockDim.x * 4) {
+      float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int t0 = 0; t0 < top; t0 += BATCH) {
+        float4 part[BATCH];
+        float weight[BATCH];
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i)
+          if (t0 + i < top) {
+            const size_t pair = (size_t)row * top + t0 + i;
+            weight[i] = weights != nullptr ? __ldcg(weights + pair) : 1.f;
+            part[i] = __ldcg(reinterpret_cast<const float4*>(y + (size_t)__ldcg(place + pair) * N + n));
+          }
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i)
+          if (t0 + i < top) {      // in the order of the row's choices
+            total.x = fmaf(weight[i], part[i].x, total.x);
+            total.y = fmaf(weight[i], part[i].y, total.y);
+            total.z = fmaf(weight[i], part[i].z, total.z);
+            total.w = fmaf(weight[i], part[i].w, total.w);
+          }
+      }
+      *reinterpret_cast<float4*>(out + (size_t)row * N + n) = total;
+    }
+    return;
+  }
   for (int n = threadIdx.x; n < N; n += blockDim.x) {
     float total = 0.f;
     for (int t = 0; t < top; ++t)
@@ -567,7 +639,7 @@ MLR_EXPORT int mlr_sort_pairs(const int* chosen, const float* weights, int* plac
                               int tile_rows, int max_tiles, cudaStream_t stream) {
   if (pairs == 0) return MLR_OK;
   if (pairs < 0 || top <= 0 || experts <= 0 || tile_rows <= 0 || max_tiles <= 0) return MLR_BAD_SIZE;
-  const size_t shared = sizeof(int) * (3 * (size_t)experts + 1);
+  const size_t shared = sizeof(int) * 2 * (size_t)experts;
   if (shared > 48 * 1024) return MLR_TOO_LARGE;
   launch_kernel(sort_pairs_kernel, dim3(1), dim3(1024), shared, stream, chosen, weights, place, token_of, sorted_weights, tiles, pairs, top, experts,
                 tile_rows, max_tiles);
@@ -587,6 +659,7 @@ MLR_EXPORT int mlr_combine_pairs(const float* y, const int* place, const float* 
                                  cudaStream_t stream) {
   if (rows == 0) return MLR_OK;
   if (rows < 0 || N <= 0 || top <= 0) return MLR_BAD_SIZE;
+  if (N % 4 == 0 && (((uintptr_t)y | (uintptr_t)out) & 15) != 0) return MLR_BAD_ALIGNMENT;
   launch_kernel(combine_pairs_kernel, dim3(rows), dim3(256), 0, stream, y, place, weights, out, N, top);
   return launch_status();
 }

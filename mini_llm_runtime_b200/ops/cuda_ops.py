@@ -1240,7 +1240,6 @@ class CudaOps:
                                  gate=gate, gate_per_head=gate_per_head)
 
     use_latent_decode_kernel = True
-    latent_decode_chunk_tiles = 4      # key tiles (of 32 keys) a CTA of the decode attention takes at least
 
     def latent_attention(self, q: torch.Tensor, pool: torch.Tensor, batch: AttentionBatch, heads: int, rank: int,
                          rot: int, scale: float, window: int, sink: torch.Tensor | None) -> torch.Tensor:
@@ -1269,10 +1268,13 @@ class CudaOps:
             # chunks so that the step's CTAs fill the device about twice
             listed = None if batch.num_decode == batch.num_segments else batch.plan["decode_seg"]
             longest = min(batch.max_kv_len, window + 31) if window else batch.max_kv_len
-            key_tiles = -(-longest // 32) + 1
+            key_tiles = -(-longest // 32) + (1 if window else 0)      # a window may begin inside a tile
             groups = batch.num_decode * -(-(-(-heads // 16)) // 2)
-            # chunks of at least ``latent_decode_chunk_tiles`` key tiles, at most 32 of them (the merge kernel's lanes)
-            chunks = max(1, min(key_tiles // self.latent_decode_chunk_tiles, 2 * self.sm_count(q.device) // groups, 32))
+            # As many chunks as run together (at most 32, the merge kernel's lanes), then as few as still take as many key tiles
+            # each: a tile costs 3 us, a second round of CTAs its tiles again.  Measured in us with 16 heads of 512 + 64, chunks of at
+            # least four tiles over two CTAs per SM / now: 8 rows at 300 keys 24 / 12, at 1,024 25 / 17, at 2,047 22 / 20.
+            together = max(1, min(self._latent_decode_per_sm(heads, rank, rot) * self.sm_count(q.device) // groups, 32, key_tiles))
+            chunks = -(-key_tiles // -(-key_tiles // together))
             partial = None
             if chunks > 1:
                 partial = torch.empty(batch.num_decode * chunks * heads * (rank + 2), dtype=torch.float32, device=q.device)
@@ -1314,6 +1316,13 @@ class CudaOps:
                 _ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_pos0), _ptr(batch.block_table),
                 _ptr(batch.seg_slot), batch.block_table.shape[1], tiles, *tail), "latent attention")
         return out
+
+    def _latent_decode_per_sm(self, heads: int, rank: int, rot: int) -> int:
+        cache = self.__dict__.setdefault("_latent_decode_together", {})
+        if (heads, rank, rot) not in cache:
+            cache[(heads, rank, rot)] = int(build.load_library("attention_latent_mma").mlr_latent_attention_mma_decode_per_sm(
+                heads, rank, rot))
+        return cache[(heads, rank, rot)]
 
     def _latent_tcgen05_fits(self, heads: int, rank: int, rot: int) -> bool:
         cache = self.__dict__.setdefault("_latent_wide_fits", {})
