@@ -26,7 +26,10 @@
 //
 // matrix_memory_pairs_kernel    all chunks at once: A, D_last and K of every chunk, q, k and v as bfloat16.
 // matrix_memory_chunks_kernel   the chunks of a (request, head) one after the other, value channels over blocks; the
-//                               state stays in registers as accumulators.
+//                               state stays in registers as accumulators.  That chain leaves SMs idle, so long segments are cut
+//                               into runs of chunks: a first launch takes every run but the last from zero, states only
+//                               (the recurrence is linear in S: a run's end is its keeps' product times the state before plus what
+//                               its own tokens leave), the second starts each run from what the runs before left.
 #include "mma_attention.cuh"
 #include "copy_async.cuh"
 #include "lane_sums.cuh"
@@ -46,6 +49,9 @@ struct MemoryArgs {
   bf16 *q16, *k16, *v16;                // chunks: [rows, heads * dim], the same, [rows, heads * vdim]
   float* states;                        // [slots, heads, vdim + 1, dim]
   float* maxima;                        // [slots, heads]
+  float* ends;                          // runs of chunks: [places, heads, vdim + 1, dim], what a run's own tokens leave (see run_place)
+  float* spans;                         // [places, heads]: product of a run's keeps
+  int run;                              // chunks of a run; 0: segments are not cut
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, dim, vdim;
   float cap, guard, eps, q_scale;
@@ -524,10 +530,21 @@ __device__ __forceinline__ void mma_cols(float (*c)[4], const uint32_t* a, const
   }
 }
 
-// grid: (segments, heads, blocks of 32 state rows).  Warp w keeps the key channels w D / 4 .. of the state.
-template <int D>
+// Where a run that starts at `row` keeps what it leaves: one place per aligned stretch of a run's rows for a segment's first run
+// and one for another run.  Of segments of several runs (the only ones with places) no two first runs start in one stretch, nor two
+// later ones: they lie more than a run's rows apart.
+__device__ __forceinline__ size_t run_place(int row, int run_rows, bool first) { return 2 * (size_t)(row / run_rows) + (first ? 1 : 0); }
+inline long long run_places(int rows, int run_rows) { return 2ll * (rows / run_rows + 1); }
+
+// grid: (segments * runs, heads, blocks of 16 state rows).  Warp w keeps the key channels w D / 4 .. of the state.
+// WHOLE: segments that are not cut (the index arithmetic of runs costs them 4 %: 100 -> 104 us for 1,300 and 748 rows).  RUNS: the
+// outputs of all runs and a segment's last state.  LEFT: only what the runs before a segment's last leave; the first run starts from the request's state and also puts a copy of that
+// where the last run has its place, since the second launch's last run overwrites the state while its first may still read it.
+enum Part { WHOLE, LEFT, RUNS };
+
+template <int D, Part PART>
 __global__ void __launch_bounds__(128)
-matrix_memory_chunks_kernel(MemoryArgs p) {
+matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
   pdl_trigger();
   constexpr int PITCH = D + 8, MT = D / 64, NT = CHUNK_COLS / 8, PIECES = D / 8;
   extern __shared__ __align__(16) uint8_t raw[];
@@ -536,9 +553,16 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
   bf16* s_parts = v_tiles + 2 * CHUNK * CHUNK_PITCH;                    // 3 x [D][CHUNK_PITCH]
   bf16* w_parts = s_parts + 3 * D * CHUNK_PITCH;                        // 3 x [64][CHUNK_PITCH]
   float2* factors = reinterpret_cast<float2*>(w_parts + 3 * CHUNK * CHUNK_PITCH);      // 2 x [64]
-  const int seg = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * CHUNK_COLS, V = p.vdim;
+  constexpr bool ENDS = PART == LEFT;
+  const int seg = PART == WHOLE ? blockIdx.x : blockIdx.x % segments, head = blockIdx.y, col0 = blockIdx.z * CHUNK_COLS, V = p.vdim;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int q_start = p.seg_q_start[seg], q_len = p.seg_q_len[seg];
+  const int segment_start = p.seg_q_start[seg], segment_rows = p.seg_q_len[seg];
+  const int run_rows = PART == WHOLE ? segment_rows : p.run * CHUNK, run = PART == WHOLE ? 0 : blockIdx.x / segments;
+  const int runs = PART == WHOLE || segment_rows <= 0 ? 1 : (segment_rows + run_rows - 1) / run_rows;
+  if (PART != WHOLE && (run >= runs || (ENDS && run == runs - 1))) return;
+  const int q_start = segment_start + run * run_rows, q_len = PART == WHOLE ? segment_rows : min(run_rows, segment_rows - run * run_rows);      // this run's
+  const size_t cells = (size_t)(V + 1) * D;
+  auto place_of = [&](int r) { return run_place(segment_start + r * run_rows, run_rows, r == 0) * p.heads + head; };
   float* state = p.states + ((size_t)p.seg_slot[seg] * p.heads + head) * (size_t)(V + 1) * D;
   // value channels beyond the last: the normaliser's is one, the others zero; no copy overwrites them
   for (int idx = threadIdx.x; idx < 2 * CHUNK * CHUNK_COLS; idx += 128) {
@@ -555,7 +579,7 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
       const int r = idx / PIECES, c = (idx - r * PIECES) * 8;
       const bool valid = r < count;
       const size_t at = valid ? (row0 + r) * p.heads * D + (size_t)head * D + c : 0;
-      cp_async_16(q_tile + r * PITCH + c, p.q16 + at, valid);
+      if (!ENDS) cp_async_16(q_tile + r * PITCH + c, p.q16 + at, valid);
       cp_async_16(k_tile + r * PITCH + c, p.k16 + at, valid);
     }
     for (int idx = threadIdx.x; idx < CHUNK * (CHUNK_COLS / 8); idx += 128) {
@@ -577,6 +601,8 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
     *d = warp * (D / 4) + mt * 16 + (lane >> 2) + 8 * (e >> 1);
     *c = col0 + nt * 8 + (lane & 3) * 2 + (e & 1);
   };
+  // the state before the run: the request's, or what the runs before leave one after the other
+  const float* start = PART == WHOLE ? state : runs == 1 || ENDS ? (run == 0 ? state : nullptr) : p.ends + place_of(run == 0 ? runs - 1 : 0) * cells;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -585,8 +611,25 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
       for (int e = 0; e < 4; ++e) {
         int d, c;
         place(mt, nt, e, &d, &c);
-        S[mt][nt][e] = c <= V ? __ldcg(state + (size_t)c * D + d) : 0.f;
+        S[mt][nt][e] = (PART == WHOLE || start != nullptr) && c <= V ? __ldcg(start + (size_t)c * D + d) : 0.f;
+        if (ENDS && run == 0 && c <= V) p.ends[place_of(runs - 1) * cells + (size_t)c * D + d] = S[mt][nt][e];
       }
+  if (PART == RUNS)
+    for (int r = 1; r < run; ++r) {
+      const float span = __ldcg(p.spans + place_of(r));
+      const float* left = p.ends + place_of(r) * cells;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            int d, c;
+            place(mt, nt, e, &d, &c);
+            S[mt][nt][e] = fmaf(S[mt][nt][e], span, c <= V ? __ldcg(left + (size_t)c * D + d) : 0.f);
+          }
+    }
+  float span = 1.f;
   int which = 0;
   for (int t0 = 0; t0 < q_len; t0 += CHUNK, which ^= 1) {
     const int count = min(CHUNK, q_len - t0);
@@ -603,6 +646,7 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
     const float* a_row[2] = {p.pairs + ((row0 + r0) * p.heads + head) * CHUNK + (lane & 3) * 2,
                              p.pairs + ((row0 + r0 + 8) * p.heads + head) * CHUNK + (lane & 3) * 2};
     float2 a_pair[CHUNK / 16][4];
+    if (!ENDS)
 #pragma unroll
     for (int ks = 0; ks < CHUNK / 16; ++ks)
 #pragma unroll
@@ -612,6 +656,7 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
           a_pair[ks][e] = __ldcg(reinterpret_cast<const float2*>(a_row[e & 1] + ks * 16 + 8 * (e >> 1)));
       }
     // the state and the weighed values in parts
+    if (!ENDS)
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -642,7 +687,7 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
     for (int n = 0; n < 3; ++n)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) o[n][nt][0] = o[n][nt][1] = o[n][nt][2] = o[n][nt][3] = 0.f;
-    if (warp * 16 < count) {
+    if (!ENDS && warp * 16 < count) {
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
         uint32_t a[4];
@@ -689,6 +734,7 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
     }
     // the state behind the chunk
     const float kept = factor[count - 1].y;
+    span *= kept;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
@@ -712,8 +758,9 @@ matrix_memory_chunks_kernel(MemoryArgs p) {
       for (int e = 0; e < 4; ++e) {
         int d, c;
         place(mt, nt, e, &d, &c);
-        if (c <= V) state[(size_t)c * D + d] = S[mt][nt][e];
+        if (c <= V && (PART != RUNS || run == runs - 1)) (ENDS ? p.ends + place_of(run) * cells : state)[(size_t)c * D + d] = S[mt][nt][e];
       }
+  if (ENDS && blockIdx.z == 0 && threadIdx.x == 0) p.spans[place_of(run)] = span;
 }
 
 template <int D>
@@ -722,15 +769,26 @@ static int launch_chunks(const MemoryArgs& p, int segments, int max_q_len, cudaS
                             sizeof(float2) * 2 * CHUNK;
   static_assert(shared <= 227 * 1024, "tiles");
   constexpr size_t pairs_shared = sizeof(bf16) * (size_t)(2 * CHUNK * (D + 8)) + sizeof(float) * CHUNK * (CHUNK + 1);
-  cudaError_t err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  cudaError_t err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D, RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D, LEFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(matrix_memory_pairs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_shared);
   if (err != cudaSuccess) return (int)err;
   launch_kernel(matrix_memory_pairs_kernel<D>, dim3((max_q_len + CHUNK - 1) / CHUNK, p.heads, segments), dim3(128), pairs_shared,
                 stream, p);
-  const int status = launch_status();
+  int status = launch_status();
   if (status != MLR_OK) return status;
-  launch_kernel(matrix_memory_chunks_kernel<D>, dim3(segments, p.heads, (p.vdim + CHUNK_COLS) / CHUNK_COLS), dim3(128), shared, stream, p);
+  const int runs = p.run > 0 ? (max_q_len + p.run * CHUNK - 1) / (p.run * CHUNK) : 1, blocks = (p.vdim + CHUNK_COLS) / CHUNK_COLS;
+  if (runs == 1) {
+    launch_kernel(matrix_memory_chunks_kernel<D, WHOLE>, dim3(segments, p.heads, blocks), dim3(128), shared, stream, p, segments);
+    return launch_status();
+  }
+  launch_kernel(matrix_memory_chunks_kernel<D, LEFT>, dim3(segments * (runs - 1), p.heads, blocks), dim3(128), shared, stream, p, segments);
+  if ((status = launch_status()) != MLR_OK) return status;
+  launch_kernel(matrix_memory_chunks_kernel<D, RUNS>, dim3(segments * runs, p.heads, blocks), dim3(128), shared, stream, p, segments);
   return launch_status();
 }
 
@@ -853,18 +911,38 @@ MLR_DEFINE_PDL_SWITCH
 // Whether prompts of these head sizes can go through the tensor cores in chunks (with `pairs`).
 MLR_EXPORT int mlr_matrix_memory_chunks_fit(int dim, int vdim) { return chunks_fit(dim, vdim); }
 
+// Chunks of a run for a step on the tensor cores (0: segments are not cut), and the float32 numbers of scratch that runs need.  So many
+// runs that the blocks of a launch still run together (two share an SM; every segment may add a short run), at least MIN_RUN chunks
+// each, and only where LEAST_RUNS or more fit (blocks that share an SM slow one another down) and a portion is long enough to pay for
+// the second launch and its scratch.  Measured in us without / with runs, heads of 128: one request of 2,048 rows, 7 heads 120 / 81,
+// 4 heads 114 / 61; 1,300 and 748 rows, 4 heads 84 / 63; 4 heads of 64, 2,048 rows 94 / 58.  Not cut: 7 heads, 1,300 and 748 rows
+// 96 / 98, 16 heads 136 / 182; 600 rows, 4 heads 52 / 57; 1,024 rows, 4 heads of 64 57 / 58.
+MLR_EXPORT int mlr_matrix_memory_run(int rows, int segments, int max_q_len, int heads, int vdim) {
+  constexpr int MIN_RUN = 4, LEAST_RUNS = 4, SHORTEST = 1024;
+  const int blocks = heads * ((vdim + CHUNK_COLS) / CHUNK_COLS), chunks = (rows + CHUNK - 1) / CHUNK;
+  const int runs = 2 * sm_count() / (blocks < 1 ? 1 : blocks) - (segments - 1);
+  if (runs < LEAST_RUNS || max_q_len <= SHORTEST) return 0;
+  int run = (chunks + runs - 1) / runs;
+  if (run < MIN_RUN) run = MIN_RUN;
+  return run * CHUNK < max_q_len ? run : 0;
+}
+MLR_EXPORT long long mlr_matrix_memory_run_scratch(int rows, int run, int heads, int dim, int vdim) {
+  return run <= 0 ? 0 : run_places(rows, run * CHUNK) * heads * ((long long)(vdim + 1) * dim + 1);
+}
+
 // q, k: float32 rows of heads * dim entries; v, gate: rows of heads * vdim; i_raw, f_raw: rows of `heads` entries (each
 // with its own row stride); i_bias, f_bias: float32 [heads]; weight: float32 [heads * vdim]; coef: float32 scratch
 // [rows, heads, 4], reads: [rows, heads, vdim], norms: [rows, heads] (all three null for steps of single rows); pairs:
 // float32 scratch [rows, heads, 64 + 2] and packed: bfloat16 scratch [rows, heads, 2 dim + vdim] (both or neither: chunks
-// on the tensor cores, or the token-by-token scan; 16-byte aligned); states:
+// on the tensor cores, or the token-by-token scan; 16-byte aligned); run, ends: chunks of a run and the scratch that needs (as the two
+// functions above say; 0 and null: no runs); states:
 // float32 [slots, heads, vdim + 1, dim], maxima: float32 [slots, heads]; out: [rows, heads * vdim] in `dtype`.
 // max_q_len: the longest segment of the step.
 MLR_EXPORT int mlr_matrix_memory(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
                                  long long v_stride, const float* i_raw, long long i_stride, const float* f_raw,
                                  long long f_stride, const float* gate, long long gate_stride, const float* i_bias,
                                  const float* f_bias, const float* weight, float* coef, float* reads, float* norms,
-                                 float* pairs, void* packed, float* states, float* maxima, void* out, const int* seg_q_start, const int* seg_q_len,
+                                 float* pairs, void* packed, float* ends, int run, float* states, float* maxima, void* out, const int* seg_q_start, const int* seg_q_len,
                                  const int* seg_slot, int rows, int segments, int max_q_len, int heads, int dim, int vdim,
                                  float cap, float guard, float eps, float q_scale, int dtype, cudaStream_t stream) {
   if (segments == 0 || rows == 0) return MLR_OK;
@@ -873,10 +951,11 @@ MLR_EXPORT int mlr_matrix_memory(const float* q, long long q_stride, const float
   bf16* q16 = (bf16*)packed;
   bf16* k16 = q16 == nullptr ? nullptr : q16 + (size_t)rows * heads * dim;
   bf16* v16 = q16 == nullptr ? nullptr : k16 + (size_t)rows * heads * dim;
-  if ((pairs == nullptr) != (packed == nullptr)) return MLR_BAD_SIZE;
+  if ((pairs == nullptr) != (packed == nullptr) || run < 0 || (run > 0 && (ends == nullptr || pairs == nullptr))) return MLR_BAD_SIZE;
   MemoryArgs p{q, k, v, i_raw, f_raw, gate, q_stride, k_stride, v_stride, i_stride, f_stride, gate_stride, i_bias, f_bias,
                weight, reinterpret_cast<float4*>(coef), reads, norms, pairs,
-               pairs == nullptr ? nullptr : reinterpret_cast<float2*>(pairs + (size_t)rows * heads * CHUNK), q16, k16, v16, states, maxima, seg_q_start, seg_q_len, seg_slot, heads,
+               pairs == nullptr ? nullptr : reinterpret_cast<float2*>(pairs + (size_t)rows * heads * CHUNK), q16, k16, v16, states, maxima, ends,
+               run <= 0 ? nullptr : ends + (size_t)run_places(rows, run * CHUNK) * heads * (vdim + 1) * dim, run, seg_q_start, seg_q_len, seg_slot, heads,
                dim, vdim, cap, guard, eps, q_scale};
   auto multiple = [](long long n) { return n % 4 == 0; };
   auto aligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };

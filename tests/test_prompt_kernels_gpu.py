@@ -207,3 +207,31 @@ def test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, mixed):
     there = {k: tuple(t.to(DEVICE) for t in v) if isinstance(v, tuple) else v.to(DEVICE) for k, v in vectors.items()}
     got = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, **there)
     close(got, want, ATTENTION_BOUND, "sigmoid attention")
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 128), (3, 64, 72)])
+@pytest.mark.parametrize("lengths,slots,order", [([1, 512, 513, 1100], [3, 0, 2, 1], None), ([515, 3, 1030], [1, 2, 0], [2, 0, 1])])
+def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
+    """Segments around the borders of runs of four chunks and more, rows of requests in any order, gates that forget and keep everything: as
+    without runs (which the 64-bit oracle vouches for elsewhere), whose products are the same and whose sums another order."""
+    ctx, rows = segments(lengths, slots, order), sum(lengths)
+    assert cuda()._memory_chunks_fit(dim, vdim)
+    q, k, v, gate = rnd(1, rows, heads * dim), rnd(2, rows, heads * dim), rnd(3, rows, heads * vdim), rnd(4, rows, heads * vdim)
+    i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
+    f_raw[rows // 3], f_raw[rows // 2] = -80.0, 80.0
+    bias, weight = torch.zeros(heads), 1 + rnd(7, heads * vdim, std=0.1)
+    state, maximum = rnd(8, len(lengths), heads, vdim + 1, dim, std=0.5), rnd(9, len(lengths), heads)
+    results = []
+    for runs in (False, True):
+        cuda().use_memory_runs = runs
+        try:
+            s, m = state.to(DEVICE), maximum.to(DEVICE)
+            out = cuda().matrix_memory(*(spaced(t, 8) for t in (q, k, v, i_raw, f_raw)), bias.to(DEVICE), bias.to(DEVICE) + 3, 15.0, 1e-6,
+                                       spaced(gate, 8), weight.to(DEVICE), 1e-6, s, m, ctx, heads, dim, vdim, torch.bfloat16)
+        finally:
+            cuda().use_memory_runs = True
+        results.append((out.cpu(), s.cpu(), m.cpu()))
+    (out, s, m), (want, want_s, want_m) = results[1], results[0]
+    assert torch.equal(m, want_m)
+    close(s.flatten(0, 1), want_s.flatten(0, 1), 200 * UNIT, "state")      # sums of 64 products at a time, once per chunk
+    close(out, want, 2.0 ** -8, "output")
