@@ -1013,8 +1013,12 @@ class CudaOps:
             maps = torch.empty((q.shape[0], 2 * heads * vdim), dtype=torch.float32, device=q.device)
             page_size = k_pool.shape[2]
             # Measured in us, 7 heads of 2 x 64 with values of 128, mma.sync / tcgen05: 2,048 rows 291 / 57, 128 rows 127 / 24,
-            # 17 rows 38 / 25, 5 rows 33 / 28, 2 rows 21 / 25 (both wait for the host there).
+            # 12 rows 27 / 23, 7 rows 21 / 23, 4 rows 20 / 23, of them 16 heads 56 / 23, 35 / 23, 23 / 23; 4 rows behind 500 41 / 27.  A
+            # step of few rows and keys has nothing but launches in it, and the older kernel's are cheaper (8 rows 20 / 23, 4 + 2
+            # rows and a decoded one 26 / 30); its time grows by 2 us a row.
             if (self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and batch.max_q_len >= 4 and page_size >= 8
+                    and (int(batch.max_kv_len) > (256 if batch.num_decode else 128)
+                         or q.shape[0] - batch.num_decode >= (16 if batch.num_decode else 12))
                     and page_size & (page_size - 1) == 0 and scale > 0 and k_pool.data_ptr() % 16 == 0
                     and v_pool.data_ptr() % 16 == 0):
                 space = self._workspace(q.device)
@@ -1292,7 +1296,12 @@ class CudaOps:
                 "latent attention (decode)")
             tiles -= batch.num_decode       # the one-row segments' tiles are the last of the list
         page_size = pool.shape[2]
+        # Measured in us, 7 / 16 heads, mma.sync -> tcgen05: 2 rows behind 500 54 -> 17 / 76 -> 23, 40 and 9 rows behind 0 and 100
+        # 17 -> 15 / 24 -> 16; 24 rows 17 -> 19 / 14 -> 16, 4 rows 13 -> 16 / 13 -> 15, 2 rows behind 40 and a
+        # decoded one 21 -> 28, behind 300 33 -> 28.  Where few rows see few keys there is nothing but launches in it, and the older
+        # kernel's are cheaper; its time grows by 3 to 5 us per tile of 32 keys.
         if (tiles > 0 and on_tensor_cores and self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and page_size >= 8
+                and (int(batch.max_kv_len) > (256 if batch.num_decode else 128) or q.shape[0] - batch.num_decode > 64)
                 and page_size & (page_size - 1) == 0 and scale > 0 and q.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0
                 and (self.use_latent_decode_kernel or batch.num_decode == 0) and self._latent_tcgen05_fits(heads, rank, rot)):
             # prompt portions with both products on tcgen05
