@@ -50,7 +50,11 @@ constexpr int FA_THREADS = FA_SOFTMAX_THREADS + 64;      // + the warp that issu
 constexpr uint32_t FA_TMEM_COLS = 256;   // S0 | S1 | O (head_dim columns)
 constexpr uint32_t FA_TMEM_O = 2 * FA_KEYS;
 constexpr int FA_P_BYTES = FA_ROWS * FA_KEYS * 2;          // one tile of probabilities
-constexpr float FA_LAZY = 8.f;      // the base exponent follows the running max in steps of more than this
+// The base exponent follows the running max in steps of more than this.  Of maps it follows every rise: relative to the max itself the
+// heavy weights lie in the upper part of a binade, where bfloat16 rounds them relatively less, relative to a lagging base anywhere.
+// The difference of two maps shows that: error against 64 bits, 290 rows of 6 heads of 2 x 64, with steps of 2^8 2.32e-3, now 2.25e-3
+// (mma.sync 2.27e-3); 2,048 rows, window 1,024, 7 heads 53.0 -> 55.2 us for it.
+constexpr float FA_LAZY = 8.f;
 
 // Sizes that depend on the head sizes (D of queries and keys, DV of values).  With 128 the shared memory of two
 // resident CTAs only fits with a two-stage ring and one buffer of probabilities.
@@ -72,7 +76,7 @@ struct FaShape {
 // leave as float32, and the first `keep` positions stay visible beside the window).  The maps' walk over the keys is
 // the softmax threads' like any head's; on mma.sync it was bound by fragment loads, one query tile's K and V fetched per
 // (head, map), and by a combination of 32 CTAs: 2,048 rows, window 1,024, 7 heads of 2 x 64 with values of 128: 290 -> 55 us,
-// 16 heads: 595 -> 72 us.
+// 16 heads: 597 -> 81 us.
 enum FaMode { FA_PLAIN, FA_SHAPED, FA_MAPS };
 
 // Barriers and the few words the warps share; behind the tiles in dynamic shared memory.
@@ -462,7 +466,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         m_run = fmaxf(m_run, tile_max * scale_log2);               // the scale is positive
         // The base follows the max only in steps: (-inf) - (-inf) is NaN and compares false (nothing
         // visible yet: no step); the first visible key gives +inf and sets the base.
-        const bool step = m_run - m_base > FA_LAZY;
+        const bool step = m_run - m_base > (MAPS ? 0.f : FA_LAZY);
         const float alpha = step ? fa_exp2(m_base - m_run) : 1.f;   // a base of -inf gives 0
         if (step) m_base = m_run;
         const float base = m_base == -INFINITY ? 0.f : m_base;     // nothing visible yet: everything stays zero

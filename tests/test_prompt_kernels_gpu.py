@@ -235,3 +235,48 @@ def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
     assert torch.equal(m, want_m)
     close(s.flatten(0, 1), want_s.flatten(0, 1), 200 * UNIT, "state")      # sums of 64 products at a time, once per chunk
     close(out, want, 2.0 ** -8, "output")
+
+
+def relative(got, want):
+    return float((got.double().cpu() - want.double()).norm() / want.double().norm())
+
+
+@pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (14, 256, 32)])
+def test_latent_prompts_are_as_close_to_64_bits_on_either_kernel(heads, rank, rot):
+    """The probabilities' rounding to 16 bits is all of the error, and the same error in both kernels; the 2-norm over 3e5 and more outputs
+    varies by far less than the two percent left to it."""
+    lengths, before = [150, 90], [200, 0]
+    (pool,), cpu, batch = paged(lengths, before, lambda p, j: j <= p, 16, [(1, rank + rot, 1.0)], 7)
+    q = rnd(6, sum(lengths), heads * (rank + rot), std=0.5).to(torch.bfloat16)
+    args = (heads, rank, rot, 0.08, 0)
+    want = FAKE.latent_attention(q.float(), pool.float(), cpu, *args, None)
+    errors = []
+    for tcgen05 in (False, True):
+        cuda().use_tcgen05_attention = tcgen05
+        try:
+            errors.append(relative(cuda().latent_attention(q.to(DEVICE), pool.to(DEVICE), batch, *args, None), want))
+        finally:
+            cuda().use_tcgen05_attention = True
+    print("error mma.sync, tcgen05:", errors)
+    assert errors[1] <= 1.02 * errors[0], errors
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 128)])
+@pytest.mark.parametrize("window", [0, 120])
+def test_differential_prompts_are_as_close_to_64_bits_on_either_kernel(dim, vdim, window):
+    """As above; the outputs' own rounding to 16 bits is in both errors."""
+    heads, kv_heads, lengths, before, keep = 6, 2, [200, 90], [150, 0], 4
+    seen = lambda p, j: j <= p and (not window or p - j < window or j < keep)      # noqa: E731
+    pools, cpu, batch = paged(lengths, before, seen, 16, [(kv_heads, 2 * dim, 1.0), (kv_heads, vdim, 0.7)], 3)
+    q = rnd(5, sum(lengths), 2 * heads * dim).to(torch.bfloat16)
+    args = (heads, kv_heads, dim, vdim, dim ** -0.5, window, keep, 0.4, 1e-6, 0.5)
+    want = FAKE.differential_attention(q.float(), *(t.float() for t in pools), cpu, *args)
+    errors = []
+    for tcgen05 in (False, True):
+        cuda().use_tcgen05_attention = tcgen05
+        try:
+            errors.append(relative(cuda().differential_attention(q.to(DEVICE), *(t.to(DEVICE) for t in pools), batch, *args), want))
+        finally:
+            cuda().use_tcgen05_attention = True
+    print("error mma.sync, tcgen05:", errors)
+    assert errors[1] <= 1.02 * errors[0], errors
