@@ -33,6 +33,7 @@ struct ChunkArgs {
   float* decays;                                 // [chunk places, heads, dim]: products over the chunk
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, weight_per_head;
+  int segments, least;                           // segments of fewer than `least` rows are another kernel's
 };
 
 // Thread (lane, warp) walks key channels [16 * slice, +16) of C neighbouring value channels; T tokens at a time are
@@ -54,16 +55,16 @@ chunk_walk_kernel(ChunkArgs p) {
   constexpr int KD = W::KD, C = W::C, T = W::T, THREADS = W::THREADS, SLICES = W::SLICES;
   pdl_trigger();
   pdl_wait();
-  const int head = blockIdx.x, chunk = blockIdx.y, seg = blockIdx.z;
-  const int length = p.seg_q_len[seg];
-  if (chunk * CHUNK >= length) return;
+  const int head = blockIdx.x;
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  if (seg < 0) return;
   extern __shared__ __align__(16) float shared[];
   float* s_o = shared + 2 * W::STAGE;                    // [SLICES][T][VDIM]
   float* s_bonus = s_o + SLICES * T * VDIM;              // [T] sum_i r c b (mode 0)
-  const int first = p.seg_q_start[seg] + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
+  const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const bool whole = length <= CHUNK;                    // the segment is this chunk
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, column = lane * C;
-  float* state = p.state + ((size_t)p.seg_slot[seg] * p.heads + head) * DIM * VDIM;
+  float* state = p.state + ((size_t)slot * p.heads + head) * DIM * VDIM;
 
   auto fetch = [&](int t0) {
     float* stage = shared + ((t0 / T) & 1) * W::STAGE;
@@ -201,8 +202,9 @@ chunk_carry_kernel(ChunkArgs p, int dim, int vdim) {
   constexpr int BATCH = 8;
   pdl_trigger();
   pdl_wait();
-  const int seg = blockIdx.y, length = p.seg_q_len[seg], first = p.seg_q_start[seg];
-  const int chunks = (length + CHUNK - 1) / CHUNK, cells = dim * vdim;
+  const auto [seg, which, length, start, slot] = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  if (seg < 0) return;
+  const int first = start, chunks = (length + CHUNK - 1) / CHUNK, cells = dim * vdim;
   const int at = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (chunks <= 1 || at >= p.heads * cells) return;
   const int head = at / cells, cell = at - head * cells, i = cell / vdim;
@@ -229,7 +231,7 @@ chunk_carry_kernel(ChunkArgs p, int dim, int vdim) {
         S.w = fmaf(a[k], S.w, own[k].w);
       }
   }
-  *reinterpret_cast<float4*>(p.state + ((size_t)p.seg_slot[seg] * p.heads + head) * cells + cell) = S;
+  *reinterpret_cast<float4*>(p.state + ((size_t)slot * p.heads + head) * cells + cell) = S;
 }
 
 // CTA per (head, chunk, segment): VDIM / 4 threads side by side take a token's value channels, eight groups of them eight
@@ -240,12 +242,12 @@ chunk_finish_kernel(ChunkArgs p, T* __restrict__ out) {
   constexpr int LANES = VDIM / 4, THREADS = 2 * VDIM, TOKENS = CHUNK / 8, PITCH = DIM + 4;
   pdl_trigger();
   pdl_wait();
-  const int head = blockIdx.x, chunk = blockIdx.y, seg = blockIdx.z;
-  const int length = p.seg_q_len[seg];
-  if (chunk * CHUNK >= length) return;
+  const int head = blockIdx.x;
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  if (seg < 0) return;
   extern __shared__ __align__(16) float shared[];
   float *s_reads = shared, *s_state = shared + CHUNK * PITCH;
-  const int first = p.seg_q_start[seg] + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
+  const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int j = (threadIdx.x % LANES) * 4, group = threadIdx.x / LANES;
   float o[TOKENS][4];
   if (chunk > 0) {
@@ -322,10 +324,10 @@ chunk_finish_kernel(ChunkArgs p, T* __restrict__ out) {
 }
 
 template <typename T, int MODE, int DIM, int VDIM>
-int launch_chunks(const ChunkArgs& args, void* out, int segments, int max_q_len, cudaStream_t stream) {
+int launch_chunks(const ChunkArgs& args, void* out, int rows, int max_q_len, cudaStream_t stream) {
   using W = WalkShape<MODE, DIM, VDIM>;
   constexpr size_t finish_shared = sizeof(float) * (CHUNK * (DIM + 4) + (size_t)DIM * VDIM);
-  const dim3 grid(args.heads, (max_q_len + CHUNK - 1) / CHUNK, segments);
+  const dim3 grid(args.heads, (unsigned)long_chunks(rows, args.segments, args.least));
   auto walk = chunk_walk_kernel<MODE, DIM, VDIM>;
   auto finish = chunk_finish_kernel<T, MODE, DIM, VDIM>;
   cudaError_t err = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::SHARED);
@@ -335,7 +337,7 @@ int launch_chunks(const ChunkArgs& args, void* out, int segments, int max_q_len,
   int status = launch_status();
   if (status != MLR_OK) return status;
   if (max_q_len > CHUNK) {
-    launch_kernel(chunk_carry_kernel, dim3((args.heads * DIM * VDIM / 4 + 255) / 256, segments), dim3(256), 0, stream, args, DIM, VDIM);
+    launch_kernel(chunk_carry_kernel, dim3((args.heads * DIM * VDIM / 4 + 255) / 256, (unsigned)long_segments(rows, args.segments, args.least)), dim3(256), 0, stream, args, DIM, VDIM);
     if ((status = launch_status()) != MLR_OK) return status;
   }
   launch_kernel(finish, grid, dim3(2 * VDIM), finish_shared, stream, args, (T*)out);
@@ -343,16 +345,16 @@ int launch_chunks(const ChunkArgs& args, void* out, int segments, int max_q_len,
 }
 
 template <int MODE>
-int launch_chunks(const ChunkArgs& args, void* out, int segments, int max_q_len, int dim, int vdim, int out_dtype,
+int launch_chunks(const ChunkArgs& args, void* out, int rows, int max_q_len, int dim, int vdim, int out_dtype,
                   cudaStream_t stream) {
   const bool wide = dim == 128;
   if (dim != vdim || (dim != 64 && dim != 128)) return MLR_TOO_LARGE;
   if (out_dtype == MLR_F32)
-    return wide ? launch_chunks<float, MODE, 128, 128>(args, out, segments, max_q_len, stream)
-                : launch_chunks<float, MODE, 64, 64>(args, out, segments, max_q_len, stream);
+    return wide ? launch_chunks<float, MODE, 128, 128>(args, out, rows, max_q_len, stream)
+                : launch_chunks<float, MODE, 64, 64>(args, out, rows, max_q_len, stream);
   if (out_dtype == MLR_BF16)
-    return wide ? launch_chunks<bf16, MODE, 128, 128>(args, out, segments, max_q_len, stream)
-                : launch_chunks<bf16, MODE, 64, 64>(args, out, segments, max_q_len, stream);
+    return wide ? launch_chunks<bf16, MODE, 128, 128>(args, out, rows, max_q_len, stream)
+                : launch_chunks<bf16, MODE, 64, 64>(args, out, rows, max_q_len, stream);
   return MLR_BAD_DTYPE;
 }
 
@@ -369,17 +371,18 @@ MLR_EXPORT long long mlr_gated_chunk_scratch(int rows, int heads, int dim, int v
 }
 
 // As mlr_gated_recurrence, for square heads of 64 or 128 and inputs (state, weights, output and scratch too) whose rows begin
-// on 16-byte boundaries.  rows: the step's rows; scratch: mlr_gated_chunk_scratch numbers.
+// on 16-byte boundaries.  rows: the step's rows; scratch: mlr_gated_chunk_scratch numbers.  Segments of fewer than least_rows rows are
+// left alone.
 MLR_EXPORT int mlr_gated_recurrence_chunks(int mode, const float* r, long long r_stride, const float* b, long long b_stride,
                                            const float* v, long long v_stride, const float* raw, long long raw_stride,
                                            const float* gate, long long gate_stride, const float* bias, const float* aux,
                                            const float* weight, float eps, float* state, void* out, float* scratch,
                                            const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments,
-                                           int rows, int max_q_len, int heads, int dim, int vdim, int out_dtype,
+                                           int rows, int max_q_len, int least_rows, int heads, int dim, int vdim, int out_dtype,
                                            cudaStream_t stream) {
-  if (segments == 0) return MLR_OK;
-  if (segments < 0 || heads <= 0 || rows <= 0 || max_q_len <= 0 || scratch == nullptr) return MLR_BAD_SIZE;
-  if (segments > 65535 || max_q_len > 65535 * CHUNK) return MLR_TOO_LARGE;
+  if (segments == 0 || max_q_len < least_rows) return MLR_OK;
+  if (segments < 0 || heads <= 0 || rows <= 0 || max_q_len <= 0 || least_rows <= 0 || scratch == nullptr) return MLR_BAD_SIZE;
+  if (long_chunks(rows, segments, least_rows) > 65535) return MLR_TOO_LARGE;
   const uintptr_t pointers = (uintptr_t)r | (uintptr_t)b | (uintptr_t)v | (uintptr_t)raw | (uintptr_t)gate | (uintptr_t)weight |
                              (uintptr_t)state | (uintptr_t)out | (uintptr_t)scratch;
   if (pointers % 16 != 0 || (r_stride | b_stride | v_stride | raw_stride | gate_stride) % 4 != 0) return MLR_BAD_ALIGNMENT;
@@ -393,8 +396,8 @@ MLR_EXPORT int mlr_gated_recurrence_chunks(int mode, const float* r, long long r
   args.ends = args.reads + (size_t)rows * heads * dim;
   args.decays = args.ends + (size_t)chunk_places(rows) * heads * dim * vdim;
   args.seg_q_start = seg_q_start; args.seg_q_len = seg_q_len; args.seg_slot = seg_slot;
-  args.heads = heads; args.weight_per_head = mode == 0 ? 1 : 0;
-  if (mode == 0) return launch_chunks<0>(args, out, segments, max_q_len, dim, vdim, out_dtype, stream);
-  if (mode == 1) return launch_chunks<1>(args, out, segments, max_q_len, dim, vdim, out_dtype, stream);
+  args.heads = heads; args.weight_per_head = mode == 0 ? 1 : 0; args.segments = segments; args.least = least_rows;
+  if (mode == 0) return launch_chunks<0>(args, out, rows, max_q_len, dim, vdim, out_dtype, stream);
+  if (mode == 1) return launch_chunks<1>(args, out, rows, max_q_len, dim, vdim, out_dtype, stream);
   return MLR_BAD_SIZE;
 }

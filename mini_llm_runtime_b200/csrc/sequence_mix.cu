@@ -10,7 +10,9 @@
 // The batch is ragged: segment s brings rows seg_q_start[s] .. +seg_q_len[s] of the request whose
 // fixed-size state lives in slot seg_slot[s].  Every row's result depends only on its own request:
 // reductions have a fixed order, recurrences run token by token, so a request's numbers do not
-// change with how its tokens are cut into steps or what else is in the batch.
+// change with how its tokens are cut into steps or what else is in the batch.  (Portions of many rows
+// may go through gated_chunks.cu, which adds in another order: then a request's numbers depend on the
+// rows of its own portion, still not on the batch.)
 #include "common.cuh"
 
 namespace mlr {
@@ -132,6 +134,7 @@ struct RecurrenceArgs {
   float* state;                                  // [slots, heads, dim, vdim]
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, dim, vdim, weight_per_head;
+  int longest;        // segments of more rows are another kernel's
   int columns;        // value channels per CTA: vdim, or a part of it (blockIdx.z picks the part)
   float* raw_out;     // with parts: the un-normalised o [rows, heads*vdim]; recurrence_finish_kernel ends the job
 };
@@ -154,6 +157,7 @@ gated_recurrence_kernel(RecurrenceArgs p, T* __restrict__ out) {
 
   const int head = blockIdx.x, seg = blockIdx.y;
   const int length = p.seg_q_len[seg], first = p.seg_q_start[seg];
+  if (length > p.longest) return;
   const int j = threadIdx.x, slice = threadIdx.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, threads = blockDim.x * blockDim.y;
   const int warp = tid >> 5, lane = tid & 31, warps = threads >> 5;
@@ -281,15 +285,21 @@ gated_recurrence_kernel(RecurrenceArgs p, T* __restrict__ out) {
 }
 
 // The end of a recurrence whose value channels were spread over CTAs: one warp per (row, head) takes
-// o / rms(o) * weight (* silu(gate)).
+// o / rms(o) * weight (* silu(gate)).  With seg_q_len: of the segments (blockIdx.y) of up to `longest` rows only.
 template <typename T>
 __global__ void __launch_bounds__(128)
 recurrence_finish_kernel(const float* raw, const float* gate, long long gate_stride, const float* __restrict__ weight,
-                         int weight_per_head, T* __restrict__ out, long long items, int heads, int vdim, float eps) {
+                         int weight_per_head, T* __restrict__ out, long long items, int heads, int vdim, float eps,
+                         const int* seg_q_start, const int* seg_q_len, int longest) {
   pdl_trigger();
   pdl_wait();
-  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (seg_q_len != nullptr) {
+    const int length = seg_q_len[blockIdx.y];
+    items = length > longest ? 0 : (long long)length * heads;
+  }
   if (item >= items) return;
+  if (seg_q_len != nullptr) item += (long long)seg_q_start[blockIdx.y] * heads;
   const int lane = threadIdx.x & 31;
   const long long row = item / heads;
   const int head = (int)(item - row * heads);
@@ -356,6 +366,8 @@ __global__ void tanh_kernel(T* x, long long count) {
 template <typename T, int MODE>
 int launch_recurrence(RecurrenceArgs args, void* out, float* raw, int segments, int rows, int max_q_len,
                       cudaStream_t stream) {
+  const bool all = args.longest >= max_q_len;      // no segment is another kernel's
+  if (!all) max_q_len = args.longest;
   // threads a CTA needs for `columns` value channels, with the fewest key channels per thread (8, 16, 32
   // or 64) that keep it within 512: more threads with shorter chains hide the latency of the
   // shared-memory loads that feed them
@@ -389,10 +401,11 @@ int launch_recurrence(RecurrenceArgs args, void* out, float* raw, int segments, 
                 (T*)out);
   int status = launch_status();
   if (status != MLR_OK || !spread) return status;
-  const long long items = (long long)rows * args.heads;
-  launch_kernel(recurrence_finish_kernel<T>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream, (const float*)raw,
+  const long long items = (long long)(all ? rows : max_q_len) * args.heads;
+  launch_kernel(recurrence_finish_kernel<T>, dim3((unsigned)((items + 3) / 4), all ? 1 : segments), dim3(128), 0, stream, (const float*)raw,
                 MODE == 0 ? args.gate : (const float*)nullptr, args.gate_stride, args.weight, args.weight_per_head,
-                (T*)out, items, args.heads, args.vdim, args.eps);
+                (T*)out, items, args.heads, args.vdim, args.eps, all ? (const int*)nullptr : args.seg_q_start,
+                all ? (const int*)nullptr : args.seg_q_len, args.longest);
   return launch_status();
 }
 
@@ -463,16 +476,16 @@ MLR_EXPORT int mlr_token_shift(const float* a, const float* coef, float* state, 
 // mode 1: forget-gate recurrence (r = raw q, v, forget raw; aux = lower bound [heads*dim]; weight [vdim]).
 // All inputs float32 views with a row stride (in elements); state float32 [slots, heads, dim, vdim];
 // out: out_dtype [rows, heads*vdim]; scratch: float32 of the same shape or null; rows: the step's
-// rows; max_q_len: its longest segment.
+// rows; max_q_len: its longest segment.  Segments of more than `longest` rows are left alone.
 MLR_EXPORT int mlr_gated_recurrence(int mode, const float* r, long long r_stride, const float* b, long long b_stride,
                                     const float* v, long long v_stride, const float* raw, long long raw_stride,
                                     const float* gate, long long gate_stride, const float* bias, const float* aux,
                                     const float* weight, float eps, float* state, void* out, float* scratch,
                                     const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments,
-                                    int rows, int max_q_len, int heads, int dim, int vdim, int out_dtype,
+                                    int rows, int max_q_len, int longest, int heads, int dim, int vdim, int out_dtype,
                                     cudaStream_t stream) {
   if (segments == 0) return MLR_OK;
-  if (segments < 0 || heads <= 0 || dim <= 0 || vdim <= 0) return MLR_BAD_SIZE;
+  if (segments < 0 || longest <= 0 || heads <= 0 || dim <= 0 || vdim <= 0) return MLR_BAD_SIZE;
   if (segments > 65535) return MLR_TOO_LARGE;
   RecurrenceArgs args;
   args.r = r; args.b = b; args.v = v; args.raw = raw; args.gate = gate;
@@ -480,7 +493,7 @@ MLR_EXPORT int mlr_gated_recurrence(int mode, const float* r, long long r_stride
   args.raw_stride = raw_stride; args.gate_stride = gate_stride;
   args.bias = bias; args.aux = aux; args.weight = weight; args.eps = eps; args.state = state;
   args.seg_q_start = seg_q_start; args.seg_q_len = seg_q_len; args.seg_slot = seg_slot;
-  args.heads = heads; args.dim = dim; args.vdim = vdim; args.weight_per_head = mode == 0 ? 1 : 0;
+  args.heads = heads; args.dim = dim; args.vdim = vdim; args.weight_per_head = mode == 0 ? 1 : 0; args.longest = longest;
   if (mode == 0 && out_dtype == MLR_F32) return launch_recurrence<float, 0>(args, out, scratch, segments, rows, max_q_len, stream);
   if (mode == 0 && out_dtype == MLR_BF16) return launch_recurrence<bf16, 0>(args, out, scratch, segments, rows, max_q_len, stream);
   if (mode == 1 && out_dtype == MLR_F32) return launch_recurrence<float, 1>(args, out, scratch, segments, rows, max_q_len, stream);
@@ -498,10 +511,10 @@ MLR_EXPORT int mlr_gated_head_norm(const float* y, const float* gate, long long 
   const dim3 grid((unsigned)((items + 3) / 4));
   if (out_dtype == MLR_F32)
     launch_kernel(recurrence_finish_kernel<float>, grid, dim3(128), 0, stream, y, gate, gate_stride, weight, 0, (float*)out,
-                  items, heads, vdim, eps);
+                  items, heads, vdim, eps, (const int*)nullptr, (const int*)nullptr, 0);
   else if (out_dtype == MLR_BF16)
     launch_kernel(recurrence_finish_kernel<bf16>, grid, dim3(128), 0, stream, y, gate, gate_stride, weight, 0, (bf16*)out,
-                  items, heads, vdim, eps);
+                  items, heads, vdim, eps, (const int*)nullptr, (const int*)nullptr, 0);
   else
     return MLR_BAD_DTYPE;
   return launch_status();

@@ -12,7 +12,8 @@
 //                          S <- a S + dt B[t, g] x[t, h]^T            (S: [state, vdim], kept as [vdim, state])
 //                          y[t, h] = S^T C[t, g] + D[h] x[t, h]
 //                        token by token in a fixed order, so a request's numbers do not depend on how its
-//                        tokens were cut into steps.
+//                        tokens were cut into steps.  (Portions of many rows may go through state_space_chunks.cu,
+//                        which adds in another order: then on the rows of its own portion, never on other requests.)
 // mlr_gated_group_norm   out = RMSnorm_parts(y * silu(z)) * weight: the row is cut into `parts` equal parts,
 //                        each divided by its own root mean square (eps inside the root).
 #include "common.cuh"
@@ -117,6 +118,7 @@ struct ScanArgs {
   float* y;
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, vdim, n, groups;
+  int longest;      // segments of more rows are another kernel's
 };
 
 // SL: threads that share one value channel's state (a power of two; SL * SCAN_NPT >= n).  Lane l of a warp
@@ -143,6 +145,7 @@ state_space_scan_kernel(ScanArgs a) {
   const float rate = expf(a.A_log[head]), bias = a.dt_bias[head], skip = a.D[head];
   pdl_wait();
   const int q_start = a.seg_q_start[seg], q_len = a.seg_q_len[seg];
+  if (q_len > a.longest) return;
 
   // rows [t0, t0 + 32) of the segment into buffer `which`: B and C of the head's group, the block's value
   // channels of x, the head's raw step sizes
@@ -306,17 +309,17 @@ MLR_EXPORT int mlr_causal_conv(const float* u, long long u_stride, const float* 
 
 // x: float32 rows of heads*vdim entries; B, C: rows of groups*n entries; dt_raw: rows of `heads` entries
 // (each with its own row stride); dt_bias, A_log, D: float32 [heads]; states: float32 [slots, heads, vdim, n];
-// y: float32 [rows, heads*vdim].
+// y: float32 [rows, heads*vdim].  Segments of more than `longest` rows are left alone.
 MLR_EXPORT int mlr_state_space_scan(const float* x, long long x_stride, const float* B, long long b_stride, const float* C,
                                     long long c_stride, const float* dt_raw, long long dt_stride, const float* dt_bias,
                                     const float* A_log, const float* D, float* states, float* y, const int* seg_q_start,
-                                    const int* seg_q_len, const int* seg_slot, int segments, int heads, int vdim, int n,
+                                    const int* seg_q_len, const int* seg_slot, int segments, int longest, int heads, int vdim, int n,
                                     int groups, cudaStream_t stream) {
   if (segments == 0) return MLR_OK;
-  if (segments < 0 || heads <= 0 || vdim <= 0 || n <= 0 || groups <= 0 || heads % groups != 0) return MLR_BAD_SIZE;
+  if (segments < 0 || longest <= 0 || heads <= 0 || vdim <= 0 || n <= 0 || groups <= 0 || heads % groups != 0) return MLR_BAD_SIZE;
   if (n > 32 * SCAN_NPT || heads > 65535) return MLR_TOO_LARGE;
   ScanArgs a{x, B, C, dt_raw, x_stride, b_stride, c_stride, dt_stride, dt_bias, A_log, D, states, y,
-             seg_q_start, seg_q_len, seg_slot, heads, vdim, n, groups};
+             seg_q_start, seg_q_len, seg_slot, heads, vdim, n, groups, longest};
   int slices = 1;
   while (slices * SCAN_NPT < n) slices *= 2;
   auto multiple = [](long long v) { return v % 4 == 0; };

@@ -34,6 +34,7 @@ struct SpaceArgs {
   float* decays;                     // [chunk places, heads]: products over the chunk
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, groups;
+  int segments, least;               // segments of fewer than `least` rows are another kernel's
 };
 
 // `count` rows of N entries into shared rows `pitch` apart; the rows up to CHUNK become zero.
@@ -48,7 +49,7 @@ __device__ __forceinline__ void fetch_rows(float* dst, int pitch, const float* s
   }
 }
 
-// grid: (chunks, segments, groups * 4): 16 of a chunk's rows against its 64 tokens; a thread takes 2 x 4 of them.
+// grid: (chunks, groups * 4): 16 of a chunk's rows against its 64 tokens; a thread takes 2 x 4 of them.
 template <int N>
 __global__ void __launch_bounds__(128)
 space_pairs_kernel(SpaceArgs p) {
@@ -57,9 +58,10 @@ space_pairs_kernel(SpaceArgs p) {
   float *s_b = shared, *s_c = shared + CHUNK * PITCH;
   pdl_trigger();
   pdl_wait();
-  const int chunk = blockIdx.x, seg = blockIdx.y, group = blockIdx.z >> 2, part = blockIdx.z & 3;
-  const int length = p.seg_q_len[seg] - chunk * CHUNK, first = p.seg_q_start[seg] + chunk * CHUNK;
-  const int count = min(CHUNK, length), t0 = part * 16;
+  const int group = blockIdx.y >> 2, part = blockIdx.y & 3;
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.x);
+  if (seg < 0) return;
+  const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK), t0 = part * 16;
   if (t0 >= count) return;
   fetch_rows<N, 128>(s_b, PITCH, p.B + (size_t)first * p.b_stride + (size_t)group * N, p.b_stride, count);
   for (int idx = threadIdx.x; idx < 16 * (N / 4); idx += 128) {
@@ -143,7 +145,7 @@ __device__ __forceinline__ void read_state(const SpaceArgs& p, const float* s_c,
   }
 }
 
-// grid: (heads, chunks, segments)
+// grid: (heads, chunks)
 template <int N>
 __global__ void __launch_bounds__(128, 3)
 space_local_kernel(SpaceArgs p) {
@@ -156,12 +158,12 @@ space_local_kernel(SpaceArgs p) {
   float* s_dt = s_g + CHUNK;                   // [CHUNK] step sizes
   float* s_to_end = s_dt + CHUNK;              // [CHUNK] decays' product behind a token
   pdl_trigger();
-  const int head = blockIdx.x, chunk = blockIdx.y, seg = blockIdx.z, tid = threadIdx.x;
+  const int head = blockIdx.x, tid = threadIdx.x;
   const float rate = expf(p.A_log[head]), bias = p.dt_bias[head], skip = p.D[head];
   pdl_wait();
-  const int length = p.seg_q_len[seg];
-  if (chunk * CHUNK >= length) return;
-  const int first = p.seg_q_start[seg] + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  if (seg < 0) return;
+  const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int group = head / (p.heads / p.groups);
   const bool whole = length <= CHUNK;
   fetch_rows<N, 128>(s_b, N, p.B + (size_t)first * p.b_stride + (size_t)group * N, p.b_stride, count);
@@ -258,7 +260,7 @@ space_local_kernel(SpaceArgs p) {
     }
   }
   const float decay = s_to_end[0] * s_g[0];
-  float* state = p.states + ((size_t)p.seg_slot[seg] * p.heads + head) * VD * N;
+  float* state = p.states + ((size_t)slot * p.heads + head) * VD * N;
   const size_t place = chunk_place(first, chunk == 0) * p.heads + head;
   if (chunk == 0) {
     // the read of the request's state: its rows and those of C take the place of what is done with
@@ -296,8 +298,9 @@ space_carry_kernel(SpaceArgs p, int cells) {
   constexpr int BATCH = 8;
   pdl_trigger();
   pdl_wait();
-  const int seg = blockIdx.y, length = p.seg_q_len[seg], first = p.seg_q_start[seg];
-  const int chunks = (length + CHUNK - 1) / CHUNK;
+  const auto [seg, which, length, start, slot] = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  if (seg < 0) return;
+  const int first = start, chunks = (length + CHUNK - 1) / CHUNK;
   const int at = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (chunks <= 1 || at >= p.heads * cells) return;
   const int head = at / cells, cell = at - head * cells;
@@ -322,10 +325,10 @@ space_carry_kernel(SpaceArgs p, int cells) {
         S.w = fmaf(g[k], S.w, own[k].w);
       }
   }
-  *reinterpret_cast<float4*>(p.states + ((size_t)p.seg_slot[seg] * p.heads + head) * cells + cell) = S;
+  *reinterpret_cast<float4*>(p.states + ((size_t)slot * p.heads + head) * cells + cell) = S;
 }
 
-// grid: (heads, chunks - 1, segments): the chunks behind a segment's first
+// grid: (heads, chunks), where a segment's first chunks have nothing to do (a single segment's is left out)
 template <int N>
 __global__ void __launch_bounds__(128, 3)
 space_read_kernel(SpaceArgs p) {
@@ -334,10 +337,11 @@ space_read_kernel(SpaceArgs p) {
   float *s_s = shared, *s_c = shared + VD * PITCH;
   pdl_trigger();
   pdl_wait();
-  const int head = blockIdx.x, chunk = blockIdx.y + 1, seg = blockIdx.z;
-  const int length = p.seg_q_len[seg];
-  if (chunk * CHUNK >= length) return;
-  const int first = p.seg_q_start[seg] + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
+  const int head = blockIdx.x;
+  const auto [seg, chunk, length, start, slot] =
+      chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y + (p.segments == 1 ? 1 : 0));
+  if (seg < 0 || chunk == 0) return;
+  const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int group = head / (p.heads / p.groups);
   const float* before = p.ends + (chunk_place(first, false) * p.heads + head) * VD * N;
   for (int idx = threadIdx.x; idx < VD * (N / 4); idx += 128)
@@ -350,24 +354,25 @@ space_read_kernel(SpaceArgs p) {
 }
 
 template <int N>
-int launch_space(const SpaceArgs& a, int segments, int max_q_len, cudaStream_t stream) {
+int launch_space(const SpaceArgs& a, int rows, int max_q_len, cudaStream_t stream) {
   constexpr size_t pairs_shared = sizeof(float) * (CHUNK + 16) * (N + 4);
   constexpr size_t local_shared = sizeof(float) * (CHUNK * (W_PITCH + VD + N + 4) + 3 * CHUNK);
   constexpr size_t read_shared = sizeof(float) * (VD + CHUNK) * (N + 4);
   static_assert(VD * (N + 4) <= CHUNK * (W_PITCH + VD), "the state takes the place of weights and inputs");
-  const int chunks = (max_q_len + CHUNK - 1) / CHUNK;
+  const unsigned chunks = (unsigned)long_chunks(rows, a.segments, a.least);
   cudaError_t err = cudaFuncSetAttribute(space_pairs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_shared);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(space_local_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local_shared);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(space_read_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)read_shared);
   if (err != cudaSuccess) return (int)err;
-  launch_kernel(space_pairs_kernel<N>, dim3(chunks, segments, a.groups * 4), dim3(128), pairs_shared, stream, a);
+  launch_kernel(space_pairs_kernel<N>, dim3(chunks, a.groups * 4), dim3(128), pairs_shared, stream, a);
   int status = launch_status();
   if (status != MLR_OK) return status;
-  launch_kernel(space_local_kernel<N>, dim3(a.heads, chunks, segments), dim3(128), local_shared, stream, a);
-  if ((status = launch_status()) != MLR_OK || chunks == 1) return status;
-  launch_kernel(space_carry_kernel, dim3((a.heads * VD * N / 4 + 255) / 256, segments), dim3(256), 0, stream, a, VD * N);
+  launch_kernel(space_local_kernel<N>, dim3(a.heads, chunks), dim3(128), local_shared, stream, a);
+  if ((status = launch_status()) != MLR_OK || max_q_len <= CHUNK) return status;
+  launch_kernel(space_carry_kernel, dim3((a.heads * VD * N / 4 + 255) / 256, (unsigned)long_segments(rows, a.segments, a.least)), dim3(256), 0,
+                stream, a, VD * N);
   if ((status = launch_status()) != MLR_OK) return status;
-  launch_kernel(space_read_kernel<N>, dim3(a.heads, chunks - 1, segments), dim3(128), read_shared, stream, a);
+  launch_kernel(space_read_kernel<N>, dim3(a.heads, chunks - (a.segments == 1 ? 1 : 0)), dim3(128), read_shared, stream, a);
   return launch_status();
 }
 
@@ -384,22 +389,22 @@ MLR_EXPORT long long mlr_state_space_chunk_scratch(int rows, int heads, int n, i
 }
 
 // As mlr_state_space_scan, for heads of 64 value channels with states of 64 or 128 entries and x, B, C, states, y and scratch whose
-// rows begin on 16-byte boundaries.  rows: the step's rows.
+// rows begin on 16-byte boundaries.  rows: the step's rows.  Segments of fewer than least_rows rows are left alone.
 MLR_EXPORT int mlr_state_space_chunks(const float* x, long long x_stride, const float* B, long long b_stride, const float* C,
                                       long long c_stride, const float* dt_raw, long long dt_stride, const float* dt_bias,
                                       const float* A_log, const float* D, float* states, float* y, float* scratch,
                                       const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments, int rows,
-                                      int max_q_len, int heads, int vdim, int n, int groups, cudaStream_t stream) {
-  if (segments == 0) return MLR_OK;
-  if (segments < 0 || rows <= 0 || max_q_len <= 0 || heads <= 0 || groups <= 0 || heads % groups != 0 || scratch == nullptr)
+                                      int max_q_len, int least_rows, int heads, int vdim, int n, int groups, cudaStream_t stream) {
+  if (segments == 0 || max_q_len < least_rows) return MLR_OK;
+  if (segments < 0 || least_rows <= 0 || rows <= 0 || max_q_len <= 0 || heads <= 0 || groups <= 0 || heads % groups != 0 || scratch == nullptr)
     return MLR_BAD_SIZE;
-  if (vdim != VD || (n != 64 && n != 128) || segments > 65535 || max_q_len > 65535 * CHUNK || groups > 65535 / 4) return MLR_TOO_LARGE;
+  if (vdim != VD || (n != 64 && n != 128) || long_chunks(rows, segments, least_rows) > 65535 || groups > 65535 / 4) return MLR_TOO_LARGE;
   const uintptr_t pointers = (uintptr_t)x | (uintptr_t)B | (uintptr_t)C | (uintptr_t)states | (uintptr_t)y | (uintptr_t)scratch;
   if (pointers % 16 != 0 || (x_stride | b_stride | c_stride) % 4 != 0) return MLR_BAD_ALIGNMENT;
   SpaceArgs a{x, B, C, dt_raw, x_stride, b_stride, c_stride, dt_stride, dt_bias, A_log, D, states, y,
-              nullptr, nullptr, scratch, nullptr, seg_q_start, seg_q_len, seg_slot, heads, groups};
+              nullptr, nullptr, scratch, nullptr, seg_q_start, seg_q_len, seg_slot, heads, groups, segments, least_rows};
   a.pairs = a.ends + (size_t)chunk_places(rows) * heads * VD * n;
   a.since = a.pairs + (size_t)rows * groups * CHUNK;
   a.decays = a.since + (size_t)rows * heads;
-  return n == 64 ? launch_space<64>(a, segments, max_q_len, stream) : launch_space<128>(a, segments, max_q_len, stream);
+  return n == 64 ? launch_space<64>(a, rows, max_q_len, stream) : launch_space<128>(a, rows, max_q_len, stream);
 }

@@ -857,8 +857,19 @@ class CudaOps:
             raise KernelError(f"{name} must be a float32 CUDA view [{rows}, {width}] with unit column stride")
         return _ptr(tensor), ctypes.c_longlong(tensor.stride(0))
 
+    @staticmethod
+    def _longest_below(ctx, rows: int) -> int:
+        """The longest portion of fewer than ``rows`` rows in a step that also has a longer one (0: none)."""
+        if ctx.num_segments == 1:
+            return 0
+        segments = getattr(ctx, "segments", None)
+        if segments is None:
+            return rows - 1       # lengths that only the device knows
+        return max((s.length for s in segments if s.length < rows), default=0)
+
     use_gated_chunks = True
-    # Longest portion of a step from which chunks pay.  Measured in us, walked by one CTA per head part / in chunks: 128 rows
+    # Portions of so many rows and more go in chunks, shorter ones beside them token by token: which way a request's rows go is a matter
+    # of its own portion only, as their numbers are.  Measured in us, walked by one CTA per head part / in chunks: 128 rows
     # 37 / 41 (14 heads of 64), 44 / 42 (32 of 64), 44 / 55 (7 and 16 of 128); 512 rows 129 / 42, 135 / 46, 157 / 70.
     GATED_CHUNK_ROWS = 192
 
@@ -874,6 +885,7 @@ class CudaOps:
             raise KernelError(f"state has shape {tuple(state.shape)}, expected [slots, {heads}, {dim}, {vdim}]")
         null = (ctypes.c_void_p(0), ctypes.c_longlong(0))
         out = torch.empty((rows, heads * vdim), dtype=out_dtype, device=r.device)
+        longest = int(ctx.max_q_len)
         views = (*self._view(r, "r", rows, heads * dim), *(null if b is None else self._view(b, "b", rows, heads * dim)),
                  *self._view(v, "v", rows, heads * vdim), *self._view(raw, "raw", rows, heads * dim),
                  *(null if gate is None else self._view(gate, "gate", rows, heads * vdim)))
@@ -883,18 +895,20 @@ class CudaOps:
             # long segments: chunks of tokens side by side
             lib = build.load_library("gated_chunks")
             lib.mlr_gated_chunk_scratch.restype = ctypes.c_longlong
-            scratch = torch.empty(lib.mlr_gated_chunk_scratch(rows, heads, dim, vdim), dtype=torch.float32, device=r.device)
+            chunk_scratch = torch.empty(lib.mlr_gated_chunk_scratch(rows, heads, dim, vdim), dtype=torch.float32, device=r.device)
             _check(lib.mlr_gated_recurrence_chunks(
-                mode, *views, _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out), _ptr(scratch),
-                _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len),
-                heads, dim, vdim, _code(out_dtype), _stream()), "gated_recurrence_chunks")
-            return out
+                mode, *views, _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out),
+                _ptr(chunk_scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows,
+                int(ctx.max_q_len), self.GATED_CHUNK_ROWS, heads, dim, vdim, _code(out_dtype), _stream()), "gated_recurrence_chunks")
+            longest = self._longest_below(ctx, self.GATED_CHUNK_ROWS)
+            if longest == 0:
+                return out
         # steps with long segments, and heads too large for one CTA, spread a head's value channels
         # over CTAs and finish in a second kernel, which reads the un-normalised rows from here
         scratch = torch.empty((rows, heads * vdim), dtype=torch.float32, device=r.device) if vdim > 32 else None
         _check(build.load_library("sequence_mix").mlr_gated_recurrence(
             mode, *views, _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out), _ptr(scratch),
-            _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len),
+            _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), longest,
             heads, dim, vdim, _code(out_dtype), _stream()),
             "gated_recurrence")
         return out
@@ -1962,7 +1976,7 @@ class CudaOps:
         return out
 
     use_state_space_chunks = True
-    # Longest portion of a step from which chunks pay.  Measured in us, token by token / in chunks: 128 rows 30 / 31 (14 heads,
+    # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us, token by token / in chunks: 128 rows 30 / 31 (14 heads,
     # states of 64), 42 / 50 (32 heads, states of 128); 512 rows 108 / 31, 161 / 64.
     STATE_SPACE_CHUNK_ROWS = 192
 
@@ -1981,6 +1995,7 @@ class CudaOps:
         if tuple(state.shape[1:]) != (heads, vdim, n):
             raise KernelError(f"state has shape {tuple(state.shape)}, expected [slots, {heads}, {vdim}, {n}]")
         y = torch.empty((rows, heads * vdim), dtype=torch.float32, device=x.device)
+        longest = int(ctx.max_q_len)
         views = (*self._view(x, "x", rows, heads * vdim), *self._view(B, "B", rows, groups * n),
                  *self._view(C, "C", rows, groups * n), *self._view(dt_raw, "dt_raw", rows, heads))
         if (self.use_state_space_chunks and ctx.max_q_len >= self.STATE_SPACE_CHUNK_ROWS and vdim == 64 and n in (64, 128)
@@ -1991,13 +2006,15 @@ class CudaOps:
             scratch = torch.empty(lib.mlr_state_space_chunk_scratch(rows, heads, n, groups), dtype=torch.float32, device=x.device)
             _check(lib.mlr_state_space_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(D), _ptr(state), _ptr(y), _ptr(scratch), _ptr(ctx.seg_q_start),
-                _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), heads, vdim, n, groups,
-                _stream()), "state_space_chunks")
-            return y
+                _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), self.STATE_SPACE_CHUNK_ROWS,
+                heads, vdim, n, groups, _stream()), "state_space_chunks")
+            longest = self._longest_below(ctx, self.STATE_SPACE_CHUNK_ROWS)
+            if longest == 0:
+                return y
         _check(build.load_library("state_space").mlr_state_space_scan(
             *views, _ptr(dt_bias), _ptr(A_log),
             _ptr(D), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot),
-            ctx.num_segments, heads, vdim, n, groups, _stream()), "state_space_scan")
+            ctx.num_segments, longest, heads, vdim, n, groups, _stream()), "state_space_scan")
         return y
 
     def gated_group_norm(self, y: torch.Tensor, gate, weight: torch.Tensor, eps: float, parts: int,

@@ -280,3 +280,69 @@ def test_differential_prompts_are_as_close_to_64_bits_on_either_kernel(dim, vdim
             cuda().use_tcgen05_attention = True
     print("error mma.sync, tcgen05:", errors)
     assert errors[1] <= 1.02 * errors[0], errors
+
+
+def gated(mode, dtype, inputs, weight, aux, bias, state, ctx, heads, dim):
+    """One call of a gated recurrence on the rows ``inputs`` (r, k, v, gate, raw); the state is advanced in place."""
+    r, k, v, gate, raw = inputs
+    if mode == "bonus":
+        return cuda().bonus_recurrence(r, k, v, raw, gate, bias, aux, weight, 1e-6, state, ctx, heads, dim, dtype)
+    return cuda().forget_gate_recurrence(r, raw, v, bias, aux, weight[:dim].contiguous(), 1e-6, state, ctx, heads, dim, dim, dtype)
+
+
+# requests whose portions are too short for chunks, each list beside a portion that is long enough
+SHORT = [[1, 1, 1], [3, 1, 60], [1, 100, 191]]
+
+
+@pytest.mark.parametrize("mode", ["bonus", "forget"])
+@pytest.mark.parametrize("heads,dim", [(3, 64), (2, 128)])
+@pytest.mark.parametrize("short", SHORT)
+@pytest.mark.parametrize("beside", [192, 400])
+def test_a_short_portion_of_a_gated_recurrence_is_the_same_beside_a_long_one(mode, heads, dim, short, beside):
+    n, rows = heads * dim, sum(short)
+    inputs = [rnd(i, rows + beside, n, std=0.7).to(DEVICE) for i in range(5)]
+    bias, weight, aux = (t.to(DEVICE) for t in (rnd(6, n) * 2 - 2, 1 + rnd(7, n, std=0.1), torch.rand(n, generator=generator(8))))
+    state = rnd(9, len(short) + 1, heads, dim, dim, std=0.5).to(DEVICE)
+    results = []
+    for lengths in (short, short + [beside]):
+        s = state.clone()
+        out = gated(mode, torch.float32, [t[:sum(lengths)].contiguous() for t in inputs], weight, aux, bias, s,
+                    segments(lengths, list(range(len(lengths)))), heads, dim)
+        results.append((out[:rows], s[:len(short)]))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("heads,n,groups", [(4, 64, 1), (6, 128, 2)])
+@pytest.mark.parametrize("short", SHORT)
+@pytest.mark.parametrize("beside", [192, 400])
+def test_a_short_portion_of_the_state_space_recurrence_is_the_same_beside_a_long_one(heads, n, groups, short, beside):
+    rows = sum(short)
+    full = [rnd(i, rows + beside, width).to(DEVICE) for i, width in enumerate((heads * 64, groups * n, groups * n, heads))]
+    vectors = [rnd(i, heads).to(DEVICE) for i in (5, 6, 7)]
+    state = rnd(8, len(short) + 1, heads, 64, n, std=0.5).to(DEVICE)
+    results = []
+    for lengths in (short, short + [beside]):
+        s = state.clone()
+        out = cuda().state_space_scan(*(t[:sum(lengths)].contiguous() for t in full), *vectors, s,
+                                      segments(lengths, list(range(len(lengths)))), heads, 64, n, groups)
+        results.append((out[:rows], s[:len(short)]))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+def test_recurrences_take_batches_without_lengths_on_the_host():
+    """A context that only says how many requests there are and which is the longest."""
+    lengths, heads, n = [400, 1, 100, 193], 4, 64
+    ctx = segments(lengths, [1, 0, 3, 2])
+    bare = types.SimpleNamespace(**{k: v for k, v in vars(ctx).items() if k != "segments"})
+    x, B, C, dt = (rnd(i, sum(lengths), width).to(DEVICE) for i, width in enumerate((heads * 64, n, n, heads)))
+    vectors = [rnd(i, heads).to(DEVICE) for i in (5, 6, 7)]
+    inputs = [rnd(i, sum(lengths), heads * 64, std=0.7).to(DEVICE) for i in range(5)]
+    weight, aux, bias = (rnd(i, heads * 64).to(DEVICE) for i in (10, 11, 12))
+    results = []
+    for context in (ctx, bare):
+        s = rnd(8, 4, heads, 64, n, std=0.5).to(DEVICE)
+        y = cuda().state_space_scan(x, B, C, dt, *vectors, s, context, heads, 64, n, 1)
+        g = rnd(9, 4, heads, 64, 64, std=0.5).to(DEVICE)
+        out = gated("bonus", torch.bfloat16, inputs, weight, aux, bias, g, context, heads, 64)
+        results.append((y, s, out, g))
+    assert all(torch.equal(a, b) for a, b in zip(*results))

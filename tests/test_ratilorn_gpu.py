@@ -446,3 +446,21 @@ def test_command_line_and_replay_program_with_a_model_folder(tmp_path):
     want = plain.forward(rs.MIXED, tensors, prompt)[0]
     rs.assert_logits_close(torch.cat([first, second[:1]]), want[[0, 3, 10]], F32)
     rs.assert_logits_close(second[1:], plain.forward(rs.MIXED, tensors, other)[0][29:], F32)
+
+
+def test_float32_logits_of_long_portions_do_not_depend_on_the_cut():
+    """Portions long enough for the chunked recurrence against short ones, alone and beside other requests."""
+    config = rs.config([rs.parallel(rs.heads(2, 1, 16, 24), (3, 64, 64, 1, 4, 1), rs.dense(40)),
+                        rs.parallel(rs.heads(2, 1, 24, 16), (2, 64, 128, 2, 4, 1)), rs.attention(2, 1, 16, 8)],
+                       width=96, vocab=131, max_positions=600)
+    engine = rs.REngine(config, F32, DEVICE, seed=4, num_pages=160, max_tokens=600, max_step_tokens=800)
+    tokens, other = rs.tokens_for(131, 400, 10), rs.tokens_for(131, 300, 11)
+    whole = engine.run_cuts("whole", tokens, [])
+    limit = 2e-5 * float(whole.abs().max())
+    rs.assert_logits_close(whole, engine.plain(tokens), F32)
+    for cuts in ([200], [191, 383], [1, 2, 64, 130, 323], list(range(50, 400, 50))):
+        assert float((engine.run_cuts("cut", tokens, cuts) - whole).abs().max()) <= limit, cuts
+    for portions in ([200, 200], [150, 250], [100, 191, 109]):
+        plan = [{"b": 1, "a": portions[0]}, {"b": 1, "a": portions[1], "c": 300}, *({"b": 1, "a": n} for n in portions[2:])]
+        got = engine.run_plan({"a": tokens, "b": other[:len(portions)], "c": other}, plan)
+        assert float((got["a"] - whole).abs().max()) <= limit, portions

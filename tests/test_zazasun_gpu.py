@@ -311,3 +311,36 @@ def test_state_heads_larger_than_one_block_of_threads_holds(dtype):
     want = engine.plain(tokens)
     zs.assert_logits_close(engine.run_cuts("a", tokens, []), want, dtype, "whole")
     zs.assert_logits_close(engine.run_cuts("b", tokens, [70, 71, 72, 80]), want, dtype, "portions and single tokens")
+
+
+def long_portions(engine, length, vocab, portions):
+    """Logits of a request's tokens in portions, beside others that decode and one that brings a long portion of its own."""
+    tokens, other = zs.tokens_for(vocab, length, 10), zs.tokens_for(vocab, 300, 11)
+    for name in ("a", "b", "c"):
+        engine.cache.create_request(name)
+    got, at = [], 0
+    for step, count in enumerate(portions):
+        entries = [("b", [other[step]], [0]), ("a", tokens[at:at + count], range(count))]
+        if step == 1:
+            entries.append(("c", other, [0]))
+        got.append(engine.step(entries)[1:1 + count])
+        at += count
+    assert at == length
+    for name in ("a", "b", "c"):
+        engine.cache.release(name)
+    return torch.cat(got)
+
+
+def test_float32_logits_of_long_portions_do_not_depend_on_the_cut():
+    """Portions long enough for the chunked recurrences against short ones, alone and beside other requests."""
+    config = zs.config([zs.wkv(2, 64, ff=48), zs.hgrn2(2, 64, 64), zs.attention(2, 1, 16, 24, window=40, keep_first=3), zs.hgrn2(1, 128, 128)],
+                       width=128, vocab=131, max_positions=600)
+    engine = zs.ZEngine(config, torch.float32, DEVICE, seed=4, long=True, num_pages=160, max_tokens=600, max_step_tokens=800)
+    tokens = zs.tokens_for(131, 400, 10)
+    whole = engine.run_cuts("whole", tokens, [])
+    limit = 2e-5 * float(whole.abs().max())
+    zs.assert_logits_close(whole, engine.plain(tokens), torch.float32)
+    for cuts in ([200], [191, 383], [1, 2, 64, 130, 323], list(range(50, 400, 50))):
+        assert float((engine.run_cuts("cut", tokens, cuts) - whole).abs().max()) <= limit, cuts
+    for portions in ([200, 200], [150, 250], [100, 191, 109]):
+        assert float((long_portions(engine, 400, 131, portions) - whole).abs().max()) <= limit, portions
