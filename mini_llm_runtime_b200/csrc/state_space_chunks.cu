@@ -203,7 +203,8 @@ space_local_kernel(SpaceArgs p) {
   }
   __syncthreads();
   {
-    // outputs of the chunk's own tokens: rows t, t + 8, .., value channels j .. j + 3; rows before a token have no part in it
+    // outputs of the chunk's own tokens: rows t, t + 8, .., value channels j .. j + 3; rows before a token have no part in it (where a
+    // step of k mixes both, the later tokens are left out rather than weighed with zero: an infinity is theirs alone)
     const int j = (tid & 15) * 4, t = tid >> 4;
     float acc[8][4] = {};
 #pragma unroll
@@ -220,8 +221,10 @@ space_local_kernel(SpaceArgs p) {
           load_columns<4>(w, s_w + (t + 8 * k) * W_PITCH + s);
 #pragma unroll
           for (int e = 0; e < 4; ++e)
+            if (k > s / 8 || s % 8 + e <= t) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) sum[k][c] = fmaf(w[e], x[e][c], sum[k][c]);
+              for (int c = 0; c < 4; ++c) sum[k][c] = fmaf(w[e], x[e][c], sum[k][c]);
+            }
         }
       }
 #pragma unroll

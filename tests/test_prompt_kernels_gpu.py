@@ -346,3 +346,22 @@ def test_recurrences_take_batches_without_lengths_on_the_host():
         out = gated("bonus", torch.bfloat16, inputs, weight, aux, bias, g, context, heads, 64)
         results.append((y, s, out, g))
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("heads,n", [(4, 64), (2, 128)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [70, 127, 199])
+def test_a_token_that_is_no_number_leaves_the_tokens_before_it_alone(heads, n, value, at):
+    lengths = [200, 193]
+    x, B, C, dt = (rnd(i, sum(lengths), width) for i, width in enumerate((heads * 64, n, n, heads)))
+    vectors = [rnd(i, heads).to(DEVICE) for i in (5, 6, 7)]
+    results = []
+    for poisoned in (False, True):
+        if poisoned:
+            x[at], B[at], C[at], dt[at] = value, value, value, value
+        s = torch.zeros(2, heads, 64, n, device=DEVICE)
+        y = cuda().state_space_scan(*(t.to(DEVICE) for t in (x, B, C, dt)), *vectors, s, segments(lengths, [0, 1]), heads, 64, n, 1)
+        results.append((y, s))
+    (want, want_s), (got, got_s) = results
+    assert torch.equal(got[:at], want[:at]) and torch.equal(got[200:], want[200:]) and torch.equal(got_s[1], want_s[1])
+    assert not torch.isfinite(got[at]).any()
