@@ -18,7 +18,7 @@
 // Bound by instructions and the barriers between the phases (1.9 of 4 instructions per cycle and SM, tensor pipe 16 %).  Measured (B200),
 // before / after sixteen warps per SM, the mixing with a weight read once per share of the heads, and a logarithm per distance
 // instead of one per pair: portions of 1,450, 401 and 197 rows 276 / 175 us (16 heads of 128), 152 / 110 us (14 of 64); eight decoded
-// rows at 2,048 keys 46 / 30 us and 47 / 35 us.
+// rows at 2,048 keys 46 / 30 us and 47 / 35 us; 8 heads of 64 with key heads of their own, two blocks per SM, 120 / 85 us.
 #include "mma_attention.cuh"
 
 namespace mlr {
@@ -58,17 +58,14 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
   bf16* k_tiles = q_tiles + (size_t)H * SM_ROWS * D;                       // [G][32][D], swizzled per head
   bf16* v_tiles = k_tiles + (size_t)G * SM_KEYS * D;                       // [G][32][V]
   bf16* w_mix = v_tiles + (size_t)G * SM_KEYS * V;                         // [H][16][SM_WSTRIDE]
-  const int HP = (H + 3) & ~3;                                             // heads in whole groups of four
-  float* w_raw = reinterpret_cast<float*>(w_mix + (size_t)H * SM_ROWS * SM_WSTRIDE);      // [HP][16][SM_WSTRIDE]
-  float* talk = w_raw + (size_t)HP * SM_ROWS * SM_WSTRIDE;                 // [SM_HEADS][SM_HEADS], zeros around [H][H]
-  float* bias = talk + SM_HEADS * SM_HEADS;                                // [SM_HEADS][SM_BIAS]: pb - r1 ln(1 + r2 distance)
-  int* key_row = reinterpret_cast<int*>(bias + SM_HEADS * SM_BIAS);        // [2][32]: the cached row of every key of this and the next tile
+  // [H][SM_HEADS]; a thread's share of the heads may end past the last one: what it reads there lies in w_raw and goes nowhere
+  float* talk = reinterpret_cast<float*>(w_mix + (size_t)H * SM_ROWS * SM_WSTRIDE);
+  float* w_raw = talk + H * SM_HEADS;                                      // [H][16][SM_WSTRIDE]
+  int* key_row = reinterpret_cast<int*>(w_raw + (size_t)H * SM_ROWS * SM_WSTRIDE);      // [2][32]: the cached row of every key of this and the next tile
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
   if (a.talk != nullptr) {
-    for (int i = threadIdx.x; i < SM_HEADS * SM_HEADS; i += SM_THREADS)
-      talk[i] = i / SM_HEADS < H && i % SM_HEADS < H ? a.talk[i / SM_HEADS * H + i % SM_HEADS] : 0.f;
-    for (int i = threadIdx.x; i < (HP - H) * SM_ROWS * SM_WSTRIDE; i += SM_THREADS) w_raw[(size_t)H * SM_ROWS * SM_WSTRIDE + i] = 0.f;
+    for (int i = threadIdx.x; i < H * H; i += SM_THREADS) talk[i / H * SM_HEADS + i % H] = a.talk[i];
   }
   pdl_wait();
   const int seg = a.tile_seg[blockIdx.x];
@@ -153,8 +150,10 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
         const float pb = a.pb != nullptr ? a.pb[h] : 0.f;
         // the bias of the 47 distances between these rows and keys, entry row - key + 31 (distances below zero are not seen); the
         // logarithm, like the exponential and the division below, is the hardware's approximate one (errors of a few units in the
-        // last place of a float32, far inside the bfloat16 rounding of the weight that follows)
-        float* head_bias = bias + h * SM_BIAS;
+        // last place of a float32, far inside the bfloat16 rounding of the weight that follows).  They lie where this warp's mixed weights
+        // of the head were (multiplied by it a phase ago) and will be (a barrier ahead): a place of their own cost some sizes the
+        // kernel and others their second block per SM.
+        float* head_bias = reinterpret_cast<float*>(w_mix + (size_t)h * SM_ROWS * SM_WSTRIDE);
 #pragma unroll
         for (int i = lane; i < SM_BIAS; i += 32) {
           const int distance = first_pos - k0 + i - (SM_KEYS - 1);
@@ -195,7 +194,8 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
       bf16* mixed = w_mix + (size_t)r * SM_WSTRIDE + j;
       if (a.talk != nullptr) {
         float2 sum[SHARE] = {};
-        for (int g = 0; g < HP; g += 4) {
+        int g = 0;
+        for (; g + 4 <= H; g += 4) {
           float2 w[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) w[e] = *reinterpret_cast<const float2*>(weights + (size_t)(g + e) * SM_ROWS * SM_WSTRIDE);
@@ -206,6 +206,14 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
             sum[h].x = fmaf(t.y, w[1].x, sum[h].x); sum[h].y = fmaf(t.y, w[1].y, sum[h].y);
             sum[h].x = fmaf(t.z, w[2].x, sum[h].x); sum[h].y = fmaf(t.z, w[2].y, sum[h].y);
             sum[h].x = fmaf(t.w, w[3].x, sum[h].x); sum[h].y = fmaf(t.w, w[3].y, sum[h].y);
+          }
+        }
+        for (; g < H; ++g) {      // heads that fill no group of four
+          const float2 w = *reinterpret_cast<const float2*>(weights + (size_t)g * SM_ROWS * SM_WSTRIDE);
+#pragma unroll
+          for (int h = 0; h < SHARE; ++h) {
+            const float t = talk[(h0 + h) * SM_HEADS + g];
+            sum[h].x = fmaf(t, w.x, sum[h].x); sum[h].y = fmaf(t, w.y, sum[h].y);
           }
         }
 #pragma unroll
@@ -289,8 +297,10 @@ add_chunks_bf16_kernel(const float* partial, bf16* __restrict__ out, long long c
 static size_t sigmoid_mma_shared(int heads, int kv_heads, int dim, int vdim) {
   return sizeof(bf16) * ((size_t)heads * SM_ROWS * dim + (size_t)kv_heads * SM_KEYS * (dim + vdim) +
                          (size_t)heads * SM_ROWS * SM_WSTRIDE) +
-         sizeof(float) * ((size_t)((heads + 3) & ~3) * SM_ROWS * SM_WSTRIDE + SM_HEADS * (SM_HEADS + SM_BIAS)) + sizeof(int) * 2 * SM_KEYS;
+         sizeof(float) * ((size_t)heads * SM_ROWS * SM_WSTRIDE + (size_t)heads * SM_HEADS) + sizeof(int) * 2 * SM_KEYS;
 }
+static_assert(SM_HEADS * SM_HEADS <= SM_ROWS * SM_WSTRIDE, "reads past the last head's shares stay within one head's weights");
+static_assert(SM_BIAS * sizeof(float) <= SM_ROWS * SM_WSTRIDE * sizeof(bf16), "a head's biases take the place of its mixed weights");
 
 }  // namespace mlr
 

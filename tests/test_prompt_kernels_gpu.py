@@ -365,3 +365,12 @@ def test_a_token_that_is_no_number_leaves_the_tokens_before_it_alone(heads, n, v
     (want, want_s), (got, got_s) = results
     assert torch.equal(got[:at], want[:at]) and torch.equal(got[200:], want[200:]) and torch.equal(got_s[1], want_s[1])
     assert not torch.isfinite(got[at]).any()
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(9, 9, 128, 128), (11, 11, 128, 64), (8, 8, 64, 64), (15, 3, 64, 64), (13, 1, 128, 128)])
+def test_sigmoid_attention_of_many_key_heads(heads, kv_heads, dim, vdim):
+    """Sizes whose tiles come close to an SM's shared memory, all on the tensor cores."""
+    from mini_llm_runtime_b200.ops import build
+    assert build.load_library("attention_sigmoid_mma").mlr_attention_sigmoid_mma_fits(heads, kv_heads, dim, vdim) == 1
+    test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, True)
+    test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, False)
