@@ -132,14 +132,15 @@ def plan_attention(lengths: np.ndarray, position_start: np.ndarray) -> tuple[dic
     ``tile_*``: tiles of at most 16 rows, those of segments longer than one row first, so that a
     split-KV kernel may take the one-row segments (``decode_seg``, ``counts["decode"]`` of them)
     instead of the last tiles.  ``wide_*`` / ``big_*``: tiles of 64 / 128 rows over the longer
-    segments only, heaviest first."""
+    segments only, heaviest first.  ``counts["prompt_keys"]``: the most keys behind a row of a longer
+    segment."""
     lengths = np.asarray(lengths, dtype=np.int32)
     position_start = np.asarray(position_start, dtype=np.int32)
     if lengths.shape[0] == 1 and lengths[0] > 1:
         # one prompt portion (the common prefill step): its tiles in order, heaviest (= last) first
         # where the general path sorts; a dozen array operations instead of forty
         rows = int(lengths[0])
-        arrays, counts = {"decode_seg": np.zeros(0, dtype=np.int32)}, {"decode": 0}
+        arrays, counts = {"decode_seg": np.zeros(0, dtype=np.int32)}, {"decode": 0, "prompt_keys": int(position_start[0]) + rows}
         for prefix, count_name, tile_rows, heavy_first in (("tile", "tiles", GENERIC_TILE_ROWS, False),
                                                            ("wide_tile", "wide", MMA_TILE_ROWS, True),
                                                            ("big_tile", "big", TCGEN05_TILE_ROWS, True)):
@@ -159,8 +160,35 @@ def plan_attention(lengths: np.ndarray, position_start: np.ndarray) -> tuple[dic
               "wide_tile_seg": wide_seg, "wide_tile_row0": wide_row0,
               "big_tile_seg": big_seg, "big_tile_row0": big_row0}
     counts = {"tiles": int(tile_seg.shape[0]), "decode": int(decode_seg.shape[0]),
-              "wide": int(wide_seg.shape[0]), "big": int(big_seg.shape[0])}
+              "wide": int(wide_seg.shape[0]), "big": int(big_seg.shape[0]),
+              "prompt_keys": int((position_start + lengths)[longer].max()) if longer.shape[0] else 0}
     return arrays, counts
+
+
+def prompt_keys(batch: AttentionBatch, window: int, keep_first: int = 0) -> int:
+    """The most keys that an item of up to 128 rows of a prompt portion walks.  (Decoded rows beside it may see many more.)"""
+    keys = int(batch.counts.get("prompt_keys", batch.max_kv_len))
+    return min(keys, int(window) + int(keep_first) + min(int(batch.max_q_len), TCGEN05_TILE_ROWS)) if window else keys
+
+
+def diff_prompt_on_tcgen05(batch: AttentionBatch, rows: int, window: int, keep_first: int) -> bool:
+    """Whether a step of ``rows`` rows has enough in its prompt portions for the tcgen05 kernel of differential attention.
+
+    A step of few rows and keys has nothing but launches in it, and those of the mma.sync kernel, whose time grows with both, are
+    cheaper.  Measured in us, mma.sync / tcgen05, 7 heads of 2 x 64 with values of 128 (16 heads): 2 rows that see 128 keys
+    20 / 22 (26 / 26); 4 rows, 32 keys 17 / 20 (30 / 26), 96 keys 22 / 22 (32 / 26), 128 keys 24 / 22, 256 keys 30 / 24; 8 rows, 32 keys
+    26 / 20 (46 / 24); beside a decoded row 4 rows, 32 keys 32 / 40 (42 / 44), 192 keys 42 / 42 (50 / 46), 8 rows, 32 keys 40 / 40
+    (58 / 44), 128 keys 44 / 40; 2,048 rows 287 / 64 (597 / 81)."""
+    few_keys = 192 if batch.num_decode else 96
+    return batch.max_q_len >= 4 and (prompt_keys(batch, window, keep_first) > few_keys or rows - batch.num_decode >= 8)
+
+
+def latent_prompt_on_tcgen05(batch: AttentionBatch, rows: int, window: int) -> bool:
+    """The same for attention over latents.  Measured in us, mma.sync / tcgen05, 14 heads of 256 + 32 (16 of 512 + 64): 2 rows that see
+    62 keys 14 / 14 (18 / 16), 128 keys 21 / 16; 4 rows, 32 keys 12 / 16 (14 / 17), 96 keys 18 / 17 (23 / 21), 128 keys 23 / 16; 8 rows, 64 keys
+    16 / 18 (21 / 23), 96 keys 20 / 19 (25 / 25); 24 rows, 96 keys 21 / 21 (27 / 25); beside a decoded row 4 rows, 64 keys 26 / 26
+    (30 / 32), 128 keys 32 / 26, 8 rows, 96 keys 30 / 30 (36 / 38), 128 keys 32 / 28."""
+    return prompt_keys(batch, window) > 96 or rows - batch.num_decode > 64
 
 
 class CudaOps:
@@ -1026,13 +1054,8 @@ class CudaOps:
             # prompt portions on the tensor cores: each map as an attention of its own, then the combination
             maps = torch.empty((q.shape[0], 2 * heads * vdim), dtype=torch.float32, device=q.device)
             page_size = k_pool.shape[2]
-            # Measured in us, 7 heads of 2 x 64 with values of 128, mma.sync / tcgen05: 2,048 rows 291 / 57, 128 rows 127 / 24,
-            # 12 rows 27 / 23, 7 rows 21 / 23, 4 rows 20 / 23, of them 16 heads 56 / 23, 35 / 23, 23 / 23; 4 rows behind 500 41 / 27.  A
-            # step of few rows and keys has nothing but launches in it, and the older kernel's are cheaper (8 rows 20 / 23, 4 + 2
-            # rows and a decoded one 26 / 30); its time grows by 2 us a row.
-            if (self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and batch.max_q_len >= 4 and page_size >= 8
-                    and (int(batch.max_kv_len) > (256 if batch.num_decode else 128)
-                         or q.shape[0] - batch.num_decode >= (16 if batch.num_decode else 12))
+            if (self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and page_size >= 8
+                    and diff_prompt_on_tcgen05(batch, q.shape[0], window, keep_first)
                     and page_size & (page_size - 1) == 0 and scale > 0 and k_pool.data_ptr() % 16 == 0
                     and v_pool.data_ptr() % 16 == 0):
                 space = self._workspace(q.device)
@@ -1310,12 +1333,8 @@ class CudaOps:
                 "latent attention (decode)")
             tiles -= batch.num_decode       # the one-row segments' tiles are the last of the list
         page_size = pool.shape[2]
-        # Measured in us, 7 / 16 heads, mma.sync -> tcgen05: 2 rows behind 500 54 -> 17 / 76 -> 23, 40 and 9 rows behind 0 and 100
-        # 17 -> 15 / 24 -> 16; 24 rows 17 -> 19 / 14 -> 16, 4 rows 13 -> 16 / 13 -> 15, 2 rows behind 40 and a
-        # decoded one 21 -> 28, behind 300 33 -> 28.  Where few rows see few keys there is nothing but launches in it, and the older
-        # kernel's are cheaper; its time grows by 3 to 5 us per tile of 32 keys.
         if (tiles > 0 and on_tensor_cores and self.use_tcgen05_attention and batch.counts.get("big", 0) > 0 and page_size >= 8
-                and (int(batch.max_kv_len) > (256 if batch.num_decode else 128) or q.shape[0] - batch.num_decode > 64)
+                and latent_prompt_on_tcgen05(batch, q.shape[0], window)
                 and page_size & (page_size - 1) == 0 and scale > 0 and q.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0
                 and (self.use_latent_decode_kernel or batch.num_decode == 0) and self._latent_tcgen05_fits(heads, rank, rot)):
             # prompt portions with both products on tcgen05

@@ -1,0 +1,36 @@
+"""The rules that send prompt portions to the tcgen05 attention kernels, on work lists made on the CPU."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from mini_llm_runtime_b200.ops import AttentionBatch
+from mini_llm_runtime_b200.ops import cuda_ops
+
+
+def batch(lengths, before):
+    lengths, before = np.array(lengths, np.int32), np.array(before, np.int32)
+    arrays, counts = cuda_ops.plan_attention(lengths, before)
+    return AttentionBatch(None, None, None, None, None, len(lengths), int(lengths.max()), int((lengths + before).max()), arrays, counts)
+
+
+@pytest.mark.parametrize("lengths,before,window,keys", [
+    ([2, 1], [40, 2000], 0, 42), ([1, 2, 7], [2000, 40, 100], 0, 107), ([9], [300], 0, 309), ([1, 1], [5, 2000], 0, 0),
+    ([2, 1], [900, 2000], 100, 102), ([300], [900], 100, 228), ([300], [0], 1000, 300)])
+def test_the_keys_that_prompt_rows_see(lengths, before, window, keys):
+    assert cuda_ops.prompt_keys(batch(lengths, before), window) == keys
+
+
+@pytest.mark.parametrize("decoded", [[], [3], [2000, 5]])
+def test_decoded_rows_contexts_do_not_move_the_borders(decoded):
+    """Few rows that see few keys stay on the older kernels however long the contexts beside them are; many rows or keys do not."""
+    ones, few = [1] * len(decoded), 192 if decoded else 96
+    for lengths, before, latent, diff in (([2], [40], False, False), ([4], [40], False, False), ([4], [few], True, True),
+                                          ([4], [few - 4], few > 96, False), ([4], [92], False, False), ([4], [93], True, not decoded),
+                                          ([2], [few], True, False), ([7], [0], False, False), ([8], [0], False, True), ([65], [0], True, True)):
+        b, rows = batch(lengths + ones, before + decoded), sum(lengths) + len(ones)
+        assert cuda_ops.latent_prompt_on_tcgen05(b, rows, 0) == latent, (lengths, before)
+        assert cuda_ops.diff_prompt_on_tcgen05(b, rows, 0, 0) == diff, (lengths, before)
+        # a window shorter than the border hides the keys behind it
+        assert cuda_ops.latent_prompt_on_tcgen05(b, rows, 50) == (rows - len(ones) > 64), (lengths, before)
