@@ -156,6 +156,19 @@ linear_simt_add_kernel(const float* partial, const TIn* __restrict__ bias, TOut*
 // their order whatever the number of rows.  Wide outputs (a vocabulary) have CTAs enough.
 inline int simt_parts(int N, int K) { return N > 16384 ? 1 : K / 1024 < 1 ? 1 : K / 1024 > 4 ? 4 : K / 1024; }
 
+// Rows whose parts are in scratch at a time, whole tiles of them: the parts of many rows and columns would be several copies of a large
+// output (4,096 rows of 16,384 in two parts 537 MB).  At most 128 MB of them; an output's additions keep their order.  Measured in us, all
+// rows together / within 64 MB / 128 MB: [M, N, K] = [4096, 3584, 4100] 2,874 / 3,144 / 2,930, [4096, 16384, 2048] 6,442 / 6,688 / 6,561,
+// [2048, 3584, 18944] 6,465 / 6,942 / 6,458 (whose parts are 117 MB): each block's last CTAs leave SMs idle.
+inline int simt_block_rows(int M, int N, int K) {
+  constexpr long long SCRATCH = 32ll << 20;      // numbers
+  const int parts = simt_parts(N, K);
+  if (parts == 1 || (long long)parts * M * N <= SCRATCH) return M;
+  const long long most = SCRATCH / ((long long)parts * N) / 64 * 64;      // N is at most 16,384: 512 and more
+  const long long blocks = (M + most - 1) / most;
+  return (int)(((M + blocks - 1) / blocks + 63) / 64 * 64);
+}
+
 template <typename TIn, typename TOut, int BM, int BN, int TM, int TN, int BK>
 int linear_simt_tiles(const void* x, const void* w, const void* bias, void* y, float* partial, int M, int N, int K, bool vec,
                       cudaStream_t stream) {
@@ -187,6 +200,9 @@ int linear_simt_tiles(const void* x, const void* w, const void* bias, void* y, f
 // rows or few columns smaller tiles that keep all SMs busy, a handful of rows 16 x 16, whose CTAs only stream weights.
 // Times in us at [N, K] = [9728, 896] / [896, 4864], tiles from large to small: 16 rows 89 38 32 37 / 86 48 22 29, 200 rows
 // 153 132 150 276 / 150 94 103 143, 1,500 rows 645 664 1017 2010 / 361 370 522 1017.
+// Whole products before these tiles and copies / now, from a flushed L2: 1 and 8 rows [9728, 896] 145 150 / 19 27, [896, 4864] 678 710 / 16 20, a head of
+// [151936, 896] 483 493 / 145 150; bfloat16 and 32-bit operands of odd lengths, which come by plain loads: 1, 64 and 600 rows
+// [4864, 897] 133 193 299 / 35 74 250 and 152 219 301 / 37 102 279, [2000, 2002] 305 453 406 / 68 145 307 and 346 510 434 / 68 201 379.
 struct SimtTile {
   int m, n, together;
   float work, step;
@@ -211,8 +227,8 @@ inline int simt_plan(int M, int N, int K) {
 }
 
 template <typename TIn, typename TOut>
-int linear_simt_launch(const void* x, const void* w, const void* bias, void* y, float* partial, int M, int N, int K,
-                       cudaStream_t stream) {
+int linear_simt_block(const void* x, const void* w, const void* bias, void* y, float* partial, int M, int N, int K,
+                      cudaStream_t stream) {
   const bool vec = K % 4 == 0 && ((uintptr_t)x | (uintptr_t)w) % 16 == 0;
   switch (simt_plan(M, N, K)) {
     case 0: return linear_simt_tiles<TIn, TOut, 64, 128, 8, 8, 16>(x, w, bias, y, partial, M, N, K, vec, stream);
@@ -222,6 +238,18 @@ int linear_simt_launch(const void* x, const void* w, const void* bias, void* y, 
   }
 }
 
+template <typename TIn, typename TOut>
+int linear_simt_launch(const void* x, const void* w, const void* bias, void* y, float* partial, int M, int N, int K,
+                       cudaStream_t stream) {
+  const int block = simt_block_rows(M, N, K);
+  for (int row = 0; row < M; row += block) {
+    const int status = linear_simt_block<TIn, TOut>((const TIn*)x + (size_t)row * K, w, bias, (TOut*)y + (size_t)row * N, partial,
+                                                    M - row < block ? M - row : block, N, K, stream);
+    if (status != MLR_OK) return status;
+  }
+  return MLR_OK;
+}
+
 }  // namespace mlr
 
 using namespace mlr;
@@ -229,8 +257,9 @@ using namespace mlr;
 MLR_DEFINE_PDL_SWITCH
 
 // How many parts a product's sums over k are taken in; with more than one mlr_linear_simt needs float32 scratch
-// [parts, M, N] in `partial`.
+// [parts, rows, N] in `partial`, for the rows it takes at a time.
 MLR_EXPORT int mlr_linear_simt_parts(int N, int K) { return N <= 0 || K <= 0 ? 1 : mlr::simt_parts(N, K); }
+MLR_EXPORT int mlr_linear_simt_block_rows(int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? M : mlr::simt_block_rows(M, N, K); }
 
 // in_dtype: storage of x, w and bias.  out_dtype: storage of y (float32 output from bfloat16
 // inputs is used for logits).

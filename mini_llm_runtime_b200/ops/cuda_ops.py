@@ -602,11 +602,12 @@ class CudaOps:
     def _linear_simt(self, x, weight, bias, out_dtype):
         out = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
         lib = build.load_library("linear_simt")
-        # long sums of narrow outputs are taken in parts, whose results meet here
+        # long sums of narrow outputs are taken in parts, whose results meet here, so many rows at a time
         parts = lib.mlr_linear_simt_parts(weight.shape[0], x.shape[1])
         partial = None
         if parts > 1:
-            partial = torch.empty((parts, x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
+            rows = lib.mlr_linear_simt_block_rows(x.shape[0], weight.shape[0], x.shape[1])
+            partial = torch.empty((parts, rows, weight.shape[0]), dtype=torch.float32, device=x.device)
         _check(lib.mlr_linear_simt(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), x.shape[0],
                                    weight.shape[0], x.shape[1], _ptr(partial), _code(x.dtype), _code(out_dtype),
                                    _stream()), "linear")

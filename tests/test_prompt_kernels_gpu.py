@@ -374,3 +374,17 @@ def test_sigmoid_attention_of_many_key_heads(heads, kv_heads, dim, vdim):
     assert build.load_library("attention_sigmoid_mma").mlr_attention_sigmoid_mma_fits(heads, kv_heads, dim, vdim) == 1
     test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, True)
     test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, False)
+
+
+def test_long_sums_of_many_rows_keep_their_scratch_bounded():
+    """4,000 rows in four parts of every sum: the rows in blocks whose parts fit the bound, with the bits of a call of their own."""
+    m, n, k = 4000, 3000, 4100
+    x, w, bias = (t.to(DEVICE) for t in (rnd(1, m, k), rnd(2, n, k, std=0.2), rnd(3, n)))
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    start = torch.cuda.memory_allocated()
+    whole = cuda().linear(x, w, bias)
+    extra = torch.cuda.max_memory_allocated() - start - whole.numel() * 4
+    assert extra <= 129 << 20, extra
+    for first, rows in ((0, 64), (1300, 500), (3937, 63)):
+        assert torch.equal(cuda().linear(x[first:first + rows].contiguous(), w, bias), whole[first:first + rows]), first
