@@ -57,11 +57,12 @@ constexpr int FA_P_BYTES = FA_ROWS * FA_KEYS * 2;          // one tile of probab
 constexpr float FA_LAZY = 8.f;
 
 // Sizes that depend on the head sizes (D of queries and keys, DV of values).  With 128 the shared memory of two
-// resident CTAs only fits with a two-stage ring and one buffer of probabilities.
+// resident CTAs only fits with a two-stage ring and one buffer of probabilities, likewise with keys of 128 beside values of 64
+// (with three stages one CTA per SM: 2,048 rows, window 1,024, 7 heads of 2 x 128: 69 us, with two 52; 16 heads 89 and 73).
 template <int D, int DV>
 struct FaShape {
   static constexpr int HALVES = D / 64, V_HALVES = DV / 64;  // 64-wide (128-byte) column blocks of a row
-  static constexpr int STAGES = D + DV == 128 ? 4 : D + DV == 192 ? 3 : 2;
+  static constexpr int STAGES = D + DV == 128 ? 4 : D + DV == 192 && D == 64 ? 3 : 2;
   static constexpr int P_BUFFERS = 1;
   static constexpr int Q_BYTES = FA_ROWS * D * 2;
   static constexpr int Q_HALF_BYTES = FA_ROWS * 128;
@@ -693,6 +694,7 @@ static int fa_launch(const void* q, const void* k_pool, const void* v_pool, void
   // dynamic shared memory then has to start on a 1024-byte boundary, which it does when the kernel
   // has no static shared memory; the kernel checks and reports through the error word if not.
   const size_t shared = (D + DV < 256 ? 1024 : 0) + (size_t)Shape::DATA_BYTES + FA_CONTROL_BYTES;
+  static_assert(2 * ((D + DV < 256 ? 1024 : 0) + Shape::DATA_BYTES + FA_CONTROL_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
   static bool configured = false;
   if (!configured) {
     cudaError_t err = cudaFuncSetAttribute(prefill_attention_tcgen05_kernel<D, DV, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
