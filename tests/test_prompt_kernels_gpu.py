@@ -65,8 +65,9 @@ CHUNKED = [([1, 64, 65, 200], [3, 0, 2, 1], None), ([193, 128, 63, 1, 127], [4, 
 @pytest.mark.parametrize("mode", ["bonus", "forget"])
 @pytest.mark.parametrize("heads,dim", [(3, 64), (2, 128)])
 @pytest.mark.parametrize("lengths,slots,order", CHUNKED)
-def test_gated_recurrences_in_chunks(mode, heads, dim, lengths, slots, order):
+def test_gated_recurrences_in_chunks(mode, heads, dim, lengths, slots, order, monkeypatch):
     """Segments around the borders of chunks of 64 tokens, rows of requests in any order, decays of zero and one."""
+    monkeypatch.setattr(cuda(), "GATED_CHUNK_ROWS", 1)      # short segments in chunks as well
     ctx, rows, n = segments(lengths, slots, order), sum(lengths), heads * dim
     r, k, v, gate = (rnd(i, rows, n, std=0.7) for i in range(4))
     raw, bias, weight = rnd(5, rows, n, std=0.5), rnd(6, n) * 2 - 2, 1 + rnd(7, n, std=0.1)
@@ -110,8 +111,9 @@ def test_products_of_the_32_bit_path_do_not_depend_on_the_rows_beside(n, k):
 
 @pytest.mark.parametrize("heads,n,groups", [(4, 64, 1), (6, 128, 2)])
 @pytest.mark.parametrize("lengths,slots,order", CHUNKED)
-def test_state_space_in_chunks(heads, n, groups, lengths, slots, order):
+def test_state_space_in_chunks(heads, n, groups, lengths, slots, order, monkeypatch):
     """Segments around the borders of chunks; decays from zero to one, among them tokens that neither keep nor forget."""
+    monkeypatch.setattr(cuda(), "STATE_SPACE_CHUNK_ROWS", 1)      # short segments in chunks as well
     ctx, rows, inner = segments(lengths, slots, order), sum(lengths), heads * 64
     x, B, C, dt = rnd(1, rows, inner), rnd(2, rows, groups * n), rnd(3, rows, groups * n), rnd(4, rows, heads, std=2.0)
     dt[rows // 3], dt[rows // 2] = 90.0, -90.0
@@ -215,7 +217,7 @@ def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
     """Segments around the borders of runs of four chunks and more, rows of requests in any order, gates that forget and keep everything: as
     without runs (which the 64-bit oracle vouches for elsewhere), whose products are the same and whose sums another order."""
     ctx, rows = segments(lengths, slots, order), sum(lengths)
-    assert cuda()._memory_chunks_fit(dim, vdim)
+    assert cuda()._memory_chunks_fit(dim, vdim) and memory_run(ctx, rows, heads, vdim) > 0
     q, k, v, gate = rnd(1, rows, heads * dim), rnd(2, rows, heads * dim), rnd(3, rows, heads * vdim), rnd(4, rows, heads * vdim)
     i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
     f_raw[rows // 3], f_raw[rows // 2] = -80.0, 80.0
@@ -235,51 +237,6 @@ def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
     assert torch.equal(m, want_m)
     close(s.flatten(0, 1), want_s.flatten(0, 1), 200 * UNIT, "state")      # sums of 64 products at a time, once per chunk
     close(out, want, 2.0 ** -8, "output")
-
-
-def relative(got, want):
-    return float((got.double().cpu() - want.double()).norm() / want.double().norm())
-
-
-@pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (14, 256, 32)])
-def test_latent_prompts_are_as_close_to_64_bits_on_either_kernel(heads, rank, rot):
-    """The probabilities' rounding to 16 bits is all of the error, and the same error in both kernels; the 2-norm over 3e5 and more outputs
-    varies by far less than the two percent left to it."""
-    lengths, before = [150, 90], [200, 0]
-    (pool,), cpu, batch = paged(lengths, before, lambda p, j: j <= p, 16, [(1, rank + rot, 1.0)], 7)
-    q = rnd(6, sum(lengths), heads * (rank + rot), std=0.5).to(torch.bfloat16)
-    args = (heads, rank, rot, 0.08, 0)
-    want = FAKE.latent_attention(q.float(), pool.float(), cpu, *args, None)
-    errors = []
-    for tcgen05 in (False, True):
-        cuda().use_tcgen05_attention = tcgen05
-        try:
-            errors.append(relative(cuda().latent_attention(q.to(DEVICE), pool.to(DEVICE), batch, *args, None), want))
-        finally:
-            cuda().use_tcgen05_attention = True
-    print("error mma.sync, tcgen05:", errors)
-    assert errors[1] <= 1.02 * errors[0], errors
-
-
-@pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 128)])
-@pytest.mark.parametrize("window", [0, 120])
-def test_differential_prompts_are_as_close_to_64_bits_on_either_kernel(dim, vdim, window):
-    """As above; the outputs' own rounding to 16 bits is in both errors."""
-    heads, kv_heads, lengths, before, keep = 6, 2, [200, 90], [150, 0], 4
-    seen = lambda p, j: j <= p and (not window or p - j < window or j < keep)      # noqa: E731
-    pools, cpu, batch = paged(lengths, before, seen, 16, [(kv_heads, 2 * dim, 1.0), (kv_heads, vdim, 0.7)], 3)
-    q = rnd(5, sum(lengths), 2 * heads * dim).to(torch.bfloat16)
-    args = (heads, kv_heads, dim, vdim, dim ** -0.5, window, keep, 0.4, 1e-6, 0.5)
-    want = FAKE.differential_attention(q.float(), *(t.float() for t in pools), cpu, *args)
-    errors = []
-    for tcgen05 in (False, True):
-        cuda().use_tcgen05_attention = tcgen05
-        try:
-            errors.append(relative(cuda().differential_attention(q.to(DEVICE), *(t.to(DEVICE) for t in pools), batch, *args), want))
-        finally:
-            cuda().use_tcgen05_attention = True
-    print("error mma.sync, tcgen05:", errors)
-    assert errors[1] <= 1.02 * errors[0], errors
 
 
 def gated(mode, dtype, inputs, weight, aux, bias, state, ctx, heads, dim):
@@ -367,6 +324,51 @@ def test_a_token_that_is_no_number_leaves_the_tokens_before_it_alone(heads, n, v
     assert not torch.isfinite(got[at]).any()
 
 
+def relative(got, want):
+    return float((got.double().cpu() - want.double()).norm() / want.double().norm())
+
+
+@pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (14, 256, 32)])
+def test_latent_prompts_are_as_close_to_64_bits_on_either_kernel(heads, rank, rot):
+    """The probabilities' rounding to 16 bits is all of the error, and the same error in both kernels; the 2-norm over 3e5 and more outputs
+    varies by far less than the two percent left to it."""
+    lengths, before = [150, 90], [200, 0]
+    (pool,), cpu, batch = paged(lengths, before, lambda p, j: j <= p, 16, [(1, rank + rot, 1.0)], 7)
+    q = rnd(6, sum(lengths), heads * (rank + rot), std=0.5).to(torch.bfloat16)
+    args = (heads, rank, rot, 0.08, 0)
+    want = FAKE.latent_attention(q.float(), pool.float(), cpu, *args, None)
+    errors = []
+    for tcgen05 in (False, True):
+        cuda().use_tcgen05_attention = tcgen05
+        try:
+            errors.append(relative(cuda().latent_attention(q.to(DEVICE), pool.to(DEVICE), batch, *args, None), want))
+        finally:
+            cuda().use_tcgen05_attention = True
+    print("error mma.sync, tcgen05:", errors)
+    assert errors[1] <= 1.02 * errors[0], errors
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (128, 128)])
+@pytest.mark.parametrize("window", [0, 120])
+def test_differential_prompts_are_as_close_to_64_bits_on_either_kernel(dim, vdim, window):
+    """As above; the outputs' own rounding to 16 bits is in both errors."""
+    heads, kv_heads, lengths, before, keep = 6, 2, [200, 90], [150, 0], 4
+    seen = lambda p, j: j <= p and (not window or p - j < window or j < keep)      # noqa: E731
+    pools, cpu, batch = paged(lengths, before, seen, 16, [(kv_heads, 2 * dim, 1.0), (kv_heads, vdim, 0.7)], 3)
+    q = rnd(5, sum(lengths), 2 * heads * dim).to(torch.bfloat16)
+    args = (heads, kv_heads, dim, vdim, dim ** -0.5, window, keep, 0.4, 1e-6, 0.5)
+    want = FAKE.differential_attention(q.float(), *(t.float() for t in pools), cpu, *args)
+    errors = []
+    for tcgen05 in (False, True):
+        cuda().use_tcgen05_attention = tcgen05
+        try:
+            errors.append(relative(cuda().differential_attention(q.to(DEVICE), *(t.to(DEVICE) for t in pools), batch, *args), want))
+        finally:
+            cuda().use_tcgen05_attention = True
+    print("error mma.sync, tcgen05:", errors)
+    assert errors[1] <= 1.02 * errors[0], errors
+
+
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(9, 9, 128, 128), (11, 11, 128, 64), (8, 8, 64, 64), (15, 3, 64, 64), (13, 1, 128, 128)])
 def test_sigmoid_attention_of_many_key_heads(heads, kv_heads, dim, vdim):
     """Sizes whose tiles come close to an SM's shared memory, all on the tensor cores."""
@@ -388,3 +390,54 @@ def test_long_sums_of_many_rows_keep_their_scratch_bounded():
     assert extra <= 129 << 20, extra
     for first, rows in ((0, 64), (1300, 500), (3937, 63)):
         assert torch.equal(cuda().linear(x[first:first + rows].contiguous(), w, bias), whole[first:first + rows]), first
+
+
+@pytest.mark.parametrize("rows,top,experts", [(2048, 6, 64), (1500, 7, 33), (1366, 6, 128), (9000, 1, 40)])
+def test_pairs_sorted_by_expert_in_several_turns(rows, top, experts):
+    """More than the 8,192 choices that the sort's threads hold at once, more experts than a warp has lanes; one expert gets none.  Weights of
+    few bits and expert matrices that only scale, so that every output is exact in 32 bits."""
+    width = 128
+    x = torch.randint(-8, 9, (rows, width), generator=generator(1)).to(torch.bfloat16)
+    chosen = torch.stack([torch.randperm(experts - 1, generator=generator(10 + r))[:top] for r in range(rows)]).int()
+    weights = torch.randint(1, 5, (rows, top), generator=generator(2)).float() / 4
+    # gate rows of zeros but for a constant would need a bias; silu(g) * u with g = x and u = x is the same for every expert, and down
+    # scales it by a power of two of the expert's own
+    eye = torch.eye(width)
+    gate_up = torch.cat([torch.cat([eye[i:i + 64], eye[i:i + 64]]) for i in range(0, width, 64)])[None].expand(experts, -1, -1)
+    scale = 2.0 ** (torch.arange(experts) % 8 - 4).float()
+    down = eye[None] * scale[:, None, None]
+    got = cuda().routed_experts(x.to(DEVICE), chosen.to(DEVICE), weights.to(DEVICE), gate_up.to(torch.bfloat16).contiguous().to(DEVICE),
+                                down.to(torch.bfloat16).contiguous().to(DEVICE), 64)
+    f = x.double()
+    hidden = f * torch.sigmoid(f) * f
+    want = hidden * (weights.double() * scale.double()[chosen.long()]).sum(1, keepdim=True)
+    # hidden is rounded to 16 bits once, with the approximate exponential before
+    assert bool(((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("lengths,slots,order", [([1, 512, 1100], [2, 0, 1], None), ([1030, 3], [1, 0], [1, 0])])
+def test_matrix_memory_in_runs_against_64_bits(lengths, slots, order):
+    heads, dim, vdim = 2, 64, 64
+    ctx, rows = segments(lengths, slots, order), sum(lengths)
+    assert memory_run(ctx, rows, heads, vdim) > 0
+    q, k, v, gate = (rnd(i, rows, heads * 64) for i in range(4))
+    i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
+    f_raw[rows // 3], f_raw[rows // 2] = -80.0, 80.0
+    bias, weight = torch.zeros(heads), 1 + rnd(7, heads * vdim, std=0.1)
+    state, maximum = rnd(8, len(lengths), heads, vdim + 1, dim, std=0.5), rnd(9, len(lengths), heads)
+    # the kernel's products take q, k and v rounded to bfloat16
+    q, k, v = (t.to(torch.bfloat16).float() for t in (q, k, v))
+    s64, m64 = state.double(), maximum.double()
+    want = FAKE.matrix_memory(*(t.double() for t in (q, k, v, i_raw, f_raw, bias, bias + 3)), 15.0, 1e-6, gate.double(), weight.double(), 1e-6,
+                              s64, m64, ctx, heads, dim, vdim, torch.float64)
+    s, m = state.to(DEVICE), maximum.to(DEVICE)
+    got = cuda().matrix_memory(*(spaced(t, 8) for t in (q, k, v, i_raw, f_raw)), bias.to(DEVICE), bias.to(DEVICE) + 3, 15.0, 1e-6,
+                               spaced(gate, 8), weight.to(DEVICE), 1e-6, s, m, ctx, heads, dim, vdim, torch.bfloat16)
+    # 32-bit sums over up to 18 chunks, whose decays and products are rounded 64 times each at most; the output in 16 bits
+    close(s.flatten(0, 1), s64.flatten(0, 1), 2000 * UNIT, "state")
+    close(got, want, 2.0 ** -8, "output")
+
+
+def memory_run(ctx, rows, heads, vdim):
+    from mini_llm_runtime_b200.ops import build
+    return build.load_library("matrix_memory").mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim)
