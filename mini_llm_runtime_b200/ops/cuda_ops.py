@@ -196,7 +196,8 @@ class CudaOps:
 
     Kernels that need scratch memory (split-K partial tiles, split-KV partial softmax states) share
     per-device buffers owned by this object; calls are ordered by the CUDA stream they run on, so
-    one stream at a time may use an instance.
+    one stream at a time may use an instance.  That holds for the prompt attention of every family on the
+    tcgen05 kernels (plain, shaped, differential, latent), which draw their items from one queue.
     """
 
     name = "cuda"
@@ -1638,7 +1639,9 @@ class CudaOps:
 
     SIGMOID_CHUNK_KEYS = 64       # keys one CTA of the sigmoid attention takes of a row, at least, when rows are few
     SIGMOID_MMA_CHUNK_KEYS = 128  # the same for the tensor-core kernel
-    SIGMOID_MMA_LONGEST = 384     # keys one CTA of the tensor-core kernel takes of a row, at most
+    # keys one CTA of the tensor-core kernel takes of a row, at most.  Measured in us with 320 / 384 / 448 / 512, portions of 1,450, 401 and 197
+    # rows: 16 heads of 128 175 / 181 / 181 / 187, 14 of 64 114 / 116 / 116 / 144; 2,048 rows 273 / 259 / 277 / 263; decoded rows the same
+    SIGMOID_MMA_LONGEST = 384
     use_mma_sigmoid = True        # bfloat16 with key and value sizes of 64 or 128: the two products on the tensor cores
 
     def sigmoid_attention(self, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, batch: AttentionBatch,
