@@ -5,7 +5,8 @@
 // and its end state is the decays' product times S plus sum_s (prod_{u > s} g_u) B_s (dt_s x_s)^T.  Four kernels:
 //   pairs    C_t . B_s of a chunk, once for all heads of a group
 //   local    per head and chunk: the masked product and what the chunk's own tokens leave behind; a segment's first chunk
-//            also reads the request's state
+//            also reads the request's state; blocks of its own take the step's shorter segments token by token (portions of 1,531, 77, 1
+//            and 439 rows, 32 heads: 139 us with all in chunks, 153 with a launch for the shorter ones, 127 so)
 //   carry    per state entry, the chunks of a segment in order
 //   read     per head and later chunk: the read of the state before it, added to the outputs
 // All 32-bit multiply-adds.  Decay products are products of numbers up to one, formed step by step, never differences of
@@ -16,6 +17,7 @@
 // request, B200: 424 -> 63 us (14 heads, states of 64), 639 -> 124 (32 heads, states of 128).
 #include "chunk_places.cuh"
 #include "copy_async.cuh"
+#include "state_space_scan.cuh"
 
 namespace mlr {
 
@@ -34,7 +36,8 @@ struct SpaceArgs {
   float* decays;                     // [chunk places, heads]: products over the chunk
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, groups;
-  int segments, least;               // segments of fewer than `least` rows are another kernel's
+  int segments, least;               // segments of `least` rows and more go in chunks
+  int scans;                         // blocks per head that take the others token by token
 };
 
 // `count` rows of N entries into shared rows `pitch` apart; the rows up to CHUNK become zero.
@@ -145,7 +148,7 @@ __device__ __forceinline__ void read_state(const SpaceArgs& p, const float* s_c,
   }
 }
 
-// grid: (heads, chunks)
+// grid: (heads, scans + chunks)
 template <int N>
 __global__ void __launch_bounds__(128, 3)
 space_local_kernel(SpaceArgs p) {
@@ -158,10 +161,18 @@ space_local_kernel(SpaceArgs p) {
   float* s_dt = s_g + CHUNK;                   // [CHUNK] step sizes
   float* s_to_end = s_dt + CHUNK;              // [CHUNK] decays' product behind a token
   pdl_trigger();
+  if ((int)blockIdx.y < p.scans) {
+    constexpr int SL = N / SCAN_NPT, PARTS = VD * SL / SCAN_THREADS;
+    const ScanArgs scan{p.x, p.B, p.C, p.dt_raw, p.x_stride, p.b_stride, p.c_stride, p.dt_stride, p.dt_bias, p.A_log, p.D, p.states, p.y,
+                        p.seg_q_start, p.seg_q_len, p.seg_slot, p.heads, VD, N, p.groups, p.least - 1};
+    scan_segment<SL, true>(scan, shared, blockIdx.y / PARTS, blockIdx.x, blockIdx.y % PARTS);
+    return;
+  }
   const int head = blockIdx.x, tid = threadIdx.x;
   const float rate = expf(p.A_log[head]), bias = p.dt_bias[head], skip = p.D[head];
   pdl_wait();
-  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  const auto [seg, chunk, length, start, slot] =
+      chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y - p.scans);
   if (seg < 0) return;
   const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int group = head / (p.heads / p.groups);
@@ -359,7 +370,9 @@ space_read_kernel(SpaceArgs p) {
 template <int N>
 int launch_space(const SpaceArgs& a, int rows, int max_q_len, cudaStream_t stream) {
   constexpr size_t pairs_shared = sizeof(float) * (CHUNK + 16) * (N + 4);
-  constexpr size_t local_shared = sizeof(float) * (CHUNK * (W_PITCH + VD + N + 4) + 3 * CHUNK);
+  constexpr size_t chunk_shared = sizeof(float) * (CHUNK * (W_PITCH + VD + N + 4) + 3 * CHUNK);
+  const size_t segment_shared = scan_shared(N, SCAN_THREADS / (N / SCAN_NPT));
+  const size_t local_shared = a.scans > 0 && segment_shared > chunk_shared ? segment_shared : chunk_shared;
   constexpr size_t read_shared = sizeof(float) * (VD + CHUNK) * (N + 4);
   static_assert(VD * (N + 4) <= CHUNK * (W_PITCH + VD), "the state takes the place of weights and inputs");
   const unsigned chunks = (unsigned)long_chunks(rows, a.segments, a.least);
@@ -370,7 +383,7 @@ int launch_space(const SpaceArgs& a, int rows, int max_q_len, cudaStream_t strea
   launch_kernel(space_pairs_kernel<N>, dim3(chunks, a.groups * 4), dim3(128), pairs_shared, stream, a);
   int status = launch_status();
   if (status != MLR_OK) return status;
-  launch_kernel(space_local_kernel<N>, dim3(a.heads, chunks), dim3(128), local_shared, stream, a);
+  launch_kernel(space_local_kernel<N>, dim3(a.heads, a.scans + chunks), dim3(128), local_shared, stream, a);
   if ((status = launch_status()) != MLR_OK || max_q_len <= CHUNK) return status;
   launch_kernel(space_carry_kernel, dim3((a.heads * VD * N / 4 + 255) / 256, (unsigned)long_segments(rows, a.segments, a.least)), dim3(256), 0,
                 stream, a, VD * N);
@@ -392,20 +405,21 @@ MLR_EXPORT long long mlr_state_space_chunk_scratch(int rows, int heads, int n, i
 }
 
 // As mlr_state_space_scan, for heads of 64 value channels with states of 64 or 128 entries and x, B, C, states, y and scratch whose
-// rows begin on 16-byte boundaries.  rows: the step's rows.  Segments of fewer than least_rows rows are left alone.
+// rows begin on 16-byte boundaries.  rows: the step's rows.  Segments of fewer than least_rows rows
+// go token by token as there; others: whether there can be any.
 MLR_EXPORT int mlr_state_space_chunks(const float* x, long long x_stride, const float* B, long long b_stride, const float* C,
                                       long long c_stride, const float* dt_raw, long long dt_stride, const float* dt_bias,
                                       const float* A_log, const float* D, float* states, float* y, float* scratch,
                                       const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments, int rows,
-                                      int max_q_len, int least_rows, int heads, int vdim, int n, int groups, cudaStream_t stream) {
-  if (segments == 0 || max_q_len < least_rows) return MLR_OK;
-  if (segments < 0 || least_rows <= 0 || rows <= 0 || max_q_len <= 0 || heads <= 0 || groups <= 0 || heads % groups != 0 || scratch == nullptr)
+                                      int max_q_len, int least_rows, int others, int heads, int vdim, int n, int groups, cudaStream_t stream) {
+  if (segments == 0) return MLR_OK;
+  if (segments < 0 || least_rows <= 0 || rows <= 0 || max_q_len < least_rows || heads <= 0 || groups <= 0 || heads % groups != 0 || scratch == nullptr)
     return MLR_BAD_SIZE;
-  if (vdim != VD || (n != 64 && n != 128) || long_chunks(rows, segments, least_rows) > 65535 || groups > 65535 / 4) return MLR_TOO_LARGE;
+  if (vdim != VD || (n != 64 && n != 128) || long_chunks(rows, segments, least_rows) + segments * 4ll > 65535 || groups > 65535 / 4) return MLR_TOO_LARGE;
   const uintptr_t pointers = (uintptr_t)x | (uintptr_t)B | (uintptr_t)C | (uintptr_t)states | (uintptr_t)y | (uintptr_t)scratch;
   if (pointers % 16 != 0 || (x_stride | b_stride | c_stride) % 4 != 0) return MLR_BAD_ALIGNMENT;
   SpaceArgs a{x, B, C, dt_raw, x_stride, b_stride, c_stride, dt_stride, dt_bias, A_log, D, states, y,
-              nullptr, nullptr, scratch, nullptr, seg_q_start, seg_q_len, seg_slot, heads, groups, segments, least_rows};
+              nullptr, nullptr, scratch, nullptr, seg_q_start, seg_q_len, seg_slot, heads, groups, segments, least_rows, others ? segments * (VD * (n / SCAN_NPT) / SCAN_THREADS) : 0};
   a.pairs = a.ends + (size_t)chunk_places(rows) * heads * VD * n;
   a.since = a.pairs + (size_t)rows * groups * CHUNK;
   a.decays = a.since + (size_t)rows * heads;

@@ -2018,7 +2018,6 @@ class CudaOps:
         if tuple(state.shape[1:]) != (heads, vdim, n):
             raise KernelError(f"state has shape {tuple(state.shape)}, expected [slots, {heads}, {vdim}, {n}]")
         y = torch.empty((rows, heads * vdim), dtype=torch.float32, device=x.device)
-        longest = int(ctx.max_q_len)
         views = (*self._view(x, "x", rows, heads * vdim), *self._view(B, "B", rows, groups * n),
                  *self._view(C, "C", rows, groups * n), *self._view(dt_raw, "dt_raw", rows, heads))
         if (self.use_state_space_chunks and ctx.max_q_len >= self.STATE_SPACE_CHUNK_ROWS and vdim == 64 and n in (64, 128)
@@ -2030,14 +2029,12 @@ class CudaOps:
             _check(lib.mlr_state_space_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(D), _ptr(state), _ptr(y), _ptr(scratch), _ptr(ctx.seg_q_start),
                 _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), self.STATE_SPACE_CHUNK_ROWS,
-                heads, vdim, n, groups, _stream()), "state_space_chunks")
-            longest = self._longest_below(ctx, self.STATE_SPACE_CHUNK_ROWS)
-            if longest == 0:
-                return y
+                int(self._longest_below(ctx, self.STATE_SPACE_CHUNK_ROWS) > 0), heads, vdim, n, groups, _stream()), "state_space_chunks")
+            return y
         _check(build.load_library("state_space").mlr_state_space_scan(
             *views, _ptr(dt_bias), _ptr(A_log),
             _ptr(D), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot),
-            ctx.num_segments, longest, heads, vdim, n, groups, _stream()), "state_space_scan")
+            ctx.num_segments, heads, vdim, n, groups, _stream()), "state_space_scan")
         return y
 
     def gated_group_norm(self, y: torch.Tensor, gate, weight: torch.Tensor, eps: float, parts: int,
