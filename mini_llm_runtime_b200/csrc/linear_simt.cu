@@ -200,8 +200,8 @@ int linear_simt_tiles(const void* x, const void* w, const void* bias, void* y, f
 // rows or few columns smaller tiles that keep all SMs busy, a handful of rows 16 x 16, whose CTAs only stream weights.
 // Times in us at [N, K] = [9728, 896] / [896, 4864], tiles from large to small: 16 rows 89 38 32 37 / 86 48 22 29, 200 rows
 // 153 132 150 276 / 150 94 103 143, 1,500 rows 645 664 1017 2010 / 361 370 522 1017.
-// Whole products before these tiles and copies / now, from a flushed L2: 1 and 8 rows [9728, 896] 145 150 / 19 27, [896, 4864] 678 710 / 16 20, a head of
-// [151936, 896] 483 493 / 145 150; bfloat16 and 32-bit operands of odd lengths, which come by plain loads: 1, 64 and 600 rows
+// Whole products before these tiles and copies / now, from a flushed L2: 1 and 8 rows [9728, 896] 145 150 / 19 27, [896, 4864] 678 710 / 16 20,
+// a head of [151936, 896] 483 493 / 145 150; bfloat16 and 32-bit operands of odd lengths, which come by plain loads: 1, 64 and 600 rows
 // [4864, 897] 133 193 299 / 35 74 250 and 152 219 301 / 37 102 279, [2000, 2002] 305 453 406 / 68 145 307 and 346 510 434 / 68 201 379.
 struct SimtTile {
   int m, n, together;
