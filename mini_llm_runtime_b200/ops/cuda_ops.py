@@ -1999,8 +1999,8 @@ class CudaOps:
         return out
 
     use_state_space_chunks = True
-    # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us, token by token / in chunks: 128 rows 30 / 31 (14 heads,
-    # states of 64), 42 / 50 (32 heads, states of 128); 512 rows 108 / 31, 161 / 64.
+    # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us, token by
+    # token / in chunks: 128 rows 30 / 31 (14 heads, states of 64), 42 / 50 (32 heads, states of 128); 512 rows 108 / 31, 161 / 64.
     STATE_SPACE_CHUNK_ROWS = 192
 
     def state_space_scan(self, x, B, C, dt_raw, dt_bias, A_log, D, state, ctx, heads: int, vdim: int, n: int,
