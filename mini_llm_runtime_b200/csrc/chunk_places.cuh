@@ -21,15 +21,16 @@ struct ChunkAt {
   int seg, chunk, length, start, slot;      // seg < 0: the step has no such chunk; start: the segment's first row
 };
 
-// The long segment (CHUNKS: the chunk of a long segment) of number `index`; every warp that asks does so as a whole.
+// The long segment (CHUNKS: the chunk of a long segment, where segments below `split` rows are one chunk) of number `index`; every warp
+// that asks does so as a whole.
 template <bool CHUNKS>
 __device__ __forceinline__ ChunkAt chunk_at(const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments, int least,
-                                            int index) {
+                                            int index, int split = 0) {
   const int lane = threadIdx.x & 31;
   for (int base = 0; base < segments; base += 32) {
     const bool in = base + lane < segments;      // all three asked for together: one trip to memory
     const int length = in ? seg_q_len[base + lane] : 0, start = in ? seg_q_start[base + lane] : 0, slot = in ? seg_slot[base + lane] : 0;
-    const int own = length < least || length <= 0 ? 0 : CHUNKS ? (length + CHUNK - 1) / CHUNK : 1;
+    const int own = length < least || length <= 0 ? 0 : CHUNKS && length >= split ? (length + CHUNK - 1) / CHUNK : 1;
     int upto = own;
     if (segments > 1) {
 #pragma unroll

@@ -4,7 +4,8 @@
 // S_t = diag(a_t) S_{t-1} + b_t v_t^T is linear in S with a diagonal factor, so a chunk's end state is its decays' product
 // times the state before it plus what the chunk's own tokens leave behind, and its outputs are those of a walk from zero
 // plus (r_t times the decays' running product)^T S.  Three kernels:
-//   walk     every chunk of CHUNK tokens at once, token by token from zero (a segment's first chunk from the request's state):
+//   walk     every chunk of CHUNK tokens at once, token by token from zero (a segment's first chunk, and a segment too short to be
+//            cut, from the request's state):
 //            outputs without norm, decay-weighted reads, the decays' product, the end state
 //   carry    per state entry, the chunks of a segment in order: the state before every chunk, and the request's new state
 //   finish   reads times the state before the chunk (a product of CHUNK x dim by dim x vdim), added to the walk's outputs, then
@@ -33,7 +34,7 @@ struct ChunkArgs {
   float* decays;                                 // [chunk places, heads, dim]: products over the chunk
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, weight_per_head;
-  int segments, least;                           // segments of fewer than `least` rows are another kernel's
+  int segments, least, split;                    // segments of fewer than `least` rows are another kernel's, below `split` not cut
 };
 
 // Thread (lane, warp) walks key channels [16 * slice, +16) of C neighbouring value channels; T tokens at a time are
@@ -56,13 +57,14 @@ chunk_walk_kernel(ChunkArgs p) {
   pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x;
-  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  const auto [seg, chunk, length, start, slot] =
+      chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y, p.split);
   if (seg < 0) return;
   extern __shared__ __align__(16) float shared[];
   float* s_o = shared + 2 * W::STAGE;                    // [SLICES][T][VDIM]
   float* s_bonus = s_o + SLICES * T * VDIM;              // [T] sum_i r c b (mode 0)
-  const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
-  const bool whole = length <= CHUNK;                    // the segment is this chunk
+  const bool whole = length <= CHUNK || length < p.split;      // the segment is this chunk
+  const int first = start + chunk * CHUNK, count = whole ? length : min(CHUNK, length - chunk * CHUNK);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, column = lane * C;
   float* state = p.state + ((size_t)slot * p.heads + head) * DIM * VDIM;
 
@@ -202,7 +204,7 @@ chunk_carry_kernel(ChunkArgs p, int dim, int vdim) {
   constexpr int BATCH = 8;
   pdl_trigger();
   pdl_wait();
-  const auto [seg, which, length, start, slot] = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  const auto [seg, which, length, start, slot] = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, max(p.least, p.split), blockIdx.y);
   if (seg < 0) return;
   const int first = start, chunks = (length + CHUNK - 1) / CHUNK, cells = dim * vdim;
   const int at = (blockIdx.x * 256 + threadIdx.x) * 4;
@@ -250,7 +252,8 @@ chunk_finish_kernel(ChunkArgs p, T* __restrict__ out) {
   const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int j = (threadIdx.x % LANES) * 4, group = threadIdx.x / LANES;
   float o[TOKENS][4];
-  if (chunk > 0) {
+  const bool behind = chunk > 0 && length >= p.split;      // a state before that the walk did not start from
+  if (behind) {
     const float* before = p.ends + (chunk_place(first, false) * p.heads + head) * DIM * VDIM;
     for (int idx = threadIdx.x; idx < DIM * VDIM / 4; idx += THREADS) copy_async_16(s_state + idx * 4, before + idx * 4);
     for (int idx = threadIdx.x; idx < count * (DIM / 4); idx += THREADS) {
@@ -264,7 +267,7 @@ chunk_finish_kernel(ChunkArgs p, T* __restrict__ out) {
     const int t = group + 8 * k;
     if (t < count) load_columns<4>(o[k], p.outputs + ((size_t)(first + t) * p.heads + head) * VDIM + j);
   }
-  if (chunk > 0) {
+  if (behind) {
     copy_async_wait<0>();
     __syncthreads();
     float add[TOKENS][4];      // sums of their own: the rest of the output joins last
@@ -336,8 +339,9 @@ int launch_chunks(const ChunkArgs& args, void* out, int rows, int max_q_len, cud
   launch_kernel(walk, grid, dim3(W::THREADS), W::SHARED, stream, args);
   int status = launch_status();
   if (status != MLR_OK) return status;
-  if (max_q_len > CHUNK) {
-    launch_kernel(chunk_carry_kernel, dim3((args.heads * DIM * VDIM / 4 + 255) / 256, (unsigned)long_segments(rows, args.segments, args.least)), dim3(256), 0, stream, args, DIM, VDIM);
+  if (max_q_len > CHUNK && max_q_len >= args.split) {
+    const int least = args.least > args.split ? args.least : args.split;
+    launch_kernel(chunk_carry_kernel, dim3((args.heads * DIM * VDIM / 4 + 255) / 256, (unsigned)long_segments(rows, args.segments, least)), dim3(256), 0, stream, args, DIM, VDIM);
     if ((status = launch_status()) != MLR_OK) return status;
   }
   launch_kernel(finish, grid, dim3(2 * VDIM), finish_shared, stream, args, (T*)out);
@@ -372,16 +376,16 @@ MLR_EXPORT long long mlr_gated_chunk_scratch(int rows, int heads, int dim, int v
 
 // As mlr_gated_recurrence, for square heads of 64 or 128 and inputs (state, weights, output and scratch too) whose rows begin
 // on 16-byte boundaries.  rows: the step's rows; scratch: mlr_gated_chunk_scratch numbers.  Segments of fewer than least_rows rows are
-// left alone.
+// left alone, those of fewer than split_rows walked in one piece.
 MLR_EXPORT int mlr_gated_recurrence_chunks(int mode, const float* r, long long r_stride, const float* b, long long b_stride,
                                            const float* v, long long v_stride, const float* raw, long long raw_stride,
                                            const float* gate, long long gate_stride, const float* bias, const float* aux,
                                            const float* weight, float eps, float* state, void* out, float* scratch,
                                            const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments,
-                                           int rows, int max_q_len, int least_rows, int heads, int dim, int vdim, int out_dtype,
+                                           int rows, int max_q_len, int least_rows, int split_rows, int heads, int dim, int vdim, int out_dtype,
                                            cudaStream_t stream) {
   if (segments == 0 || max_q_len < least_rows) return MLR_OK;
-  if (segments < 0 || heads <= 0 || rows <= 0 || max_q_len <= 0 || least_rows <= 0 || scratch == nullptr) return MLR_BAD_SIZE;
+  if (segments < 0 || heads <= 0 || rows <= 0 || max_q_len <= 0 || least_rows <= 0 || split_rows < 0 || scratch == nullptr) return MLR_BAD_SIZE;
   if (long_chunks(rows, segments, least_rows) > 65535) return MLR_TOO_LARGE;
   const uintptr_t pointers = (uintptr_t)r | (uintptr_t)b | (uintptr_t)v | (uintptr_t)raw | (uintptr_t)gate | (uintptr_t)weight |
                              (uintptr_t)state | (uintptr_t)out | (uintptr_t)scratch;
@@ -396,7 +400,7 @@ MLR_EXPORT int mlr_gated_recurrence_chunks(int mode, const float* r, long long r
   args.ends = args.reads + (size_t)rows * heads * dim;
   args.decays = args.ends + (size_t)chunk_places(rows) * heads * dim * vdim;
   args.seg_q_start = seg_q_start; args.seg_q_len = seg_q_len; args.seg_slot = seg_slot;
-  args.heads = heads; args.weight_per_head = mode == 0 ? 1 : 0; args.segments = segments; args.least = least_rows;
+  args.heads = heads; args.weight_per_head = mode == 0 ? 1 : 0; args.segments = segments; args.least = least_rows; args.split = split_rows;
   if (mode == 0) return launch_chunks<0>(args, out, rows, max_q_len, dim, vdim, out_dtype, stream);
   if (mode == 1) return launch_chunks<1>(args, out, rows, max_q_len, dim, vdim, out_dtype, stream);
   return MLR_BAD_SIZE;

@@ -898,10 +898,13 @@ class CudaOps:
         return max((s.length for s in segments if s.length < rows), default=0)
 
     use_gated_chunks = True
-    # Portions of so many rows and more go in chunks, shorter ones beside them token by token: which way a request's rows go is a matter
-    # of its own portion only, as their numbers are.  Measured in us, walked by one CTA per head part / in chunks: 128 rows
-    # 37 / 41 (14 heads of 64), 44 / 42 (32 of 64), 44 / 55 (7 and 16 of 128); 512 rows 129 / 42, 135 / 46, 157 / 70.
-    GATED_CHUNK_ROWS = 192
+    # By head size: portions of fewer rows than the first number go token by token in a launch of their own, those from the second on in
+    # chunks, those between token by token in the chunks' launches.  Which way a request's rows go is a matter of its own portion
+    # only, as their numbers are.  Measured in us from a flushed L2, by sequence_mix.cu / walked in the chunks' launches / in chunks:
+    # 14 heads of 64: 16 rows 14, 32 rows 21 / 21, 64 34 / 32, 100 48 / 40, 127 56 / 48, 128 56 / 48 / 38, 160 69 / - / 38; 7 heads of 128,
+    # whose walk keeps a head on one CTA: 64 rows 34 / 42, 128 58 / 71 / 58 (44 / - / 55 from the L2), 160 71 / - / 58.  A launch of its own
+    # beside long portions: 1,531, 77, 1 and 439 rows 104 with it, 71 walked, 67 all in chunks (14 heads of 64).
+    GATED_ROWS = {64: (32, 128), 128: (160, 160)}
 
     def _recurrence(self, mode, r, b, v, raw, gate, bias, aux, weight, eps, state, ctx, heads, dim, vdim, out_dtype):
         rows = r.shape[0]
@@ -919,7 +922,8 @@ class CudaOps:
         views = (*self._view(r, "r", rows, heads * dim), *(null if b is None else self._view(b, "b", rows, heads * dim)),
                  *self._view(v, "v", rows, heads * vdim), *self._view(raw, "raw", rows, heads * dim),
                  *(null if gate is None else self._view(gate, "gate", rows, heads * vdim)))
-        if (self.use_gated_chunks and ctx.max_q_len >= self.GATED_CHUNK_ROWS and dim == vdim and dim in (64, 128)
+        least, split = self.GATED_ROWS.get(dim, (0, 0))
+        if (self.use_gated_chunks and least and dim == vdim and ctx.max_q_len >= least
                 and all(t is None or (t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0) for t in (r, b, v, raw, gate))
                 and weight.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0):
             # long segments: chunks of tokens side by side
@@ -929,8 +933,8 @@ class CudaOps:
             _check(lib.mlr_gated_recurrence_chunks(
                 mode, *views, _ptr(bias), _ptr(aux), _ptr(weight), ctypes.c_float(eps), _ptr(state), _ptr(out),
                 _ptr(chunk_scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows,
-                int(ctx.max_q_len), self.GATED_CHUNK_ROWS, heads, dim, vdim, _code(out_dtype), _stream()), "gated_recurrence_chunks")
-            longest = self._longest_below(ctx, self.GATED_CHUNK_ROWS)
+                int(ctx.max_q_len), least, split, heads, dim, vdim, _code(out_dtype), _stream()), "gated_recurrence_chunks")
+            longest = self._longest_below(ctx, least)
             if longest == 0:
                 return out
         # steps with long segments, and heads too large for one CTA, spread a head's value channels

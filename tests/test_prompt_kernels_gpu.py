@@ -67,7 +67,7 @@ CHUNKED = [([1, 64, 65, 200], [3, 0, 2, 1], None), ([193, 128, 63, 1, 127], [4, 
 @pytest.mark.parametrize("lengths,slots,order", CHUNKED)
 def test_gated_recurrences_in_chunks(mode, heads, dim, lengths, slots, order, monkeypatch):
     """Segments around the borders of chunks of 64 tokens, rows of requests in any order, decays of zero and one."""
-    monkeypatch.setattr(cuda(), "GATED_CHUNK_ROWS", 1)      # short segments in chunks as well
+    monkeypatch.setattr(cuda(), "GATED_ROWS", {64: (1, 1), 128: (1, 1)})      # short segments in chunks as well
     ctx, rows, n = segments(lengths, slots, order), sum(lengths), heads * dim
     r, k, v, gate = (rnd(i, rows, n, std=0.7) for i in range(4))
     raw, bias, weight = rnd(5, rows, n, std=0.5), rnd(6, n) * 2 - 2, 1 + rnd(7, n, std=0.1)
@@ -248,7 +248,7 @@ def gated(mode, dtype, inputs, weight, aux, bias, state, ctx, heads, dim):
 
 
 # requests whose portions are too short for chunks, each list beside a portion that is long enough
-SHORT = [[1, 1, 1], [3, 1, 60], [1, 100, 191]]
+SHORT = [[1, 1, 1], [3, 1, 31], [32, 1, 63], [1, 100, 127], [1, 159, 191]]
 
 
 @pytest.mark.parametrize("mode", ["bonus", "forget"])
