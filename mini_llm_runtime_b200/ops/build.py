@@ -35,6 +35,7 @@ COMMON_FLAGS = ("-O3", "-lineinfo", "-std=c++17", "--shared", "-Xcompiler", "-fP
 LIBRARIES: dict[str, tuple[str, ...]] = {
     "elementwise": (),
     "linear_simt": (),
+    "linear_split": (),
     "attention_generic": (),
     "sampling": (),
     "gemm_tcgen05": (),

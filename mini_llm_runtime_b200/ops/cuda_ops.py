@@ -368,6 +368,8 @@ class CudaOps:
             out = self._linear_tcgen05(x, weight, None, torch.bfloat16, swiglu=code)
             if out is not None:
                 return out
+        if (activation == "silu" and self.use_fused_swiglu and block == self.SWIGLU_BLOCK and self._split_fits(x, weight)):
+            return self._linear_split(x if rms_eps is None else self.rms_norm(x, None, rms_eps), weight, None, gated=True)
         product = self.linear(x, weight, rms_eps=rms_eps)
         return self.swiglu(product, block) if activation == "silu" else self.gated_activation(product, block, activation)
 
@@ -492,7 +494,10 @@ class CudaOps:
             x = self.rms_norm(x, None, rms_eps)
         out = self._linear_tcgen05(x, weight, bias, out_dtype) if tensor_cores else None
         if out is None:
-            out = self._linear_simt(x, weight, bias, out_dtype)
+            if out_dtype == torch.float32 and self._split_fits(x, weight):
+                out = self._linear_split(x, weight, bias)
+            else:
+                out = self._linear_simt(x, weight, bias, out_dtype)
         return self.add_inplace(residual, out) if residual is not None else out
 
     # Rows up to which the few-rows kernel is chosen.  It accepts up to 64, but measured on the
@@ -598,6 +603,27 @@ class CudaOps:
                                     ctypes.c_float(gate[1]), _ptr(space["gemm_scratch"]),
                                     _ptr(space["gemm_counters"]), _ptr(space["error_word"]), _stream()),
                "linear (tcgen05)")
+        return out
+
+    # Elements of a weight from which 32-bit products run on the tensor cores in bfloat16 parts; a rule on the weight alone, so that a
+    # row's result does not depend on how many rows come with it.  In us, CUDA cores / parts, at 1, 8, 24, 60, 100, 600, 1,500
+    # rows: [1024, 512] 10 10 10 14 15 39 55 / 13 13 15 19 25 28 46; [896, 896] 12 12 14 18 22 43 90 / 13 13 15 17 22 36 52;
+    # [2048, 2048] 15 17 24 38 50 169 355 / 17 17 19 24 28 70 136; [9728, 896] 18 25 37 63 88 302 670 / 19 19 21 24 32 75 157.
+    SPLIT_WEIGHT = 3 << 18
+
+    def _split_fits(self, x, weight) -> bool:
+        """Rows of whole 16-byte pieces on 16-byte boundaries, as the bulk copies want them."""
+        return (self.use_tensor_cores and x.dtype == torch.float32 and x.shape[0] > 0 and x.shape[1] % 4 == 0
+                and weight.data_ptr() % 16 == 0 and weight.numel() >= self.SPLIT_WEIGHT)
+
+    def _linear_split(self, x, weight, bias, gated=False):
+        M, K = x.shape
+        N = weight.shape[0]
+        lib = build.load_library("linear_split")
+        out = torch.empty((M, N // 2 if gated else N), dtype=torch.float32, device=x.device)
+        parts = torch.empty((3, lib.mlr_linear_split_rows(M, K), -(-K // 8) * 8), dtype=torch.bfloat16, device=x.device)
+        _check(lib.mlr_linear_split(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), M, N, K, int(gated), _ptr(parts),
+                                    _ptr(self._workspace(x.device)["error_word"]), _stream()), "linear (32-bit operands in parts)")
         return out
 
     def _linear_simt(self, x, weight, bias, out_dtype):

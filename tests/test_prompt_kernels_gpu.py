@@ -441,3 +441,42 @@ def test_matrix_memory_in_runs_against_64_bits(lengths, slots, order):
 def memory_run(ctx, rows, heads, vdim):
     from mini_llm_runtime_b200.ops import build
     return build.load_library("matrix_memory").mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim)
+
+
+# Tiles of 128 outputs, of 16, 32, 64 and 128 rows, blocks of 64 k; 1, 2, 4 and 8 parts of the sums over k; more tiles than SMs.
+@pytest.mark.parametrize("n,k", [(1024, 832), (1152, 896), (896, 4864), (130, 6148), (7000, 132), (9728, 200), (33, 30000)])
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 300])
+def test_products_in_parts(m, n, k):
+    """32-bit products on the tensor cores: dropped products of parts are below 2^-26 of sum |x||w|, a block's accumulator drops up to
+    2^-23 of its sum at some dozen steps, each block and part is one 32-bit addition; rows keep their bits in other batches."""
+    x, w, bias = (t.to(DEVICE) for t in (rnd(m, m, k), rnd(2, n, k, std=0.2), rnd(3, n)))
+    ops_ = cuda()
+    assert ops_._split_fits(x, w) == (n * k >= ops_.SPLIT_WEIGHT)
+    got, shifted = ops_._linear_split(x, w, bias), torch.cat([torch.zeros(1, device=DEVICE), x.flatten()])[1:].view(m, k)
+    torch.cuda.synchronize()
+    ops_.raise_if_device_error()
+    bound = (k / 64 + 48) * UNIT * (x.abs() @ w.abs().T + bias.abs())
+    assert bool(((got.double() - (x.double() @ w.double().T + bias.double())).abs() <= bound.double()).all())
+    assert torch.equal(ops_._linear_split(shifted, w, bias), got)          # x on no 16-byte boundary
+    for first in {0, m // 2, m - 1}:
+        assert torch.equal(ops_._linear_split(x[first:first + 1].contiguous(), w, bias), got[first:first + 1])
+    if n % 128 == 0:
+        gated = ops_.linear_swiglu(x, w, 64) if ops_._split_fits(x, w) else ops_._linear_split(x, w, None, gated=True)
+        assert torch.equal(gated, ops_.swiglu(ops_._linear_split(x, w, None), 64))
+
+
+@pytest.mark.parametrize("n,k", [(1152, 896), (9728, 100)])
+def test_products_in_parts_with_infinities(n, k):
+    """Infinities, NaN, zeros beside them, numbers at the ends of the range: what a chain of 32-bit multiply-adds makes of them."""
+    x, w = rnd(1, 40, k), rnd(2, n, k, std=0.2)
+    x[3, 5], x[4, 7], x[5, 9], x[6] = float("inf"), -float("inf"), float("nan"), 3.4e38
+    w[10] = 0.0
+    w[11, 5], w[12, 7], w[13, 0] = 1.0, float("inf"), float("nan")
+    x[7], w[14] = 1e-38, 1e-3
+    got, want = cuda()._linear_split(x.to(DEVICE), w.to(DEVICE), None).cpu(), cuda()._linear_simt(x.to(DEVICE), w.to(DEVICE), None, torch.float32).cpu()
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        rows = torch.arange(40) != 6                 # of row 6 the order of the sum decides what overflows
+        assert torch.equal(kind(got)[rows], kind(want)[rows])
+    fine = torch.isfinite(got) & torch.isfinite(want)
+    bound = (k + 48) * UNIT * (x.double().abs() @ w.double().abs().T) + k * 2.0 ** -134
+    assert bool(((got.double() - want.double()).abs() <= bound)[fine].all())
