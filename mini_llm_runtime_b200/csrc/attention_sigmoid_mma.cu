@@ -283,15 +283,26 @@ attention_sigmoid_mma_kernel(const bf16* q, const bf16* k_pool, const bf16* v_po
   }
 }
 
+// The chunks' sums in their order, four neighbouring numbers per thread, all chunks asked for together (number by number, one chunk behind
+// the other: 20 us for four chunks of 2,048 rows of 2,048, bound by the latency of its loads; 12 now, 151 MB).
 __global__ void __launch_bounds__(256)
 add_chunks_bf16_kernel(const float* partial, bf16* __restrict__ out, long long count, int chunks) {
+  constexpr int BATCH = 4;
   pdl_trigger();
   pdl_wait();
-  const long long index = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long index = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (index >= count) return;
-  float sum = 0.f;
-  for (int c = 0; c < chunks; ++c) sum += __ldcg(partial + (size_t)c * count + index);
-  out[index] = __float2bfloat16_rn(sum);
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int c0 = 0; c0 < chunks; c0 += BATCH) {
+    float4 part[BATCH];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i)
+      if (c0 + i < chunks) part[i] = __ldcg(reinterpret_cast<const float4*>(partial + (size_t)(c0 + i) * count + index));
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i)
+      if (c0 + i < chunks) { sum.x += part[i].x; sum.y += part[i].y; sum.z += part[i].z; sum.w += part[i].w; }
+  }
+  *reinterpret_cast<uint2*>(out + index) = make_uint2(pack_bf16(sum.x, sum.y), pack_bf16(sum.z, sum.w));
 }
 
 static size_t sigmoid_mma_shared(int heads, int kv_heads, int dim, int vdim) {
@@ -344,8 +355,8 @@ MLR_EXPORT int mlr_attention_sigmoid_mma(const void* q, const void* k_pool, cons
     int status = launch_status();
     if (status != MLR_OK || chunks == 1) return status;
     const long long count = (long long)total_rows * heads * vdim;
-    launch_kernel(add_chunks_bf16_kernel, dim3((unsigned)((count + 255) / 256)), dim3(256), 0, stream,
-                  (const float*)partial, (bf16*)out, count, chunks);
+    launch_kernel(add_chunks_bf16_kernel, dim3((unsigned)((count / 4 + 255) / 256)), dim3(256), 0, stream,
+                  (const float*)partial, (bf16*)out, count, chunks);      // vdim is a multiple of 64
     return launch_status();
   };
   if (dim == 64 && vdim == 64) return launch(attention_sigmoid_mma_kernel<64, 64>, SigmoidShape<64, 64>::THREADS);

@@ -42,6 +42,7 @@ struct DeltaArgs {
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, kv_heads, dim, vdim;
   float unit_eps, q_scale;
+  int below;                            // segments of so many rows and more are left out (0: none)
 };
 
 __device__ __forceinline__ float delta_decay(float raw, float bias, float a_log) {
@@ -64,7 +65,7 @@ delta_prepare_kernel(DeltaArgs p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q_len = p.seg_q_len[seg];
   const int t0 = (blockIdx.x * PREP_WARPS + warp) * 4;
-  if (t0 >= q_len) return;
+  if (t0 >= q_len || (p.below > 0 && q_len >= p.below)) return;
   const size_t row0 = (size_t)p.seg_q_start[seg] + t0;
   const int count = min(4, q_len - t0);
   float kk[4][4], qk[4][4], qq[4];      // kk[t][s] for s <= t, qk[t][s] = q_t . k_s for s <= t
@@ -165,6 +166,7 @@ delta_scan_kernel(DeltaArgs p) {
   const float a_log = p.A_log[head], bias = p.dt_bias[head];
   pdl_wait();
   const int q_start = p.seg_q_start[seg], q_len = p.seg_q_len[seg];
+  if (p.below > 0 && q_len >= p.below) return;
 
   // zeros that no copy overwrites: behind the rows' D entries
   if (D < pitch) {
@@ -437,19 +439,20 @@ MLR_DEFINE_PDL_SWITCH
 // q, k: float32 rows of kv_heads * dim entries; v: rows of heads * vdim entries; a, b: rows of `heads` entries
 // (each with its own row stride); dt_bias, A_log: float32 [heads]; coef: float32 scratch [rows, heads, 12], or
 // null (then tokens are taken one by one); states: float32 [slots, heads, vdim, dim] (the transposed S);
-// y: float32 [rows, heads * vdim].  max_q_len: the longest segment of the step.
+// y: float32 [rows, heads * vdim].  max_q_len: the longest segment of the step (of those below `below` rows, if that is not 0:
+// the others are left out, states and outputs).
 MLR_EXPORT int mlr_delta_rule_scan(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
                                    long long v_stride, const float* a, long long a_stride, const float* b, long long b_stride,
                                    const float* dt_bias, const float* A_log, float* coef, float* states, float* y,
                                    const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments,
-                                   int max_q_len, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
+                                   int max_q_len, int below, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
                                    cudaStream_t stream) {
   if (segments == 0) return MLR_OK;
   if (segments < 0 || max_q_len <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || dim <= 0 || vdim <= 0)
     return MLR_BAD_SIZE;
   if (dim > 512 || heads > 65535 || segments > 65535 || vdim > 65535) return MLR_TOO_LARGE;
   DeltaArgs p{q, k, v, a, b, q_stride, k_stride, v_stride, a_stride, b_stride, dt_bias, A_log, coef, states, y,
-              seg_q_start, seg_q_len, seg_slot, heads, kv_heads, dim, vdim, unit_eps, q_scale};
+              seg_q_start, seg_q_len, seg_slot, heads, kv_heads, dim, vdim, unit_eps, q_scale, below};
   auto multiple = [](long long n) { return n % 4 == 0; };
   auto aligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
   const bool wide = multiple(dim) && multiple(vdim) && multiple(q_stride) && multiple(k_stride) && multiple(v_stride) &&

@@ -28,6 +28,7 @@
 // 3.4 TB/s; 600 rows [9728, 896] with its gate 318 / 83, [896, 4864] 173 / 70.  Errors against 64 bits (2-norm) at 896, 4,864 and
 // 8,192 k: 1.1e-7, 1.1e-7, 1.2e-7, on the CUDA cores 5.4e-7, 6.2e-7, 8.1e-7.  One MMA of 128 x 128 x 16 takes 64 cycles
 // either way, but of 128 x 16 x 16 takes 12 with its rows in tensor memory and 39 with them in shared memory.
+#include "float_parts.cuh"
 #include "tcgen05.cuh"
 
 namespace mlr {
@@ -61,15 +62,6 @@ struct LinearSplitShape {
   static_assert(SHARED <= 226 * 1024, "tiles fit the shared memory");
   static_assert((size_t)BN * LS_ROWS * 4 <= RAW_STAGES * (size_t)LS_RAW_BYTES, "a tile's sums fit where W's tiles were");
 };
-
-// two neighbours' next part, taken off them
-__device__ __forceinline__ uint32_t take_part(float& a, float& b) {
-  const __nv_bfloat162 pair = __floats2bfloat162_rn(a, b);
-  const uint32_t bits = *reinterpret_cast<const uint32_t*>(&pair);
-  a -= __uint_as_float(bits << 16);
-  b -= __uint_as_float(bits & 0xffff0000u);
-  return bits;
-}
 
 // parts [3][M][pitch], pitch = K rounded up to 8; what lies behind K becomes zero.  K % 4 == 0.
 __global__ void __launch_bounds__(256)

@@ -58,6 +58,7 @@ LIBRARIES: dict[str, tuple[str, ...]] = {
     "state_space": (),
     "state_space_chunks": (),
     "delta_rule": (),
+    "delta_chunks": (),
     "attention_shaped_mma": (),
     "matrix_memory": (),
 }

@@ -1960,6 +1960,12 @@ class CudaOps:
         return out
 
     # ------------------------------------------------------------------ gated delta rule
+    use_delta_chunks = True
+    # Rows from which a request's portion goes in chunks: three launches, of which the first alone takes 20 us.  In us from a flushed L2,
+    # token by token / in chunks, 14 heads of 64 x 64: 128 rows 26 / 32, 256 38 / 40, 384 50 / 42, 1,024 112 / 60, 2,048 214 / 99; 32 heads of
+    # 128 x 64: 128 rows 36 / 52, 256 56 / 58, 384 75 / 65, 1,024 181 / 103, 2,048 346 / 202.
+    DELTA_CHUNK_ROWS = 288
+
     def delta_rule_scan(self, q, k, v, a, b, dt_bias, A_log, state, ctx, heads: int, kv_heads: int, dim: int, vdim: int,
                         unit_eps: float) -> torch.Tensor:
         """Per request and head h (q and k of head h // (heads / kv_heads)), token after token: u_t = beta_t (v_t -
@@ -1976,13 +1982,28 @@ class CudaOps:
         if tuple(state.shape[1:]) != (heads, vdim, dim):
             raise KernelError(f"state has shape {tuple(state.shape)}, expected [slots, {heads}, {vdim}, {dim}]")
         y = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device)
+        views = (*self._view(q, "q", rows, kv_heads * dim), *self._view(k, "k", rows, kv_heads * dim),
+                 *self._view(v, "v", rows, heads * vdim), *self._view(a, "a", rows, heads), *self._view(b, "b", rows, heads))
+        longest, below = int(ctx.max_q_len), 0
+        if (self.use_delta_chunks and longest >= self.DELTA_CHUNK_ROWS and dim in (64, 128) and vdim % 16 == 0
+                and all(t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0 for t in (q, k, v)) and state.data_ptr() % 16 == 0):
+            # long segments: chunks of tokens, all but the state's way through them side by side
+            lib, below = build.load_library("delta_chunks"), self.DELTA_CHUNK_ROWS
+            lib.mlr_delta_chunk_scratch.restype = ctypes.c_longlong
+            scratch = torch.empty(lib.mlr_delta_chunk_scratch(rows, ctx.num_segments, below, heads, kv_heads, dim, vdim),
+                                  dtype=torch.float32, device=q.device)
+            _check(lib.mlr_delta_rule_chunks(
+                *views, _ptr(dt_bias), _ptr(A_log), _ptr(scratch), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
+                _ptr(ctx.seg_slot), ctx.num_segments, rows, below, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+                ctypes.c_float(float(dim) ** -0.5), _ptr(self._workspace(q.device)["error_word"]), _stream()), "delta_rule_chunks")
+            longest = int(self._longest_below(ctx, below))
+            if longest == 0:
+                return y
         # steps with longer segments take four tokens at once; a first kernel leaves their inner products here
-        coef = torch.empty((rows, heads, 12), dtype=torch.float32, device=q.device) if ctx.max_q_len > 1 else None
+        coef = torch.empty((rows, heads, 12), dtype=torch.float32, device=q.device) if longest > 1 else None
         _check(build.load_library("delta_rule").mlr_delta_rule_scan(
-            *self._view(q, "q", rows, kv_heads * dim), *self._view(k, "k", rows, kv_heads * dim),
-            *self._view(v, "v", rows, heads * vdim), *self._view(a, "a", rows, heads), *self._view(b, "b", rows, heads),
-            _ptr(dt_bias), _ptr(A_log), _ptr(coef), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
-            _ptr(ctx.seg_slot), ctx.num_segments, int(ctx.max_q_len), heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+            *views, _ptr(dt_bias), _ptr(A_log), _ptr(coef), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
+            _ptr(ctx.seg_slot), ctx.num_segments, longest, below, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
             ctypes.c_float(float(dim) ** -0.5), _stream()), "delta_rule_scan")
         return y
 

@@ -480,3 +480,51 @@ def test_products_in_parts_with_infinities(n, k):
     fine = torch.isfinite(got) & torch.isfinite(want)
     bound = (k + 48) * UNIT * (x.double().abs() @ w.double().abs().T) + k * 2.0 ** -134
     assert bool(((got.double() - want.double()).abs() <= bound)[fine].all())
+
+
+def delta_inputs(rows, heads, kv_heads, dim, vdim, alike):
+    """``alike``: keys that nearly repeat one another, steps near one, hardly any decay: the triangular systems at their hardest."""
+    q, k, v = rnd(1, rows, kv_heads * dim), rnd(2, rows, kv_heads * dim), rnd(3, rows, heads * vdim)
+    a, b, bias, a_log = rnd(4, rows, heads, std=2.0), rnd(5, rows, heads), rnd(6, heads), rnd(7, heads)
+    if alike:
+        k, a, b = k[:1] + 0.05 * k, a - 9.0, b + 6.0
+    else:
+        a[rows // 3], a[rows // 2], k[rows // 2 + 1] = 90.0, -90.0, 0.0      # all forgotten, nothing forgotten, no key at all
+    return q, k, v, a, b, bias, a_log
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 64, 64), (3, 1, 128, 48), (2, 2, 128, 80)])
+@pytest.mark.parametrize("alike", [False, True])
+@pytest.mark.parametrize("lengths,slots,order", CHUNKED)
+def test_delta_rule_in_chunks(heads, kv_heads, dim, vdim, alike, lengths, slots, order, monkeypatch):
+    """Segments around the borders of chunks, all of them in chunks or the short ones token by token beside."""
+    ctx, rows = segments(lengths, slots, order), sum(lengths)
+    q, k, v, a, b, bias, a_log = delta_inputs(rows, heads, kv_heads, dim, vdim, alike)
+    state = rnd(8, len(lengths), heads, vdim, dim, std=0.3)
+    want_state = state.double()
+    want = FAKE.delta_rule_scan(*(t.double() for t in (q, k, v, a, b, bias, a_log)), want_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
+    for least in (1, cuda().DELTA_CHUNK_ROWS):
+        monkeypatch.setattr(cuda(), "DELTA_CHUNK_ROWS", least)
+        got_state = state.to(DEVICE)
+        got = cuda().delta_rule_scan(*(spaced(t) for t in (q, k, v, a, b)), bias.to(DEVICE), a_log.to(DEVICE), got_state, ctx, heads,
+                                     kv_heads, dim, vdim, 1e-6)
+        # sums of up to dim + CHUNK products behind a triangular system of CHUNK rows
+        close(got, want, 200 * UNIT, "delta rule outputs")
+        close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "delta rule state")
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("which,at", [("k", 70), ("k", 110), ("v", 127), ("q", 199), ("a", 130), ("a", 105), ("b", 120)])
+def test_a_token_that_is_no_number_leaves_the_tokens_of_a_delta_rule_before_it_alone(value, which, at):
+    heads, kv_heads, dim, vdim, rows = 2, 1, 128, 64, 200
+    inputs = dict(zip("qkvab", delta_inputs(rows, heads, kv_heads, dim, vdim, False)))
+    bias, a_log = rnd(6, heads).to(DEVICE), rnd(7, heads).to(DEVICE)
+    ctx, results = segments([rows], [0], None), []
+    for broken in (False, True):
+        given = {name: t.clone() for name, t in inputs.items()}
+        if broken:
+            given[which][at, 0] = value
+        state = rnd(8, 1, heads, vdim, dim, std=0.3).to(DEVICE)
+        results.append(cuda().delta_rule_scan(*(given[name].to(DEVICE) for name in "qkvab"), bias, a_log, state, ctx, heads, kv_heads, dim,
+                                              vdim, 1e-6).cpu())
+    assert torch.equal(results[0][:at], results[1][:at])
