@@ -802,7 +802,18 @@ static GemmPlan plan_many_rows(int M, int N, int K, bool swiglu, int sms) {
 
 static GemmPlan plan_gemm(int M, int N, int K, bool swiglu) {
   const int sms = sm_count();
-  if (M > 128) return plan_many_rows(M, N, K, swiglu, sms);
+  if (M > 128) {
+    // The model above is asked about some eighty plans, 2 us; a step's layers ask for the same few products, so plans are kept by what they
+    // depend on.  (As with the tensor maps, kernels are launched from one host thread.)
+    struct Kept { int M, N, K, swiglu, sms; GemmPlan plan; };
+    static Kept kept[64] = {};
+    const bool by_rule = forced_bn == 0 && forced_stages == 0 && forced_splits == 0 && forced_bm == 0 && forced_pair == 0;
+    Kept& at = kept[((unsigned)M * 0x9E3779B1u ^ (unsigned)N * 0x85EBCA77u ^ (unsigned)K * 0xC2B2AE3Du ^ (swiglu ? 0x27D4EB2Fu : 0u)) >> 26];
+    if (by_rule && at.M == M && at.N == N && at.K == K && at.swiglu == (int)swiglu && at.sms == sms) return at.plan;
+    const GemmPlan plan = plan_many_rows(M, N, K, swiglu, sms);
+    if (by_rule) at = {M, N, K, (int)swiglu, sms, plan};
+    return plan;
+  }
   GemmPlan plan;
   plan.bm = TILE_ROWS;
   plan.pair = false;
@@ -869,14 +880,7 @@ MLR_EXPORT void mlr_gemm_tcgen05_debug(int bn, int stages, int splits, int bm) {
 // allows, with rings of six stages (one CTA per SM); 2: the same with three stages (two CTAs per SM).
 MLR_EXPORT void mlr_gemm_tcgen05_debug_pair(int pair) { forced_pair = pair; }
 
-// Scratch needed for a product of this shape (bytes of float32 partial tiles); 0 without split-K.
-// `splits_out` receives the split count the launcher will use, `tiles_out` the number of tiles.
-MLR_EXPORT long long mlr_gemm_tcgen05_plan(int M, int N, int K, int swiglu, int* splits_out, int* tiles_out) {
-  const GemmPlan plan = plan_gemm(M, N, K, swiglu != 0);
-  if (splits_out) *splits_out = plan.splits;
-  if (tiles_out) *tiles_out = plan.tiles;
-  return plan.splits > 1 ? (long long)plan.tiles * plan.splits * plan.bn * TILE_ROWS * 4 : 0;
-}
+#define MLR_NO_ROOM (-6)
 
 // x [M,K], w [N,K], bias [N] or null, all bfloat16; out [M,N] bfloat16 (out_f32 = 0) or float32.
 // swiglu != 0: w holds blocks of 64 gate rows followed by the 64 up rows of the same outputs and the
@@ -884,11 +888,11 @@ MLR_EXPORT long long mlr_gemm_tcgen05_plan(int M, int N, int K, int swiglu, int*
 // (swiglu == 3) the clamped gate g * sigmoid(gate_slope * g) * (u + 1) with g = min(gate, gate_limit) and
 // u = clamp(up, -gate_limit, gate_limit)
 // (N % 128 == 0; the bias comes first) and out is act(gate) * up, [M, N/2] bfloat16.
-// scratch: at least mlr_gemm_tcgen05_plan(...) bytes; counters: one zeroed int per tile;
+// scratch: scratch_bytes of it; counters: counters_len zeroed ints; a plan that needs more than either is refused with MLR_NO_ROOM;
 // error_word: host-visible int that receives a non-zero code if a wait inside the kernel runs out.
 MLR_EXPORT int mlr_gemm_tcgen05(const void* x, const void* w, const void* bias, void* out, int M, int N, int K,
-                                int out_f32, int swiglu, float gate_limit, float gate_slope, void* scratch, int* counters,
-                                int* error_word, cudaStream_t stream) {
+                                int out_f32, int swiglu, float gate_limit, float gate_slope, void* scratch, long long scratch_bytes,
+                                int* counters, int counters_len, int* error_word, cudaStream_t stream) {
   if (M == 0) return MLR_OK;
   if (M < 0 || N <= 0 || K <= 0) return MLR_BAD_SIZE;
   if (K % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return MLR_BAD_ALIGNMENT;
@@ -912,6 +916,8 @@ MLR_EXPORT int mlr_gemm_tcgen05(const void* x, const void* w, const void* bias, 
   p.group_tiles = nullptr;
   p.row_scale = nullptr;
   if (plan.splits > 1 && (scratch == nullptr || counters == nullptr)) return MLR_BAD_SIZE;
+  if (plan.splits > 1 && ((long long)plan.tiles * plan.splits * plan.bn * TILE_ROWS * 4 > scratch_bytes || plan.tiles > counters_len))
+    return MLR_NO_ROOM;
   if (swiglu) {
     if (M <= 16) return launch<16, true, true>(x, w, p, plan.splits, stream);
     if (M <= 32) return launch<32, true, true>(x, w, p, plan.splits, stream);

@@ -198,6 +198,9 @@ def compile_library(name: str, *, verbose_ptxas: bool = False) -> Path:
 
 def load_library(name: str) -> ctypes.CDLL:
     """The loaded library ``name``; compiled first if no current build exists."""
+    library = _loaded.get(name)
+    if library is not None:
+        return library
     with _lock:
         if name not in _loaded:
             path = compile_library(name)

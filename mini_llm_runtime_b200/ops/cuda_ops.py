@@ -30,6 +30,9 @@ _STATUS_TEXT = {
 }
 
 
+_NO_ROOM = -6
+
+
 class KernelError(RuntimeError):
     pass
 
@@ -73,6 +76,37 @@ def _stream() -> ctypes.c_void_p:
     """The current stream of the current device (the raw handle: the wrapper object of
     ``torch.cuda.current_stream`` costs microseconds, and a step asks hundreds of times)."""
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+
+
+# What the entry points of a prompt step's products, norms and attention take: p a pointer, i an int, l a long long, f a float.  Declared, they
+# take Python's own integers (tensor.data_ptr()) and floats; an object made for each of some twenty arguments costs as much as the launch.
+# Steps of up to about 1,400 rows of a 0.5B model are bound by the host (170 launches); with a product's plan kept by its sizes instead of asked
+# for twice, one step of 64 rows 3,120 -> 2,840 us, of 1,000 rows 3,380 -> 3,020.
+_PROTOTYPES = {
+    "gemm_tcgen05": {"mlr_gemm_tcgen05": "ppppiiiiiffplpipp"},
+    "elementwise": {"mlr_rms_norm": "ppppiifiip", "mlr_rope_kv_write": "pppppppiiiiiiip"},
+    "attention_tcgen05": {"mlr_attention_prefill_tcgen05": "ppppppppppp" "iiiiiiiii" "fi" "ppp" "l" "pip"},
+}
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
+_declared: dict[str, ctypes.CDLL] = {}
+
+
+def _declared_library(name: str) -> ctypes.CDLL:
+    """The library with the prototypes above."""
+    library = build.load_library(name)
+    if _declared.get(name) is not library:
+        for symbol, codes in _PROTOTYPES[name].items():
+            getattr(library, symbol).argtypes = [_CTYPES[code] for code in codes]
+        _declared[name] = library
+    return library
+
+
+def _address(tensor: torch.Tensor | None) -> int | None:
+    return None if tensor is None else tensor.data_ptr()
+
+
+def _raw_stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 @dataclass
@@ -322,10 +356,9 @@ class CudaOps:
             if weight.shape[0] != x.shape[1]:
                 raise KernelError(f"norm weight has {weight.shape[0]} entries, rows have {x.shape[1]}")
         out = torch.empty_like(x)
-        lib = build.load_library("elementwise")
-        _check(lib.mlr_rms_norm(_ptr(x), _ptr(delta), _ptr(weight), _ptr(out), x.shape[0], x.shape[1],
-                                ctypes.c_float(eps), _code(x.dtype),
-                                _code(x.dtype if weight is None else weight.dtype), _stream()), "rms_norm")
+        _check(_declared_library("elementwise").mlr_rms_norm(
+            x.data_ptr(), _address(delta), _address(weight), out.data_ptr(), x.shape[0], x.shape[1], eps, _code(x.dtype),
+            _code(x.dtype if weight is None else weight.dtype), _raw_stream()), "rms_norm")
         return out
 
     def swiglu(self, gate_up: torch.Tensor, block: int | None = None) -> torch.Tensor:
@@ -396,12 +429,11 @@ class CudaOps:
         if k_pool.shape != v_pool.shape or k_pool.shape[1] != num_kv_heads or k_pool.shape[3] != head_dim:
             raise KernelError(f"page pools have shape {tuple(k_pool.shape)}, expected "
                               f"[pages, {num_kv_heads}, page_size, {head_dim}]")
-        q = torch.empty((tokens, num_heads * head_dim), dtype=qkv.dtype, device=qkv.device)
-        lib = build.load_library("elementwise")
-        _check(lib.mlr_rope_kv_write(_ptr(qkv), _ptr(positions), _ptr(inv_freq), _ptr(slots), _ptr(q),
-                                     _ptr(k_pool), _ptr(v_pool), tokens, num_heads, num_kv_heads,
-                                     head_dim, k_pool.shape[2], int(bool(write_kv)), _code(qkv.dtype),
-                                     _stream()), "rope_kv_write")
+        q = qkv.new_empty((tokens, num_heads * head_dim))
+        _check(_declared_library("elementwise").mlr_rope_kv_write(
+            qkv.data_ptr(), positions.data_ptr(), inv_freq.data_ptr(), slots.data_ptr(), q.data_ptr(), k_pool.data_ptr(),
+            v_pool.data_ptr(), tokens, num_heads, num_kv_heads, head_dim, k_pool.shape[2], int(bool(write_kv)), _code(qkv.dtype),
+            _raw_stream()), "rope_kv_write")
         return q
 
     # ------------------------------------------------------------------ resident tables and slot records
@@ -536,6 +568,8 @@ class CudaOps:
         measured at 1152 x 896 and 32 rows, 3.0 against 7.1 us; a batch-32 decode step 1.50 -> 1.44 ms.
         (At 64 rows it wins alone, 6.3 against 8.4 us, but loses inside a step: 1.96 -> 2.20 ms.)"""
         rows = x.shape[0]
+        if rows > self.SKINNY_ROWS and rows > self.SKINNY_ROWS_SMALL_WEIGHT:
+            return False
         # a weight with a 128-row tile for every SM keeps the tcgen05 kernel's tensor-memory tiles busy
         if (not self.use_skinny or weight.shape[0] >= 128 * self.sm_count(x.device)
                 or (swiglu and x.shape[1] > 2048)):
@@ -590,19 +624,16 @@ class CudaOps:
     def _linear_tcgen05(self, x, weight, bias, out_dtype, swiglu=False, gate=(0.0, 0.0)):
         M, K = x.shape
         N = weight.shape[0]
-        lib = build.load_library("gemm_tcgen05")
-        lib.mlr_gemm_tcgen05_plan.restype = ctypes.c_longlong
-        splits, tiles = ctypes.c_int(0), ctypes.c_int(0)
-        need = lib.mlr_gemm_tcgen05_plan(M, N, K, int(swiglu), ctypes.byref(splits), ctypes.byref(tiles))
         space = self._workspace(x.device)
-        if need > space["gemm_scratch"].numel() or (splits.value > 1 and tiles.value > space["gemm_counters"].numel()):
+        out = x.new_empty((M, N // 2 if swiglu else N), dtype=out_dtype)
+        scratch, counters = space["gemm_scratch"], space["gemm_counters"]
+        status = _declared_library("gemm_tcgen05").mlr_gemm_tcgen05(
+            x.data_ptr(), weight.data_ptr(), _address(bias), out.data_ptr(), M, N, K, int(out_dtype == torch.float32), int(swiglu),
+            gate[0], gate[1], scratch.data_ptr(), self.GEMM_SCRATCH_BYTES, counters.data_ptr(), self.GEMM_COUNTERS,
+            space["error_word"].data_ptr(), _raw_stream())
+        if status == _NO_ROOM:      # its partial tiles do not fit the scratch memory
             return None
-        out = torch.empty((M, N // 2 if swiglu else N), dtype=out_dtype, device=x.device)
-        _check(lib.mlr_gemm_tcgen05(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), M, N, K,
-                                    int(out_dtype == torch.float32), int(swiglu), ctypes.c_float(gate[0]),
-                                    ctypes.c_float(gate[1]), _ptr(space["gemm_scratch"]),
-                                    _ptr(space["gemm_counters"]), _ptr(space["error_word"]), _stream()),
-               "linear (tcgen05)")
+        _check(status, "linear (tcgen05)")
         return out
 
     # Elements of a weight from which 32-bit products run on the tensor cores in bfloat16 parts; a rule on the weight alone, so that a
@@ -695,14 +726,14 @@ class CudaOps:
                               f"[pages, {num_kv_heads}, page_size, {head_dim}] and [.., {value_dim}]")
         if "tile_seg" not in batch.plan:
             raise KernelError("the batch carries no attention work lists (plan_attention)")
-        out = torch.empty((q.shape[0], num_heads * value_dim), dtype=q.dtype, device=q.device)
+        out = q.new_empty((q.shape[0], num_heads * value_dim))
         plan, counts = batch.plan, batch.counts
         generic_tiles = counts["tiles"]
         group = num_heads // num_kv_heads
         page_size = k_pool.shape[2]
         paged_by_tma = page_size >= 8 and page_size & (page_size - 1) == 0
         common = (_ptr(batch.seg_q_start), _ptr(batch.seg_q_len), _ptr(batch.seg_pos0), _ptr(batch.block_table),
-                  _ptr(batch.seg_slot), batch.block_table.shape[1])
+                  _ptr(batch.seg_slot), batch.block_table.shape[1])      # declared entry points take them too
         equal_sizes = value_dim == head_dim
         if (self.use_mma_attention and equal_sizes and q.dtype == torch.bfloat16 and head_dim in (64, 128) and group <= 16
                 and batch.num_decode * num_kv_heads <= self.ATTENTION_COUNTERS):
@@ -712,14 +743,14 @@ class CudaOps:
             if counts["big"] > 0 and self.use_tcgen05_attention and paged_by_tma:
                 # S = Q K^T and P V on tcgen05 with tensor-memory accumulators
                 space = self._workspace(q.device)
-                _check(build.load_library("attention_tcgen05").mlr_attention_prefill_tcgen05(
-                    _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(plan["big_tile_seg"]),
-                    _ptr(plan["big_tile_row0"]), *common, counts["big"], q.shape[0], num_heads,
-                    num_kv_heads, head_dim, page_size, k_pool.shape[0], int(window or 0), ctypes.c_float(scale),
-                    int(batch.max_kv_len), _ptr(space["prefill_queue"]), _ptr(space["error_word"]),
-                    _ptr(space["prefill_scratch"] if self.split_prefill_items else None),
-                    ctypes.c_longlong(space["prefill_scratch"].numel()),
-                    _ptr(space["prefill_counters"]), space["prefill_counters"].numel(), _stream()),
+                scratch, counters = space["prefill_scratch"], space["prefill_counters"]
+                _check(_declared_library("attention_tcgen05").mlr_attention_prefill_tcgen05(
+                    q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(), plan["big_tile_seg"].data_ptr(),
+                    plan["big_tile_row0"].data_ptr(), *common, counts["big"], q.shape[0], num_heads,
+                    num_kv_heads, head_dim, page_size, k_pool.shape[0], int(window or 0), scale,
+                    int(batch.max_kv_len), space["prefill_queue"].data_ptr(), space["error_word"].data_ptr(),
+                    scratch.data_ptr() if self.split_prefill_items else None, scratch.numel(),
+                    counters.data_ptr(), counters.numel(), _raw_stream()),
                     "prefill attention (tcgen05)")
             elif counts["wide"] > 0 and self.use_tma_attention and paged_by_tma:
                 space = self._workspace(q.device)
