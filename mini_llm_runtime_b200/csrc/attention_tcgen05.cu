@@ -76,7 +76,7 @@ struct FaShape {
 // (a map is a head of its own here: head = 2 * head + map; keys hold the maps side by side; the normalised rows
 // leave as float32, and the first `keep` positions stay visible beside the window).  The maps' walk over the keys is
 // the softmax threads' like any head's; on mma.sync it was bound by fragment loads, one query tile's K and V fetched per
-// (head, map), and by a combination of 32 CTAs: 2,048 rows, window 1,024, 7 heads of 2 x 64 with values of 128: 290 -> 55 us,
+// (head, map), and by a combination of 32 CTAs: 2,048 rows, window 1,024, 7 heads of 2 x 64 with values of 128: 290 -> 50 us,
 // 16 heads: 597 -> 81 us.
 enum FaMode { FA_PLAIN, FA_SHAPED, FA_MAPS };
 
@@ -817,35 +817,34 @@ struct FaSizes {
   static constexpr int D = KEY_SIZE, DV = VALUE_SIZE;
 };
 
-// o = a1 - lambda * a2, o / rms(o) * out_scale, a warp per row.  grid: (tiles, FA_ROWS / 4)
+// o = a1 - lambda * a2, o / rms(o) * out_scale, a warp per row and head.  A warp that took a row's heads one after the other waited for each:
+// 2,048 rows of 7 heads of 128, from cold caches, 9.5 us, 6.8 now (22 MB); the whole attention 55.5 / 50.3.  grid: (tiles * heads, FA_ROWS / 4)
 __global__ void __launch_bounds__(128)
 combine_maps_kernel(const float* maps, bf16* __restrict__ out, const int* __restrict__ tile_seg, const int* __restrict__ tile_row0,
                     const int* __restrict__ seg_q_start, const int* __restrict__ seg_q_len, int heads, int vdim, float lambda,
                     float eps, float out_scale) {
   pdl_trigger();
-  pdl_wait();
-  const int tile = blockIdx.x, seg = tile_seg[tile], r = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / heads, head = blockIdx.x - tile * heads, seg = tile_seg[tile];
+  const int r = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (tile_row0[tile] + r >= seg_q_len[seg]) return;
   const size_t row = (size_t)(seg_q_start[seg] + tile_row0[tile] + r);
-#pragma unroll 4
-  for (int head = 0; head < heads; ++head) {
-    const float* a1 = maps + (row * heads + head) * 2 * vdim + lane * 2;
-    float2 o[2];
-    float sq = 0.f;
+  const float* a1 = maps + (row * heads + head) * 2 * vdim + lane * 2;
+  pdl_wait();
+  float2 o[2];
+  float sq = 0.f;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h * 64 >= vdim) break;
-      const float2 x = __ldcg(reinterpret_cast<const float2*>(a1 + h * 64)), y = __ldcg(reinterpret_cast<const float2*>(a1 + vdim + h * 64));
-      o[h] = make_float2(x.x - lambda * y.x, x.y - lambda * y.y);
-      sq = fmaf(o[h].x, o[h].x, fmaf(o[h].y, o[h].y, sq));
-    }
-    const float factor = out_scale / sqrtf(warp_sum(sq) / (float)vdim + eps);
+  for (int h = 0; h < 2; ++h) {
+    if (h * 64 >= vdim) break;
+    const float2 x = __ldcg(reinterpret_cast<const float2*>(a1 + h * 64)), y = __ldcg(reinterpret_cast<const float2*>(a1 + vdim + h * 64));
+    o[h] = make_float2(x.x - lambda * y.x, x.y - lambda * y.y);
+    sq = fmaf(o[h].x, o[h].x, fmaf(o[h].y, o[h].y, sq));
+  }
+  const float factor = out_scale / sqrtf(warp_sum(sq) / (float)vdim + eps);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h * 64 >= vdim) break;
-      *reinterpret_cast<__nv_bfloat162*>(out + (row * heads + head) * vdim + h * 64 + lane * 2) =
-          __floats2bfloat162_rn(o[h].x * factor, o[h].y * factor);
-    }
+  for (int h = 0; h < 2; ++h) {
+    if (h * 64 >= vdim) break;
+    *reinterpret_cast<__nv_bfloat162*>(out + (row * heads + head) * vdim + h * 64 + lane * 2) =
+        __floats2bfloat162_rn(o[h].x * factor, o[h].y * factor);
   }
 }
 
@@ -884,7 +883,7 @@ MLR_EXPORT int mlr_attention_diff_prefill_tcgen05(
   const int status = dim == 64 ? (vdim == 64 ? launch(FaSizes<64, 64>()) : launch(FaSizes<64, 128>()))
                                : (vdim == 64 ? launch(FaSizes<128, 64>()) : launch(FaSizes<128, 128>()));
   if (status != MLR_OK) return status;
-  launch_kernel(combine_maps_kernel, dim3(tiles, FA_ROWS / 4), dim3(128), 0, stream, (const float*)maps, (bf16*)out, tile_seg,
+  launch_kernel(combine_maps_kernel, dim3(tiles * heads, FA_ROWS / 4), dim3(128), 0, stream, (const float*)maps, (bf16*)out, tile_seg,
                 tile_row0, seg_q_start, seg_q_len, heads, vdim, lambda, eps, out_scale);
   return launch_status();
 }
