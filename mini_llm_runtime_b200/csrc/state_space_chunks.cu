@@ -306,10 +306,11 @@ space_local_kernel(SpaceArgs p) {
   if (chunk == 0) read_state<N>(p, s_b, shared, first, count, head);
 }
 
-// A thread owns four neighbouring entries and takes the chunks of its segment in order; BATCH chunks are asked for together.
+// A thread owns four neighbouring entries and takes the chunks of its segment in order; BATCH chunks are asked for together (8: 126.4 us
+// for 1,531 + 77 + 1 + 439 rows of 32 heads, all launches; 16: 125.4).
 __global__ void __launch_bounds__(256)
 space_carry_kernel(SpaceArgs p, int cells) {
-  constexpr int BATCH = 8;
+  constexpr int BATCH = 16;
   pdl_trigger();
   pdl_wait();
   const auto [seg, which, length, start, slot] = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
