@@ -8,7 +8,7 @@
 // The columns of S are independent of each other given u, so a thread group of SL lanes owns a few columns
 // and splits the key channels among its lanes.
 //
-// Several tokens are taken at once (TB = 4 in long segments).  Within such a block the state before it, S0,
+// Several tokens are taken at once (TB = 4 in segments of more than one row; delta_chunks.cu takes the long ones).  Within such a block the state before it, S0,
 // enters every token's reads linearly: with G_t = g_1 .. g_t,
 //
 //   u_t = beta_t (v_t - G_t S0^T k_t - sum_{s<t} (G_t / G_s) (k_s . k_t) u_s)

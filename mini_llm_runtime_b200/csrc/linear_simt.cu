@@ -1,6 +1,6 @@
 // y[M,N] = x[M,K] * W[N,K]^T (+ bias[N]) on the CUDA cores, float32 multiply-add throughout.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores, no TF32) and the fallback
+// This is the matrix product of the true 32-bit path (no TF32) for weights that linear_split.cu does not take, and the fallback
 // of the bfloat16 path for shapes the tensor-core kernel refuses.  Weights keep the checkpoint's
 // [out, in] layout, as the reference's F.linear calls do (qwen_model_runner.py:88-102,183,215-217).
 //
