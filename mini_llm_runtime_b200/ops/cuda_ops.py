@@ -1992,10 +1992,12 @@ class CudaOps:
 
     # ------------------------------------------------------------------ gated delta rule
     use_delta_chunks = True
-    # Rows from which a request's portion goes in chunks: three launches, of which the first alone takes 20 us.  In us from a flushed L2,
-    # token by token / in chunks, 14 heads of 64 x 64: 128 rows 26 / 32, 256 38 / 40, 384 50 / 42, 1,024 112 / 60, 2,048 214 / 99; 32 heads of
-    # 128 x 64: 128 rows 36 / 52, 256 56 / 58, 384 75 / 65, 1,024 181 / 103, 2,048 346 / 202.
-    DELTA_CHUNK_ROWS = 288
+    # Rows from which a request's portion goes in chunks, whatever else is in the step: three launches, of which the first alone takes 20 us,
+    # in front of the one for shorter portions.  In us, token by token / in chunks, 14 heads of 64 x 64: 256 rows 38 / 40, 384 50 / 42, 512 62 / 48,
+    # 1,024 112 / 60, 2,048 214 / 99; 32 heads of 128 x 64: 256 rows 56 / 58, 384 75 / 65, 512 95 / 71, 1,024 181 / 103, 2,048 346 / 202.  Alone they
+    # pay from 288 rows on, but beside other portions of a few hundred rows, which take their time all the same, they do not: 281, 76, 9, 324,
+    # 127 and 176 rows 130 token by token, 153 with the 324 in chunks.
+    DELTA_CHUNK_ROWS = 512
 
     def delta_rule_scan(self, q, k, v, a, b, dt_bias, A_log, state, ctx, heads: int, kv_heads: int, dim: int, vdim: int,
                         unit_eps: float) -> torch.Tensor:
