@@ -8,12 +8,17 @@
 // delta_chain_kernel   the chunks of a (segment, head) one after the other, 16 value channels per CTA; leaves every chunk's S and u
 // delta_read_kernel    all chunks at once: o
 //
-// The products of the last two run on the tensor cores (mma.sync) in 32 bits: operands in three bfloat16 parts, six of the nine
-// products (the rest is below 2^-26), the leading product and the small ones in sums of their own, at most 64 k long (the tensor cores'
-// sums drop bits at every step), added in float32.  Decays are products throughout: nothing divides, they may be zero.
+// Products run on the tensor cores (mma.sync) in 32 bits: operands in three bfloat16 parts, six of the nine products (the rest is below
+// 2^-26), the leading product and the small ones in sums of their own, at most 64 k long (the tensor cores' sums drop bits at every
+// step: with_dropped), added in float32.  Decays are products throughout: nothing divides, they may be zero.
 //
-// Measured (B200), token by token / in chunks: 2,048 rows of 32 heads of 128 x 64 340 / 188 us (solve 60, chain 78, read 43), of 14 heads of
-// 64 x 64 207 / 92; error against 64 bits 1.2e-7 / 1.6e-7.  The first and the last kernel are bound by instructions (splitting operands,
+// Roundings that every output sees are saved: norms, decays and P are computed in 64 bits and rounded once, beta v - G .. and u's share of
+// the state are each one rounding.  Error against 64 bits (2-norm, outputs / states, means of four inputs), token by token, here without and
+// with all that, in 1e-7: 2,048 rows of 32 heads of 128 x 64 1.21 / 1.24, 1.65 / 1.25, 1.09 / 1.11; 14 heads of 64 x 64 1.29 / 1.27, 1.84 / 1.49,
+// 1.11 / 1.12.  It costs 12 us of the 32 heads' 212, 6 of the 14 heads' 105.
+//
+// Measured (B200), token by token / in chunks: 2,048 rows of 32 heads of 128 x 64 340 / 203 us, of 14 heads of 64 x 64 207 / 97 (188 and 92
+// before those roundings were saved: solve 60, chain 78, read 43).  The first and the last kernel are bound by instructions (splitting operands,
 // decays) and shared memory, the chain by the latency of its steps, 4,500 cycles per chunk, of which 1,900 are MMAs.
 //
 // In the chain four warps issue MMAs, each with 16 channels x a quarter of dim of the state in its registers (as accumulators, whose
@@ -129,6 +134,12 @@ __device__ __forceinline__ void add_products(float (&lead)[2 * PAIRS][4], float 
         }
   }
 }
+// A tensor core's sum is cut off, not rounded, at every step.  What that took from `lead` is given back on average, as `share` halves of the last
+// place's unit (one for sums over the key channels, of steps that mostly agree in sign, three quarters for the others, found by the errors
+// above), with the sum of the small products.
+__device__ __forceinline__ float with_dropped(float lead, float low, float share) {
+  return fmaf(__uint_as_float(__float_as_uint(lead) & 0xff800000u), share * 5.9604644775390625e-8f, low);      // its sign and power of two
+}
 template <int N>
 __device__ __forceinline__ void clear(float (&x)[N][4]) {
 #pragma unroll
@@ -157,7 +168,8 @@ delta_solve_kernel(DeltaChunkArgs p) {
   bf16* keys = reinterpret_cast<bf16*>(solve_shared);                                        // in parts
   float* queries = reinterpret_cast<float*>(solve_shared + 3 * Shape::KEY_APART * sizeof(bf16));
   float *kk = reinterpret_cast<float*>(solve_shared), *qk = kk + CHUNK * SQUARE_PITCH, *matrix = qk + CHUNK * SQUARE_PITCH;
-  __shared__ float rk[CHUNK], rq[CHUNK], decay[2][CHUNK], beta[2][CHUNK], upto[2][CHUNK];
+  __shared__ double rq[CHUNK];
+  __shared__ float rk[CHUNK], decay[2][CHUNK], beta[2][CHUNK], upto[2][CHUNK];
   pdl_trigger();
   pdl_wait();
   const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.x);
@@ -181,11 +193,13 @@ delta_solve_kernel(DeltaChunkArgs p) {
       for (int i = 0; i < PIECES; ++i) {
         const int idx = t + i * 256, row = idx / ROW_LANES, d = idx % ROW_LANES * 4;
         const float4 x = piece[i];
-        float sum = fmaf(x.x, x.x, x.y * x.y) + fmaf(x.z, x.z, x.w * x.w);
+        double sum = fmaf(x.x, x.x, x.y * x.y) + fmaf(x.z, x.z, x.w * x.w);
 #pragma unroll
         for (int offset = ROW_LANES / 2; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
-        const float inverse = row < count ? 1.f / sqrtf(sum + p.unit_eps) : 0.f;      // rows behind the segment are nothing, whatever unit_eps
-        if (d == 0) (which ? rq : rk)[row] = which ? p.q_scale * inverse : inverse;
+        const double inverse = row < count ? rsqrt(sum + p.unit_eps) : 0.;      // rows behind the segment are nothing, whatever unit_eps
+        if (d == 0) {
+          if (which) rq[row] = p.q_scale * inverse; else rk[row] = (float)inverse;
+        }
         if (which) {
           *reinterpret_cast<float4*>(queries + row * Shape::QUERY_PITCH + d) = x;
         } else {
@@ -232,7 +246,10 @@ delta_solve_kernel(DeltaChunkArgs p) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) total[j][e] += lead[j][e];
+          for (int e = 0; e < 4; ++e) {
+            total[j][e] += lead[j][e];
+            low[j][e] = with_dropped(lead[j][e], low[j][e], 1.f);
+          }
         clear(lead);
       }
     }
@@ -262,20 +279,24 @@ delta_solve_kernel(DeltaChunkArgs p) {
     __syncthreads();      // also: kk and qk are there, the heads before are done
     float* A = matrix + half * CHUNK * SQUARE_PITCH;
     const float own = rk[s];
-    float since = 1.f;      // D(row, s)
+    double since = 1.;      // D(row, s)
     float* P = p.P + at * DC_SQUARE;
     {      // two threads per column, one for the earlier rows and one for the later
       const int row0 = row_half * HALF;
-#pragma unroll 8
-      for (int row = 1; row < row0; ++row)
-        if (row > s) since *= decay[half][row];
+      if (row_half == 1) {      // four chains of products instead of one: 2,048 rows of 32 heads 218 -> 212 us
+        double chain[4] = {1., 1., 1., 1.};
+#pragma unroll
+        for (int row = 0; row < HALF; ++row)
+          if (row > s) chain[row & 3] *= decay[half][row];
+        since = (chain[0] * chain[1]) * (chain[2] * chain[3]);
+      }
 #pragma unroll 8
       for (int row = row0; row < row0 + HALF; ++row) {
         if (row > s) since *= decay[half][row];
-        const float weight = row >= s ? since * own : 0.f;
-        if (mine) P[row * CHUNK + s] = row >= s ? weight * rq[row] * qk[row * SQUARE_PITCH + s] : 0.f;
-        A[row * SQUARE_PITCH + s] = row > s ? weight * rk[row] * beta[half][row] * kk[row * SQUARE_PITCH + s] : 0.f;
-        if (s == 0) upto[half][row] = decay[half][0] * since;
+        const double weight = since * own;
+        if (mine) P[row * CHUNK + s] = row >= s ? (float)(weight * rq[row] * qk[row * SQUARE_PITCH + s]) : 0.f;
+        A[row * SQUARE_PITCH + s] = row > s ? (float)weight * rk[row] * beta[half][row] * kk[row * SQUARE_PITCH + s] : 0.f;
+        if (s == 0) upto[half][row] = (float)(decay[half][0] * since);
       }
     }
     __syncthreads();
@@ -283,8 +304,8 @@ delta_solve_kernel(DeltaChunkArgs p) {
       float* factors = p.factors + at * DC_FACTORS;
       factors[s] = step * upto[half][s] * own;
       factors[CHUNK + s] = step;
-      factors[2 * CHUNK + s] = since * own;
-      factors[3 * CHUNK + s] = upto[half][s] * rq[s];
+      factors[2 * CHUNK + s] = (float)(since * own);
+      factors[3 * CHUNK + s] = (float)(upto[half][s] * rq[s]);
       if (s == 0) p.decays[at] = upto[half][CHUNK - 1];
     }
     float x[HALF];      // column s of its triangle's inverse
@@ -368,7 +389,7 @@ struct ChainShape {
   static constexpr int KEY_PITCH = D + 8, KEY_APART = CHUNK * KEY_PITCH, T_APART = CHUNK * DC_PITCH, LEFT_APART = DC_COLS * DC_PITCH;
   static constexpr size_t KEYS = 3 * KEY_APART * sizeof(bf16), SQUARE = 3 * T_APART * sizeof(bf16);
   static constexpr size_t VALUES = DC_COLS * DC_PITCH * sizeof(float), ROW = CHUNK * sizeof(float);
-  static constexpr size_t BUFFER = KEYS + SQUARE + VALUES + 2 * ROW;
+  static constexpr size_t BUFFER = KEYS + SQUARE + VALUES + 3 * ROW;
   static constexpr size_t LEFT = 3 * LEFT_APART * sizeof(bf16);
   static constexpr size_t SHARED = 2 * BUFFER + 4 * VALUES + 2 * LEFT + 4 * DC_COLS * sizeof(int);      // the four warps' sums, R and u in parts
   static_assert(KEYS % 16 == 0 && SQUARE % 16 == 0 && BUFFER % 16 == 0, "bulk copies");
@@ -425,7 +446,7 @@ delta_chain_kernel(DeltaChunkArgs p) {
   // The last four warps fetch: parts of keys and T by a bulk copy each, values and factors through registers, asked for a chunk before.
   constexpr int V_PIECES = CHUNK * DC_COLS / 4 / 128;
   float4 v_piece[V_PIECES];
-  float v_factor[V_PIECES], factor;
+  float factor, beta;
   const int i0 = threadIdx.x - 128;
   auto copy = [&](int chunk, int which) {
     const size_t place = (size_t)(first_chunk + chunk);
@@ -445,9 +466,9 @@ delta_chain_kernel(DeltaChunkArgs p) {
       const int idx = i0 + n * 128, row = idx / (DC_COLS / 4), c = idx % (DC_COLS / 4) * 4;
       v_piece[n] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (row < count) v_piece[n] = __ldcg(reinterpret_cast<const float4*>(p.v + (size_t)(row0 + row) * p.v_stride + (size_t)head * V + col0 + c));
-      v_factor[n] = __ldcg(factors + CHUNK + row);
     }
-    factor = __ldcg(factors + (i0 < CHUNK ? i0 : i0 + CHUNK));      // beta G rk | D(last, .) rk
+    factor = __ldcg(factors + (i0 < CHUNK ? i0 : i0 + CHUNK));      // beta G rk | D(last, .) rk | beta
+    beta = __ldcg(factors + CHUNK + i0 % CHUNK);
   };
   auto put = [&](int which) {
     float *values = values_of(which), *row_factor = values + DC_COLS * DC_PITCH;
@@ -455,12 +476,13 @@ delta_chain_kernel(DeltaChunkArgs p) {
     for (int n = 0; n < V_PIECES; ++n) {
       const int idx = i0 + n * 128, row = idx / (DC_COLS / 4), c = idx % (DC_COLS / 4) * 4;
       const float4 x = v_piece[n];
-      values[c * DC_PITCH + row] = v_factor[n] * x.x;
-      values[(c + 1) * DC_PITCH + row] = v_factor[n] * x.y;
-      values[(c + 2) * DC_PITCH + row] = v_factor[n] * x.z;
-      values[(c + 3) * DC_PITCH + row] = v_factor[n] * x.w;
+      values[c * DC_PITCH + row] = x.x;
+      values[(c + 1) * DC_PITCH + row] = x.y;
+      values[(c + 2) * DC_PITCH + row] = x.z;
+      values[(c + 3) * DC_PITCH + row] = x.w;
     }
     row_factor[i0] = factor;
+    if (i0 < CHUNK) row_factor[2 * CHUNK + i0] = beta;
   };
   // The fetching warps wait for the copies; the block's barrier behind it tells the others, who would pay for a look of their own.
   bool gave_up = false;
@@ -515,8 +537,11 @@ delta_chain_kernel(DeltaChunkArgs p) {
         float* mine = sums + warp * DC_COLS * DC_PITCH;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          *reinterpret_cast<float2*>(mine + r * DC_PITCH + j * 8 + c2) = make_float2(lead[j][0] + low[j][0], lead[j][1] + low[j][1]);
-          *reinterpret_cast<float2*>(mine + (r + 8) * DC_PITCH + j * 8 + c2) = make_float2(lead[j][2] + low[j][2], lead[j][3] + low[j][3]);
+          float z[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) z[e] = lead[j][e] + with_dropped(lead[j][e], low[j][e], 0.75f);
+          *reinterpret_cast<float2*>(mine + r * DC_PITCH + j * 8 + c2) = make_float2(z[0], z[1]);
+          *reinterpret_cast<float2*>(mine + (r + 8) * DC_PITCH + j * 8 + c2) = make_float2(z[2], z[3]);
         }
       }
       // the state before the chunk, for the outputs
@@ -533,7 +558,7 @@ delta_chain_kernel(DeltaChunkArgs p) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int t = warp * 16 + j * 8 + c2;
-          const float2 f = *reinterpret_cast<const float2*>(row_factor + t);
+          const float2 f = *reinterpret_cast<const float2*>(row_factor + t), beta = *reinterpret_cast<const float2*>(row_factor + 2 * CHUNK + t);
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const int cell = (r + 8 * i) * DC_PITCH + t;
@@ -545,8 +570,8 @@ delta_chain_kernel(DeltaChunkArgs p) {
               z.y += add.y;
             }
             const float2 v = *reinterpret_cast<const float2*>(values + cell);
-            R[j][2 * i] = fmaf(-f.x, z.x, v.x);
-            R[j][2 * i + 1] = fmaf(-f.y, z.y, v.y);
+            R[j][2 * i] = fmaf(beta.x, v.x, -f.x * z.x);
+            R[j][2 * i + 1] = fmaf(beta.y, v.y, -f.y * z.y);
           }
         }
         if (take_out(R, warp * 16 + c2, broken)) earliest_of_row(broken);
@@ -592,19 +617,21 @@ delta_chain_kernel(DeltaChunkArgs p) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int t = warp * 16 + j * 8 + c2;
+          const float2 f = *reinterpret_cast<const float2*>(row_factor + CHUNK + t);
           float total[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            total[e] = part[0][j][e];
+            float low = part[0][j][e], lead = part[5][j][e];
 #pragma unroll
-            for (int q = 1; q < 6; ++q) total[e] += part[q][j][e];      // the leading product last
-            if (t + (e & 1) >= broken[e >> 1]) total[e] = NAN;
+            for (int q = 1; q < 5; ++q) low += part[q][j][e];
+            low = with_dropped(lead, low, 0.75f);
+            if (t + (e & 1) >= broken[e >> 1]) lead = NAN;
+            const float factor = e & 1 ? f.y : f.x;
+            total[e] = lead + low;
+            scaled[j][e] = fmaf(lead, factor, low * factor);
           }
           *reinterpret_cast<float2*>(u + r * CHUNK + t) = make_float2(total[0], total[1]);
           *reinterpret_cast<float2*>(u + (r + 8) * CHUNK + t) = make_float2(total[2], total[3]);
-          const float2 f = *reinterpret_cast<const float2*>(row_factor + CHUNK + t);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) scaled[j][e] = total[e] * (e & 1 ? f.y : f.x);
         }
         store_operand(u_parts, warp * 16, scaled[0], scaled[1], r, c2);
       }
@@ -623,7 +650,7 @@ delta_chain_kernel(DeltaChunkArgs p) {
 #pragma unroll
         for (int j = 0; j < TILES; ++j)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) S[j][e] = fmaf(last, S[j][e], lead[j][e] + low[j][e]);
+          for (int e = 0; e < 4; ++e) S[j][e] = fmaf(last, S[j][e], lead[j][e] + with_dropped(lead[j][e], low[j][e], 0.75f));
       }
     }
     __syncthreads();      // the next chunk's tiles are there, this one's are read
@@ -693,7 +720,10 @@ delta_read_kernel(DeltaChunkArgs p) {
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) total[j][e] += lead[j][e];
+      for (int e = 0; e < 4; ++e) {
+        total[j][e] += lead[j][e];
+        low[j][e] = with_dropped(lead[j][e], low[j][e], 1.f);
+      }
     clear(lead);
   };
   clear(total);
@@ -750,7 +780,7 @@ delta_read_kernel(DeltaChunkArgs p) {
     for (int e = 0; e < 4; ++e) {
       const int t = j * 8 + c2 + (e & 1);
       if (t < count)
-        p.y[((size_t)(first + t) * p.heads + head) * V + col0 + r + (e >> 1) * 8] = t < broken[e >> 1] ? total[j][e] + (lead[j][e] + low[j][e]) : NAN;
+        p.y[((size_t)(first + t) * p.heads + head) * V + col0 + r + (e >> 1) * 8] = t < broken[e >> 1] ? total[j][e] + (lead[j][e] + with_dropped(lead[j][e], low[j][e], 1.f)) : NAN;
     }
 }
 

@@ -529,3 +529,24 @@ def test_a_token_that_is_no_number_leaves_the_tokens_of_a_delta_rule_before_it_a
         results.append(cuda().delta_rule_scan(*(given[name].to(DEVICE) for name in "qkvab"), bias, a_log, state, ctx, heads, kv_heads, dim,
                                               vdim, 1e-6).cpu())
     assert torch.equal(results[0][:at], results[1][:at])
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 4, 128), (8, 4, 64)])
+def test_delta_rule_in_chunks_is_no_further_from_64_bits(heads, kv_heads, dim, monkeypatch):
+    """Inputs as behind a convolution's silu, whose keys have a common direction: the sums of their products grow, and with them what the
+    tensor cores cut off.  The states' errors are sums of few roundings and differ from draw to draw, by a tenth in the mean of two."""
+    vdim, rows = 64, 1024
+    errors = {True: [0.0, 0.0], False: [0.0, 0.0]}
+    for seed in (0, 20):
+        silu = lambda index, width: torch.nn.functional.silu(rnd(seed + index, rows, width))      # noqa: E731
+        inputs = (silu(1, kv_heads * dim), silu(2, kv_heads * dim), silu(3, heads * vdim), rnd(seed + 4, rows, heads), rnd(seed + 5, rows, heads),
+                  torch.rand(heads, generator=generator(seed + 6)) * 4 - 4, torch.rand(heads, generator=generator(seed + 7)) * 2.5)
+        ctx, want_state = segments([rows], [0]), torch.zeros(1, heads, vdim, dim, dtype=torch.float64)
+        want = FAKE.delta_rule_scan(*(t.double() for t in inputs), want_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
+        for chunks in errors:
+            monkeypatch.setattr(cuda(), "use_delta_chunks", chunks)
+            state = torch.zeros(1, heads, vdim, dim, device=DEVICE)
+            got = cuda().delta_rule_scan(*(t.to(DEVICE) for t in inputs), state, ctx, heads, kv_heads, dim, vdim, 1e-6)
+            for index, (a, b) in enumerate(((got, want), (state, want_state))):
+                errors[chunks][index] += float((a.double().cpu() - b).norm() / b.norm())
+    assert errors[True][0] <= errors[False][0] and errors[True][1] <= 1.1 * errors[False][1], errors
