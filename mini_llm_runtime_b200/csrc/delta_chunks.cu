@@ -50,6 +50,7 @@ struct DeltaChunkArgs {
   float* before;                        // [chunks, heads, vdim, dim]: S
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int segments, least, heads, kv_heads, vdim;
+  int first_chunk, chunks;              // of this round; scratch is indexed from the first on
   float unit_eps, q_scale;
   int* error_word;
 };
@@ -172,7 +173,7 @@ delta_solve_kernel(DeltaChunkArgs p) {
   __shared__ float rk[CHUNK], decay[2][CHUNK], beta[2][CHUNK], upto[2][CHUNK];
   pdl_trigger();
   pdl_wait();
-  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.x);
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, p.first_chunk + blockIdx.x);
   if (seg < 0) return;
   const int kv = blockIdx.y, first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -435,7 +436,10 @@ delta_chain_kernel(DeltaChunkArgs p) {
   if (segment.seg < 0) return;
   const int seg = segment.seg, length = segment.length, start = segment.start, slot = segment.slot;
   const int head = blockIdx.y, kv = head / (p.heads / p.kv_heads), col0 = blockIdx.z * DC_COLS, V = p.vdim;
-  const int chunks = (length + CHUNK - 1) / CHUNK, first_chunk = chunks_before(p.seg_q_len, seg, p.least);
+  // of the segment's chunks those of this round; `place` of the first chunk is where its numbers would lie in scratch
+  const int place = chunks_before(p.seg_q_len, seg, p.least) - p.first_chunk;
+  const int begin = max(0, -place), end = min((length + CHUNK - 1) / CHUNK, p.chunks - place);
+  if (begin >= end) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = lane >> 2, c2 = (lane & 3) * 2;      // of an accumulator: rows r and r + 8, columns c2 and c2 + 1
 
@@ -449,18 +453,18 @@ delta_chain_kernel(DeltaChunkArgs p) {
   float factor, beta;
   const int i0 = threadIdx.x - 128;
   auto copy = [&](int chunk, int which) {
-    const size_t place = (size_t)(first_chunk + chunk);
+    const size_t at = (size_t)(place + chunk);
     mbar_expect_tx(&there[which], (uint32_t)(Shape::KEYS + Shape::SQUARE));
     auto bulk = [&](bf16* dst, const bf16* src, size_t bytes) {
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                    ::"r"(shared_address(dst)), "l"(src), "r"((uint32_t)bytes), "r"(smem_u32(&there[which])) : "memory");
     };
-    bulk(keys_of(which), p.key_parts + (place * p.kv_heads + kv) * 3 * Shape::KEY_APART, Shape::KEYS);
-    bulk(square_of(which), p.T + (place * p.heads + head) * 3 * Shape::T_APART, Shape::SQUARE);
+    bulk(keys_of(which), p.key_parts + (at * p.kv_heads + kv) * 3 * Shape::KEY_APART, Shape::KEYS);
+    bulk(square_of(which), p.T + (at * p.heads + head) * 3 * Shape::T_APART, Shape::SQUARE);
   };
   auto ask = [&](int chunk) {
     const int row0 = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
-    const float* factors = p.factors + ((size_t)(first_chunk + chunk) * p.heads + head) * DC_FACTORS;
+    const float* factors = p.factors + ((size_t)(place + chunk) * p.heads + head) * DC_FACTORS;
 #pragma unroll
     for (int n = 0; n < V_PIECES; ++n) {
       const int idx = i0 + n * 128, row = idx / (DC_COLS / 4), c = idx % (DC_COLS / 4) * 4;
@@ -487,17 +491,17 @@ delta_chain_kernel(DeltaChunkArgs p) {
   // The fetching warps wait for the copies; the block's barrier behind it tells the others, who would pay for a look of their own.
   bool gave_up = false;
   auto arrived = [&](int chunk) {
-    if (!gave_up) gave_up = !mbar_wait(&there[chunk & 1], (chunk >> 1) & 1, p.error_word, 51);
+    if (!gave_up) gave_up = !mbar_wait(&there[(chunk - begin) & 1], ((chunk - begin) >> 1) & 1, p.error_word, 51);
   };
   float* state = p.states + ((size_t)slot * p.heads + head) * V * D + (size_t)col0 * D;
   float S[TILES][4];
   __syncthreads();      // the barriers are set up
   if (warp >= 4) {
-    if (i0 == 0) copy(0, 0);
-    ask(0);
+    if (i0 == 0) copy(begin, 0);
+    ask(begin);
     put(0);
-    if (chunks > 1) ask(1);
-    arrived(0);
+    if (begin + 1 < end) ask(begin + 1);
+    arrived(begin);
   } else {
 #pragma unroll
     for (int j = 0; j < TILES; ++j) {
@@ -508,20 +512,20 @@ delta_chain_kernel(DeltaChunkArgs p) {
   }
   __syncthreads();
 
-  for (int chunk = 0; chunk < chunks; ++chunk) {
-    const int which = chunk & 1;
+  for (int chunk = begin; chunk < end; ++chunk) {
+    const int which = (chunk - begin) & 1;
     if (warp >= 4) {
-      if (chunk + 1 < chunks) {
+      if (chunk + 1 < end) {
         if (i0 == 0) copy(chunk + 1, which ^ 1);
         put(which ^ 1);
       }
-      if (chunk + 2 < chunks) ask(chunk + 2);
-      if (chunk + 1 < chunks) arrived(chunk + 1);
+      if (chunk + 2 < end) ask(chunk + 2);
+      if (chunk + 1 < end) arrived(chunk + 1);
     } else {
 
       const bf16 *keys = keys_of(which), *square = square_of(which);
       const float *values = values_of(which), *row_factor = values + DC_COLS * DC_PITCH;
-      const size_t at = (size_t)(first_chunk + chunk) * p.heads + head;
+      const size_t at = (size_t)(place + chunk) * p.heads + head;
       const float last = __ldcg(p.decays + at);
       {      // this warp's share of S^T k_t
         float lead[8][4], low[8][4];
@@ -680,7 +684,7 @@ delta_read_kernel(DeltaChunkArgs p) {
   bf16 *queries = reinterpret_cast<bf16*>(read_shared), *pairs = queries + 3 * Shape::Q_APART;
   pdl_trigger();
   pdl_wait();
-  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, p.first_chunk + blockIdx.y);
   if (seg < 0) return;
   const int head = blockIdx.x, kv = head / (p.heads / p.kv_heads), V = p.vdim;
   const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
@@ -784,23 +788,42 @@ delta_read_kernel(DeltaChunkArgs p) {
     }
 }
 
+// Scratch of a chunk, in float32 numbers (two bfloat16 numbers count for one).
+inline long long scratch_of_chunk(int heads, int kv_heads, int dim, int vdim) {
+  return (long long)heads * (DC_SQUARE + 3ll * CHUNK * DC_PITCH / 2 + DC_FACTORS + 4 + (long long)vdim * (CHUNK + dim)) + (long long)kv_heads * (3ll * CHUNK * (dim + 8) / 2);
+}
+
+// Chunks that a round of launches takes: as many as have their scratch in DC_SCRATCH_BYTES, the rounds as even as can be.  The state goes from one
+// to the next where it lies.  8,192 rows of 32 heads of 128 x 64 in rounds of 64, 160 MB and without a bound (470 MB): 826, 811, 732 us, 4,096 rows
+// 417, 416, 388; this bound takes 4,400 of these rows at a time, 13,300 of 14 heads of 64 x 64.
+constexpr long long DC_SCRATCH_BYTES = 256ll << 20;
+inline int chunks_of_round(int chunks, int heads, int kv_heads, int dim, int vdim) {
+  const long long most = DC_SCRATCH_BYTES / 4 / scratch_of_chunk(heads, kv_heads, dim, vdim), room = most < 1 ? 1 : most;
+  const long long rounds = (chunks + room - 1) / room;
+  return (int)((chunks + rounds - 1) / rounds);
+}
+
 template <int D>
-int launch_delta_chunks(const DeltaChunkArgs& p, int rows, cudaStream_t stream) {
+int launch_delta_chunks(DeltaChunkArgs p, int rows, int chunks, cudaStream_t stream) {
   constexpr size_t solve_shared = SolveShape<D>::SHARED;
   static_assert(ChainShape<D>::SHARED <= 227 * 1024 && 2 * (ReadShape<D>::SHARED + 1024) <= 227 * 1024, "one and two CTAs per SM");
   cudaError_t err = cudaFuncSetAttribute(delta_solve_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_shared);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(delta_chain_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChainShape<D>::SHARED);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(delta_read_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ReadShape<D>::SHARED);
   if (err != cudaSuccess) return (int)err;
-  const unsigned chunks = (unsigned)long_chunks(rows, p.segments, p.least);
-  launch_kernel(delta_solve_kernel<D>, dim3(chunks, p.kv_heads), dim3(256), solve_shared, stream, p);
-  int status = launch_status();
-  if (status != MLR_OK) return status;
-  launch_kernel(delta_chain_kernel<D>, dim3((unsigned)long_segments(rows, p.segments, p.least), p.heads, p.vdim / DC_COLS), dim3(256),
-                ChainShape<D>::SHARED, stream, p);
-  if ((status = launch_status()) != MLR_OK) return status;
-  launch_kernel(delta_read_kernel<D>, dim3(p.heads, chunks, (p.vdim + 63) / 64), dim3(128), ReadShape<D>::SHARED, stream, p);
-  return launch_status();
+  const int round = p.chunks;
+  for (p.first_chunk = 0; p.first_chunk < chunks; p.first_chunk += round) {
+    p.chunks = chunks - p.first_chunk < round ? chunks - p.first_chunk : round;
+    launch_kernel(delta_solve_kernel<D>, dim3(p.chunks, p.kv_heads), dim3(256), solve_shared, stream, p);
+    int status = launch_status();
+    if (status != MLR_OK) return status;
+    launch_kernel(delta_chain_kernel<D>, dim3((unsigned)long_segments(rows, p.segments, p.least), p.heads, p.vdim / DC_COLS), dim3(256),
+                  ChainShape<D>::SHARED, stream, p);
+    if ((status = launch_status()) != MLR_OK) return status;
+    launch_kernel(delta_read_kernel<D>, dim3(p.heads, p.chunks, (p.vdim + 63) / 64), dim3(128), ReadShape<D>::SHARED, stream, p);
+    if ((status = launch_status()) != MLR_OK) return status;
+  }
+  return MLR_OK;
 }
 
 }  // namespace mlr
@@ -809,35 +832,38 @@ using namespace mlr;
 
 MLR_DEFINE_PDL_SWITCH
 
-// float32 scratch of a step, in numbers.
-MLR_EXPORT long long mlr_delta_chunk_scratch(int rows, int segments, int least_rows, int heads, int kv_heads, int dim, int vdim) {
-  const long long chunks = long_chunks(rows, segments, least_rows);      // two bfloat16 numbers count for one
-  return chunks * heads * (DC_SQUARE + 3ll * CHUNK * DC_PITCH / 2 + DC_FACTORS + 4 + (long long)vdim * (CHUNK + dim)) + chunks * kv_heads * (3ll * CHUNK * (dim + 8) / 2);
+// float32 scratch of a step whose long segments have `chunks` chunks, in numbers.
+MLR_EXPORT long long mlr_delta_chunk_scratch(int chunks, int heads, int kv_heads, int dim, int vdim) {
+  if (chunks <= 0 || heads <= 0 || kv_heads <= 0 || dim <= 0 || vdim <= 0) return 0;
+  return chunks_of_round(chunks, heads, kv_heads, dim, vdim) * scratch_of_chunk(heads, kv_heads, dim, vdim);
 }
 
-// As mlr_delta_rule_scan, for the segments of least_rows rows and more: dim 64 or 128, vdim a multiple of 16, every row of q, k and v, states
-// and scratch on 16-byte boundaries.  rows: the step's rows.  error_word: host-visible int that receives a code if a wait runs out.
+// As mlr_delta_rule_scan, for the segments of least_rows rows and more, which have `chunks` chunks of 64 rows or fewer in all: dim 64 or 128,
+// vdim a multiple of 16, every row of q, k and v, states and scratch on 16-byte boundaries.  rows: the step's rows.  error_word:
+// host-visible int that receives a code if a wait runs out.
 MLR_EXPORT int mlr_delta_rule_chunks(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
                                      long long v_stride, const float* a, long long a_stride, const float* b, long long b_stride,
                                      const float* dt_bias, const float* A_log, float* scratch, float* states, float* y,
                                      const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments, int rows,
-                                     int least_rows, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
+                                     int least_rows, int chunks, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
                                      int* error_word, cudaStream_t stream) {
-  if (segments == 0) return MLR_OK;
-  if (segments < 0 || rows <= 0 || least_rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || scratch == nullptr) return MLR_BAD_SIZE;
+  if (segments == 0 || chunks == 0) return MLR_OK;
+  if (segments < 0 || rows <= 0 || chunks < 0 || least_rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || scratch == nullptr)
+    return MLR_BAD_SIZE;
   if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % DC_COLS != 0) return MLR_BAD_SIZE;
-  const long long chunks = long_chunks(rows, segments, least_rows);
-  if (heads > 65535 || chunks > 65535 || vdim > 65535) return MLR_TOO_LARGE;
+  if (heads > 65535 || vdim > 65535) return MLR_TOO_LARGE;
   const uintptr_t pointers = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)states | (uintptr_t)scratch;
   if (pointers % 16 != 0 || (q_stride | k_stride | v_stride) % 4 != 0) return MLR_BAD_ALIGNMENT;
+  const int round = chunks_of_round(chunks, heads, kv_heads, dim, vdim);      // a few thousand at most: a grid's y
   DeltaChunkArgs p{q, k, v, a, b, q_stride, k_stride, v_stride, a_stride, b_stride, dt_bias, A_log, states, y, nullptr, nullptr, scratch, nullptr,
-                   nullptr, nullptr, nullptr, seg_q_start, seg_q_len, seg_slot, segments, least_rows, heads, kv_heads, vdim, unit_eps, q_scale, error_word};
-  const long long places = chunks * heads;
+                   nullptr, nullptr, nullptr, seg_q_start, seg_q_len, seg_slot, segments, least_rows, heads, kv_heads, vdim, 0, round, unit_eps,
+                   q_scale, error_word};
+  const long long places = (long long)round * heads;
   p.factors = p.P + places * DC_SQUARE;
   p.u = p.factors + places * DC_FACTORS;
   p.before = p.u + places * vdim * CHUNK;
   p.T = reinterpret_cast<bf16*>(p.before + places * vdim * dim);
   p.key_parts = p.T + places * 3 * CHUNK * DC_PITCH;
-  p.decays = reinterpret_cast<float*>(p.key_parts + chunks * kv_heads * 3 * CHUNK * (dim + 8));
-  return dim == 64 ? launch_delta_chunks<64>(p, rows, stream) : launch_delta_chunks<128>(p, rows, stream);
+  p.decays = reinterpret_cast<float*>(p.key_parts + (long long)round * kv_heads * 3 * CHUNK * (dim + 8));
+  return dim == 64 ? launch_delta_chunks<64>(p, rows, chunks, stream) : launch_delta_chunks<128>(p, rows, chunks, stream);
 }

@@ -954,6 +954,14 @@ class CudaOps:
             return rows - 1       # lengths that only the device knows
         return max((s.length for s in segments if s.length < rows), default=0)
 
+    @staticmethod
+    def _chunks_from(ctx, rows: int, least: int) -> int:
+        """Chunks of 64 rows that the portions of ``least`` rows and more have, or the most there can be."""
+        segments = getattr(ctx, "segments", None)
+        if segments is not None:
+            return sum(-(-s.length // 64) for s in segments if s.length >= least)
+        return -(-rows // 64) if ctx.num_segments == 1 else rows // 64 + min(ctx.num_segments, rows // least)
+
     use_gated_chunks = True
     # By head size: portions of fewer rows than the first number go token by token in a launch of their own, those from the second on in
     # chunks, those between token by token in the chunks' launches.  Which way a request's rows go is a matter of its own portion
@@ -2023,11 +2031,11 @@ class CudaOps:
             # long segments: chunks of tokens, all but the state's way through them side by side
             lib, below = build.load_library("delta_chunks"), self.DELTA_CHUNK_ROWS
             lib.mlr_delta_chunk_scratch.restype = ctypes.c_longlong
-            scratch = torch.empty(lib.mlr_delta_chunk_scratch(rows, ctx.num_segments, below, heads, kv_heads, dim, vdim),
-                                  dtype=torch.float32, device=q.device)
+            chunks = self._chunks_from(ctx, rows, below)
+            scratch = torch.empty(lib.mlr_delta_chunk_scratch(chunks, heads, kv_heads, dim, vdim), dtype=torch.float32, device=q.device)
             _check(lib.mlr_delta_rule_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(scratch), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
-                _ptr(ctx.seg_slot), ctx.num_segments, rows, below, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+                _ptr(ctx.seg_slot), ctx.num_segments, rows, below, chunks, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
                 ctypes.c_float(float(dim) ** -0.5), _ptr(self._workspace(q.device)["error_word"]), _stream()), "delta_rule_chunks")
             longest = int(self._longest_below(ctx, below))
             if longest == 0:

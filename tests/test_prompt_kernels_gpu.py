@@ -550,3 +550,22 @@ def test_delta_rule_in_chunks_is_no_further_from_64_bits(heads, kv_heads, dim, m
             for index, (a, b) in enumerate(((got, want), (state, want_state))):
                 errors[chunks][index] += float((a.double().cpu() - b).norm() / b.norm())
     assert errors[True][0] <= errors[False][0] and errors[True][1] <= 1.1 * errors[False][1], errors
+
+
+def test_delta_rule_of_many_chunks_keeps_its_scratch_bounded():
+    """More chunks than have their scratch in the bound: rounds of them, borders between rounds inside a portion and between portions."""
+    heads, kv_heads, dim, vdim, lengths = 32, 16, 128, 64, [2700, 40, 600, 2300]
+    ctx, rows = segments(lengths, [2, 0, 3, 1], [3, 1, 0, 2]), sum(lengths)
+    q, k, v, a, b, bias, a_log = delta_inputs(rows, heads, kv_heads, dim, vdim, False)
+    state = rnd(8, len(lengths), heads, vdim, dim, std=0.3)
+    given, got_state = [t.to(DEVICE) for t in (q, k, v, a, b, bias, a_log)], state.to(DEVICE)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    start = torch.cuda.memory_allocated()
+    got = cuda().delta_rule_scan(*given, got_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
+    extra = torch.cuda.max_memory_allocated() - start - got.numel() * 4
+    assert extra <= (257 << 20) + rows * heads * 48, extra      # and the inner products of the portions token by token
+    want_state = state.to(DEVICE).double()
+    want = FAKE.delta_rule_scan(*(t.double() for t in given), want_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
+    close(got, want.cpu(), 200 * UNIT, "delta rule outputs")
+    close(got_state.flatten(0, 1), want_state.cpu().flatten(0, 1), 200 * UNIT, "delta rule state")
