@@ -15,11 +15,14 @@
 // Roundings that every output sees are saved: norms, decays and P are computed in 64 bits and rounded once, beta v - G .. and u's share of
 // the state are each one rounding.  Error against 64 bits (2-norm, outputs / states, means of four inputs), token by token, here without and
 // with all that, in 1e-7: 2,048 rows of 32 heads of 128 x 64 1.21 / 1.24, 1.65 / 1.25, 1.09 / 1.11; 14 heads of 64 x 64 1.29 / 1.27, 1.84 / 1.49,
-// 1.11 / 1.12.  It costs 12 us of the 32 heads' 212, 6 of the 14 heads' 105.
+// 1.11 / 1.12.  It costs 12 us of 2,048 rows of the 32 heads, 6 of the 14.
 //
-// Measured (B200), token by token / in chunks: 2,048 rows of 32 heads of 128 x 64 340 / 203 us, of 14 heads of 64 x 64 207 / 97 (188 and 92
-// before those roundings were saved: solve 60, chain 78, read 43).  The first and the last kernel are bound by instructions (splitting operands,
+// Measured (B200), token by token / in chunks: 2,048 rows of 32 heads of 128 x 64 340 / 191 us, from a flushed L2 347 / 206 (first kernel
+// 71, second 83, third 48), of 14 heads of 64 x 64 214 / 105 (23, 62, 16).  The first and the last kernel are bound by instructions (splitting operands,
 // decays) and shared memory, the chain by the latency of its steps, 4,500 cycles per chunk, of which 1,900 are MMAs.
+//
+// The first two kernels do not bring in the next one early: its waiting CTAs slow them down (512 rows of 14 heads of 64 x 64: the first
+// kernel 17 -> 25 us, all three 46 -> 56; of 32 heads of 128 x 64 71 -> 77).
 //
 // In the chain four warps issue MMAs, each with 16 channels x a quarter of dim of the state in its registers (as accumulators, whose
 // layout is that of the next product's left operand), while four fetch the next chunk's keys and T, whose parts the first kernel left.
@@ -51,6 +54,7 @@ struct DeltaChunkArgs {
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int segments, least, heads, kv_heads, vdim;
   int first_chunk, chunks;              // of this round; scratch is indexed from the first on
+  int beside;                           // the launch just before is the recurrence of the short segments, which runs beside the first kernel
   float unit_eps, q_scale;
   int* error_word;
 };
@@ -159,6 +163,8 @@ struct SolveShape {
 // A CTA per chunk and key/value head: the products k_t . k_s and q_t . k_s of s <= t on the tensor cores, then its heads two at a time.
 // T is a triangular inverse: the two triangles of 32 rows at once, a thread per column, then T_21 = -T_22 A_21 T_11.  Bound by
 // shared-memory reads; on the CUDA cores the products alone took 24,000 cycles of a CTA, and 64 rows one behind the other 19,000.
+// Behind delta_scan_kernel, which triggers its successor only once all that came before it is complete, it starts without a wait: the two
+// share nothing.  One thread waits at the end, so that whoever waits for this kernel has waited for that one as well.
 // grid: (chunks, kv heads)
 template <int D>
 __global__ void __launch_bounds__(256, 2)
@@ -171,10 +177,13 @@ delta_solve_kernel(DeltaChunkArgs p) {
   float *kk = reinterpret_cast<float*>(solve_shared), *qk = kk + CHUNK * SQUARE_PITCH, *matrix = qk + CHUNK * SQUARE_PITCH;
   __shared__ double rq[CHUNK];
   __shared__ float rk[CHUNK], decay[2][CHUNK], beta[2][CHUNK], upto[2][CHUNK];
-  pdl_trigger();
-  pdl_wait();
+  if (!p.beside) pdl_wait();
   const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, p.first_chunk + blockIdx.x);
-  if (seg < 0) return;
+  const bool waits = p.beside && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
+  if (seg < 0) {
+    if (waits) pdl_wait();
+    return;
+  }
   const int kv = blockIdx.y, first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 
@@ -382,6 +391,7 @@ delta_solve_kernel(DeltaChunkArgs p) {
     }
     __syncthreads();      // A, decays and factors are rewritten by the next heads
   }
+  if (waits) pdl_wait();
 }
 
 // ---------------------------------------------------------------- the chain
@@ -430,7 +440,6 @@ delta_chain_kernel(DeltaChunkArgs p) {
     mbar_init(&there[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  pdl_trigger();
   pdl_wait();
   const ChunkAt segment = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.x);
   if (segment.seg < 0) return;
@@ -822,6 +831,7 @@ int launch_delta_chunks(DeltaChunkArgs p, int rows, int chunks, cudaStream_t str
     if ((status = launch_status()) != MLR_OK) return status;
     launch_kernel(delta_read_kernel<D>, dim3(p.heads, p.chunks, (p.vdim + 63) / 64), dim3(128), ReadShape<D>::SHARED, stream, p);
     if ((status = launch_status()) != MLR_OK) return status;
+    p.beside = 0;
   }
   return MLR_OK;
 }
@@ -839,13 +849,14 @@ MLR_EXPORT long long mlr_delta_chunk_scratch(int chunks, int heads, int kv_heads
 }
 
 // As mlr_delta_rule_scan, for the segments of least_rows rows and more, which have `chunks` chunks of 64 rows or fewer in all: dim 64 or 128,
-// vdim a multiple of 16, every row of q, k and v, states and scratch on 16-byte boundaries.  rows: the step's rows.  error_word:
-// host-visible int that receives a code if a wait runs out.
+// vdim a multiple of 16, every row of q, k and v, states and scratch on 16-byte boundaries.  rows: the step's rows.  beside: the stream's last
+// launch was mlr_delta_rule_scan for the segments below least_rows, and scratch is older than it.  error_word: host-visible int that
+// receives a code if a wait runs out.
 MLR_EXPORT int mlr_delta_rule_chunks(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
                                      long long v_stride, const float* a, long long a_stride, const float* b, long long b_stride,
                                      const float* dt_bias, const float* A_log, float* scratch, float* states, float* y,
                                      const int* seg_q_start, const int* seg_q_len, const int* seg_slot, int segments, int rows,
-                                     int least_rows, int chunks, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
+                                     int least_rows, int chunks, int beside, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
                                      int* error_word, cudaStream_t stream) {
   if (segments == 0 || chunks == 0) return MLR_OK;
   if (segments < 0 || rows <= 0 || chunks < 0 || least_rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || scratch == nullptr)
@@ -856,7 +867,7 @@ MLR_EXPORT int mlr_delta_rule_chunks(const float* q, long long q_stride, const f
   if (pointers % 16 != 0 || (q_stride | k_stride | v_stride) % 4 != 0) return MLR_BAD_ALIGNMENT;
   const int round = chunks_of_round(chunks, heads, kv_heads, dim, vdim);      // a few thousand at most: a grid's y
   DeltaChunkArgs p{q, k, v, a, b, q_stride, k_stride, v_stride, a_stride, b_stride, dt_bias, A_log, states, y, nullptr, nullptr, scratch, nullptr,
-                   nullptr, nullptr, nullptr, seg_q_start, seg_q_len, seg_slot, segments, least_rows, heads, kv_heads, vdim, 0, round, unit_eps,
+                   nullptr, nullptr, nullptr, seg_q_start, seg_q_len, seg_slot, segments, least_rows, heads, kv_heads, vdim, 0, round, beside, unit_eps,
                    q_scale, error_word};
   const long long places = (long long)round * heads;
   p.factors = p.P + places * DC_SQUARE;

@@ -152,7 +152,7 @@ delta_prepare_kernel(DeltaArgs p) {
 template <int E, int SL, int C, int TB, bool WIDE, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 delta_scan_kernel(DeltaArgs p) {
-  pdl_trigger();
+  if (p.below == 0) pdl_trigger();
   extern __shared__ __align__(16) float shared[];
   constexpr int GROUPS = THREADS / SL, COLS = GROUPS * C;
   constexpr int N = TB * C;
@@ -165,6 +165,7 @@ delta_scan_kernel(DeltaArgs p) {
   const int lane = threadIdx.x & 31, s = threadIdx.x % SL, group = threadIdx.x / SL;
   const float a_log = p.A_log[head], bias = p.dt_bias[head];
   pdl_wait();
+  if (p.below > 0) pdl_trigger();      // the long segments' first kernel takes this as the end of all that came before
   const int q_start = p.seg_q_start[seg], q_len = p.seg_q_len[seg];
   if (p.below > 0 && q_len >= p.below) return;
 

@@ -2000,12 +2000,13 @@ class CudaOps:
 
     # ------------------------------------------------------------------ gated delta rule
     use_delta_chunks = True
-    # Rows from which a request's portion goes in chunks, whatever else is in the step: three launches, of which the first alone takes 20 us,
-    # in front of the one for shorter portions.  In us, token by token / in chunks, 14 heads of 64 x 64: 256 rows 38 / 40, 384 50 / 42, 512 62 / 48,
-    # 1,024 112 / 60, 2,048 214 / 99; 32 heads of 128 x 64: 256 rows 56 / 58, 384 75 / 65, 512 95 / 71, 1,024 181 / 103, 2,048 346 / 202.  Alone they
-    # pay from 288 rows on, but beside other portions of a few hundred rows, which take their time all the same, they do not: 281, 76, 9, 324,
-    # 127 and 176 rows 130 token by token, 153 with the 324 in chunks.
-    DELTA_CHUNK_ROWS = 512
+    # Rows from which a request's portion goes in chunks, whatever else is in the step.  In us from a flushed L2, token by token / in chunks,
+    # 14 heads of 64 x 64: 256 rows 38 / 38, 320 44 / 40, 384 50 / 42, 512 62 / 46, 2,048 214 / 105; 32 heads of 128 x 64: 256 rows 56 / 56, 320
+    # 67 / 62, 384 77 / 65, 512 95 / 71, 2,048 347 / 206.  Alone they pay from 256 rows on, but shorter portions of the same step take their time
+    # before the chunks' last two kernels: 600 and 280 rows 89 / 80 and 142 / 131, 600 and 500 (all in chunks) 89 / 52 and 142 / 120, 400 and 380 rows
+    # 65 / 86 and 103 / 137.  Of 70 steps of two to six portions of 1 to 3,000 rows, drawn over their logarithms, borders of 256, 320, 384 and 512
+    # leave 6, 4, 1 and 2 more than 4 % slower than token by token (by 21, 24, 12 and 8 %); the mean gain is 19, 18, 18 and 14 %.
+    DELTA_CHUNK_ROWS = 384
 
     def delta_rule_scan(self, q, k, v, a, b, dt_bias, A_log, state, ctx, heads: int, kv_heads: int, dim: int, vdim: int,
                         unit_eps: float) -> torch.Tensor:
@@ -2025,27 +2026,28 @@ class CudaOps:
         y = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device)
         views = (*self._view(q, "q", rows, kv_heads * dim), *self._view(k, "k", rows, kv_heads * dim),
                  *self._view(v, "v", rows, heads * vdim), *self._view(a, "a", rows, heads), *self._view(b, "b", rows, heads))
-        longest, below = int(ctx.max_q_len), 0
+        longest, below, chunks = int(ctx.max_q_len), 0, 0
         if (self.use_delta_chunks and longest >= self.DELTA_CHUNK_ROWS and dim in (64, 128) and vdim % 16 == 0
                 and all(t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0 for t in (q, k, v)) and state.data_ptr() % 16 == 0):
             # long segments: chunks of tokens, all but the state's way through them side by side
-            lib, below = build.load_library("delta_chunks"), self.DELTA_CHUNK_ROWS
+            below = self.DELTA_CHUNK_ROWS
+            longest, chunks = int(self._longest_below(ctx, below)), self._chunks_from(ctx, rows, below)
+            lib = build.load_library("delta_chunks")
             lib.mlr_delta_chunk_scratch.restype = ctypes.c_longlong
-            chunks = self._chunks_from(ctx, rows, below)
             scratch = torch.empty(lib.mlr_delta_chunk_scratch(chunks, heads, kv_heads, dim, vdim), dtype=torch.float32, device=q.device)
+        if longest > 0 or chunks == 0:
+            # steps with longer segments take four tokens at once; a first kernel leaves their inner products here
+            coef = torch.empty((rows, heads, 12), dtype=torch.float32, device=q.device) if longest > 1 else None
+            _check(build.load_library("delta_rule").mlr_delta_rule_scan(
+                *views, _ptr(dt_bias), _ptr(A_log), _ptr(coef), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
+                _ptr(ctx.seg_slot), ctx.num_segments, longest, below, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+                ctypes.c_float(float(dim) ** -0.5), _stream()), "delta_rule_scan")
+        if chunks > 0:      # last: their first kernel runs beside the one above, in scratch that is older than it
             _check(lib.mlr_delta_rule_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(scratch), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
-                _ptr(ctx.seg_slot), ctx.num_segments, rows, below, chunks, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
-                ctypes.c_float(float(dim) ** -0.5), _ptr(self._workspace(q.device)["error_word"]), _stream()), "delta_rule_chunks")
-            longest = int(self._longest_below(ctx, below))
-            if longest == 0:
-                return y
-        # steps with longer segments take four tokens at once; a first kernel leaves their inner products here
-        coef = torch.empty((rows, heads, 12), dtype=torch.float32, device=q.device) if longest > 1 else None
-        _check(build.load_library("delta_rule").mlr_delta_rule_scan(
-            *views, _ptr(dt_bias), _ptr(A_log), _ptr(coef), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
-            _ptr(ctx.seg_slot), ctx.num_segments, longest, below, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
-            ctypes.c_float(float(dim) ** -0.5), _stream()), "delta_rule_scan")
+                _ptr(ctx.seg_slot), ctx.num_segments, rows, below, chunks, int(longest > 0), heads, kv_heads, dim, vdim,
+                ctypes.c_float(unit_eps), ctypes.c_float(float(dim) ** -0.5), _ptr(self._workspace(q.device)["error_word"]), _stream()),
+                "delta_rule_chunks")
         return y
 
     def gated_head_norm(self, y: torch.Tensor, gate, weight: torch.Tensor, eps: float, heads: int,

@@ -11,7 +11,7 @@ import torch
 
 from fake_ops import FakeOps
 from mini_llm_runtime_b200 import ops
-from mini_llm_runtime_b200.ops import AttentionBatch
+from mini_llm_runtime_b200.ops import AttentionBatch, cuda_ops
 
 pytestmark = pytest.mark.gpu
 
@@ -503,7 +503,7 @@ def test_delta_rule_in_chunks(heads, kv_heads, dim, vdim, alike, lengths, slots,
     state = rnd(8, len(lengths), heads, vdim, dim, std=0.3)
     want_state = state.double()
     want = FAKE.delta_rule_scan(*(t.double() for t in (q, k, v, a, b, bias, a_log)), want_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
-    for least in (1, cuda().DELTA_CHUNK_ROWS):
+    for least in (1, 65, 128):
         monkeypatch.setattr(cuda(), "DELTA_CHUNK_ROWS", least)
         got_state = state.to(DEVICE)
         got = cuda().delta_rule_scan(*(spaced(t) for t in (q, k, v, a, b)), bias.to(DEVICE), a_log.to(DEVICE), got_state, ctx, heads,
@@ -569,3 +569,38 @@ def test_delta_rule_of_many_chunks_keeps_its_scratch_bounded():
     want = FAKE.delta_rule_scan(*(t.double() for t in given), want_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
     close(got, want.cpu(), 200 * UNIT, "delta rule outputs")
     close(got_state.flatten(0, 1), want_state.cpu().flatten(0, 1), 200 * UNIT, "delta rule state")
+
+
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(14, 7, 64, 64), (4, 1, 128, 32)])
+def test_delta_rule_at_the_border_of_chunks(heads, kv_heads, dim, vdim, known, monkeypatch):
+    """Portions on both sides of the border in one step, side by side; each has the bits of a step of its own.  ``known``: the lengths are on
+    the host as well."""
+    least, launched, load = cuda().DELTA_CHUNK_ROWS, [], cuda_ops.build.load_library
+    lengths = [1, least - 1, least, 40, least + 65, 2, least - 30]
+    ctx, rows = segments(lengths, [3, 0, 2, 1, 6, 5, 4], [4, 1, 6, 0, 5, 2, 3]), sum(lengths)
+    parts = ctx.segments
+    if not known:
+        del ctx.segments
+    q, k, v, a, b, bias, a_log = (t.to(DEVICE) for t in delta_inputs(rows, heads, kv_heads, dim, vdim, False))
+    state = rnd(8, len(lengths), heads, vdim, dim, std=0.3)
+    want_state = state.double()
+    want = FAKE.delta_rule_scan(*(t.double().cpu() for t in (q, k, v, a, b, bias, a_log)), want_state, types.SimpleNamespace(
+        seg_q_start=ctx.seg_q_start.cpu(), seg_q_len=ctx.seg_q_len.cpu(), seg_slot=ctx.seg_slot.cpu(), num_segments=len(lengths), segments=parts),
+        heads, kv_heads, dim, vdim, 1e-6)
+    monkeypatch.setattr(cuda_ops.build, "load_library", lambda name: launched.append(name) or load(name))
+    for _ in range(3):
+        launched.clear()
+        got_state = state.to(DEVICE)
+        got = cuda().delta_rule_scan(q, k, v, a, b, bias, a_log, got_state, ctx, heads, kv_heads, dim, vdim, 1e-6)
+        following = got + got                   # behind both kernels' rows, those whose last launch it does not follow directly
+        assert {"delta_rule", "delta_chunks"} <= set(launched)
+        close(got, want, 200 * UNIT, "delta rule outputs")
+        close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "delta rule state")
+        assert torch.equal(following, got * 2)
+    for part in parts:
+        at, own_state = slice(part.row_start, part.row_start + part.length), state.to(DEVICE)
+        own = cuda().delta_rule_scan(*(t[at] for t in (q, k, v, a, b)), bias, a_log, own_state, segments([part.length], [part.slot]), heads,
+                                     kv_heads, dim, vdim, 1e-6)
+        if part.length > 1:                     # a decoded row is walked another way beside longer portions
+            assert torch.equal(own, got[at]) and torch.equal(own_state[part.slot], got_state[part.slot]), part.length
