@@ -88,20 +88,21 @@ __device__ __forceinline__ void split_operand(uint32_t (&parts)[3][4], const flo
     for (int i = 0; i < 4; ++i) parts[q][i] = take_part(v[2 * i], v[2 * i + 1]);
 }
 
-// Of a left operand whose columns are tokens from t0 on: numbers that are not finite become zeros, else a zero weight would carry them to
-// the tokens before; first: the earliest of them, in this lane's two rows.
+// Of a left operand whose columns are tokens from t0 on: numbers whose parts are not finite become zeros, else a zero weight would carry them
+// to the tokens before; first: the earliest of them, in this lane's two rows.  That is infinities, NaN and what rounds to an infinite part.
 __device__ __forceinline__ bool take_out(float (&v)[2][4], int t0, int (&first)[2]) {
-  float probe = 0.f;
+  constexpr float LIMIT = 3.39617752923046e38f;      // half a last place above the largest bfloat16 number
+  bool any = false;
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) probe = fmaf(v[j][e], 0.f, probe);
-  if (!__any_sync(0xffffffffu, probe != 0.f)) return false;
+    for (int e = 0; e < 4; ++e) any |= !(fabsf(v[j][e]) < LIMIT);
+  if (!__any_sync(0xffffffffu, any)) return false;
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      if (!(fabsf(v[j][e]) <= 3.402823466e38f)) {
+      if (!(fabsf(v[j][e]) < LIMIT)) {
         first[e >> 1] = min(first[e >> 1], t0 + j * 8 + (e & 1));
         v[j][e] = 0.f;
       }

@@ -513,12 +513,14 @@ def test_delta_rule_in_chunks(heads, kv_heads, dim, vdim, alike, lengths, slots,
         close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "delta rule state")
 
 
-@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+# 3.4e38: the largest bfloat16 number is below it
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
 @pytest.mark.parametrize("which,at", [("k", 70), ("k", 110), ("v", 127), ("q", 199), ("a", 130), ("a", 105), ("b", 120)])
 def test_a_token_that_is_no_number_leaves_the_tokens_of_a_delta_rule_before_it_alone(value, which, at, monkeypatch):
     monkeypatch.setattr(cuda(), "DELTA_CHUNK_ROWS", 64)
     heads, kv_heads, dim, vdim, rows = 2, 1, 128, 64, 200
     inputs = dict(zip("qkvab", delta_inputs(rows, heads, kv_heads, dim, vdim, False)))
+    inputs["b"][at] = 90.0           # a value goes in whole
     bias, a_log = rnd(6, heads).to(DEVICE), rnd(7, heads).to(DEVICE)
     ctx, results = segments([rows], [0], None), []
     for broken in (False, True):
