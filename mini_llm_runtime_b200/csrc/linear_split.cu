@@ -64,10 +64,12 @@ struct LinearSplitShape {
 };
 
 // parts [3][M][pitch], pitch = K rounded up to 8; what lies behind K becomes zero.  K % 4 == 0.
+// It brings in the product only behind its own wait: so all that came before is complete when the product's first copies read W, which may
+// have been written by the kernel just before.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* x, uint2* parts, int M, int K, int pitch) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int per_row = pitch / 4;
   const bool wide = ((uintptr_t)x & 15) == 0;
   const long long count = (long long)M * per_row;
@@ -164,7 +166,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   bool gave_up = false;
 
   if (warp == 0) {
-    if (lane == 0) {      // W does not depend on the kernel before this one: no wait for it
+    if (lane == 0) {      // W does not depend on the kernel before this one (split_rows_kernel): no wait for it
       int raw = 0;
       uint32_t turn = 0;
       for (int item = first_item; item < items; item += item_step) {

@@ -606,3 +606,14 @@ def test_delta_rule_at_the_border_of_chunks(heads, kv_heads, dim, vdim, known, m
                                      kv_heads, dim, vdim, 1e-6)
         if part.length > 1:                     # a decoded row is walked another way beside longer portions
             assert torch.equal(own, got[at]) and torch.equal(own_state[part.slot], got_state[part.slot]), part.length
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8192, 2048), (40, 896, 4864), (300, 4864, 896)])
+def test_products_in_parts_of_a_weight_just_written(m, n, k):
+    """The product follows the kernel that writes its weight without anything between them."""
+    x, base, step = (t.to(DEVICE) for t in (rnd(1, m, k), rnd(2, n, k, std=0.2), rnd(3, n, k, std=0.2)))
+    assert cuda()._split_fits(x, base)
+    want = cuda().linear(x, base + step)
+    for _ in range(20):
+        w = base.clone()
+        assert torch.equal(cuda().linear(x, cuda().add_inplace(w, step)), want)
