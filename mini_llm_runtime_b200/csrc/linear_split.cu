@@ -13,7 +13,11 @@
 //                 so one barrier per block tells all: x is there, W's parts are there, the accumulator is read
 //   warps 2..9    split W, four warps the even blocks and four the odd ones: a thread takes one row, stores its parts to tensor memory
 //   warps 10..17  add each block's accumulator to their sums; write the tile
-// x is split once by a kernel of its own (every W tile uses it), W inside (it is read from memory once, in float32).
+// x is split once by a kernel of its own (every W tile uses it), W inside (it is read from memory once, in float32).  Up to 32 rows
+// warps 10..17 split x themselves, two blocks ahead of the accumulators they read, in every CTA: a launch less, and the tiles of W are asked for
+// as soon as the kernel before is complete (1 row, cold weights, us per product of a chain: [896, 896] 7.9 with the launch, 6.2 without, 6.5 on
+// the CUDA cores; [9728, 896] 14.3, 12.6, 14.2).  One more warp for all of x would have been the bound: [16384, 2048] 31 us at 1 row, 48 at 16;
+// 27 and 28 so.
 //
 // Long sums of narrow outputs are cut into 2 to 8 parts along k, one CTA each, that form a cluster and exchange their
 // sums through shared memory.  How k is cut depends on N and K alone and an element's additions on nothing else, so results do not
@@ -24,10 +28,11 @@
 // Every wait is bounded; one that runs out stores a code into the error word and the CTA stops issuing work and returns.
 //
 // For many rows bound by the MMAs, six per product: 1,500 rows [16384, 2048] 2,461 us on the CUDA cores (41 TFLOP/s), 505 us here, 1.2
-// PFLOP/s of bfloat16 multiply-adds, near what the power limit sustains.  For few by the stream of W: 8 rows [16384, 2048] 54 / 40 us,
-// 3.4 TB/s; 600 rows [9728, 896] with its gate 318 / 83, [896, 4864] 173 / 70.  Errors against 64 bits (2-norm) at 896, 4,864 and
+// PFLOP/s of bfloat16 multiply-adds, near what the power limit sustains.  For few by the stream of W: 8 rows [16384, 2048] 51 / 28 us,
+// 4.8 TB/s; 600 rows [9728, 896] with its gate 318 / 83, [896, 4864] 173 / 70.  Errors against 64 bits (2-norm) at 896, 4,864 and
 // 8,192 k: 1.1e-7, 1.1e-7, 1.2e-7, on the CUDA cores 5.4e-7, 6.2e-7, 8.1e-7.  One MMA of 128 x 128 x 16 takes 64 cycles
 // either way, but of 128 x 16 x 16 takes 12 with its rows in tensor memory and 39 with them in shared memory.
+#include "copy_async.cuh"
 #include "float_parts.cuh"
 #include "tcgen05.cuh"
 
@@ -50,15 +55,18 @@ struct LinearSplitArgs {
 
 template <int BN>
 struct LinearSplitShape {
+  static constexpr bool OWN_X = BN <= 32;                      // x is split here
+  static constexpr int OWN_X_STAGES = BN == 16 ? 8 : BN == 32 ? 4 : 0;      // its tiles under way, in float32
   static constexpr uint32_t X_BYTES = 3u * BN * LS_K * 2;      // the three parts of a tile of x
   // even, so that a stage of the ring of W tiles is always converted by the same warps: a barrier's parity only tells phases apart to
   // those who wait for every one of them
   static constexpr int RAW_STAGES = BN >= 128 ? 2 : 4;
-  static constexpr int X_STAGES = BN >= 64 ? 3 : BN >= 32 ? 6 : 8;
+  static constexpr int X_STAGES = OWN_X ? 4 : 3;
   static_assert(RAW_STAGES % 2 == 0 && X_STAGES >= 3, "see above; arrivals for a block's stage come up to two blocks ahead of its MMAs");
   static constexpr uint32_t TMEM_COLS = 2 * BN + 192 <= 256 ? 256 : 512;      // two accumulators, two slots of three W parts of 32 columns
   static constexpr size_t EXCHANGE_BYTES = 2ull * LS_EXCHANGE * LS_ROWS * 4;
-  static constexpr size_t SHARED = 1024 + RAW_STAGES * (size_t)LS_RAW_BYTES + X_STAGES * (size_t)X_BYTES + EXCHANGE_BYTES;
+  static constexpr size_t SHARED = 1024 + RAW_STAGES * (size_t)LS_RAW_BYTES + X_STAGES * (size_t)X_BYTES + EXCHANGE_BYTES +
+                                    OWN_X_STAGES * (size_t)BN * LS_K * 4;
   static_assert(SHARED <= 226 * 1024, "tiles fit the shared memory");
   static_assert((size_t)BN * LS_ROWS * 4 <= RAW_STAGES * (size_t)LS_RAW_BYTES, "a tile's sums fit where W's tiles were");
 };
@@ -134,7 +142,8 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   uint8_t* raw_tiles = (uint8_t*)(((uintptr_t)ls_shared + 1023) & ~(uintptr_t)1023);
   uint8_t* x_tiles = raw_tiles + RAW_STAGES * LS_RAW_BYTES;
   float* exchange = reinterpret_cast<float*>(x_tiles + X_STAGES * Shape::X_BYTES);
-  // of every block: its x (1 arrival with the copies' bytes), its parts of W (4 warps) and the accumulator two blocks before (8 warps)
+  // of every block: its x (1 arrival with the copies' bytes), its parts of W (4 warps) and the accumulator two blocks before (8 warps; where
+  // they split x as well, these arrivals stand for it too)
   __shared__ uint64_t ready[X_STAGES];
   __shared__ uint64_t raw_full[RAW_STAGES], raw_empty[RAW_STAGES], x_empty[X_STAGES], done[2];      // done: a block's MMAs, by its parity
   __shared__ uint32_t tmem_holder;
@@ -142,7 +151,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < RAW_STAGES; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4); }
-    for (int s = 0; s < X_STAGES; ++s) { mbar_init(&ready[s], 13); mbar_init(&x_empty[s], 1); }
+    for (int s = 0; s < X_STAGES; ++s) { mbar_init(&ready[s], Shape::OWN_X ? 12 : 13); mbar_init(&x_empty[s], 1); }
     mbar_init(&done[0], 1);
     mbar_init(&done[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -166,7 +175,8 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   bool gave_up = false;
 
   if (warp == 0) {
-    if (lane == 0) {      // W does not depend on the kernel before this one (split_rows_kernel): no wait for it
+    if (lane == 0) {
+      if (Shape::OWN_X) pdl_wait();      // else W does not depend on the kernel before this one, split_rows_kernel
       int raw = 0;
       uint32_t turn = 0;
       for (int item = first_item; item < items; item += item_step) {
@@ -184,7 +194,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       }
     }
   } else if (warp == 18) {
-    if (lane == 0) {
+    if (!Shape::OWN_X && lane == 0) {
       pdl_wait();
       int xs = 0;
       uint32_t turn = 0;
@@ -280,6 +290,67 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     constexpr int COLS = BN / 2;      // columns (rows of x) of this warp
     const int quarter = warp & 3, side = (warp - 10) >> 2, row = quarter * 32 + lane;
     uint32_t n = 0;      // blocks so far
+    // Own x: half a warp per row, 2 (w + 8 i) and the next for piece i of the w-th warp; a lane reads only what it has copied itself.  A stage
+    // is free: block n + 2 takes that of block n - 2, whose accumulator has been read.  Rows and columns behind the last are zeros.
+    constexpr int PIECES = BN / 16, AHEAD = Shape::OWN_X ? Shape::OWN_X_STAGES - 1 : 0;
+    const int c = lane & 15, pair = 2 * (warp - 10), turns = end_block - first_block;
+    const int count = first_item < items ? ((items - first_item - 1) / item_step + 1) * turns : 0;
+    const bool wide = ((uintptr_t)p.x & 15) == 0;
+    uint8_t* raw_x = reinterpret_cast<uint8_t*>(exchange) + Shape::EXCHANGE_BYTES + (warp - 10) * (Shape::OWN_X_STAGES * PIECES * 512) + lane * 16;
+    auto x_slot = [&](int stage, int i) {
+      const int x_row = pair + 16 * i + (lane >> 4);
+      return x_tiles + stage * Shape::X_BYTES + x_row * 128 + (((c >> 1) ^ (x_row & 7)) << 4) + (c & 1) * 8;
+    };
+    auto ask = [&](int block) {
+      if (block < count) {
+        const int k = (first_block + block % turns) * LS_K + c * 4;
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+          const int x_row = pair + 16 * i + (lane >> 4);
+          float* dst = reinterpret_cast<float*>(raw_x + ((block % (AHEAD + 1)) * PIECES + i) * 512);
+          const float* src = p.x + (size_t)x_row * p.K + k;
+          if (x_row >= p.M || k >= p.K) {
+            *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+          } else if (wide) {
+            copy_async_16(dst, src);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) copy_async_4(dst + e, src + e);
+          }
+        }
+      }
+      copy_async_commit();
+    };
+    auto split_x = [&](int block) {
+      ask(block + AHEAD);
+      copy_async_wait<AHEAD>();
+      if (block >= count) return;
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i)
+        if (pair + 16 * i < p.M) {
+          float4 v = *reinterpret_cast<const float4*>(raw_x + ((block % (AHEAD + 1)) * PIECES + i) * 512);
+          uint8_t* dst = x_slot(block % X_STAGES, i);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            const uint32_t low = take_part(v.x, v.y), high = take_part(v.z, v.w);
+            *reinterpret_cast<uint2*>(dst + q * (BN * LS_K * 2)) = make_uint2(low, high);
+          }
+        }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    };
+    if constexpr (Shape::OWN_X) {
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i)
+        if (pair + 16 * i >= p.M) {
+          for (int stage = 0; stage < X_STAGES; ++stage)
+            for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(x_slot(stage, i) + q * (BN * LS_K * 2)) = make_uint2(0u, 0u);
+        }
+      pdl_wait();
+      for (int block = 0; block < AHEAD; ++block) ask(block);
+      split_x(0);
+      split_x(1);
+      __syncwarp();
+    }
     if (lane == 0) {     // both accumulators are free
       mbar_arrive(&ready[0]);
       mbar_arrive(&ready[1]);
@@ -291,6 +362,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       for (int c = 0; c < COLS; ++c) sum[c] = 0.f;
       for (int block = first_block; block < end_block; ++block, ++n) {
         const uint32_t slot = n & 1;
+        if constexpr (Shape::OWN_X) split_x((int)n + 2);
         fa_wait(&done[slot], (n >> 1) & 1, p.error_word, 48, gave_up);
         __syncwarp();
         fa_fence_after();
@@ -442,7 +514,9 @@ static int launch_split(const LinearSplitArgs& p, const void* parts, int pitch, 
     configured = true;
   }
   CUtensorMap w_map, x_map;
-  if (!float_tile_map(&w_map, p.w, p.N, p.K) || !make_tile_map(&x_map, parts, 3ll * p.M, pitch, BN)) return MLR_BAD_ALIGNMENT;
+  if (!float_tile_map(&w_map, p.w, p.N, p.K)) return MLR_BAD_ALIGNMENT;
+  if (Shape::OWN_X) x_map = w_map;      // not read
+  else if (!make_tile_map(&x_map, parts, 3ll * p.M, pitch, BN)) return MLR_BAD_ALIGNMENT;
   const int items = p.n_tiles * p.m_tiles;
   if (p.parts > 1) {
     launch_kernel_clustered(kernel, dim3(items * p.parts), dim3(LS_THREADS), Shape::SHARED, stream, p.parts, w_map, x_map, p);
@@ -468,8 +542,8 @@ using namespace mlr;
 
 MLR_DEFINE_PDL_SWITCH
 
-// Rows that mlr_linear_split takes at a time; its scratch holds the parts of that many: 3 x rows x (K rounded up to 8) bfloat16.
-MLR_EXPORT int mlr_linear_split_rows(int M, int K) { return M <= 0 || K <= 0 ? M : mlr::split_block_rows(M, K); }
+// Rows whose parts the scratch of mlr_linear_split holds: 3 x rows x (K rounded up to 8) bfloat16.  0: it needs none.
+MLR_EXPORT int mlr_linear_split_rows(int M, int K) { return M <= 32 || K <= 0 ? 0 : mlr::split_block_rows(M, K); }
 
 // x [M,K], w [N,K], bias [N] or null, out [M,N] (gated: [M, N/2], w in blocks of 64 gate rows and their 64 up rows,
 // silu(gate) * up), all float32.  K % 4 == 0, w and scratch on 16-byte boundaries.  error_word: host-visible int that receives a
@@ -477,7 +551,7 @@ MLR_EXPORT int mlr_linear_split_rows(int M, int K) { return M <= 0 || K <= 0 ? M
 MLR_EXPORT int mlr_linear_split(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int gated,
                                 void* scratch, int* error_word, cudaStream_t stream) {
   if (M == 0) return MLR_OK;
-  if (M < 0 || N <= 0 || K <= 0 || scratch == nullptr) return MLR_BAD_SIZE;
+  if (M < 0 || N <= 0 || K <= 0 || (scratch == nullptr && M > 32)) return MLR_BAD_SIZE;
   if (K % 4 != 0 || ((uintptr_t)w & 15) || ((uintptr_t)scratch & 15)) return MLR_BAD_ALIGNMENT;
   if (gated && N % LS_ROWS != 0) return MLR_BAD_SIZE;
   const int pitch = (K + 7) / 8 * 8, block = split_block_rows(M, K), width = gated ? N / 2 : N;
@@ -493,11 +567,13 @@ MLR_EXPORT int mlr_linear_split(const float* x, const float* w, const float* bia
     p.bias = bias;
     p.out = out + (size_t)row * width;
     p.error_word = error_word;
-    const long long pieces = (long long)p.M * (pitch / 4), blocks = (pieces + 255) / 256;
-    launch_kernel(split_rows_kernel, dim3((unsigned)(blocks < 8 * sm_count() ? blocks : 8 * sm_count())), dim3(256), 0, stream,
-                  p.x, (uint2*)scratch, p.M, K, pitch);
-    int status = launch_status();
-    if (status != MLR_OK) return status;
+    int status = MLR_OK;
+    if (p.M > 32) {
+      const long long pieces = (long long)p.M * (pitch / 4), blocks = (pieces + 255) / 256;
+      launch_kernel(split_rows_kernel, dim3((unsigned)(blocks < 8 * sm_count() ? blocks : 8 * sm_count())), dim3(256), 0, stream,
+                    p.x, (uint2*)scratch, p.M, K, pitch);
+      if ((status = launch_status()) != MLR_OK) return status;
+    }
     status = gated ? launch_split_width<true>(p, scratch, pitch, stream) : launch_split_width<false>(p, scratch, pitch, stream);
     if (status != MLR_OK) return status;
   }

@@ -637,9 +637,10 @@ class CudaOps:
         return out
 
     # Elements of a weight from which 32-bit products run on the tensor cores in bfloat16 parts; a rule on the weight alone, so that a
-    # row's result does not depend on how many rows come with it.  In us, CUDA cores / parts, at 1, 8, 24, 60, 100, 600, 1,500
-    # rows: [1024, 512] 10 10 10 14 15 39 55 / 13 13 15 19 25 28 46; [896, 896] 12 12 14 18 22 43 90 / 13 13 15 17 22 36 52;
-    # [2048, 2048] 15 17 24 38 50 169 355 / 17 17 19 24 28 70 136; [9728, 896] 18 25 37 63 88 302 670 / 19 19 21 24 32 75 157.
+    # row's result does not depend on how many rows come with it.  In us per product of a captured chain with cold weights, CUDA cores / parts,
+    # at 1, 8, 24, 60, 100, 600, 1,500 rows: [1024, 512] 4 5 8 18 25 33 49 / 6 6 7 11 15 16 29; [896, 896] 6.5 7.5 12 21 42 79 83 / 6.2 6.3 6.9
+    # 10 14 25 39; [2048, 2048] 15 19 27 63 83 163 349 / 9 10 11 14 19 53 105; [9728, 896] 14 23 43 57 83 294 664 / 13 13 16 19 28 68 151.
+    # Short sums of very many outputs pay at few rows: [20000, 132] 6.1 6.9 12 18 28 97 225 / 7.8 8.7 11 16 25 60 122.
     SPLIT_WEIGHT = 3 << 18
 
     def _split_fits(self, x, weight) -> bool:
@@ -652,7 +653,8 @@ class CudaOps:
         N = weight.shape[0]
         lib = build.load_library("linear_split")
         out = torch.empty((M, N // 2 if gated else N), dtype=torch.float32, device=x.device)
-        parts = torch.empty((3, lib.mlr_linear_split_rows(M, K), -(-K // 8) * 8), dtype=torch.bfloat16, device=x.device)
+        rows = lib.mlr_linear_split_rows(M, K)
+        parts = torch.empty((3, rows, -(-K // 8) * 8), dtype=torch.bfloat16, device=x.device) if rows else None
         _check(lib.mlr_linear_split(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), M, N, K, int(gated), _ptr(parts),
                                     _ptr(self._workspace(x.device)["error_word"]), _stream()), "linear (32-bit operands in parts)")
         return out

@@ -443,9 +443,9 @@ def memory_run(ctx, rows, heads, vdim):
     return build.load_library("matrix_memory").mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim)
 
 
-# Tiles of 128 outputs, of 16, 32, 64 and 128 rows, blocks of 64 k; 1, 2, 4 and 8 parts of the sums over k; more tiles than SMs.
-@pytest.mark.parametrize("n,k", [(1024, 832), (1152, 896), (896, 4864), (130, 6148), (7000, 132), (9728, 200), (33, 30000)])
-@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 300])
+# Tiles of 128 outputs, of 16, 32, 64 and 128 rows, blocks of 64 k; 1, 2, 4 and 8 parts of the sums over k; more tiles than SMs, few rows too.
+@pytest.mark.parametrize("n,k", [(1024, 832), (1152, 896), (896, 4864), (130, 6148), (7000, 132), (9728, 200), (33, 30000), (20100, 132)])
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 300])
 def test_products_in_parts(m, n, k):
     """32-bit products on the tensor cores: dropped products of parts are below 2^-26 of sum |x||w|, a block's accumulator drops up to
     2^-23 of its sum at some dozen steps, each block and part is one 32-bit addition; rows keep their bits in other batches."""
