@@ -24,7 +24,9 @@
 // depend on how rows are batched.
 //
 // An output that is not finite is computed again as one chain of fmaf over k: a part of an infinity times a part that is zero
-// would have made NaN of it, and sums may pass the largest float on the way.
+// would have made NaN of it, and sums may pass the largest float on the way.  All warps of the CTA do so at its end, on the CUDA cores:
+// 600 rows of NaN, [9728, 896], 0.85 ms.  (A chain per thread in the epilogue took 50 ms, while the MMA warp's bounded waits ran on, and its call
+// cost the epilogue registers: 600 rows of a feed-forward, all finite, 141 us with it, 128 without.)
 // Every wait is bounded; one that runs out stores a code into the error word and the CTA stops issuing work and returns.
 //
 // For many rows bound by the MMAs, six per product: 1,500 rows [16384, 2048] 2,461 us on the CUDA cores (41 TFLOP/s), 505 us here, 1.2
@@ -117,24 +119,83 @@ __device__ __forceinline__ void ls_tmem_load8(uint32_t taddr, uint32_t* r) {
                : "r"(taddr) : "memory");
 }
 
-// An output whose sum by parts is not finite, as one chain over k.
-__device__ __noinline__ float ls_chain(const float* x, const float* w, int K) {
-  float sum = 0.f;
-  for (int k = 0; k < K; ++k) sum = fmaf(__ldcg(x + k), __ldcg(w + k), sum);
-  return sum;
-}
-__device__ __forceinline__ float ls_output(const LinearSplitArgs& p, float v, int m, int n) {
-  if (!(fabsf(v) <= 3.402823466e38f)) v = ls_chain(p.x + (size_t)m * p.K, p.w + (size_t)n * p.K, p.K);
-  return p.bias != nullptr ? v + p.bias[n] : v;
-}
+__device__ __forceinline__ float ls_output(const LinearSplitArgs& p, float v, int n) { return p.bias != nullptr ? v + p.bias[n] : v; }
 __device__ __forceinline__ float ls_gated(float gate, float up) { return (gate / (1.f + expf(-gate))) * up; }
+
+// Of the tile of 128 weight rows from n0 on and the rows of x from `m_begin` to below `m_end`, the outputs in memory that are not finite, again: sums as
+// chains over k.  A thread of the first 512 takes weight rows 2 a, 2 a + 1 and the two 64 rows on (of a gated tile the ups of the same
+// outputs) and X rows of x.  The whole CTA comes here; `tiles`: shared memory, 64 (132 + 16 X) numbers.
+template <bool GATED, int X>
+__device__ __noinline__ void ls_chains(const LinearSplitArgs& p, int n0, int m_begin, int m_end, float* tiles) {
+  constexpr int STEP = 64, W_PITCH = 132, X_ROWS = 16 * X;
+  float *w_tile = tiles, *x_tile = tiles + STEP * W_PITCH;      // [k][row]
+  const int t = threadIdx.x, a = t & 31, group = t >> 5, width = GATED ? p.N >> 1 : p.N;
+  const bool wide = ((uintptr_t)p.x & 15) == 0;
+  for (int m0 = m_begin; m0 < m_end; m0 += X_ROWS) {
+    // outputs: of row m0 + group * X + i columns column(0) .. column(3), gated columns column(0) and column(1)
+    auto column = [&](int j) { return GATED ? (n0 >> 1) + 2 * a + j : n0 + 2 * a + (j & 1) + (j >> 1) * 64; };
+    auto broken = [&](int i, int j) {
+      const int m = m0 + group * X + i;
+      return t < 512 && m < m_end && column(j) < width && !(fabsf(__ldcg(p.out + (size_t)m * width + column(j))) <= 3.402823466e38f);
+    };
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < X; ++i)
+#pragma unroll
+      for (int j = 0; j < (GATED ? 2 : 4); ++j) any |= broken(i, j);
+    if (!__syncthreads_or(any)) continue;
+    float sum[X][4];
+#pragma unroll
+    for (int i = 0; i < X; ++i) sum[i][0] = sum[i][1] = sum[i][2] = sum[i][3] = 0.f;
+    for (int k0 = 0; k0 < p.K; k0 += STEP) {
+#pragma unroll
+      for (int at = t; at < (LS_ROWS + X_ROWS) * (STEP / 4); at += LS_THREADS) {
+        const int row = at / (STEP / 4), k = at % (STEP / 4) * 4;
+        const bool of_w = row < LS_ROWS;
+        const int from = of_w ? n0 + row : m0 + row - LS_ROWS;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (from < (of_w ? p.N : m_end) && k0 + k < p.K) {
+          const float* src = (of_w ? p.w : p.x) + (size_t)from * p.K + k0 + k;
+          if (of_w || wide) v = __ldcg(reinterpret_cast<const float4*>(src));
+          else v = make_float4(__ldcg(src), __ldcg(src + 1), __ldcg(src + 2), __ldcg(src + 3));
+        }
+        const int pitch = of_w ? W_PITCH : X_ROWS;
+        float* dst = (of_w ? w_tile + row : x_tile + row - LS_ROWS) + k * pitch;
+        dst[0] = v.x; dst[pitch] = v.y; dst[2 * pitch] = v.z; dst[3 * pitch] = v.w;
+      }
+      __syncthreads();
+      const int steps = min(STEP, p.K - k0);
+      if (t < 512) {
+        for (int k = 0; k < steps; ++k) {
+          const float2 low = *reinterpret_cast<const float2*>(w_tile + k * W_PITCH + 2 * a), high = *reinterpret_cast<const float2*>(w_tile + k * W_PITCH + 64 + 2 * a);
+#pragma unroll
+          for (int i = 0; i < X; ++i) {
+            const float x = x_tile[k * X_ROWS + group * X + i];
+            sum[i][0] = fmaf(x, low.x, sum[i][0]); sum[i][1] = fmaf(x, low.y, sum[i][1]);
+            sum[i][2] = fmaf(x, high.x, sum[i][2]); sum[i][3] = fmaf(x, high.y, sum[i][3]);
+          }
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < X; ++i)
+#pragma unroll
+      for (int j = 0; j < (GATED ? 2 : 4); ++j)
+        if (broken(i, j)) {
+          const int n = n0 + 2 * a + (j & 1) + (j >> 1) * 64;
+          p.out[(size_t)(m0 + group * X + i) * width + column(j)] =
+              GATED ? ls_gated(ls_output(p, sum[i][j], n), ls_output(p, sum[i][2 + (j & 1)], n + 64)) : ls_output(p, sum[i][j], n);
+        }
+  }
+}
 
 // grid: parts == 1: as many CTAs as fill the device (or tiles, if those are fewer), each taking every gridDim.x-th tile; else one
 // cluster of `parts` CTAs per tile.  GATED: weight rows come in blocks of 64 gate rows and the 64 up rows of the same
 // outputs; the tile's results are silu(gate) * up.
 template <int BN, bool GATED>
 __global__ void __launch_bounds__(LS_THREADS, 1)
-linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const LinearSplitArgs p) {
+linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ LinearSplitArgs p) {
   using Shape = LinearSplitShape<BN>;
   constexpr int RAW_STAGES = Shape::RAW_STAGES, X_STAGES = Shape::X_STAGES;
   constexpr uint32_t W_COLUMNS = 2 * BN;      // tensor memory: accumulators at 0 and BN, then W's parts
@@ -173,6 +234,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   const int all_blocks = (p.K + LS_K - 1) / LS_K;
   const int first_block = (int)((long long)all_blocks * part / p.parts), end_block = (int)((long long)all_blocks * (part + 1) / p.parts);
   bool gave_up = false;
+  float probe = 0.f;      // not zero: this thread has written an output that is not finite
 
   if (warp == 0) {
     if (lane == 0) {
@@ -399,7 +461,11 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
 #pragma unroll
           for (int c = 0; c < COLS; ++c) {
             const int m = m0 + side * COLS + c;
-            if (m < p.M) p.out[(size_t)m * p.N + n0 + row] = ls_output(p, sum[c], m, n0 + row);
+            if (m < p.M) {
+              const float v = ls_output(p, sum[c], n0 + row);
+              p.out[(size_t)m * p.N + n0 + row] = v;
+              probe = fmaf(v, 0.f, probe);
+            }
           }
         }
       } else {
@@ -416,9 +482,11 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
 #pragma unroll
           for (int c = t >> 6; c < STEP; c += 2) {
             const int m = m0 + side * COLS + c0 + c;
-            if (m < p.M)
-              p.out[(size_t)m * inner + out_col] = ls_gated(ls_output(p, mine[c * LS_ROWS + j], m, n0 + j),
-                                                            ls_output(p, mine[c * LS_ROWS + 64 + j], m, n0 + 64 + j));
+            if (m < p.M) {
+              const float v = ls_gated(ls_output(p, mine[c * LS_ROWS + j], n0 + j), ls_output(p, mine[c * LS_ROWS + 64 + j], n0 + 64 + j));
+              p.out[(size_t)m * inner + out_col] = v;
+              probe = fmaf(v, 0.f, probe);
+            }
           }
         }
       }
@@ -444,7 +512,10 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           if (q < p.parts) { v[0] += piece[q].x; v[1] += piece[q].y; v[2] += piece[q].z; v[3] += piece[q].w; }
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (n + e < p.N) v[e] = ls_output(p, v[e], m, n + e);
+          if (n + e < p.N) {
+            v[e] = ls_output(p, v[e], n + e);
+            if (!GATED) probe = fmaf(v[e], 0.f, probe);
+          }
         if constexpr (!GATED) {
           float* dst = p.out + (size_t)m * p.N + n;
           if ((p.N & 3) == 0) {
@@ -458,8 +529,11 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
           float r[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) r[e] = ls_gated(v[e], __shfl_down_sync(0xffffffffu, v[e], 16));
-          if (lane < 16)
+          if (lane < 16) {
             *reinterpret_cast<float4*>(p.out + (size_t)m * (p.N >> 1) + (n0 >> 1) + 4 * lane) = make_float4(r[0], r[1], r[2], r[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) probe = fmaf(r[e], 0.f, probe);
+          }
         }
       }
     }
@@ -467,10 +541,20 @@ linear_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     ls_cluster_sync();      // the others have read this CTA's sums
   }
   fa_fence_before();
-  __syncthreads();
+  const bool chains = __syncthreads_or(probe != 0.f);
   if (warp == 1) {
     fa_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Shape::TMEM_COLS) : "memory");
+  }
+  if (chains && !__syncthreads_or(gave_up)) {      // every copy has arrived and been read: the tiles' memory is free
+    float* tiles = reinterpret_cast<float*>(raw_tiles);
+    constexpr int X = BN < 64 ? 1 : 4;
+    static_assert(64 * (132 + 16 * X) * 4 <= RAW_STAGES * (size_t)LS_RAW_BYTES, "tiles of the chains");
+    const int mine = BN / p.parts;      // rows of x of this CTA's share
+    for (int item = first_item; item < items; item += item_step) {
+      const int m_begin = item / p.n_tiles * BN + part * mine;
+      ls_chains<GATED, X>(p, (item % p.n_tiles) * LS_ROWS, m_begin, min(p.M, m_begin + mine), tiles);
+    }
   }
 }
 

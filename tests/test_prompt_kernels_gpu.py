@@ -617,3 +617,40 @@ def test_products_in_parts_of_a_weight_just_written(m, n, k):
     for _ in range(20):
         w = base.clone()
         assert torch.equal(cuda().linear(x, cuda().add_inplace(w, step)), want)
+
+
+@pytest.mark.parametrize("n,k", [(1152, 896), (9728, 200), (896, 4864), (20100, 132), (33, 30000)])
+@pytest.mark.parametrize("m", [1, 17, 40, 300])
+def test_products_in_parts_whose_outputs_are_all_no_numbers(m, n, k):
+    """Every output through the chains over k: values, and a time that is a batch's on the CUDA cores and not a thread's per output (a
+    few microseconds per 64 k, where a CTA's steps over k follow one another)."""
+    def timed(x):
+        best = float("inf")
+        for _ in range(3):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            got = cuda()._linear_split(x, w, bias)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end))
+        cuda().raise_if_device_error()
+        return got, best
+
+    x, w, bias = rnd(1, m, k).to(DEVICE), rnd(2, n, k, std=0.2).to(DEVICE), rnd(3, n).to(DEVICE)
+    w[n // 2], w[n // 3, k - 1] = 0.0, -w[n // 3, k - 1]
+    fine, plain = timed(x)
+    broken = x.clone()
+    broken[:, k - 1] = float("inf")
+    got, took = timed(broken)
+    assert torch.equal(torch.isnan(got), (w[:, k - 1] == 0).expand(m, n))
+    assert torch.equal(got == float("inf"), (w[:, k - 1] > 0).expand(m, n)) and torch.equal(got == -float("inf"), (w[:, k - 1] < 0).expand(m, n))
+    assert took <= 20 * plain + 0.1 + 1e-4 * k, (took, plain)
+    if n % 128 == 0:
+        assert torch.equal(cuda()._linear_split(broken, w, None, gated=True).nan_to_num(7.0),
+                           cuda().swiglu(cuda()._linear_split(broken, w, None), 64).nan_to_num(7.0))
+    broken.fill_(float("nan"))
+    got, took = timed(broken)
+    assert bool(torch.isnan(got).all()) and took <= 20 * plain + 0.1 + 1e-4 * k, (took, plain)
+    x[m // 2, 0] = float("nan")                     # one row: the others keep their bits
+    got, others = timed(x)[0], torch.arange(m, device=DEVICE) != m // 2
+    assert bool(torch.isnan(got[m // 2]).all()) and torch.equal(got[others], fine[others])
