@@ -244,6 +244,7 @@ class CudaOps:
 
     def __init__(self) -> None:
         self._workspaces: dict[int, dict[str, torch.Tensor]] = {}
+        self._error_words: dict[int, torch.Tensor] = {}
         # Switches for tests and measurements: each takes one kernel family out, and the next one
         # in line (see the dispatch in linear / paged_attention) serves instead.
         self.use_tensor_cores = True
@@ -264,6 +265,14 @@ class CudaOps:
         self.decode_chunk: int | None = None      # None: chosen per call from the batch's shape
         self.decode_max_splits: int | None = None  # None: just enough for the longest context
 
+    def _error_word(self, device: torch.device) -> torch.Tensor:
+        """Written by a kernel whose bounded wait ran out; read by the host without a copy.  It is host memory alone, so that the first
+        call of a kernel that needs nothing else may be captured: a workspace made then would hold its zeros only after a replay."""
+        index = device.index if device.type == "cuda" and device.index is not None else torch.cuda.current_device()
+        if index not in self._error_words:
+            self._error_words[index] = torch.zeros(1, dtype=torch.int32).pin_memory()
+        return self._error_words[index]
+
     def _workspace(self, device: torch.device) -> dict[str, torch.Tensor]:
         index = device.index if device.type == "cuda" and device.index is not None else torch.cuda.current_device()
         if index not in self._workspaces:
@@ -274,8 +283,7 @@ class CudaOps:
                 "attention_counters": torch.zeros(self.ATTENTION_COUNTERS, dtype=torch.int32, device=device),
                 "attention_scratch": torch.empty(self.ATTENTION_SCRATCH_BYTES, dtype=torch.uint8, device=device),
                 "sm_count": torch.cuda.get_device_properties(device).multi_processor_count,
-                # written by a kernel whose bounded wait ran out; read by the host without a copy
-                "error_word": torch.zeros(1, dtype=torch.int32).pin_memory(),
+                "error_word": self._error_word(device),
                 "prefill_queue": torch.zeros(2, dtype=torch.int32, device=device),
                 # states of prompt-attention items that are cut into parts, and one counter per item
                 "prefill_scratch": torch.empty(64 << 20, dtype=torch.uint8, device=device),
@@ -287,12 +295,14 @@ class CudaOps:
         """Call after a synchronisation point: raises if a kernel gave up on a bounded wait.  Such
         a kernel may have left its work queue and its split counters half-used, which every later
         launch would trip over, so they are cleared before the exception leaves."""
-        for space in self._workspaces.values():
-            code = int(space["error_word"][0])
+        for index, word in self._error_words.items():
+            code = int(word[0])
             if code != 0:
-                space["error_word"][0] = 0
+                word[0] = 0
+                space = self._workspaces.get(index, {})
                 for name in ("gemm_counters", "attention_counters", "prefill_queue", "prefill_counters"):
-                    space[name].zero_()
+                    if name in space:
+                        space[name].zero_()
                 raise KernelError(f"a kernel's bounded wait ran out (code {code}); the results of the "
                                   "steps since the last check are invalid")
 
@@ -656,7 +666,7 @@ class CudaOps:
         rows = lib.mlr_linear_split_rows(M, K)
         parts = torch.empty((3, rows, -(-K // 8) * 8), dtype=torch.bfloat16, device=x.device) if rows else None
         _check(lib.mlr_linear_split(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), M, N, K, int(gated), _ptr(parts),
-                                    _ptr(self._workspace(x.device)["error_word"]), _stream()), "linear (32-bit operands in parts)")
+                                    _ptr(self._error_word(x.device)), _stream()), "linear (32-bit operands in parts)")
         return out
 
     def _linear_simt(self, x, weight, bias, out_dtype):
@@ -2048,7 +2058,7 @@ class CudaOps:
             _check(lib.mlr_delta_rule_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(scratch), _ptr(state), _ptr(y), _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len),
                 _ptr(ctx.seg_slot), ctx.num_segments, rows, below, chunks, int(longest > 0), heads, kv_heads, dim, vdim,
-                ctypes.c_float(unit_eps), ctypes.c_float(float(dim) ** -0.5), _ptr(self._workspace(q.device)["error_word"]), _stream()),
+                ctypes.c_float(unit_eps), ctypes.c_float(float(dim) ** -0.5), _ptr(self._error_word(q.device)), _stream()),
                 "delta_rule_chunks")
         return y
 

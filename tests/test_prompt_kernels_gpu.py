@@ -654,3 +654,27 @@ def test_products_in_parts_whose_outputs_are_all_no_numbers(m, n, k):
     x[m // 2, 0] = float("nan")                     # one row: the others keep their bits
     got, others = timed(x)[0], torch.arange(m, device=DEVICE) != m // 2
     assert bool(torch.isnan(got[m // 2]).all()) and torch.equal(got[others], fine[others])
+
+
+def test_a_first_call_in_32_bits_may_be_captured():
+    """A set of operations whose first calls are captured: no workspace is made inside a graph, where its counters would be zero only after
+    a replay, and the products in bfloat16 that come next find theirs as they should be."""
+    fresh = type(cuda())()
+    x, w = rnd(1, 8, 896).to(DEVICE), rnd(2, 1152, 896, std=0.2).to(DEVICE)
+    ctx, rows = segments([600], [0]), 600
+    q, k, v, a, b, bias, a_log = (t.to(DEVICE) for t in delta_inputs(rows, 4, 2, 64, 64, False))
+    state = torch.zeros(1, 4, 64, 64, device=DEVICE)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        product = fresh.linear(x, w)
+        y = fresh.delta_rule_scan(q, k, v, a, b, bias, a_log, state, ctx, 4, 2, 64, 64, 1e-6)
+    assert not fresh._workspaces
+    rows = rnd(3, 64, 4864).to(DEVICE, torch.bfloat16), rnd(4, 896, 4864, std=0.02).to(DEVICE, torch.bfloat16)
+    assert torch.equal(fresh.linear(*rows), cuda().linear(*rows))          # sums in parts, counted
+    graph.replay()
+    torch.cuda.synchronize()
+    fresh.raise_if_device_error()
+    assert torch.equal(product, cuda().linear(x, w))
+    other = torch.zeros_like(state)
+    assert torch.equal(y, cuda().delta_rule_scan(q, k, v, a, b, bias, a_log, other, ctx, 4, 2, 64, 64, 1e-6)) and torch.equal(state, other)
