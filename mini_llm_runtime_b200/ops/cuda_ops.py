@@ -639,7 +639,7 @@ class CudaOps:
         scratch, counters = space["gemm_scratch"], space["gemm_counters"]
         status = _declared_library("gemm_tcgen05").mlr_gemm_tcgen05(
             x.data_ptr(), weight.data_ptr(), _address(bias), out.data_ptr(), M, N, K, int(out_dtype == torch.float32), int(swiglu),
-            gate[0], gate[1], scratch.data_ptr(), self.GEMM_SCRATCH_BYTES, counters.data_ptr(), self.GEMM_COUNTERS,
+            gate[0], gate[1], scratch.data_ptr(), scratch.numel(), counters.data_ptr(), counters.numel(),
             space["error_word"].data_ptr(), _raw_stream())
         if status == _NO_ROOM:      # its partial tiles do not fit the scratch memory
             return None

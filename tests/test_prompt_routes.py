@@ -2,8 +2,11 @@
 
 from __future__ import annotations
 
+import types
+
 import numpy as np
 import pytest
+import torch
 
 from mini_llm_runtime_b200.ops import AttentionBatch
 from mini_llm_runtime_b200.ops import cuda_ops
@@ -34,3 +37,19 @@ def test_decoded_rows_contexts_do_not_move_the_borders(decoded):
         assert cuda_ops.diff_prompt_on_tcgen05(b, rows, 0, 0) == diff, (lengths, before)
         # a window shorter than the border hides the keys behind it
         assert cuda_ops.latent_prompt_on_tcgen05(b, rows, 50) == (rows - len(ones) > 64), (lengths, before)
+
+
+def test_a_product_is_told_the_room_that_its_workspace_has(monkeypatch):
+    """The kernel refuses plans that do not fit; what counts is the memory there is, not what a workspace made later would get."""
+    asked = []
+    library = types.SimpleNamespace(mlr_gemm_tcgen05=lambda *args: asked.append((args[12], args[14])) or cuda_ops._NO_ROOM)
+    monkeypatch.setattr(cuda_ops, "_declared_library", lambda name: library)
+    monkeypatch.setattr(cuda_ops, "_raw_stream", lambda: 0)
+    operations = cuda_ops.CudaOps()
+    space = {"gemm_scratch": torch.empty(512, dtype=torch.uint8), "gemm_counters": torch.zeros(7, dtype=torch.int32),
+             "error_word": torch.zeros(1, dtype=torch.int32)}
+    monkeypatch.setattr(operations, "_workspace", lambda device: space)
+    operations.GEMM_SCRATCH_BYTES = operations.GEMM_COUNTERS = 1 << 20
+    x, w = torch.zeros(64, 128, dtype=torch.bfloat16), torch.zeros(256, 128, dtype=torch.bfloat16)
+    assert operations._linear_tcgen05(x, w, None, torch.bfloat16) is None
+    assert asked == [(512, 7)]
