@@ -198,8 +198,9 @@ chunk_walk_kernel(ChunkArgs p) {
 }
 
 // A thread owns four neighbouring value channels of one key channel and takes the chunks of its segment in order; BATCH chunks
-// are asked for together.  Bound by round trips to the L2, where most of the states lie (2,048 rows of 14 heads of 64, all three launches:
-// 64.6 us with batches of 8, 63.0 with 16).
+// are asked for together.  Bound by round trips to the L2, where most of the states lie.  All launches from a flushed L2, batches of
+// 8 / 16: 14 heads of 64 66.6 / 65.4 us at 2,048 rows and 116.5 / 112.1 at 4,000, 32 heads 118.4 / 115.9 and 209 / 207, 16 heads of 128 162.9 / 156.8 and
+// 291 / 283; segments of few chunks pay for the registers, 200 rows of 32 heads of 64 38.2 / 39.6, 512 rows of 14 39.8 / 40.2.
 __global__ void __launch_bounds__(256)
 chunk_carry_kernel(ChunkArgs p, int dim, int vdim) {
   constexpr int BATCH = 16;

@@ -306,8 +306,9 @@ space_local_kernel(SpaceArgs p) {
   if (chunk == 0) read_state<N>(p, s_b, shared, first, count, head);
 }
 
-// A thread owns four neighbouring entries and takes the chunks of its segment in order; BATCH chunks are asked for together (8: 126.4 us
-// for 1,531 + 77 + 1 + 439 rows of 32 heads, all launches; 16: 125.4).
+// A thread owns four neighbouring entries and takes the chunks of its segment in order; BATCH chunks are asked for together.
+// All launches from a flushed L2, batches of 8 / 16: 32 heads 132.4 / 128.0 us at 2,048 rows, 235 / 223 at 4,000, 128.4 / 126.7 for 1,531 + 77 + 1 + 439; 14
+// heads 59.8 / 58.3 and 97.8 / 89.5; segments of few chunks pay for the registers, 512 rows of 14 heads 37.3 / 38.8.
 __global__ void __launch_bounds__(256)
 space_carry_kernel(SpaceArgs p, int cells) {
   constexpr int BATCH = 16;

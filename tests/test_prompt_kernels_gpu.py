@@ -678,3 +678,26 @@ def test_a_first_call_in_32_bits_may_be_captured():
     assert torch.equal(product, cuda().linear(x, w))
     other = torch.zeros_like(state)
     assert torch.equal(y, cuda().delta_rule_scan(q, k, v, a, b, bias, a_log, other, ctx, 4, 2, 64, 64, 1e-6)) and torch.equal(state, other)
+
+
+@pytest.mark.parametrize("lengths", [[576, 577, 640], [1088, 1089, 65], [2177]])
+def test_states_carried_over_many_chunks(lengths):
+    """Segments around the numbers of chunks that the carrying kernels ask for at a time: one turn, two and three."""
+    ctx, rows, heads, n = segments(lengths, list(reversed(range(len(lengths)))), None), sum(lengths), 3, 64
+    inner, bound = heads * 64, 200 * UNIT
+    x, B, C, dt = rnd(1, rows, inner), rnd(2, rows, n), rnd(3, rows, n), rnd(4, rows, heads, std=2.0)
+    vectors = rnd(5, heads), rnd(6, heads), rnd(7, heads)
+    state = rnd(8, len(lengths), heads, 64, n, std=0.5)
+    want_state, got_state = state.double(), state.to(DEVICE)
+    want = FAKE.state_space_scan(*(t.double() for t in (x, B, C, dt, *vectors)), want_state, ctx, heads, 64, n, 1)
+    got = cuda().state_space_scan(*(spaced(t) for t in (x, B, C, dt)), *(t.to(DEVICE) for t in vectors), got_state, ctx, heads, 64, n, 1)
+    close(got, want, bound, "state-space outputs")
+    close(got_state.flatten(0, 1), want_state.flatten(0, 1), bound, "state-space state")
+    r, k, v, gate, raw = (rnd(10 + i, rows, inner, std=0.7) for i in range(5))
+    bias, bonus, weight = rnd(16, inner) * 2 - 2, rnd(17, inner, std=0.3), 1 + rnd(18, inner, std=0.1)
+    want_state, got_state = state.double(), state.to(DEVICE)
+    want = FAKE.bonus_recurrence(*(t.double() for t in (r, k, v, raw, gate, bias, bonus, weight)), 1e-6, want_state, ctx, heads, 64, torch.float32)
+    got = cuda().bonus_recurrence(*(spaced(t) for t in (r, k, v, raw, gate)), *(t.to(DEVICE) for t in (bias, bonus, weight)), 1e-6, got_state, ctx,
+                                  heads, 64, torch.float32)
+    close(got, want, bound, "recurrence outputs")
+    close(got_state.flatten(0, 1), want_state.flatten(0, 1), bound, "recurrence state")
