@@ -457,6 +457,11 @@ def test_products_in_parts(m, n, k):
     ops_.raise_if_device_error()
     bound = (k / 64 + 48) * UNIT * (x.abs() @ w.abs().T + bias.abs())
     assert bool(((got.double() - (x.double() @ w.double().T + bias.double())).abs() <= bound.double()).all())
+    # .. and in the 2-norm, where roundings average out: 1.1e-7 is what float32 itself gives; without the products of second and third parts 4e-6
+    exact = x.double() @ w.double().T
+    error, simt = ((t.double() - exact).norm(dim=1) / exact.norm(dim=1) for t in (ops_._linear_split(x, w, None),
+                                                                                   ops_._linear_simt(x, w, None, torch.float32)))
+    assert float(error.max()) <= 4e-7 and (k < 800 or float(error.mean()) <= float(simt.mean())), (float(error.max()), float(simt.mean()))
     assert torch.equal(ops_._linear_split(shifted, w, bias), got)          # x on no 16-byte boundary
     for first in {0, m // 2, m - 1}:
         assert torch.equal(ops_._linear_split(x[first:first + 1].contiguous(), w, bias), got[first:first + 1])
@@ -701,3 +706,59 @@ def test_states_carried_over_many_chunks(lengths):
                                   heads, 64, torch.float32)
     close(got, want, bound, "recurrence outputs")
     close(got_state.flatten(0, 1), want_state.flatten(0, 1), bound, "recurrence state")
+
+
+@pytest.mark.parametrize("m", [9, 27, 60, 200])
+@pytest.mark.parametrize("places", [(0, 1, 2), (3, 40, 17), (63, 64, 895), (500, 130, 129)])
+def test_products_in_parts_take_each_product_of_parts(m, places):
+    """Numbers of one to three parts (1, 2^-9 and 2^-18 beside it) whose leading products cancel, so that what is left is one product of
+    smaller parts; those left out are 2^-27 and less, every sum is exact."""
+    n, k, (a, b, c) = 1152, 896, places
+    x, w = torch.zeros(m, k), torch.zeros(n, k)
+    numbers = torch.tensor([1.0, 1 + 2.0 ** -18, 1 + 2.0 ** -9, 1 + 2.0 ** -9 + 2.0 ** -18])
+    x[:, a], x[:, b], x[:, c] = numbers[torch.arange(m) % 4], -1.0, torch.where(torch.arange(m) % 3 == 0, -2.0 ** -8, 0.0)
+    w[:, a], w[:, b], w[:, c] = numbers[torch.arange(n) % 4], 1.0, 1.0
+    got, want = cuda()._linear_split(x.to(DEVICE), w.to(DEVICE), None).double().cpu(), x.double() @ w.double().T
+    assert float((got - want).abs().max()) <= 3 * 2.0 ** -27
+
+
+@pytest.mark.parametrize("m,n,k,gated", [(641, 33, 30000, False), (1300, 33, 30000, False), (672, 256, 30000, True)])
+def test_products_in_parts_of_rows_in_blocks(m, n, k, gated):
+    """More rows than have their parts in scratch at a time (640 of 30,000 k): blocks of rows with the bits of calls of their own, the last of one
+    row, of 20 and of 32."""
+    x, w, bias = (t.to(DEVICE) for t in (rnd(1, m, k), rnd(2, n, k, std=0.02), rnd(3, n)))
+    product = lambda rows: cuda()._linear_split(rows, w, None if gated else bias, gated=gated)      # noqa: E731
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    start = torch.cuda.memory_allocated()
+    whole = product(x)
+    extra = torch.cuda.max_memory_allocated() - start - whole.numel() * 4
+    assert extra <= 129 << 20, extra
+    exact = x.double() @ w.double().T
+    if gated:
+        gate, up = exact.view(m, -1, 2, 64).unbind(2)
+        exact = (torch.nn.functional.silu(gate) * up).reshape(m, -1)
+    else:
+        exact += bias.double()
+    assert float((whole.double() - exact).norm() / exact.norm()) <= 1e-6
+    for first, rows in ((0, 640), (640, min(m, 1280) - 640), (m - 1, 1), (m - 20, 20), (630, 11)):
+        assert torch.equal(product(x[first:first + rows].contiguous()), whole[first:first + rows]), first
+
+
+@pytest.mark.parametrize("n,k", [(16400, 73), (3000, 4101)])
+def test_products_that_the_tensor_cores_do_not_take(n, k):
+    """Rows of no whole 16-byte pieces: the product on the CUDA cores, more than 16,384 outputs, long sums in parts of many rows in blocks."""
+    m = 4000 if k > 4000 else 300
+    x, w, bias = (t.to(DEVICE) for t in (rnd(1, m, k), rnd(2, n, k, std=0.2), rnd(3, n)))
+    assert not cuda()._split_fits(x, w)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    start = torch.cuda.memory_allocated()
+    whole = cuda().linear(x, w, bias)
+    extra = torch.cuda.max_memory_allocated() - start - whole.numel() * 4
+    assert extra <= 129 << 20, extra
+    for first, rows in ((0, 64), (m // 3, 100), (m - 63, 63), (m - 1, 1)):
+        exact = x[first:first + rows].double() @ w.double().T + bias.double()
+        assert bool(((whole[first:first + rows].double() - exact).abs()
+                     <= k * UNIT * (x[first:first + rows].abs() @ w.abs().T + bias.abs()).double()).all())
+        assert torch.equal(cuda().linear(x[first:first + rows].contiguous(), w, bias), whole[first:first + rows]), first
