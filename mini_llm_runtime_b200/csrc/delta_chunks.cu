@@ -18,8 +18,9 @@
 // 1.11 / 1.12.  It costs 12 us of 2,048 rows of the 32 heads, 6 of the 14.
 //
 // Measured (B200), token by token / in chunks: 2,048 rows of 32 heads of 128 x 64 340 / 191 us, from a flushed L2 347 / 206 (first kernel
-// 71, second 83, third 48), of 14 heads of 64 x 64 214 / 105 (23, 62, 16).  The first and the last kernel are bound by instructions (splitting operands,
-// decays) and shared memory, the chain by the latency of its steps, 4,500 cycles per chunk, of which 1,900 are MMAs.
+// 71, second 83, third 48), of 14 heads of 64 x 64 214 / 105 (23, 62, 16).  The first kernel waits for shared memory (chains of reads of
+// triangles and decays) and for its code, the chain is the latency of its steps, 4,800 cycles per chunk, of which the tensor pipe is busy for
+// 1,900, the last waits for its loads.
 //
 // The first two kernels do not bring in the next one early: its waiting CTAs slow them down (512 rows of 14 heads of 64 x 64: the first
 // kernel 17 -> 25 us, all three 46 -> 56; of 32 heads of 128 x 64 71 -> 77).

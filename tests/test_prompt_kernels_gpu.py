@@ -605,6 +605,12 @@ def test_delta_rule_at_the_border_of_chunks(heads, kv_heads, dim, vdim, known, m
         close(got, want, 200 * UNIT, "delta rule outputs")
         close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "delta rule state")
         assert torch.equal(following, got * 2)
+    graph, captured_state = torch.cuda.CUDAGraph(), state.to(DEVICE)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        captured = cuda().delta_rule_scan(q, k, v, a, b, bias, a_log, captured_state, ctx, heads, kv_heads, dim, vdim, 1e-6) * 2
+    graph.replay()
+    assert torch.equal(captured, following) and torch.equal(captured_state, got_state)
     for part in parts:
         at, own_state = slice(part.row_start, part.row_start + part.length), state.to(DEVICE)
         own = cuda().delta_rule_scan(*(t[at] for t in (q, k, v, a, b)), bias, a_log, own_state, segments([part.length], [part.slot]), heads,
