@@ -651,6 +651,7 @@ class CudaOps:
     # at 1, 8, 24, 60, 100, 600, 1,500 rows: [1024, 512] 4 5 8 18 25 33 49 / 6 6 7 11 15 16 29; [896, 896] 6.5 7.5 12 21 42 79 83 / 6.0 6.2 6.9
     # 10 12 23 36; [2048, 2048] 15 19 28 63 82 163 348 / 9 10 10 14 18 49 98; [9728, 896] 14 23 43 57 83 294 664 / 13 13 15 19 26 64 142.
     # Short sums of very many outputs pay at few rows: [20000, 132] 6.1 6.9 12 18 28 97 225 / 7.8 8.7 11 16 25 60 122.
+    # Whole decode steps of the 0.5B sizes in 32 bits, 1, 8 and 32 requests: 3,256 3,831 6,412 / 2,961 2,897 3,147.
     SPLIT_WEIGHT = 3 << 18
 
     def _split_fits(self, x, weight) -> bool:
