@@ -55,6 +55,7 @@ LIBRARIES: dict[str, tuple[str, ...]] = {
     "routed_experts": (),
     "attention_sigmoid": (),
     "attention_sigmoid_mma": (),
+    "attention_sigmoid_tcgen05": (),
     "state_space": (),
     "state_space_chunks": (),
     "delta_rule": (),

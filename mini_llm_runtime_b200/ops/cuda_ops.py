@@ -86,6 +86,8 @@ _PROTOTYPES = {
     "gemm_tcgen05": {"mlr_gemm_tcgen05": "ppppiiiiiffplpipp"},
     "elementwise": {"mlr_rms_norm": "ppppiifiip", "mlr_rope_kv_write": "pppppppiiiiiiip"},
     "attention_tcgen05": {"mlr_attention_prefill_tcgen05": "ppppppppppp" "iiiiiiiii" "fi" "ppp" "l" "pip"},
+    "attention_sigmoid_tcgen05": {"mlr_attention_sigmoid_tcgen05": "ppppp" "ppppppp" "iiiiiiii" "f" "pppp" "iii" "pp",
+                                  "mlr_attention_sigmoid_tcgen05_scratch": "iiiii"},
 }
 _CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
 _declared: dict[str, ctypes.CDLL] = {}
@@ -1752,6 +1754,26 @@ class CudaOps:
         tiles = batch.counts["tiles"]
         if (self.use_mma_sigmoid and self.use_mma_attention and q.dtype == torch.bfloat16 and dim in (64, 128)
                 and vdim in (64, 128) and q.data_ptr() % 16 == 0):
+            wide = _declared_library("attention_sigmoid_tcgen05")
+            if (self.use_tcgen05_attention and int(batch.max_kv_len) > dim // 2 and k_pool.data_ptr() % 16 == 0
+                    and v_pool.data_ptr() % 16 == 0 and tiles <= wide.mlr_attention_sigmoid_tcgen05_most()
+                    and wide.mlr_attention_sigmoid_tcgen05_fits(heads, kv_heads, dim, vdim, k_pool.shape[2])):
+                # both products on tcgen05.  Its tiles have 128 keys whatever the rows see, so the shortest contexts stay where they were:
+                # us with mma.sync / so, 16 heads of 128, 1 row that sees 21 keys 9 / 18, 8 rows 48 keys 15 / 18, 60 rows 17 / 20, 1 row 65 keys 20 / 18,
+                # 90 rows 23 / 20; 14 heads of 64, 1 row 21 keys 8 / 12, 8 rows 48 keys 13 / 12, 60 rows 16 / 14
+                most = -(-int(batch.max_kv_len) // 128)      # key tiles of an entry
+                ctas = min(self.sm_count(q.device), tiles * most)
+                wide.mlr_attention_sigmoid_tcgen05_scratch.restype = ctypes.c_longlong
+                scratch = torch.empty(wide.mlr_attention_sigmoid_tcgen05_scratch(tiles, ctas, int(batch.max_q_len), heads, vdim),
+                                      dtype=torch.float32, device=q.device)
+                plan = batch.plan
+                _check(wide.mlr_attention_sigmoid_tcgen05(
+                    q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(), scratch.data_ptr(), plan["tile_seg"].data_ptr(),
+                    plan["tile_row0"].data_ptr(), batch.seg_q_start.data_ptr(), batch.seg_q_len.data_ptr(), batch.seg_pos0.data_ptr(),
+                    batch.block_table.data_ptr(), _address(batch.seg_slot), batch.block_table.shape[1], tiles, heads, kv_heads, dim, vdim,
+                    k_pool.shape[2], k_pool.shape[0], scale, _address(r1), _address(r2), _address(score_bias), _address(head_mix), ctas, most,
+                    int(batch.max_q_len), self._error_word(q.device).data_ptr(), _raw_stream()), "sigmoid attention (tcgen05)")
+                return out
             mma = build.load_library("attention_sigmoid_mma")
             if mma.mlr_attention_sigmoid_mma_fits(heads, kv_heads, dim, vdim):
                 # one CTA per entry of 16 rows and chunk of keys: steps of few rows share a row's keys out over

@@ -211,6 +211,51 @@ def test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, mixed):
     close(got, want, ATTENTION_BOUND, "sigmoid attention")
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,page_size", [(16, 4, 128, 128, 8), (14, 2, 64, 64, 16), (9, 3, 128, 64, 64), (5, 1, 64, 128, 256),
+                                                               (4, 4, 64, 64, 128)])
+@pytest.mark.parametrize("lengths,before", [([129], [0]), ([16, 1, 8], [112, 640, 300]), ([1] * 7, [127, 128, 63, 64, 1000, 200, 500]),
+                                            ([70, 260, 9, 1], [250, 0, 127, 383])])
+def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, lengths, before):
+    """Keys around tiles of 128 and their halves, rows around the 8 of half an entry, entries cut and whole, pages smaller and larger than a
+    tile and its halves, heads that do not fill fours; places that no row sees hold NaN.  Mixing factors large enough that what mixing in fewer
+    than 32 bits would leave of the weights shows.  The second call finds the first one's scratch."""
+    (k_pool, v_pool), cpu, batch = paged(lengths, before, lambda p, j: j <= p, page_size, [(kv_heads, dim, 1.0), (kv_heads, vdim, 0.5)], 11)
+    assert cuda().use_tcgen05_attention and cuda_ops.build.load_library("attention_sigmoid_tcgen05").mlr_attention_sigmoid_tcgen05_fits(
+        heads, kv_heads, dim, vdim, page_size)
+    q = rnd(6, sum(lengths), heads * dim).to(torch.bfloat16)
+    vectors = dict(distance=(torch.rand(heads, generator=generator(1)), torch.rand(heads, generator=generator(2))), score_bias=rnd(3, heads, std=0.3),
+                   head_mix=rnd(4, heads, heads))
+    args = (heads, kv_heads, dim, vdim, dim ** -0.5)
+    want = FAKE.sigmoid_attention(q.float(), k_pool.float(), v_pool.float(), cpu, *args, **vectors)
+    there = {k: tuple(t.to(DEVICE) for t in v) if isinstance(v, tuple) else v.to(DEVICE) for k, v in vectors.items()}
+    first = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, **there)
+    got = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, **there)
+    torch.cuda.synchronize()
+    cuda().raise_if_device_error()
+    # mixed weights and results are rounded to 8 bits, 2^-9 each at most; mixed with signs, weights lose size against the keys' sum of squares no
+    # more than in ATTENTION_BOUND's own margin
+    close(got, want, ATTENTION_BOUND, "sigmoid attention")
+    assert torch.equal(first, got)
+
+
+def test_heads_mixed_by_parts_are_mixed_in_32_bits():
+    """Weights that cancel in the mixing, to results that 16 bits of them would not show: twelve equal heads, factors whose sum is 2^-12."""
+    heads, dim, rows = 12, 64, 40
+    (k_pool, v_pool), cpu, batch = paged([rows], [100], lambda p, j: j <= p, 16, [(1, dim, 1.0), (1, dim, 0.5)], 12)
+    q = rnd(6, rows, 1, dim).expand(rows, heads, dim).reshape(rows, heads * dim).to(torch.bfloat16)
+    mix = rnd(4, heads, heads)
+    mix[:, -1] += 2.0 ** -12 - mix.double().sum(1).float()
+    mix[:, -1] += (2.0 ** -12 - mix.double().sum(1)).float()
+    args = (heads, 1, dim, dim, dim ** -0.5)
+    sums = mix.double().sum(1)
+    plain = FAKE.sigmoid_attention(q.double(), k_pool.double(), v_pool.double(), cpu, *args).double().view(rows, heads, dim)
+    want = (plain[:, :1] * sums[None, :, None]).reshape(rows, heads * dim)
+    got = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, head_mix=mix.to(DEVICE))
+    # a mixed weight is a sum of twelve products of numbers around one, each rounded to 2^-24 (the tensor cores' sums drop as much), beside a result
+    # of 2^-12 / 2: below 12 * 2 * 2^-24 / 2^-13 = 2^-6.4 of it, independent from key to key
+    close(got, want, ATTENTION_BOUND + 2.0 ** -6.4, "mixed weights")
+
+
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 128), (3, 64, 72)])
 @pytest.mark.parametrize("lengths,slots,order", [([1, 512, 513, 1100], [3, 0, 2, 1], None), ([515, 3, 1030], [1, 2, 0], [2, 0, 1])])
 def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
