@@ -2129,8 +2129,9 @@ class CudaOps:
 
     use_state_space_chunks = True
     # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us, token by
-    # token / in chunks: 128 rows 30 / 31 (14 heads, states of 64), 42 / 50 (32 heads, states of 128); 512 rows 108 / 31, 161 / 64.
-    STATE_SPACE_CHUNK_ROWS = 192
+    # token / in chunks, 14 heads with states of 64 (32 heads, 128): 77 rows 18 / 24 (26 / 32), 96 rows 22 / 24 (32 / 33), 112 rows 25 / 24 (37 / 33), 160 rows
+    # 35 / 26 (52 / 35), 512 rows 108 / 24 (161 / 39); three of 100 rows beside one of 1,000 57 / 34 (95 / 81).
+    STATE_SPACE_CHUNK_ROWS = 97
 
     def state_space_scan(self, x, B, C, dt_raw, dt_bias, A_log, D, state, ctx, heads: int, vdim: int, n: int,
                          groups: int) -> torch.Tensor:
@@ -2149,16 +2150,17 @@ class CudaOps:
         y = torch.empty((rows, heads * vdim), dtype=torch.float32, device=x.device)
         views = (*self._view(x, "x", rows, heads * vdim), *self._view(B, "B", rows, groups * n),
                  *self._view(C, "C", rows, groups * n), *self._view(dt_raw, "dt_raw", rows, heads))
-        if (self.use_state_space_chunks and ctx.max_q_len >= self.STATE_SPACE_CHUNK_ROWS and vdim == 64 and n in (64, 128)
+        least = max(self.STATE_SPACE_CHUNK_ROWS, 65)      # one chunk is token by token's
+        if (self.use_state_space_chunks and ctx.max_q_len >= least and vdim == 64 and n in (64, 128)
                 and all(t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0 for t in (x, B, C)) and state.data_ptr() % 16 == 0):
             # long segments: chunks of tokens side by side
             lib = build.load_library("state_space_chunks")
             lib.mlr_state_space_chunk_scratch.restype = ctypes.c_longlong
-            scratch = torch.empty(lib.mlr_state_space_chunk_scratch(rows, heads, n, groups), dtype=torch.float32, device=x.device)
+            scratch = torch.empty(lib.mlr_state_space_chunk_scratch(rows, ctx.num_segments, least, heads, n, groups), dtype=torch.float32, device=x.device)
             _check(lib.mlr_state_space_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(D), _ptr(state), _ptr(y), _ptr(scratch), _ptr(ctx.seg_q_start),
-                _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), self.STATE_SPACE_CHUNK_ROWS,
-                int(self._longest_below(ctx, self.STATE_SPACE_CHUNK_ROWS) > 0), heads, vdim, n, groups, _stream()), "state_space_chunks")
+                _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), least,
+                int(self._longest_below(ctx, least) > 0), heads, vdim, n, groups, _stream()), "state_space_chunks")
             return y
         _check(build.load_library("state_space").mlr_state_space_scan(
             *views, _ptr(dt_bias), _ptr(A_log),

@@ -128,6 +128,35 @@ def test_state_space_in_chunks(heads, n, groups, lengths, slots, order, monkeypa
     close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "state-space state")
 
 
+@pytest.mark.parametrize("heads,n,groups", [(2, 64, 1), (4, 128, 2)])
+@pytest.mark.parametrize("where", ["x", "B", "C", "state", "before"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+def test_state_space_chunks_with_numbers_that_have_no_parts(heads, n, groups, where, value):
+    """One such number among ordinary ones goes by multiply-adds in its chunk: outputs that are no numbers where token by token has them, the
+    others as there.  ``before``: a state that only later chunks see."""
+    lengths, slots = [130, 65], [1, 0]
+    ctx, rows, inner = segments(lengths, slots), sum(lengths), heads * 64
+    x, B, C, dt = rnd(1, rows, inner), rnd(2, rows, groups * n), rnd(3, rows, groups * n), rnd(4, rows, heads, std=0.5) - 3
+    state = rnd(8, 2, heads, 64, n, std=0.5)
+    {"x": x, "B": B, "C": C, "state": state[1, 0], "before": x}[where][70 if where in ("x", "B", "C") else 3, 5] = value
+    vectors = rnd(5, heads), rnd(6, heads), rnd(7, heads)
+    results = []
+    for chunks in (False, True):
+        cuda().use_state_space_chunks = chunks
+        try:
+            s = state.to(DEVICE)
+            y = cuda().state_space_scan(*(spaced(t) for t in (x, B, C, dt)), *(v.to(DEVICE) for v in vectors), s, ctx, heads, 64, n, groups)
+        finally:
+            cuda().use_state_space_chunks = True
+        results.append((y.cpu().double(), s.cpu().double()))
+    for want, got in zip(*results):
+        # beside 3.4e38 sums overflow in one order and not in the other; the outputs and states that it has no part in are ordinary
+        if value != 3.4e38:
+            assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+        normal = torch.isfinite(want) & (want.abs() < 1e30)
+        assert float((got[normal] - want[normal]).norm()) <= 200 * UNIT * float(want[normal].norm())
+
+
 def paged(lengths, before, visible, page_size, pools, seed):
     """Pools [pages, heads, page_size, entries] and the batch, on the CPU and on the device.  Page 0 belongs to nobody; it and every
     place that no row of its request sees (``visible(position, key)``) hold NaN, and pages without a visible key are given back."""
