@@ -139,7 +139,7 @@ struct GemmParams {
   // the stacked matrix [groups * N, K]; rows at or beyond the end row are computed and not written;
   // an entry whose group is negative is unused.  The list is device memory written by an earlier kernel.
   const int* group_tiles;
-  const float* row_scale;    // grouped form: factor of every row's product (before the gate), or null
+  const float* row_scale;    // grouped form: factor of every row's product, or null
 };
 
 constexpr int MAX_STAGES = 8;
@@ -331,7 +331,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int stages = p.stages;
   // grouped form: the grid is (column tiles, row tiles), so that the CTAs that share a row tile's
   // activations run together; every weight tile of a group is read by one CTA per row tile anyway
-  const bool grouped = !SWAP && !PAIR && p.group_tiles != nullptr;
+  const bool grouped = !SWAP && !PAIR && !SWIGLU && p.group_tiles != nullptr;
   const int tile_x = grouped ? blockIdx.y : blockIdx.x;
   const int tile_y = grouped ? blockIdx.x : blockIdx.y;
   int a_row0 = tile_x * BM;                    // first row of the 128-row (or 256-row) operand
@@ -532,14 +532,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           tmem_issue_load16(from + 64 + c0 + 16, u + 16);
           tmem_wait_loads();
           if (m >= row_limit) continue;
-          if (grouped && p.row_scale != nullptr) {
-            const float scale = __ldcg(p.row_scale + m);
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              g[c] = __float_as_uint(scale * __uint_as_float(g[c]));
-              u[c] = __float_as_uint(scale * __uint_as_float(u[c]));
-            }
-          }
           if (p.bias != nullptr) {
             const uint4* gate_bias = reinterpret_cast<const uint4*>(p.bias + (tile_y * (BN / 128) + block) * 128 + c0);
 #pragma unroll
@@ -941,38 +933,37 @@ MLR_EXPORT int mlr_gemm_tcgen05(const void* x, const void* w, const void* bias, 
 
 // ---------------------------------------------------------------- grouped form
 namespace mlr {
-template <int BN, bool SWIGLU, int BM = TILE_ROWS>
+template <int BN, int BM = TILE_ROWS>
 static int launch_grouped(const void* x, const void* w, const GemmParams& p, int rows, int groups, int max_tiles,
                           cudaStream_t stream) {
   const size_t shared = (size_t)p.stages * (BM * TILE_K * 2 + BN * TILE_K * 2) + 1024;
-  if (int err = allow_shared<BN, false, SWIGLU, BM>(shared)) return err;
+  if (int err = allow_shared<BN, false, false, BM>(shared)) return err;
   CUtensorMap map_a, map_b;
   if (!cached_tile_map(&map_a, x, rows, p.K, TILE_ROWS) || !cached_tile_map(&map_b, w, groups * p.N, p.K, BN))
     return MLR_BAD_ALIGNMENT;
   if (max_tiles > 65535) return MLR_TOO_LARGE;
   dim3 grid((p.N + BN - 1) / BN, max_tiles, 1);
-  launch_kernel(gemm_tcgen05_kernel<BN, false, SWIGLU, BM>, dim3(grid), dim3(GEMM_THREADS), shared, stream, map_a,
+  launch_kernel(gemm_tcgen05_kernel<BN, false, false, BM>, dim3(grid), dim3(GEMM_THREADS), shared, stream, map_a,
                 map_b, p);
   return launch_status();
 }
 }  // namespace mlr
 
 // The product of rows that are sorted by group with each group's own matrix: x [rows, K], w [groups, N, K]
-// (stacked), out [rows, N] (or [rows, N/2] bfloat16 with swiglu, as in mlr_gemm_tcgen05).  `tiles` is
+// (stacked), out [rows, N].  (With the gate in the epilogue: experts_tcgen05.cu.)  `tiles` is
 // device memory, int32 [max_tiles][3] = (group, first row, end row) per tile of up to `tile_rows` (128,
 // or 256 where N is a multiple of 256: two accumulators from one load of the weight tile, one CTA
 // per SM) rows of one group, group < 0 for unused entries; it may be written by the kernel just
 // before this one.  A 128-row load may run into the next group's rows (or past the last row: zeros);
-// those rows are computed and dropped.  `row_scale` (float32 [rows] or null) multiplies each row's product,
-// before the gate (the same as scaling the rows of x).  N % BN need not hold only without swiglu: a weight tile that would run into
+// those rows are computed and dropped.  `row_scale` (float32 [rows] or null) multiplies each row's product
+// (the same as scaling the rows of x).  A weight tile that would run into
 // the next group's rows is loaded but its columns beyond N are never written.
 MLR_EXPORT int mlr_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* tiles, int max_tiles, int rows,
-                                        int groups, int N, int K, int out_f32, int swiglu, int tile_rows,
+                                        int groups, int N, int K, int out_f32, int tile_rows,
                                         const float* row_scale, int* error_word, cudaStream_t stream) {
   if (rows == 0 || max_tiles == 0) return MLR_OK;
   if (rows < 0 || max_tiles < 0 || groups <= 0 || N <= 0 || K <= 0 || tiles == nullptr) return MLR_BAD_SIZE;
   if (K % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return MLR_BAD_ALIGNMENT;
-  if (swiglu && (N % 128 != 0 || out_f32)) return MLR_BAD_SIZE;
   if ((long long)groups * N > 0x7fffffffll) return MLR_TOO_LARGE;
   const int total_kb = (K + TILE_K - 1) / TILE_K;
   const bool wide = N % 256 == 0 && N >= 512;
@@ -992,7 +983,7 @@ MLR_EXPORT int mlr_gemm_tcgen05_grouped(const void* x, const void* w, void* out,
   p.bias = nullptr;
   p.out = out;
   p.out_f32 = out_f32;
-  p.gate_act = swiglu >= 2 ? swiglu - 1 : 0;
+  p.gate_act = 0;
   p.gate_limit = 0.f;
   p.gate_slope = 0.f;
   p.scratch = nullptr;
@@ -1000,10 +991,6 @@ MLR_EXPORT int mlr_gemm_tcgen05_grouped(const void* x, const void* w, void* out,
   p.error_word = error_word;
   p.group_tiles = tiles;
   p.row_scale = row_scale;
-  if (tall) return swiglu ? launch_grouped<256, true, 2 * TILE_ROWS>(x, w, p, rows, groups, max_tiles, stream)
-                          : launch_grouped<256, false, 2 * TILE_ROWS>(x, w, p, rows, groups, max_tiles, stream);
-  if (swiglu) return wide ? launch_grouped<256, true>(x, w, p, rows, groups, max_tiles, stream)
-                          : launch_grouped<128, true>(x, w, p, rows, groups, max_tiles, stream);
-  return wide ? launch_grouped<256, false>(x, w, p, rows, groups, max_tiles, stream)
-              : launch_grouped<128, false>(x, w, p, rows, groups, max_tiles, stream);
+  if (tall) return launch_grouped<256, 2 * TILE_ROWS>(x, w, p, rows, groups, max_tiles, stream);
+  return wide ? launch_grouped<256>(x, w, p, rows, groups, max_tiles, stream) : launch_grouped<128>(x, w, p, rows, groups, max_tiles, stream);
 }

@@ -53,6 +53,7 @@ LIBRARIES: dict[str, tuple[str, ...]] = {
     "attention_latent_tcgen05": (),
     "attention_rotated": (),
     "routed_experts": (),
+    "experts_tcgen05": (),
     "attention_sigmoid": (),
     "attention_sigmoid_mma": (),
     "attention_sigmoid_tcgen05": (),

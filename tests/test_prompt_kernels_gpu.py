@@ -466,6 +466,32 @@ def test_long_sums_of_many_rows_keep_their_scratch_bounded():
         assert torch.equal(cuda().linear(x[first:first + rows].contiguous(), w, bias), whole[first:first + rows]), first
 
 
+@pytest.mark.parametrize("width,inner", [(72, 64), (200, 192), (512, 128)])
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("weigh_input", [False, True])
+def test_experts_of_any_number_of_rows(width, inner, activation, weigh_input):
+    """Rows of an expert around the multiples of 16 and 32 of an MMA and a copy, of the 64 and 128 of half a tile and a tile, none at all; columns
+    that fill no copy of 64, weight rows that fill no tile of 256, and so many tiles that a CTA takes several."""
+    counts = [1, 15, 0, 16, 17, 31, 33, 63, 64, 65, 96, 127, 128, 129, 255, 256, 257] + [3] * 300
+    experts, rows = len(counts), sum(counts)
+    chosen = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(rows, generator=generator(1))]
+    x, weights = rnd(2, rows, width).to(torch.bfloat16), torch.rand(rows, 1, generator=generator(3)) + 0.5
+    gate_up, down = (rnd(4, experts, 2 * inner, width, std=width ** -0.5).to(torch.bfloat16),
+                     rnd(5, experts, width, inner, std=inner ** -0.5).to(torch.bfloat16))
+    got = cuda().routed_experts(x.to(DEVICE), chosen[:, None].int().to(DEVICE), weights.to(DEVICE), gate_up.to(DEVICE), down.to(DEVICE), 64,
+                                activation, weigh_input)
+    torch.cuda.synchronize()
+    cuda().raise_if_device_error()
+    act = torch.nn.functional.silu if activation == "silu" else lambda z: torch.nn.functional.gelu(z, approximate="tanh")
+    want = torch.zeros(rows, width, dtype=torch.float64)
+    for e in range(experts):
+        mine = chosen == e
+        both = (x[mine].double() @ gate_up[e].double().T * (weights[mine].double() if weigh_input else 1.0)).view(-1, inner // 64, 2, 64)
+        want[mine] = (act(both[:, :, 0]) * both[:, :, 1]).flatten(1) @ down[e].double().T * (1.0 if weigh_input else weights[mine].double())
+    # the hidden numbers' rounding to 8 bits, 2^-9 each at most and independent
+    close(got, want, 2.0 ** -8, "experts")
+
+
 @pytest.mark.parametrize("rows,top,experts", [(2048, 6, 64), (1500, 7, 33), (1366, 6, 128), (9000, 1, 40)])
 def test_pairs_sorted_by_expert_in_several_turns(rows, top, experts):
     """More than the 8,192 choices that the sort's threads hold at once, more experts than a warp has lanes; one expert gets none.  Weights of
