@@ -24,12 +24,15 @@
 //   S^T q_t (of token t) = K_t S_before^T q_t + sum_{s <= t} A_ts v_s    with  A_ts = D_ts (k_s . q_t)
 //   S_behind = K_last S_before + sum_s k_s (D_last,s v_s)^T
 //
+// Chunks side by side (value heads of up to 128, portions of more than two chunks), which is linear in S as well:
+// memory_ends_kernel            per chunk and head: what its own tokens leave behind, sum_s k_s (D_last,s v_s)^T.
+// memory_carry_kernel           per state entry, the chunks of a segment in order: the state before each.
+// memory_outputs_kernel         per chunk and head: A, both products, normaliser, head norm, weight and gate.
+// One behind the other:
 // matrix_memory_pairs_kernel    all chunks at once: A, D_last and K of every chunk, q, k and v as bfloat16.
 // matrix_memory_chunks_kernel   the chunks of a (request, head) one after the other, value channels over blocks; the
-//                               state stays in registers as accumulators.  That chain leaves SMs idle, so long segments are cut
-//                               into runs of chunks: a first launch takes every run but the last from zero, states only
-//                               (the recurrence is linear in S: a run's end is its keeps' product times the state before plus what
-//                               its own tokens leave), the second starts each run from what the runs before left.
+//                               state stays in registers as accumulators.
+#include "chunk_places.cuh"
 #include "mma_attention.cuh"
 #include "copy_async.cuh"
 #include "lane_sums.cuh"
@@ -49,11 +52,10 @@ struct MemoryArgs {
   bf16 *q16, *k16, *v16;                // chunks: [rows, heads * dim], the same, [rows, heads * vdim]
   float* states;                        // [slots, heads, vdim + 1, dim]
   float* maxima;                        // [slots, heads]
-  float* ends;                          // runs of chunks: [places, heads, vdim + 1, dim], what a run's own tokens leave (see run_place)
-  float* spans;                         // [places, heads]: product of a run's keeps
-  int run;                              // chunks of a run; 0: segments are not cut
+  float* ends;                          // chunks side by side: [chunks, heads, vdim + 1, dim], what a chunk's tokens leave, then the state before it
+  float* spans;                         // [chunks, heads]: product of a chunk's keeps
   const int *seg_q_start, *seg_q_len, *seg_slot;
-  int heads, dim, vdim;
+  int segments, heads, dim, vdim;
   float cap, guard, eps, q_scale;
 };
 
@@ -424,7 +426,6 @@ static int launch_scan(const MemoryArgs& p, int segments, cudaStream_t stream) {
 }
 
 // ------------------------------------------------------------------ chunks on the tensor cores
-constexpr int CHUNK = 64;         // tokens
 constexpr int CHUNK_COLS = 16;    // value channels of a block of the sequential kernel
 constexpr int CHUNK_PITCH = CHUNK_COLS + 8;
 
@@ -530,21 +531,10 @@ __device__ __forceinline__ void mma_cols(float (*c)[4], const uint32_t* a, const
   }
 }
 
-// Where a run that starts at `row` keeps what it leaves: one place per aligned stretch of a run's rows for a segment's first run
-// and one for another run.  Of segments of several runs (the only ones with places) no two first runs start in one stretch, nor two
-// later ones: they lie more than a run's rows apart.
-__device__ __forceinline__ size_t run_place(int row, int run_rows, bool first) { return 2 * (size_t)(row / run_rows) + (first ? 1 : 0); }
-inline long long run_places(int rows, int run_rows) { return 2ll * (rows / run_rows + 1); }
-
-// grid: (segments * runs, heads, blocks of 16 state rows).  Warp w keeps the key channels w D / 4 .. of the state.
-// WHOLE: segments that are not cut (the index arithmetic of runs costs them 4 %: 100 -> 104 us for 1,300 and 748 rows).  RUNS: the
-// outputs of all runs and a segment's last state.  LEFT: only what the runs before a segment's last leave; the first run starts from the request's state and also puts a copy of that
-// where the last run has its place, since the second launch's last run overwrites the state while its first may still read it.
-enum Part { WHOLE, LEFT, RUNS };
-
-template <int D, Part PART>
+// grid: (segments, heads, blocks of 16 state rows).  Warp w keeps the key channels w D / 4 .. of the state.
+template <int D>
 __global__ void __launch_bounds__(128)
-matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
+matrix_memory_chunks_kernel(MemoryArgs p) {
   pdl_trigger();
   constexpr int PITCH = D + 8, MT = D / 64, NT = CHUNK_COLS / 8, PIECES = D / 8;
   extern __shared__ __align__(16) uint8_t raw[];
@@ -553,16 +543,9 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
   bf16* s_parts = v_tiles + 2 * CHUNK * CHUNK_PITCH;                    // 3 x [D][CHUNK_PITCH]
   bf16* w_parts = s_parts + 3 * D * CHUNK_PITCH;                        // 3 x [64][CHUNK_PITCH]
   float2* factors = reinterpret_cast<float2*>(w_parts + 3 * CHUNK * CHUNK_PITCH);      // 2 x [64]
-  constexpr bool ENDS = PART == LEFT;
-  const int seg = PART == WHOLE ? blockIdx.x : blockIdx.x % segments, head = blockIdx.y, col0 = blockIdx.z * CHUNK_COLS, V = p.vdim;
+  const int seg = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * CHUNK_COLS, V = p.vdim;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int segment_start = p.seg_q_start[seg], segment_rows = p.seg_q_len[seg];
-  const int run_rows = PART == WHOLE ? segment_rows : p.run * CHUNK, run = PART == WHOLE ? 0 : blockIdx.x / segments;
-  const int runs = PART == WHOLE || segment_rows <= 0 ? 1 : (segment_rows + run_rows - 1) / run_rows;
-  if (PART != WHOLE && (run >= runs || (ENDS && run == runs - 1))) return;
-  const int q_start = segment_start + run * run_rows, q_len = PART == WHOLE ? segment_rows : min(run_rows, segment_rows - run * run_rows);      // this run's
-  const size_t cells = (size_t)(V + 1) * D;
-  auto place_of = [&](int r) { return run_place(segment_start + r * run_rows, run_rows, r == 0) * p.heads + head; };
+  const int q_start = p.seg_q_start[seg], q_len = p.seg_q_len[seg];
   float* state = p.states + ((size_t)p.seg_slot[seg] * p.heads + head) * (size_t)(V + 1) * D;
   // value channels beyond the last: the normaliser's is one, the others zero; no copy overwrites them
   for (int idx = threadIdx.x; idx < 2 * CHUNK * CHUNK_COLS; idx += 128) {
@@ -579,7 +562,7 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
       const int r = idx / PIECES, c = (idx - r * PIECES) * 8;
       const bool valid = r < count;
       const size_t at = valid ? (row0 + r) * p.heads * D + (size_t)head * D + c : 0;
-      if (!ENDS) cp_async_16(q_tile + r * PITCH + c, p.q16 + at, valid);
+      cp_async_16(q_tile + r * PITCH + c, p.q16 + at, valid);
       cp_async_16(k_tile + r * PITCH + c, p.k16 + at, valid);
     }
     for (int idx = threadIdx.x; idx < CHUNK * (CHUNK_COLS / 8); idx += 128) {
@@ -601,8 +584,6 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
     *d = warp * (D / 4) + mt * 16 + (lane >> 2) + 8 * (e >> 1);
     *c = col0 + nt * 8 + (lane & 3) * 2 + (e & 1);
   };
-  // the state before the run: the request's, or what the runs before leave one after the other
-  const float* start = PART == WHOLE ? state : runs == 1 || ENDS ? (run == 0 ? state : nullptr) : p.ends + place_of(run == 0 ? runs - 1 : 0) * cells;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -611,25 +592,8 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
       for (int e = 0; e < 4; ++e) {
         int d, c;
         place(mt, nt, e, &d, &c);
-        S[mt][nt][e] = (PART == WHOLE || start != nullptr) && c <= V ? __ldcg(start + (size_t)c * D + d) : 0.f;
-        if (ENDS && run == 0 && c <= V) p.ends[place_of(runs - 1) * cells + (size_t)c * D + d] = S[mt][nt][e];
+        S[mt][nt][e] = c <= V ? __ldcg(state + (size_t)c * D + d) : 0.f;
       }
-  if (PART == RUNS)
-    for (int r = 1; r < run; ++r) {
-      const float span = __ldcg(p.spans + place_of(r));
-      const float* left = p.ends + place_of(r) * cells;
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            int d, c;
-            place(mt, nt, e, &d, &c);
-            S[mt][nt][e] = fmaf(S[mt][nt][e], span, c <= V ? __ldcg(left + (size_t)c * D + d) : 0.f);
-          }
-    }
-  float span = 1.f;
   int which = 0;
   for (int t0 = 0; t0 < q_len; t0 += CHUNK, which ^= 1) {
     const int count = min(CHUNK, q_len - t0);
@@ -646,7 +610,6 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
     const float* a_row[2] = {p.pairs + ((row0 + r0) * p.heads + head) * CHUNK + (lane & 3) * 2,
                              p.pairs + ((row0 + r0 + 8) * p.heads + head) * CHUNK + (lane & 3) * 2};
     float2 a_pair[CHUNK / 16][4];
-    if (!ENDS)
 #pragma unroll
     for (int ks = 0; ks < CHUNK / 16; ++ks)
 #pragma unroll
@@ -656,7 +619,6 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
           a_pair[ks][e] = __ldcg(reinterpret_cast<const float2*>(a_row[e & 1] + ks * 16 + 8 * (e >> 1)));
       }
     // the state and the weighed values in parts
-    if (!ENDS)
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -687,7 +649,7 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
     for (int n = 0; n < 3; ++n)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) o[n][nt][0] = o[n][nt][1] = o[n][nt][2] = o[n][nt][3] = 0.f;
-    if (!ENDS && warp * 16 < count) {
+    if (warp * 16 < count) {
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
         uint32_t a[4];
@@ -734,7 +696,6 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
     }
     // the state behind the chunk
     const float kept = factor[count - 1].y;
-    span *= kept;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
@@ -758,9 +719,8 @@ matrix_memory_chunks_kernel(MemoryArgs p, int segments) {
       for (int e = 0; e < 4; ++e) {
         int d, c;
         place(mt, nt, e, &d, &c);
-        if (c <= V && (PART != RUNS || run == runs - 1)) (ENDS ? p.ends + place_of(run) * cells : state)[(size_t)c * D + d] = S[mt][nt][e];
+        if (c <= V) state[(size_t)c * D + d] = S[mt][nt][e];
       }
-  if (ENDS && blockIdx.z == 0 && threadIdx.x == 0) p.spans[place_of(run)] = span;
 }
 
 template <int D>
@@ -769,26 +729,481 @@ static int launch_chunks(const MemoryArgs& p, int segments, int max_q_len, cudaS
                             sizeof(float2) * 2 * CHUNK;
   static_assert(shared <= 227 * 1024, "tiles");
   constexpr size_t pairs_shared = sizeof(bf16) * (size_t)(2 * CHUNK * (D + 8)) + sizeof(float) * CHUNK * (CHUNK + 1);
-  cudaError_t err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D, RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D, LEFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  cudaError_t err = cudaFuncSetAttribute(matrix_memory_chunks_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(matrix_memory_pairs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_shared);
   if (err != cudaSuccess) return (int)err;
   launch_kernel(matrix_memory_pairs_kernel<D>, dim3((max_q_len + CHUNK - 1) / CHUNK, p.heads, segments), dim3(128), pairs_shared,
                 stream, p);
+  const int status = launch_status();
+  if (status != MLR_OK) return status;
+  launch_kernel(matrix_memory_chunks_kernel<D>, dim3(segments, p.heads, (p.vdim + CHUNK_COLS) / CHUNK_COLS), dim3(128), shared, stream, p);
+  return launch_status();
+}
+
+// ------------------------------------------------------------------ chunks side by side
+// Bound by the tensor cores' rate for three products of parts with a warp's instructions between them: a block of the outputs takes some 23,000
+// cycles alone on an SM, of which 8,500 are the products with the state before (loads, split and products of a part after another), 3,000 the chunk's
+// own tokens and 6,500 normaliser, norm and gate; the ends 10,000, 4,100 of them products.  The carry moves the states of all chunks through L2.
+// 16 warps of half the columns each were slower (splits and fragments of A twice: 56 -> 61 us at the time), a branch around a pair that a warp does not have cost
+// 10 % of the products, and rows one after the other with their divisions and roots 4,500 cycles.  Whole calls, chunks one behind the other (or in runs of
+// four and more, which these kernels replace) / side by side, 7 heads of 128 x 128: 1,300 and 748 rows 86 / 44 us, 2,048 rows 78 / 46, 4,000 rows 153 / 76,
+// 512 rows 41 / 26; 16 heads: 2,048 rows 148 / 86, 8 of 200 rows 104 / 79.
+constexpr int SIDE_THREADS = 256;
+constexpr int SIDE_V = 128;               // value channels at most
+constexpr int SIDE_PAIRS = SIDE_V / 16 + 1;      // pairs of eight columns, the normaliser's among them
+constexpr int SIDE_PITCH = 16 * SIDE_PAIRS + 8;  // rows of value columns: an odd number of 16-byte pieces
+
+// Column pairs of a head: its value channels, the normaliser and zeros.
+__host__ __device__ __forceinline__ int side_pairs(int V) { return (V / 8 + 2) / 2; }
+// A token's gates: keep and write; a place without a token keeps everything and writes nothing.
+__device__ __forceinline__ void side_gates(const MemoryArgs& p, float* keep, float* write, float* floor_of, size_t row0, int count, int head) {
+  const int t = threadIdx.x;
+  if (t >= CHUNK) return;
+  float4 gate = make_float4(1.f, 0.f, 0.f, 0.f);
+  if (t < count) gate = __ldcg(p.coef + (row0 + t) * p.heads + head);
+  keep[t] = gate.x;
+  write[t] = gate.y;
+  if (floor_of != nullptr) floor_of[t] = gate.z;
+}
+
+// A chunk's rows of float32 numbers, asked for with all loads in flight together and kept as bfloat16: COLUMNS pieces of four, `used` of them
+// (and `rows` of the rows) are there, PER of them a thread's.
+template <int COLUMNS, int THREADS>
+struct SideRows {
+  static constexpr int PER = (CHUNK * COLUMNS + THREADS - 1) / THREADS;
+  float4 piece[PER];
+  __device__ __forceinline__ void ask(const float* from, long long stride, int rows, int used) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int idx = threadIdx.x + i * THREADS, r = idx / COLUMNS, c = idx % COLUMNS;
+      piece[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < rows && c < used) piece[i] = __ldcg(reinterpret_cast<const float4*>(from + r * stride) + c);
+    }
+  }
+  template <typename F>
+  __device__ __forceinline__ void each(F&& f) {      // f(row, first column, numbers)
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int idx = threadIdx.x + i * THREADS;
+      if (idx < CHUNK * COLUMNS) f(idx / COLUMNS, idx % COLUMNS * 4, piece[i]);
+    }
+  }
+};
+
+// A warp takes 16 key channels and its share of the column pairs.  grid: (heads, chunks)
+template <int D, int PAIRS>
+__global__ void __launch_bounds__(SIDE_THREADS, 2)
+memory_ends_kernel(MemoryArgs p) {
+  constexpr int PITCH = D + 8, W_APART = CHUNK * SIDE_PITCH, KEY_TILES = D / 16;
+  constexpr int GROUPS = SIDE_THREADS / 32 / KEY_TILES, MOST = (PAIRS + GROUPS - 1) / GROUPS;      // of column pairs, and pairs of a group
+  extern __shared__ __align__(16) uint8_t raw[];
+  bf16 *k_tile = reinterpret_cast<bf16*>(raw), *w_parts = k_tile + CHUNK * PITCH;      // [64][PITCH], 3 x [64][SIDE_PITCH]
+  __shared__ float keep[CHUNK], write[CHUNK], share[CHUNK], kept;
+  pdl_wait();
+  const int head = blockIdx.x, V = p.vdim, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, 1, blockIdx.y);
+  if (seg < 0) return;
+  const int count = min(CHUNK, length - chunk * CHUNK);
+  const size_t row0 = (size_t)start + chunk * CHUNK;
+  side_gates(p, keep, write, nullptr, row0, count, head);
+  SideRows<D / 4, SIDE_THREADS> keys;
+  keys.ask(p.k + row0 * p.k_stride + (size_t)head * D, p.k_stride, count, D / 4);
+  SideRows<4 * PAIRS, SIDE_THREADS> values;
+  values.ask(p.v + row0 * p.v_stride + (size_t)head * V, p.v_stride, count, V / 4);
+  __syncthreads();
+  if (warp == 0) {      // what the chunk's last token has of each, two to a lane: places behind the last token keep it
+    const float near = keep[2 * lane], far = keep[2 * lane + 1];
+    float all = near * far;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const float later = __shfl_down_sync(0xffffffffu, all, offset);
+      if (lane + offset < 32) all *= later;
+    }
+    float behind = __shfl_down_sync(0xffffffffu, all, 1);
+    if (lane == 31) behind = 1.f;
+    share[2 * lane + 1] = write[2 * lane + 1] * behind;
+    share[2 * lane] = write[2 * lane] * (far * behind);
+    if (lane == 0) p.spans[(size_t)blockIdx.y * p.heads + head] = kept = all;
+  }
+  keys.each([&](int r, int d, const float4& x) { *reinterpret_cast<uint2*>(k_tile + r * PITCH + d) = pack4(x); });
+  __syncthreads();
+  values.each([&](int r, int c, const float4& x) {
+    const float weight = share[r];
+    const uint2 rounded = pack4(x);
+    float4 v = make_float4(weight * __uint_as_float(rounded.x << 16), weight * __uint_as_float(rounded.x & 0xffff0000u),
+                           weight * __uint_as_float(rounded.y << 16), weight * __uint_as_float(rounded.y & 0xffff0000u));
+    if (c >= V) v = make_float4(c == V ? weight : 0.f, 0.f, 0.f, 0.f);
+    uint32_t low[3], high[3];
+    split_pair(v.x, v.y, low);
+    split_pair(v.z, v.w, high);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) *reinterpret_cast<uint2*>(w_parts + n * W_APART + r * SIDE_PITCH + c) = make_uint2(low[n], high[n]);
+  });
+  __syncthreads();
+  float E[2 * MOST][4];
+#pragma unroll
+  for (int j = 0; j < 2 * MOST; ++j) E[j][0] = E[j][1] = E[j][2] = E[j][3] = 0.f;
+  const int tile = warp % KEY_TILES, all_pairs = side_pairs(V), share_of = (all_pairs + GROUPS - 1) / GROUPS;
+  const int pair0 = warp / KEY_TILES * share_of, pairs = min(share_of, all_pairs - pair0);
+#pragma unroll
+  for (int ks = 0; ks < CHUNK / 16; ++ks) {
+    if (ks * 16 >= count) break;
+    uint32_t a[4];      // keys transposed: channels are the product's rows
+    ldmatrix_x4_trans(a, k_tile + (ks * 16 + ((lane >> 4) << 3) + (lane & 7)) * PITCH + tile * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+    for (int n = 2; n >= 0; --n)
+#pragma unroll
+      for (int j = 0; j < MOST; ++j) {      // a pair beyond the last is multiplied and dropped: a branch here would keep loads and products apart
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, w_parts + n * W_APART + (ks * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * SIDE_PITCH +
+                                 (min(pair0 + j, PAIRS - 1) * 2 + (lane >> 4)) * 8);
+        mma_bf16(E[2 * j], a, b[0], b[1]);
+        mma_bf16(E[2 * j + 1], a, b[2], b[3]);
+      }
+  }
+  const int c0 = pair0 * 16 + (lane & 3) * 2;
+  const size_t mine = (size_t)c0 * D + tile * 16 + (lane >> 2);
+  float* to = p.ends + ((size_t)blockIdx.y * p.heads + head) * (size_t)(V + 1) * D + mine;
+  float* state = p.states + ((size_t)slot * p.heads + head) * (size_t)(V + 1) * D + mine;
+  auto entry = [&](int j, int e) { return (j * 8 + (e & 1)) * D + 8 * (e >> 1); };
+  auto there = [&](int j, int e) { return j < 2 * pairs && c0 + j * 8 + (e & 1) <= V; };
+  if (length > CHUNK) {
+#pragma unroll
+    for (int j = 0; j < 2 * MOST; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (there(j, e)) to[entry(j, e)] = E[j][e];
+    pdl_trigger();      // late, as in the kernel behind
+    return;
+  }
+  // the segment's only chunk: nothing is left for the carry
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    float before[MOST][4];
+#pragma unroll
+    for (int j = 0; j < MOST; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (there(half * MOST + j, e)) before[j][e] = __ldcg(state + entry(half * MOST + j, e));
+#pragma unroll
+    for (int j = 0; j < MOST; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (there(half * MOST + j, e)) {
+          to[entry(half * MOST + j, e)] = before[j][e];
+          state[entry(half * MOST + j, e)] = fmaf(kept, before[j][e], E[half * MOST + j][e]);
+        }
+  }
+}
+
+// A thread owns four neighbouring entries and takes the chunks of its segment in order, BATCH of them asked for together.  Leaves the state before
+// every chunk where what its tokens left behind was.  grid: (entries, segments)
+__global__ void __launch_bounds__(256)
+memory_carry_kernel(MemoryArgs p, int cells) {
+  constexpr int BATCH = 8;
+  pdl_wait();
+  const int seg = blockIdx.y, length = p.seg_q_len[seg], at = (blockIdx.x * 256 + threadIdx.x) * 4;
+  if (length <= CHUNK) return;
+  int first = 0;
+  for (int i = threadIdx.x & 31; i < seg; i += 32) first += (max(p.seg_q_len[i], 0) + CHUNK - 1) / CHUNK;
+  first = __reduce_add_sync(0xffffffffu, first);
+  if (at >= p.heads * cells) return;
+  const int head = at / cells, cell = at - head * cells, chunks = (length + CHUNK - 1) / CHUNK;
+  float4* state = reinterpret_cast<float4*>(p.states + ((size_t)p.seg_slot[seg] * p.heads + head) * cells + cell);
+  float4 S = *state;
+  const size_t step = (size_t)p.heads * cells / 4;
+  float4* end = reinterpret_cast<float4*>(p.ends + ((size_t)first * p.heads + head) * cells + cell);
+  const float* span = p.spans + (size_t)first * p.heads + head;
+  for (int c0 = 0; c0 < chunks; c0 += BATCH, end += BATCH * step, span += BATCH * p.heads) {
+    float4 own[BATCH];
+    float g[BATCH];
+#pragma unroll
+    for (int k = 0; k < BATCH; ++k)
+      if (c0 + k < chunks) {
+        own[k] = end[k * step];
+        g[k] = span[k * p.heads];
+      }
+#pragma unroll
+    for (int k = 0; k < BATCH; ++k)
+      if (c0 + k < chunks) {
+        end[k * step] = S;
+        S.x = fmaf(g[k], S.x, own[k].x);
+        S.y = fmaf(g[k], S.y, own[k].y);
+        S.z = fmaf(g[k], S.z, own[k].z);
+        S.w = fmaf(g[k], S.w, own[k].w);
+      }
+  }
+  *state = S;
+  // The outputs' blocks, brought in while these still fill some SMs, would land two to an SM beside empty ones: a step of 512 rows, 7 heads, takes
+  // 34.8 us with the trigger in front, 26.6 so, and one of 2,048 rows 50.4 and (with that of the ends) 45.6.
+  pdl_trigger();
+}
+
+constexpr int SIDE_D = 32;                // key channels of the state taken at a time
+constexpr int SIDE_D_PITCH = SIDE_D + 8;
+constexpr int SIDE_A_PITCH = CHUNK + 8;
+constexpr int SIDE_SUMS = SIDE_V + 8;     // float32 sums of a row, the normaliser among them
+
+template <int D>
+struct SideShape {
+  static constexpr int QK_PITCH = D + 8, S_APART = 16 * SIDE_PAIRS * SIDE_D_PITCH;
+  static constexpr size_t Q = CHUNK * QK_PITCH * sizeof(bf16), VALUES = CHUNK * SIDE_PITCH * sizeof(bf16), A = CHUNK * SIDE_A_PITCH * sizeof(float);
+  static constexpr size_t S = 3 * S_APART * sizeof(bf16);      // keys before
+  static_assert(S >= Q && A + S >= CHUNK * SIDE_SUMS * sizeof(float), "keys, sums");
+  static constexpr size_t SHARED = Q + VALUES + A + S;
+  static constexpr size_t ENDS = Q + 3 * CHUNK * SIDE_PITCH * sizeof(bf16);
+};
+
+// 1 / (1 + e^-z) without a branch: one step of Newton's on the approximate reciprocal, which leaves it within an ulp of the exact one; beyond 1e37 the
+// approximation stands (also for infinity and NaN, where the step would give NaN).
+__device__ __forceinline__ float even_sigmoid(float z) {
+  const float d = 1.f + expf(-z), r = __fdividef(1.f, d);
+  return d < 1e37f ? fmaf(r, fmaf(-d, r, 1.f), r) : r;
+}
+
+// Warps 4 i .. 4 i + 3 take 16 rows each with the i-th share of the column pairs (of the tokens for A).  grid: (heads, chunks)
+template <int D, int PAIRS>
+__global__ void __launch_bounds__(SIDE_THREADS, 2)
+memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
+  using Shape = SideShape<D>;
+  constexpr int PITCH = Shape::QK_PITCH, SIDES = SIDE_THREADS / 128, MOST = (PAIRS + SIDES - 1) / SIDES;      // column pairs of a warp
+  extern __shared__ __align__(16) uint8_t raw[];
+  bf16 *q_tile = reinterpret_cast<bf16*>(raw), *v_tile = q_tile + CHUNK * PITCH;
+  float* A = reinterpret_cast<float*>(raw + Shape::Q + Shape::VALUES);                      // [64][SIDE_A_PITCH]
+  bf16* s_parts = reinterpret_cast<bf16*>(raw + Shape::Q + Shape::VALUES + Shape::A);      // 3 x [columns][SIDE_D_PITCH]; keys before
+  bf16* k_tile = s_parts;
+  __shared__ __align__(16) float keep[CHUNK];
+  __shared__ float write[CHUNK], floor_of[CHUNK], since[CHUNK];
+  pdl_trigger();
+  pdl_wait();
+  const int head = blockIdx.x, V = p.vdim, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, 1, blockIdx.y);
+  if (seg < 0) return;
+  const int count = min(CHUNK, length - chunk * CHUNK);
+  const size_t row0 = (size_t)start + chunk * CHUNK;
+  side_gates(p, keep, write, floor_of, row0, count, head);
+  {
+    SideRows<D / 4, SIDE_THREADS> queries, keys;
+    queries.ask(p.q + row0 * p.q_stride + (size_t)head * D, p.q_stride, count, D / 4);
+    keys.ask(p.k + row0 * p.k_stride + (size_t)head * D, p.k_stride, count, D / 4);
+    queries.each([&](int r, int d, const float4& x) { *reinterpret_cast<uint2*>(q_tile + r * PITCH + d) = pack4(x); });
+    keys.each([&](int r, int d, const float4& x) { *reinterpret_cast<uint2*>(k_tile + r * PITCH + d) = pack4(x); });
+  }
+  SideRows<4 * PAIRS, SIDE_THREADS> values;      // on their way until the products of queries and keys are done
+  values.ask(p.v + row0 * p.v_stride + (size_t)head * V, p.v_stride, count, V / 4);
+  const int all_pairs = side_pairs(V);
+  // a part of the state before the chunk
+  const float* before = p.ends + ((size_t)blockIdx.y * p.heads + head) * (size_t)(V + 1) * D;
+  constexpr int S_PIECES = (16 * PAIRS * (SIDE_D / 4) + SIDE_THREADS - 1) / SIDE_THREADS;
+  float4 piece[S_PIECES];
+  auto ask = [&](int d0) {
+#pragma unroll
+    for (int k = 0; k < S_PIECES; ++k) {
+      const int idx = threadIdx.x + k * SIDE_THREADS, c = idx / (SIDE_D / 4), d = idx % (SIDE_D / 4) * 4;
+      piece[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c <= V) piece[k] = __ldcg(reinterpret_cast<const float4*>(before + (size_t)c * D + d0 + d));
+    }
+  };
+  ask(0);
+  __syncthreads();
+  {      // thread (s, eighth): token s's share at the eighth's rows
+    constexpr int ROWS = CHUNK * CHUNK / SIDE_THREADS;
+    const int s = threadIdx.x & (CHUNK - 1), t0 = threadIdx.x / CHUNK * ROWS;
+    float x = write[s], all = 1.f;
+    auto four = [&](int t, auto&& at) {
+      const float4 k4 = *reinterpret_cast<const float4*>(keep + t);
+      const float own[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (t + i > s) x *= own[i];
+        all *= own[i];
+        at(t + i);
+      }
+    };
+#pragma unroll 4
+    for (int t = 0; t < t0; t += 4) four(t, [](int) {});
+#pragma unroll
+    for (int t = 0; t < ROWS; t += 4)
+      four(t0 + t, [&](int row) {
+        A[row * SIDE_A_PITCH + s] = row >= s ? x : 0.f;
+        if (s == 0) since[row] = all;
+      });
+  }
+  const int tile = warp & 3, side = warp >> 2, r = lane >> 2, c2 = (lane & 3) * 2;
+  const bf16* q_at = q_tile + (tile * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * PITCH + (lane >> 4) * 8;
+  constexpr int BLOCKS = 4 / SIDES;      // blocks of 16 tokens of a warp; those behind its rows are not seen
+  float s[BLOCKS][2][4];
+#pragma unroll
+  for (int n = 0; n < BLOCKS; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[n][0][e] = s[n][1][e] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) {
+    uint32_t a[4];
+    ldmatrix_x4(a, q_at + ks * 16);
+#pragma unroll
+    for (int n = 0; n < BLOCKS; ++n)
+      {
+        uint32_t b[4];
+        ldmatrix_x4(b, k_tile + ((n * SIDES + side) * 16 + (lane & 7) + ((lane >> 4) << 3)) * PITCH + ks * 16 + ((lane >> 3) & 1) * 8);
+        mma_bf16(s[n][0], a, b[0], b[1]);
+        mma_bf16(s[n][1], a, b[2], b[3]);
+      }
+  }
+  __syncthreads();      // the shares are there, the keys have been read
+#pragma unroll
+  for (int n = 0; n < BLOCKS; ++n)
+    if (n * SIDES + side <= tile) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int row = tile * 16 + r + 8 * i, token = (n * SIDES + side) * 16 + j * 8 + c2;      // later tokens are not seen, whatever numbers they hold
+          float2* at = reinterpret_cast<float2*>(A + row * SIDE_A_PITCH + token);
+          const float2 d = *at;
+          *at = make_float2(token <= row ? s[n][j][2 * i] * d.x : 0.f, token < row ? s[n][j][2 * i + 1] * d.y : 0.f);
+        }
+    }
+  values.each([&](int row, int c, const float4& x) {
+    *reinterpret_cast<uint2*>(v_tile + row * SIDE_PITCH + c) = c < V ? pack4(x) : make_uint2(c == V ? 0x3f80u : 0u, 0u);      // the normaliser's value is one
+  });
+  const int share_of = (all_pairs + SIDES - 1) / SIDES, pair0 = side * share_of, pairs = min(share_of, all_pairs - pair0);
+  float o[2 * MOST][4];
+#pragma unroll
+  for (int j = 0; j < 2 * MOST; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+#pragma unroll 1
+  for (int d0 = 0; d0 < D; d0 += SIDE_D) {
+    if (d0 > 0) __syncthreads();      // the part before has been read
+#pragma unroll
+    for (int k = 0; k < S_PIECES; ++k) {
+      const int idx = threadIdx.x + k * SIDE_THREADS, c = idx / (SIDE_D / 4), d = idx % (SIDE_D / 4) * 4;
+      if (c >= 16 * PAIRS) continue;
+      uint32_t first[3], second[3];
+      split_pair(piece[k].x, piece[k].y, first);
+      split_pair(piece[k].z, piece[k].w, second);
+#pragma unroll
+      for (int n = 0; n < 3; ++n) *reinterpret_cast<uint2*>(s_parts + n * Shape::S_APART + c * SIDE_D_PITCH + d) = make_uint2(first[n], second[n]);
+    }
+    __syncthreads();
+    if (d0 + SIDE_D < D) ask(d0 + SIDE_D);
+    if (tile * 16 < count) {
+#pragma unroll
+      for (int ks = 0; ks < SIDE_D / 16; ++ks) {
+        uint32_t a[4];
+        ldmatrix_x4(a, q_at + d0 + ks * 16);
+#pragma unroll
+        for (int n = 2; n >= 0; --n)
+#pragma unroll
+          for (int j = 0; j < MOST; ++j) {
+            uint32_t b[4];
+            ldmatrix_x4(b, s_parts + n * Shape::S_APART + (min(pair0 + j, PAIRS - 1) * 16 + (lane & 7) + ((lane >> 4) << 3)) * SIDE_D_PITCH + ks * 16 +
+                               ((lane >> 3) & 1) * 8);
+            mma_bf16(o[2 * j], a, b[0], b[1]);
+            mma_bf16(o[2 * j + 1], a, b[2], b[3]);
+          }
+      }
+    }
+  }
+  const float kept[2] = {since[tile * 16 + r], since[tile * 16 + r + 8]};
+#pragma unroll
+  for (int j = 0; j < 2 * MOST; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] *= kept[e >> 1];
+  if (tile * 16 < count) {
+#pragma unroll 1
+    for (int ks = 0; ks <= tile; ++ks) {      // the chunk's own tokens; later ones are not seen
+      uint32_t part[4][3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = *reinterpret_cast<const float2*>(A + (tile * 16 + r + 8 * (e & 1)) * SIDE_A_PITCH + ks * 16 + 8 * (e >> 1) + c2);
+        split_pair(x.x, x.y, part[e]);
+      }
+#pragma unroll
+      for (int j = 0; j < MOST; ++j) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, v_tile + (ks * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * SIDE_PITCH + (min(pair0 + j, PAIRS - 1) * 2 + (lane >> 4)) * 8);
+#pragma unroll
+        for (int n = 2; n >= 0; --n) {
+          const uint32_t a[4] = {part[0][n], part[1][n], part[2][n], part[3][n]};
+          mma_bf16(o[2 * j], a, b[0], b[1]);
+          mma_bf16(o[2 * j + 1], a, b[2], b[3]);
+        }
+      }
+    }
+  }
+  // Normaliser, head norm, weight and gate: a warp takes ROWS rows, its lanes the channels; what a row needs once, a lane works out for each row.
+  // No branches between the rows (those behind the last are dropped when they are stored), or each waits for the one before.
+  __syncthreads();      // A has been read
+  float* sums = A;      // [64][SIDE_SUMS]
+#pragma unroll
+  for (int j = 0; j < 2 * MOST; ++j) {
+    const int c = pair0 * 16 + j * 8 + c2;
+    if (j < 2 * pairs && c <= V) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(sums + (tile * 16 + r + 8 * i) * SIDE_SUMS + c) = make_float2(o[j][2 * i], o[j][2 * i + 1]);
+    }
+  }
+  constexpr int ROWS = CHUNK / (SIDE_THREADS / 32), COLUMNS = SIDE_V / 32;      // rows of a warp, channels of a lane
+  const int first = warp * ROWS;
+  const bool full = V == SIDE_V && first + ROWS <= count;
+  const float* gate_at = p.gate + (row0 + first) * p.gate_stride + (size_t)head * V + lane;
+  float gate[ROWS][COLUMNS], weight[COLUMNS], x[ROWS][COLUMNS], sq[ROWS];
+#pragma unroll
+  for (int j = 0; j < COLUMNS; ++j) weight[j] = lane + 32 * j < V ? p.weight[(size_t)head * V + lane + 32 * j] : 0.f;
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+    for (int j = 0; j < COLUMNS; ++j) gate[i][j] = full || (first + i < count && lane + 32 * j < V) ? __ldcg(gate_at + i * p.gate_stride + 32 * j) : 0.f;
+  __syncthreads();
+  const int own_row = first + (lane & (ROWS - 1));
+  const float own_scale = p.q_scale / (fmaxf(fabsf(sums[own_row * SIDE_SUMS + V] * p.q_scale), floor_of[own_row]) + p.guard);
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const float scale = __shfl_sync(0xffffffffu, own_scale, i);
+    sq[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < COLUMNS; ++j) {
+      x[i][j] = lane + 32 * j < V ? sums[(first + i) * SIDE_SUMS + lane + 32 * j] * scale : 0.f;
+      sq[i] = fmaf(x[i][j], x[i][j], sq[i]);
+    }
+  }
+  float own_sq = 0.f;
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1)
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], offset);
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i)
+    if ((lane & (ROWS - 1)) == i) own_sq = sq[i];
+  const float own_factor = 1.f / sqrtf(own_sq / (float)V + p.eps);
+  bf16* dst = out + ((row0 + first) * p.heads + head) * V + lane;
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const float factor = __shfl_sync(0xffffffffu, own_factor, i);
+#pragma unroll
+    for (int j = 0; j < COLUMNS; ++j) {
+      const bf16 y = __float2bfloat16(x[i][j] * factor * weight[j] * even_sigmoid(gate[i][j]));
+      if (full || (first + i < count && lane + 32 * j < V)) dst[(size_t)i * p.heads * V + 32 * j] = y;
+    }
+  }
+}
+
+template <int D, int PAIRS>
+static int launch_side(const MemoryArgs& p, bf16* out, int rows, int segments, cudaStream_t stream) {
+  const unsigned chunks = (unsigned)long_chunks(rows, segments, 1);
+  const int cells = (p.vdim + 1) * D;
+  cudaError_t err = cudaFuncSetAttribute(memory_ends_kernel<D, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::ENDS);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(memory_outputs_kernel<D, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::SHARED);
+  if (err != cudaSuccess) return (int)err;
+  launch_kernel(memory_ends_kernel<D, PAIRS>, dim3(p.heads, chunks), dim3(SIDE_THREADS), SideShape<D>::ENDS, stream, p);
   int status = launch_status();
   if (status != MLR_OK) return status;
-  const int runs = p.run > 0 ? (max_q_len + p.run * CHUNK - 1) / (p.run * CHUNK) : 1, blocks = (p.vdim + CHUNK_COLS) / CHUNK_COLS;
-  if (runs == 1) {
-    launch_kernel(matrix_memory_chunks_kernel<D, WHOLE>, dim3(segments, p.heads, blocks), dim3(128), shared, stream, p, segments);
-    return launch_status();
-  }
-  launch_kernel(matrix_memory_chunks_kernel<D, LEFT>, dim3(segments * (runs - 1), p.heads, blocks), dim3(128), shared, stream, p, segments);
+  launch_kernel(memory_carry_kernel, dim3((p.heads * cells / 4 + 255) / 256, segments), dim3(256), 0, stream, p, cells);
   if ((status = launch_status()) != MLR_OK) return status;
-  launch_kernel(matrix_memory_chunks_kernel<D, RUNS>, dim3(segments * runs, p.heads, blocks), dim3(128), shared, stream, p, segments);
+  launch_kernel(memory_outputs_kernel<D, PAIRS>, dim3(p.heads, chunks), dim3(SIDE_THREADS), SideShape<D>::SHARED, stream, p, out);
   return launch_status();
 }
 
@@ -860,6 +1275,7 @@ matrix_memory_finish_kernel(MemoryArgs p, T* __restrict__ out, long long items) 
     dst[c] = from_float<T>(__ldcg(reads + c) * inverse * factor * weight[c] * sigmoid(__ldcg(gate + c)));
 }
 
+static bool side_fits(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim % 8 == 0 && vdim <= SIDE_V; }
 static bool chunks_fit(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim % 8 == 0; }
 
 template <typename T>
@@ -874,10 +1290,19 @@ static int launch_memory(const MemoryArgs& p, T* out, int rows, int segments, in
     else launch_kernel(matrix_memory_decode_kernel<T, 4>, grid, dim3(DECODE_THREADS), shared, stream, p, out);
     return launch_status();
   }
-  if (p.coef == nullptr || p.reads == nullptr || p.norms == nullptr) return MLR_BAD_SIZE;
+  if (p.coef == nullptr || (p.ends == nullptr && (p.reads == nullptr || p.norms == nullptr))) return MLR_BAD_SIZE;
   launch_kernel(matrix_memory_gates_kernel, dim3(segments, p.heads), dim3(GATE_THREADS), 0, stream, p);
   int status = launch_status();
   if (status != MLR_OK) return status;
+  if (p.ends != nullptr) {
+    if constexpr (sizeof(T) == 2) {
+      if (!wide || !side_fits(D, p.vdim) || long_chunks(rows, segments, 1) > 65535) return MLR_BAD_SIZE;
+      if (side_pairs(p.vdim) <= 6)
+        return D == 64 ? launch_side<64, 6>(p, out, rows, segments, stream) : launch_side<128, 6>(p, out, rows, segments, stream);
+      return D == 64 ? launch_side<64, SIDE_PAIRS>(p, out, rows, segments, stream) : launch_side<128, SIDE_PAIRS>(p, out, rows, segments, stream);
+    }
+    return MLR_BAD_DTYPE;
+  }
   if (p.pairs != nullptr) {
     if (!wide || !chunks_fit(D, p.vdim)) return MLR_BAD_SIZE;
     status = D == 64 ? launch_chunks<64>(p, segments, max_q_len, stream) : launch_chunks<128>(p, segments, max_q_len, stream);
@@ -911,38 +1336,30 @@ MLR_DEFINE_PDL_SWITCH
 // Whether prompts of these head sizes can go through the tensor cores in chunks (with `pairs`).
 MLR_EXPORT int mlr_matrix_memory_chunks_fit(int dim, int vdim) { return chunks_fit(dim, vdim); }
 
-// Chunks of a run for a step on the tensor cores (0: segments are not cut), and the float32 numbers of scratch that runs need.  So many
-// runs that the blocks of a launch still run together (two share an SM; every segment may add a short run), at least MIN_RUN chunks
-// each, and only where LEAST_RUNS or more fit (blocks that share an SM slow one another down) and a portion is long enough to pay for
-// the second launch and its scratch.  Measured in us without / with runs, heads of 128: one request of 2,048 rows, 7 heads 120 / 81,
-// 4 heads 114 / 61; 1,300 and 748 rows, 4 heads 84 / 63; 4 heads of 64, 2,048 rows 94 / 58.  Not cut: 7 heads, 1,300 and 748 rows
-// 96 / 98, 16 heads 136 / 182; 600 rows, 4 heads 52 / 57; 1,024 rows, 4 heads of 64 57 / 58.
+// Chunks that a block walks one behind the other: 1 where a step's chunks go side by side, 0 where all of a segment's go one behind the other: where
+// no portion has more than two (one behind the other / side by side: 65 rows of 7 heads 21.5 / 24.4 us, 128 rows 22.5 / 24.4, 129 rows 24.9 / 24.8, 192 rows
+// 25.5 / 24.9, 16 heads of 129 rows 25.2 / 25.2; short portions beside a longer one take no time of their own).
 MLR_EXPORT int mlr_matrix_memory_run(int rows, int segments, int max_q_len, int heads, int vdim) {
-  constexpr int MIN_RUN = 4, LEAST_RUNS = 4, SHORTEST = 1024;
-  const int blocks = heads * ((vdim + CHUNK_COLS) / CHUNK_COLS), chunks = (rows + CHUNK - 1) / CHUNK;
-  const int runs = 2 * sm_count() / (blocks < 1 ? 1 : blocks) - (segments - 1);
-  if (runs < LEAST_RUNS || max_q_len <= SHORTEST) return 0;
-  int run = (chunks + runs - 1) / runs;
-  if (run < MIN_RUN) run = MIN_RUN;
-  return run * CHUNK < max_q_len ? run : 0;
+  return side_fits(64, vdim) && max_q_len > 2 * CHUNK && long_chunks(rows, segments, 1) <= 65535 ? 1 : 0;
 }
-MLR_EXPORT long long mlr_matrix_memory_run_scratch(int rows, int run, int heads, int dim, int vdim) {
-  return run <= 0 ? 0 : run_places(rows, run * CHUNK) * heads * ((long long)(vdim + 1) * dim + 1);
+// .. and the float32 numbers of scratch that side by side needs.
+MLR_EXPORT long long mlr_matrix_memory_run_scratch(int rows, int segments, int heads, int dim, int vdim) {
+  return long_chunks(rows, segments, 1) * heads * ((long long)(vdim + 1) * dim + 1);
 }
 
 // q, k: float32 rows of heads * dim entries; v, gate: rows of heads * vdim; i_raw, f_raw: rows of `heads` entries (each
 // with its own row stride); i_bias, f_bias: float32 [heads]; weight: float32 [heads * vdim]; coef: float32 scratch
 // [rows, heads, 4], reads: [rows, heads, vdim], norms: [rows, heads] (all three null for steps of single rows); pairs:
 // float32 scratch [rows, heads, 64 + 2] and packed: bfloat16 scratch [rows, heads, 2 dim + vdim] (both or neither: chunks
-// on the tensor cores, or the token-by-token scan; 16-byte aligned); run, ends: chunks of a run and the scratch that needs (as the two
-// functions above say; 0 and null: no runs); states:
+// on the tensor cores, or the token-by-token scan; 16-byte aligned); ends: null, or the scratch of chunks side by side (as the two
+// functions above say, for bfloat16 results; reads, norms, pairs and packed are then not asked for); states:
 // float32 [slots, heads, vdim + 1, dim], maxima: float32 [slots, heads]; out: [rows, heads * vdim] in `dtype`.
 // max_q_len: the longest segment of the step.
 MLR_EXPORT int mlr_matrix_memory(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
                                  long long v_stride, const float* i_raw, long long i_stride, const float* f_raw,
                                  long long f_stride, const float* gate, long long gate_stride, const float* i_bias,
                                  const float* f_bias, const float* weight, float* coef, float* reads, float* norms,
-                                 float* pairs, void* packed, float* ends, int run, float* states, float* maxima, void* out, const int* seg_q_start, const int* seg_q_len,
+                                 float* pairs, void* packed, float* ends, float* states, float* maxima, void* out, const int* seg_q_start, const int* seg_q_len,
                                  const int* seg_slot, int rows, int segments, int max_q_len, int heads, int dim, int vdim,
                                  float cap, float guard, float eps, float q_scale, int dtype, cudaStream_t stream) {
   if (segments == 0 || rows == 0) return MLR_OK;
@@ -951,15 +1368,15 @@ MLR_EXPORT int mlr_matrix_memory(const float* q, long long q_stride, const float
   bf16* q16 = (bf16*)packed;
   bf16* k16 = q16 == nullptr ? nullptr : q16 + (size_t)rows * heads * dim;
   bf16* v16 = q16 == nullptr ? nullptr : k16 + (size_t)rows * heads * dim;
-  if ((pairs == nullptr) != (packed == nullptr) || run < 0 || (run > 0 && (ends == nullptr || pairs == nullptr))) return MLR_BAD_SIZE;
+  if ((pairs == nullptr) != (packed == nullptr)) return MLR_BAD_SIZE;
   MemoryArgs p{q, k, v, i_raw, f_raw, gate, q_stride, k_stride, v_stride, i_stride, f_stride, gate_stride, i_bias, f_bias,
                weight, reinterpret_cast<float4*>(coef), reads, norms, pairs,
                pairs == nullptr ? nullptr : reinterpret_cast<float2*>(pairs + (size_t)rows * heads * CHUNK), q16, k16, v16, states, maxima, ends,
-               run <= 0 ? nullptr : ends + (size_t)run_places(rows, run * CHUNK) * heads * (vdim + 1) * dim, run, seg_q_start, seg_q_len, seg_slot, heads,
-               dim, vdim, cap, guard, eps, q_scale};
+               ends == nullptr ? nullptr : ends + (size_t)long_chunks(rows, segments, 1) * heads * (vdim + 1) * dim, seg_q_start, seg_q_len, seg_slot,
+               segments, heads, dim, vdim, cap, guard, eps, q_scale};
   auto multiple = [](long long n) { return n % 4 == 0; };
   auto aligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
-  if (!aligned(coef) || !aligned(pairs) || !aligned(packed)) return MLR_BAD_ALIGNMENT;
+  if (!aligned(coef) || !aligned(pairs) || !aligned(packed) || !aligned(ends)) return MLR_BAD_ALIGNMENT;
   const bool wide = multiple(dim) && multiple(vdim) && multiple(q_stride) && multiple(k_stride) && multiple(v_stride) &&
                     aligned(q) && aligned(k) && aligned(v) && aligned(states);
   if (dtype == MLR_F32) return launch_memory(p, (float*)out, rows, segments, max_q_len, wide, stream);

@@ -1977,7 +1977,7 @@ class CudaOps:
     # ------------------------------------------------------------------ matrix memory
     use_memory_chunks = True      # bfloat16 prompts in chunks of 64 tokens on the tensor cores
     MEMORY_CHUNK_ROWS = 16        # longest portion of a step from which that pays
-    use_memory_runs = True        # long portions in runs of chunks side by side
+    use_memory_runs = True        # chunks side by side
 
     def _memory_chunks_fit(self, dim: int, vdim: int) -> bool:
         cache = self.__dict__.setdefault("_memory_fits", {})
@@ -2007,27 +2007,28 @@ class CudaOps:
                               "one maximum per slot and head")
         out = torch.empty((rows, heads * vdim), dtype=out_dtype, device=q.device)
         coef = reads = norms = pairs = packed = ends = None
-        run = 0
         if ctx.max_q_len > 1:
+            coef = torch.empty((rows, heads, 4), dtype=torch.float32, device=q.device)
             if (out_dtype == torch.bfloat16 and self.use_memory_chunks and ctx.max_q_len >= self.MEMORY_CHUNK_ROWS
                     and all(t.data_ptr() % 16 == 0 and t.stride(0) % 4 == 0 for t in (q, k, v))
                     and self._memory_chunks_fit(dim, vdim)):
-                pairs = torch.empty((rows, heads, 66), dtype=torch.float32, device=q.device)
-                packed = torch.empty((rows, heads, 2 * dim + vdim), dtype=torch.bfloat16, device=q.device)
                 lib = build.load_library("matrix_memory")
-                run = lib.mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim) if self.use_memory_runs else 0
-                if run > 0:
+                if self.use_memory_runs and lib.mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim) > 0:
                     lib.mlr_matrix_memory_run_scratch.restype = ctypes.c_longlong
-                    ends = torch.empty(lib.mlr_matrix_memory_run_scratch(rows, run, heads, dim, vdim), dtype=torch.float32, device=q.device)
-            coef = torch.empty((rows, heads, 4), dtype=torch.float32, device=q.device)
-            reads = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device)
-            norms = torch.empty((rows, heads), dtype=torch.float32, device=q.device)
+                    ends = torch.empty(lib.mlr_matrix_memory_run_scratch(rows, ctx.num_segments, heads, dim, vdim), dtype=torch.float32,
+                                       device=q.device)
+                else:
+                    pairs = torch.empty((rows, heads, 66), dtype=torch.float32, device=q.device)
+                    packed = torch.empty((rows, heads, 2 * dim + vdim), dtype=torch.bfloat16, device=q.device)
+            if ends is None:
+                reads = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device)
+                norms = torch.empty((rows, heads), dtype=torch.float32, device=q.device)
         _check(build.load_library("matrix_memory").mlr_matrix_memory(
             *self._view(q, "q", rows, heads * dim), *self._view(k, "k", rows, heads * dim),
             *self._view(v, "v", rows, heads * vdim), *self._view(i_raw, "i_raw", rows, heads),
             *self._view(f_raw, "f_raw", rows, heads), *self._view(gate, "gate", rows, heads * vdim), _ptr(i_bias),
             _ptr(f_bias), _ptr(weight), _ptr(coef), _ptr(reads), _ptr(norms), _ptr(pairs),
-            _ptr(packed), _ptr(ends), run, _ptr(state), _ptr(maximum), _ptr(out),
+            _ptr(packed), _ptr(ends), _ptr(state), _ptr(maximum), _ptr(out),
             _ptr(ctx.seg_q_start), _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), rows, ctx.num_segments, int(ctx.max_q_len), heads,
             dim, vdim, ctypes.c_float(cap), ctypes.c_float(guard), ctypes.c_float(eps), ctypes.c_float(float(dim) ** -0.5),
             _code(out_dtype), _stream()), "matrix_memory")

@@ -538,6 +538,42 @@ def test_matrix_memory_in_runs_against_64_bits(lengths, slots, order):
     close(got, want, 2.0 ** -8, "output")
 
 
+@pytest.mark.parametrize("heads,dim,vdim", [(1, 64, 8), (3, 128, 88), (2, 64, 96), (2, 128, 128)])
+@pytest.mark.parametrize("lengths,slots,order", [([129, 1, 64, 65], [0, 3, 2, 1], None), ([63, 192, 128, 2], [1, 0, 3, 2], [2, 1, 3, 0])])
+def test_matrix_memory_side_by_side(heads, dim, vdim, lengths, slots, order):
+    """Portions of one chunk, one row more, one less and several beside each other, few and many value channels: as one chunk behind the other.  A number
+    that is none leaves the rows before it as they are."""
+    ctx, rows = segments(lengths, slots, order), sum(lengths)
+    assert memory_run(ctx, rows, heads, vdim) > 0
+    q, k, v, gate = rnd(1, rows, heads * dim), rnd(2, rows, heads * dim), rnd(3, rows, heads * vdim), rnd(4, rows, heads * vdim)
+    i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
+    gate[5], gate[6], gate[7] = -200.0, 200.0, -87.0
+    bias, weight = torch.zeros(heads), 1 + rnd(7, heads * vdim, std=0.1)
+    state, maximum = rnd(8, len(lengths), heads, vdim + 1, dim, std=0.5), rnd(9, len(lengths), heads)
+
+    def call(runs, v):
+        cuda().use_memory_runs = runs
+        try:
+            s, m = state.to(DEVICE), maximum.to(DEVICE)
+            out = cuda().matrix_memory(*(spaced(t, 8) for t in (q, k, v, i_raw, f_raw)), bias.to(DEVICE), bias.to(DEVICE) + 3, 15.0, 1e-6,
+                                       spaced(gate, 8), weight.to(DEVICE), 1e-6, s, m, ctx, heads, dim, vdim, torch.bfloat16)
+        finally:
+            cuda().use_memory_runs = True
+        return out.cpu(), s.cpu(), m.cpu()
+
+    (out, s, m), (want, want_s, want_m) = call(True, v), call(False, v)
+    assert torch.equal(m, want_m)
+    close(s.flatten(0, 1), want_s.flatten(0, 1), 200 * UNIT, "state")      # sums of 64 products at a time, once per chunk
+    close(out, want, 2.0 ** -8, "output")
+    last = int(ctx.seg_q_start[lengths.index(max(lengths))]) + max(lengths) - 1      # of the longest portion, in a block of 16 rows of its own
+    broken = v.clone()
+    broken[last] = float("nan")
+    after = call(True, broken)[0]
+    kept = torch.arange(rows) != last
+    kept[last - (max(lengths) - 1) % 16:last] = False      # rows of the same block meet it with a weight of nothing
+    assert torch.equal(after[kept], out[kept]) and bool(after[last].isnan().any())
+
+
 def memory_run(ctx, rows, heads, vdim):
     from mini_llm_runtime_b200.ops import build
     return build.load_library("matrix_memory").mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim)
