@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(WalkShape<MODE, DIM, VDIM>::THREADS)
 chunk_walk_kernel(ChunkArgs p) {
   using W = WalkShape<MODE, DIM, VDIM>;
   constexpr int KD = W::KD, C = W::C, T = W::T, THREADS = W::THREADS, SLICES = W::SLICES;
-  pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x;
   const auto [seg, chunk, length, start, slot] =
@@ -195,6 +194,10 @@ chunk_walk_kernel(ChunkArgs p) {
 #pragma unroll
   for (int i = 0; i < KD; ++i) store_columns<C>(end + (size_t)(warp * KD + i) * VDIM + column, S[i]);
   if (chunk > 0 && tid < DIM) p.decays[place * DIM + tid] = product;
+  // At the end, in all three kernels: blocks of the next that come in while these still fill some SMs land two to an SM beside empty ones, and each of
+  // them runs long.  Trigger in front / at the end: 7 heads of 128 x 128, 512 rows 72 / 47 us, 2,048 rows 81 / 77, 16 heads 73 / 48 and 151 / 150; 14 heads of
+  // 64 x 64, 300 rows 41 / 28, 512 rows 46 / 29, 2,048 rows 58 / 53, 32 heads, 512 rows 50 / 36.
+  pdl_trigger();
 }
 
 // A thread owns four neighbouring value channels of one key channel and takes the chunks of its segment in order; BATCH chunks
@@ -204,7 +207,6 @@ chunk_walk_kernel(ChunkArgs p) {
 __global__ void __launch_bounds__(256)
 chunk_carry_kernel(ChunkArgs p, int dim, int vdim) {
   constexpr int BATCH = 16;
-  pdl_trigger();
   pdl_wait();
   const auto [seg, which, length, start, slot] = chunk_at<false>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, max(p.least, p.split), blockIdx.y);
   if (seg < 0) return;
@@ -236,6 +238,7 @@ chunk_carry_kernel(ChunkArgs p, int dim, int vdim) {
       }
   }
   *reinterpret_cast<float4*>(p.state + ((size_t)slot * p.heads + head) * cells + cell) = S;
+  pdl_trigger();
 }
 
 // CTA per (head, chunk, segment): VDIM / 4 threads side by side take a token's value channels, eight groups of them eight
@@ -244,7 +247,6 @@ template <typename T, int MODE, int DIM, int VDIM>
 __global__ void __launch_bounds__(2 * VDIM)
 chunk_finish_kernel(ChunkArgs p, T* __restrict__ out) {
   constexpr int LANES = VDIM / 4, THREADS = 2 * VDIM, TOKENS = CHUNK / 8, PITCH = DIM + 4;
-  pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x;
   const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
@@ -326,6 +328,7 @@ chunk_finish_kernel(ChunkArgs p, T* __restrict__ out) {
     else
       *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(y);
   }
+  pdl_trigger();
 }
 
 template <typename T, int MODE, int DIM, int VDIM>

@@ -975,7 +975,6 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
   bf16* k_tile = s_parts;
   __shared__ __align__(16) float keep[CHUNK];
   __shared__ float write[CHUNK], floor_of[CHUNK], since[CHUNK];
-  pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x, V = p.vdim, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, 1, blockIdx.y);
@@ -1189,6 +1188,7 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
       if (full || (first + i < count && lane + 32 * j < V)) dst[(size_t)i * p.heads * V + 32 * j] = y;
     }
   }
+  pdl_trigger();
 }
 
 template <int D, int PAIRS>
