@@ -66,6 +66,11 @@ skinny_gemm_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* __rest
   float (*partial)[GROUPS * TOKENS8 * 4][32] = reinterpret_cast<float (*)[GROUPS * TOKENS8 * 4][32]>(partial_raw);
   __shared__ float squares[WARPS][TOKENS8 * 8];     // per warp: sum of x^2 over its share of K, per token
   __shared__ float row_scale[TOKENS8 * 8];
+  // Steps of up to eight rows let the next kernel in only after their own wait.  With the trigger in front the kernels behind came in one after the other
+  // while this one still waited, held room on the SMs and asked for weights before this one's were there: eight decoding requests of a 24-layer
+  // model of width 896, 12 tokens and their prompts 10,900 us, 9,900 so (behind the activations' loads 10,200, behind all products 10,930); one request,
+  // 24 tokens 14,810 and 13,380.  With more rows the loads of x take longer and the early start pays: 12 requests 20,570 and 20,790, 16 20,250 and 20,600.
+  if (TOKENS8 > 1) pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int k_blocks = (K + 31) / 32;
@@ -142,11 +147,7 @@ skinny_gemm_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* __rest
     if (!waited) {
       pdl_wait();                                             // x comes from the kernel before this one
       waited = true;
-      // Only now may the next kernel come in and ask for its weights.  With the trigger in front of the wait the kernels behind it came in one after
-      // the other while this one still waited, held room on the SMs and asked for weights before this one's were there: eight decoding requests of a
-      // 24-layer model of width 896, 12 tokens and their prompts 10,900 us, 9,900 so; after the wait but behind the activations' loads 10,200, behind
-      // all products 10,930.
-      pdl_trigger();
+      if (TOKENS8 == 1) pdl_trigger();
       fetch_residual();
     }
 #pragma unroll
