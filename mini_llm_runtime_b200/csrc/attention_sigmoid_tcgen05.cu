@@ -138,7 +138,7 @@ __device__ __forceinline__ float sg_log2(float x) {
 __device__ __forceinline__ void sg_half_barrier(int half) { asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(SG_COMPUTE / 2) : "memory"); }
 
 // Entries take a place per key tile and SG_ENTRY before them, for what a CTA spends on an entry whatever its keys (queries, sums out); the run of
-// CTA b begins at place sg_run(b): equal shares.
+// CTA b begins at place sg_run(b): equal shares, and as many runs as there are places where those are fewer than CTAs.
 constexpr int SG_ENTRY = 1;
 __device__ __forceinline__ int sg_run(int b, int total, int ctas) { return (int)((long long)b * total / ctas); }
 
@@ -257,12 +257,13 @@ attention_sigmoid_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, cons
     }
     if (blockIdx.x == 0 && lane == 0) a.before[0] = 0;
     __syncwarp();
-    const int first = sg_run(blockIdx.x, total, gridDim.x);
+    const int runs = min((int)gridDim.x, total), mine = blockIdx.x;      // a CTA without a run has an empty one at place 0
+    const int first = mine < runs ? sg_run(mine, total, runs) : 0;
     int entry = 0;
     for (int base = 0; base < a.tiles; base += 32) entry += __popc(__ballot_sync(0xffffffffu, base + lane < a.tiles && places[base + lane] <= first));
     if (lane == 0) {
       ctl.begin = first;
-      ctl.end = sg_run(blockIdx.x + 1, total, gridDim.x);
+      ctl.end = mine < runs ? sg_run(mine + 1, total, runs) : 0;
       ctl.entry = entry;
       ctl.entry_at = entry > 0 ? places[entry - 1] : 0;
     }
@@ -600,30 +601,29 @@ attention_sigmoid_tcgen05_kernel(const __grid_constant__ CUtensorMap k_map, cons
 
 // Entries that lie in several runs: their sums added in the order of the keys.  grid: (entries, parts), four neighbouring numbers per thread.
 __global__ void __launch_bounds__(256)
-sigmoid_add_runs_kernel(const SgArgs a, int vdim, int ctas) {
+sigmoid_add_runs_kernel(const SgArgs a, int vdim, int most_runs) {
   constexpr int BATCH = 4;
   pdl_trigger();
   pdl_wait();
   const int total = __ldcg(a.before + a.tiles), begin = __ldcg(a.before + blockIdx.x) + SG_ENTRY, end = __ldcg(a.before + blockIdx.x + 1);
   // the run that holds place x is the last one to begin at x or before
-  const int first = (int)(((long long)(begin + 1) * ctas - 1) / total), last = (int)(((long long)end * ctas - 1) / total);
+  const int runs = min(most_runs, total);
+  const int first = (int)(((long long)(begin + 1) * runs - 1) / total), last = (int)(((long long)end * runs - 1) / total);
   if (first == last) return;
   const int seg = a.tile_seg[blockIdx.x], row0 = a.tile_row0[blockIdx.x];
   const int width = a.heads * vdim, count = min(a.slot_rows, a.seg_q_len[seg] - row0) * width;
   bf16* out = a.out + (size_t)(a.seg_q_start[seg] + row0) * width;
   const size_t slot = (size_t)a.slot_rows * width;
-  const bool sparse = total < ctas;      // some runs are empty
-  auto holds = [&](int b) { return b <= last && (!sparse || sg_run(b, total, ctas) < sg_run(b + 1, total, ctas)); };
   for (int index = (blockIdx.y * 256 + threadIdx.x) * 4; index < count; index += gridDim.y * 1024) {
     float4 sum = __ldcg(reinterpret_cast<const float4*>(a.partial + (2 * (size_t)first + 1) * slot + index));
     for (int b0 = first + 1; b0 <= last; b0 += BATCH) {
       float4 part[BATCH];
 #pragma unroll
       for (int i = 0; i < BATCH; ++i)
-        if (holds(b0 + i)) part[i] = __ldcg(reinterpret_cast<const float4*>(a.partial + 2 * (size_t)(b0 + i) * slot + index));
+        if (b0 + i <= last) part[i] = __ldcg(reinterpret_cast<const float4*>(a.partial + 2 * (size_t)(b0 + i) * slot + index));
 #pragma unroll
       for (int i = 0; i < BATCH; ++i)
-        if (holds(b0 + i)) { sum.x += part[i].x; sum.y += part[i].y; sum.z += part[i].z; sum.w += part[i].w; }
+        if (b0 + i <= last) { sum.x += part[i].x; sum.y += part[i].y; sum.z += part[i].z; sum.w += part[i].w; }
     }
     *reinterpret_cast<uint2*>(out + index) = make_uint2(pack_bf16(sum.x, sum.y), pack_bf16(sum.z, sum.w));
   }
