@@ -1756,13 +1756,17 @@ class CudaOps:
         if (self.use_mma_sigmoid and self.use_mma_attention and q.dtype == torch.bfloat16 and dim in (64, 128)
                 and vdim in (64, 128) and q.data_ptr() % 16 == 0):
             wide = _declared_library("attention_sigmoid_tcgen05")
-            if (self.use_tcgen05_attention and int(batch.max_kv_len) > dim // 2 and k_pool.data_ptr() % 16 == 0
+            longest = int(batch.max_kv_len)
+            # A tile has 128 keys whatever the rows see, so the shortest contexts and, in a step of few rows with heads of 128, those that have half a second
+            # tile or less stay on mma.sync.  In us with mma.sync / on tcgen05, 16 heads of 128: 1 row that sees 21 keys 9 / 18, 8 rows 48 keys 15 / 18, 60 rows
+            # 17 / 20, 1 row 65 keys 20 / 18, 90 rows 23 / 20, 130 rows 25 / 24, 160 rows 25 / 28, 192 rows 25 / 28, 224 rows 31 / 28, 16 rows 192 keys 22 / 24, 224
+            # keys 28 / 24; nine portions of 160 rows (90 entries) 28 / 28, of 176 (99) 39 / 29; 14 heads of 64, 1 row 21 keys 8 / 12, 8 rows 48 keys 13 / 12, 60 rows
+            # 16 / 14, 239 keys 30 / 21.
+            few = longest <= dim // 2 or (dim == 128 and 128 < longest <= 192 and tiles <= 90)
+            if (self.use_tcgen05_attention and not few and k_pool.data_ptr() % 16 == 0
                     and v_pool.data_ptr() % 16 == 0 and tiles <= wide.mlr_attention_sigmoid_tcgen05_most()
                     and wide.mlr_attention_sigmoid_tcgen05_fits(heads, kv_heads, dim, vdim, k_pool.shape[2])):
-                # both products on tcgen05.  Its tiles have 128 keys whatever the rows see, so the shortest contexts stay where they were:
-                # us with mma.sync / so, 16 heads of 128, 1 row that sees 21 keys 9 / 18, 8 rows 48 keys 15 / 18, 60 rows 17 / 20, 1 row 65 keys 20 / 18,
-                # 90 rows 23 / 20; 14 heads of 64, 1 row 21 keys 8 / 12, 8 rows 48 keys 13 / 12, 60 rows 16 / 14
-                most = -(-int(batch.max_kv_len) // 128)      # key tiles of an entry
+                most = -(-longest // 128)      # key tiles of an entry
                 ctas = min(self.sm_count(q.device), tiles * most)
                 wide.mlr_attention_sigmoid_tcgen05_scratch.restype = ctypes.c_longlong
                 scratch = torch.empty(wide.mlr_attention_sigmoid_tcgen05_scratch(tiles, ctas, int(batch.max_q_len), heads, vdim),
@@ -1781,9 +1785,8 @@ class CudaOps:
                 # several CTAs; and no CTA takes more than SIGMOID_MMA_LONGEST keys, so that the rows at the end
                 # of a long prompt (which see all of it) do not keep one SM busy long after the others
                 want = max(1, 2 * self.sm_count(q.device) // max(tiles, 1))
-                longest = int(batch.max_kv_len)
                 chunks = max(-(-longest // self.SIGMOID_MMA_LONGEST), min(want, -(-longest // self.SIGMOID_MMA_CHUNK_KEYS)), 1)
-                chunk_keys = max(32, -(-(-(-int(batch.max_kv_len) // chunks)) // 32) * 32)
+                chunk_keys = max(32, -(-(-(-longest // chunks)) // 32) * 32)
                 partial = None
                 if chunks > 1:
                     partial = torch.empty((chunks, rows, heads * vdim), dtype=torch.float32, device=q.device)

@@ -242,7 +242,7 @@ def test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, mixed):
 
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,page_size", [(16, 4, 128, 128, 8), (14, 2, 64, 64, 16), (9, 3, 128, 64, 64), (5, 1, 64, 128, 256),
                                                                (4, 4, 64, 64, 128)])
-@pytest.mark.parametrize("lengths,before", [([129], [0]), ([16, 1, 8], [112, 640, 300]), ([1] * 7, [127, 128, 63, 64, 1000, 200, 500]),
+@pytest.mark.parametrize("lengths,before", [([129], [0]), ([16, 1, 8], [112, 640, 300]), ([1] * 7, [127, 128, 63, 64, 1000, 200, 500]), ([1] * 6, [2700, 3, 60, 127, 128, 11]),
                                             ([70, 260, 9, 1], [250, 0, 127, 383])])
 def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, lengths, before):
     """Keys around tiles of 128 and their halves, rows around the 8 of half an entry, entries cut and whole, pages smaller and larger than a
