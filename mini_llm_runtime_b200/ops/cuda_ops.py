@@ -2133,10 +2133,11 @@ class CudaOps:
         return out
 
     use_state_space_chunks = True
-    # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us, token by
-    # token / in chunks, 14 heads with states of 64 (32 heads, 128): 77 rows 18 / 24 (26 / 32), 96 rows 22 / 24 (32 / 33), 112 rows 25 / 24 (37 / 33), 160 rows
-    # 35 / 26 (52 / 35), 512 rows 108 / 24 (161 / 39); three of 100 rows beside one of 1,000 57 / 34 (95 / 81).
-    STATE_SPACE_CHUNK_ROWS = 97
+    # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us from a flushed L2, token by
+    # token / in chunks, 14 heads with states of 64 (32 heads, 128): 97 rows 29 / 34 (31 / 40), 112 rows 31 / 33 (33 / 39), 128 rows 35 / 34 (37 / 38), 140 rows
+    # 37 / 34 (39 / 41), 160 rows 41 / 34 (44 / 41), 512 rows 108 / 24 (161 / 39) repeated.  Three of 100 rows beside one of 1,000 would gain from chunks too (55 / 45
+    # and 108 / 97), but which way a portion goes is a matter of its own rows, as its numbers are.
+    STATE_SPACE_CHUNK_ROWS = 144
 
     def state_space_scan(self, x, B, C, dt_raw, dt_bias, A_log, D, state, ctx, heads: int, vdim: int, n: int,
                          groups: int) -> torch.Tensor:
