@@ -131,9 +131,12 @@ def test_state_space_in_chunks(heads, n, groups, lengths, slots, order, monkeypa
 @pytest.mark.parametrize("heads,n,groups", [(2, 64, 1), (4, 128, 2)])
 @pytest.mark.parametrize("where", ["x", "B", "C", "state", "before"])
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
-def test_state_space_chunks_with_numbers_that_have_no_parts(heads, n, groups, where, value):
+def test_state_space_chunks_with_numbers_that_have_no_parts(heads, n, groups, where, value, monkeypatch):
     """One such number among ordinary ones goes by multiply-adds in its chunk: outputs that are no numbers where token by token has them, the
     others as there.  ``before``: a state that only later chunks see."""
+    monkeypatch.setattr(cuda(), "STATE_SPACE_CHUNK_ROWS", 65)
+    launched, load = [], cuda_ops.build.load_library
+    monkeypatch.setattr(cuda_ops.build, "load_library", lambda name: launched.append(name) or load(name))
     lengths, slots = [130, 65], [1, 0]
     ctx, rows, inner = segments(lengths, slots), sum(lengths), heads * 64
     x, B, C, dt = rnd(1, rows, inner), rnd(2, rows, groups * n), rnd(3, rows, groups * n), rnd(4, rows, heads, std=0.5) - 3
@@ -149,6 +152,7 @@ def test_state_space_chunks_with_numbers_that_have_no_parts(heads, n, groups, wh
         finally:
             cuda().use_state_space_chunks = True
         results.append((y.cpu().double(), s.cpu().double()))
+    assert [name for name in launched if name.startswith("state_space")] == ["state_space", "state_space_chunks"]
     for want, got in zip(*results):
         # beside 3.4e38 sums overflow in one order and not in the other; the outputs and states that it has no part in are ordinary
         if value != 3.4e38:
