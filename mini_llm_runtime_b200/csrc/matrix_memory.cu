@@ -33,7 +33,7 @@
 // matrix_memory_chunks_kernel   the chunks of a (request, head) one after the other, value channels over blocks; the
 //                               state stays in registers as accumulators.
 #include "chunk_places.cuh"
-#include "mma_attention.cuh"
+#include "part_products.cuh"
 #include "copy_async.cuh"
 #include "lane_sums.cuh"
 
@@ -943,6 +943,13 @@ memory_carry_kernel(MemoryArgs p, int cells) {
 constexpr int SIDE_D = 32;                // key channels of the state taken at a time
 constexpr int SIDE_D_PITCH = SIDE_D + 8;
 constexpr int SIDE_A_PITCH = CHUNK + 8;
+// Sums of the outputs: the leading part's products in an accumulator of their own; the smaller ones' sums of 32 key channels (16 tokens) are added with
+// what the leading sum's steps dropped on average (with_dropped).  Sums that cancel to some 2^-18 of their products, heads of 128 (64), errors with one chunk
+// behind the other / all in one accumulator / so: reads of the state 1.23e-2 (0.66e-2) / 5.9e-2 (3.5e-2) / 0.99e-2 (0.66e-2), with tokens 3.1e-2 (2.3e-2) /
+// 13.5e-2 (10.2e-2) / 2.8e-2 (2.1e-2); 0.0 and 0.0 give 1.39e-2 (0.80e-2) and 3.3e-2 (2.7e-2).  1,300 and 748 rows of 7
+// heads: 48.3 us in one accumulator, 50.4 so.
+constexpr float STATE_DROPPED = 0.6f, TOKENS_DROPPED = 0.25f;
+constexpr int SIDE_LOW = 2;               // column pairs whose smaller products are summed at a time
 constexpr int SIDE_SUMS = SIDE_V + 8;     // float32 sums of a row, the normaliser among them
 
 template <int D>
@@ -1089,20 +1096,29 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
     __syncthreads();
     if (d0 + SIDE_D < D) ask(d0 + SIDE_D);
     if (tile * 16 < count) {
+      uint32_t a[SIDE_D / 16][4];
 #pragma unroll
-      for (int ks = 0; ks < SIDE_D / 16; ++ks) {
-        uint32_t a[4];
-        ldmatrix_x4(a, q_at + d0 + ks * 16);
+      for (int ks = 0; ks < SIDE_D / 16; ++ks) ldmatrix_x4(a[ks], q_at + d0 + ks * 16);
 #pragma unroll
-        for (int n = 2; n >= 0; --n)
+      for (int j0 = 0; j0 < MOST; j0 += SIDE_LOW) {
+        float low[2 * SIDE_LOW][4] = {};
 #pragma unroll
-          for (int j = 0; j < MOST; ++j) {
-            uint32_t b[4];
-            ldmatrix_x4(b, s_parts + n * Shape::S_APART + (min(pair0 + j, PAIRS - 1) * 16 + (lane & 7) + ((lane >> 4) << 3)) * SIDE_D_PITCH + ks * 16 +
-                               ((lane >> 3) & 1) * 8);
-            mma_bf16(o[2 * j], a, b[0], b[1]);
-            mma_bf16(o[2 * j + 1], a, b[2], b[3]);
-          }
+        for (int ks = 0; ks < SIDE_D / 16; ++ks)
+#pragma unroll
+          for (int n = 2; n >= 0; --n)
+#pragma unroll
+            for (int j = j0; j < j0 + SIDE_LOW && j < MOST; ++j) {
+              uint32_t b[4];
+              ldmatrix_x4(b, s_parts + n * Shape::S_APART + (min(pair0 + j, PAIRS - 1) * 16 + (lane & 7) + ((lane >> 4) << 3)) * SIDE_D_PITCH + ks * 16 +
+                                 ((lane >> 3) & 1) * 8);
+              float (*sum)[4] = n > 0 ? low + 2 * (j - j0) : o + 2 * j;
+              mma_bf16(sum[0], a[ks], b[0], b[1]);
+              mma_bf16(sum[1], a[ks], b[2], b[3]);
+            }
+#pragma unroll
+        for (int i = 0; i < 2 * SIDE_LOW && 2 * j0 + i < 2 * MOST; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[2 * j0 + i][e] += with_dropped(o[2 * j0 + i][e], low[i][e], STATE_DROPPED);
       }
     }
   }
@@ -1121,15 +1137,24 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
         split_pair(x.x, x.y, part[e]);
       }
 #pragma unroll
-      for (int j = 0; j < MOST; ++j) {
-        uint32_t b[4];
-        ldmatrix_x4_trans(b, v_tile + (ks * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * SIDE_PITCH + (min(pair0 + j, PAIRS - 1) * 2 + (lane >> 4)) * 8);
+      for (int j0 = 0; j0 < MOST; j0 += SIDE_LOW) {
+        float low[2 * SIDE_LOW][4] = {};
+        uint32_t b[SIDE_LOW][4];
 #pragma unroll
-        for (int n = 2; n >= 0; --n) {
-          const uint32_t a[4] = {part[0][n], part[1][n], part[2][n], part[3][n]};
-          mma_bf16(o[2 * j], a, b[0], b[1]);
-          mma_bf16(o[2 * j + 1], a, b[2], b[3]);
-        }
+        for (int n = 2; n >= 0; --n)
+#pragma unroll
+          for (int j = j0; j < j0 + SIDE_LOW && j < MOST; ++j) {
+            if (n == 2)
+              ldmatrix_x4_trans(b[j - j0], v_tile + (ks * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * SIDE_PITCH + (min(pair0 + j, PAIRS - 1) * 2 + (lane >> 4)) * 8);
+            const uint32_t a[4] = {part[0][n], part[1][n], part[2][n], part[3][n]};
+            float (*sum)[4] = n > 0 ? low + 2 * (j - j0) : o + 2 * j;
+            mma_bf16(sum[0], a, b[j - j0][0], b[j - j0][1]);
+            mma_bf16(sum[1], a, b[j - j0][2], b[j - j0][3]);
+          }
+#pragma unroll
+        for (int i = 0; i < 2 * SIDE_LOW && 2 * j0 + i < 2 * MOST; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[2 * j0 + i][e] += with_dropped(o[2 * j0 + i][e], low[i][e], TOKENS_DROPPED);
       }
     }
   }

@@ -578,6 +578,44 @@ def test_matrix_memory_side_by_side(heads, dim, vdim, lengths, slots, order):
     assert torch.equal(after[kept], out[kept]) and bool(after[last].isnan().any())
 
 
+@pytest.mark.parametrize("heads,dim,vdim", [(64, 128, 128), (64, 64, 96)])
+@pytest.mark.parametrize("what", ["state", "state and tokens"])
+def test_matrix_memory_side_by_side_loses_no_bits_of_its_sums(heads, dim, vdim, what):
+    """Sums that cancel to some 2^-18 of their products, which shows in 16 bits what was lost of 32: no more than one chunk behind the other loses.
+    A head's norm takes the small sums to ordinary size."""
+    rows, ctx = 192, segments([192], [0])
+    query, k, v = (rnd(i, *shape).to(torch.bfloat16).double() for i, shape in ((1, (heads, dim)), (2, (rows, heads, dim)), (3, (rows, heads, vdim))))
+    along = query / (query * query).sum(1, keepdim=True)
+    state = rnd(4, heads, vdim + 1, dim).double()
+    state -= torch.einsum("hcd,hd->hc", state, query)[..., None] * along[:, None]      # across the query
+    rest = rnd(5, heads, vdim + 1) * dim ** 0.5 * 2.0 ** -18
+    i_raw, maximum, take = torch.full((rows, heads), -15.0), torch.full((1, heads), 15.0), slice(0, 64)      # tokens write e^-30
+    if what == "state":
+        v.zero_()
+    else:                                       # the state takes back what a chunk's tokens write, as its last row reads them
+        i_raw, maximum, take = torch.zeros(rows, heads), torch.zeros(1, heads), slice(63, 64)
+        written = torch.einsum("shd,hd,shc->hc", k[:64], query, torch.cat([v[:64], torch.ones(64, heads, 1)], 2))
+        rest = rest * 8 - written
+    state = (state + rest[..., None] * along[:, None]).float()[None]
+    q, k, v = query.flatten().expand(rows, -1).float().contiguous(), k.flatten(1).float(), v.flatten(1).float()
+    gate, weight = torch.zeros(rows, heads * vdim), torch.ones(heads * vdim)
+    f_raw, zero = torch.full((rows, heads), 200.0), torch.zeros(heads)      # kept whole
+    s64 = state.double()
+    want = FAKE.matrix_memory(*(t.double() for t in (q, k, v, i_raw, f_raw, zero, zero)), 100.0, 1e-6, gate.double(), weight.double(), 1e-30,
+                              s64, maximum.double(), types.SimpleNamespace(**{**vars(ctx), "seg_slot": ctx.seg_slot.cpu()}), heads, dim, vdim, torch.float64)
+    errors, take = [], slice(0, 64) if what == "state" else slice(63, 64)
+    for together in (False, True):
+        cuda().use_memory_runs = together
+        try:
+            got = cuda().matrix_memory(*(t.to(DEVICE) for t in (q, k, v, i_raw, f_raw, zero, zero)), 100.0, 1e-6, gate.to(DEVICE), weight.to(DEVICE),
+                                       1e-30, state.to(DEVICE), maximum.to(DEVICE), ctx, heads, dim, vdim, torch.bfloat16)
+        finally:
+            cuda().use_memory_runs = True
+        errors.append(float((got.double().cpu() - want)[take].norm() / want[take].norm()))
+    # 2^-18 of a sum's 24 bits leave six.  Thousands of numbers that were lost alike: the two means of squares differ by a few in a hundred by chance
+    assert 2.0 ** -8 < errors[0] and errors[1] <= 1.03 * errors[0], errors
+
+
 def memory_run(ctx, rows, heads, vdim):
     from mini_llm_runtime_b200.ops import build
     return build.load_library("matrix_memory").mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim)
