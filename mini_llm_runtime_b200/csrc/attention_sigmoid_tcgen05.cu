@@ -6,8 +6,9 @@
 //   O^T = V^T W'^T  128 value columns (lanes) x (query heads, 16 rows), kept in tensor memory over all key tiles
 // and the columns of S^T stand in an order (SG_SLOTS below) in which a tensor-memory load leaves in each thread of four the heads that mma.sync
 // wants there as its second operand: W'^T = talk W^T is a third product (16 heads x 16 heads x 8 keys) without a weight leaving its
-// thread.  Its operands are split exactly into three bfloat16 parts each, six of the nine products (the others are below 2^-23 of the
-// result), float32 sums.  By multiply-adds (a thread owning one key and eight rows with all heads) every factor of the mixing came from shared
+// thread.  Its operands are split exactly into three bfloat16 parts each, six of the nine products (the others are below 2^-26 of the
+// magnitudes' sum; parts cut off instead of rounded would leave 2^-22 of one sign), float32 sums.  Equal heads whose factors cancel to 2^-17, errors by
+// multiply-adds / with cut / with rounded parts: 3.3e-2 / 2.2e-2 / 0.5e-2 (16 heads of 128), 2.6e-2 / 2.1e-2 / 0.5e-2 (12 of 64).  By multiply-adds (a thread owning one key and eight rows with all heads) every factor of the mixing came from shared
 // memory, four wavefronts per 16 bytes, whose bandwidth the MMAs' operands and the copies want.  A thread ends with eight rows of a
 // (key, head), the 16 bytes that the second product reads together.  Value heads of 64 lie two to the 128 lanes; what a head's rows make of its
 // neighbour's values is never read.
@@ -26,7 +27,7 @@
 // its keys (5,000 to 12,000 cycles until its first scores, of which 3 or 4 stages' copies at a time, 4,000 for its sums).  Measured (B200), mma.sync kernel / this one, with
 // the adding: portions of 1,450, 401 and 197 rows, 16 heads of 128 166 / 68 us, 14 of 64 102 / 56; 2,048 rows 243 / 89 and 170 / 76; 4,000 rows
 // 844 / 238 and 516 / 206; eight decoded rows at 2,000 keys 29 / 29 and 33 / 24, 32 at 3,000 140 / 62 and 81 / 45.
-#include "mma_attention.cuh"
+#include "part_products.cuh"
 #include "tcgen05.cuh"
 
 namespace mlr {
@@ -108,13 +109,10 @@ __device__ __forceinline__ void sg_tmem_load_scores(uint32_t taddr, float* r) {
                  "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
                : "r"(taddr) : "memory");
 }
-// Two numbers as three parts of 8 bits each, exactly: the upper halves of x, of what is left of it, and of what is left then.
+// Two numbers as three parts each.
 __device__ __forceinline__ void sg_parts(float2 x, uint32_t (&part)[3]) {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    part[i] = __byte_perm(__float_as_uint(x.x), __float_as_uint(x.y), 0x7632);
-    if (i < 2) x.x -= __uint_as_float(__float_as_uint(x.x) & 0xffff0000u), x.y -= __uint_as_float(__float_as_uint(x.y) & 0xffff0000u);
-  }
+  for (int i = 0; i < 3; ++i) part[i] = take_part(x.x, x.y);
 }
 __device__ __forceinline__ void sg_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {      // may be moved among other products
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"

@@ -289,6 +289,36 @@ def test_heads_mixed_by_parts_are_mixed_in_32_bits():
     close(got, want, ATTENTION_BOUND + 2.0 ** -6.4, "mixed weights")
 
 
+def on_tcgen05(monkeypatch):
+    """Every sigmoid attention of sizes that fit on tcgen05, whatever it costs; how many calls went there."""
+    lib, calls = cuda_ops._declared_library("attention_sigmoid_tcgen05"), []
+    kernel = lib.mlr_attention_sigmoid_tcgen05
+    monkeypatch.setattr(lib, "mlr_attention_sigmoid_tcgen05", lambda *args: calls.append(1) or kernel(*args))
+    return calls
+
+
+@pytest.mark.parametrize("heads,dim", [(12, 64), (16, 128)])
+def test_heads_mixed_by_parts_lose_no_more_than_multiply_adds(heads, dim, monkeypatch):
+    """Equal heads, factors whose sum is 2^-17: what the mixing lost of 32 bits shows in the 8 bits of the mixed weights."""
+    rows = 300
+    (k_pool, v_pool), cpu, batch = paged([rows], [0], lambda p, j: j <= p, 16, [(1, dim, 1.0), (1, dim, 0.5)], 12)
+    q = rnd(6, rows, 1, dim).expand(rows, heads, dim).reshape(rows, heads * dim).to(torch.bfloat16)
+    mix = rnd(4, heads, heads)
+    for _ in range(3):
+        mix[:, -1] += (2.0 ** -17 - mix.double().sum(1)).float()
+    args = (heads, 1, dim, dim, dim ** -0.5)
+    plain = FAKE.sigmoid_attention(q.double(), k_pool.double(), v_pool.double(), cpu, *args).double().view(rows, heads, dim)
+    want = (plain[:, :1] * mix.double().sum(1)[None, :, None]).reshape(rows, heads * dim)
+    calls, errors = on_tcgen05(monkeypatch), []
+    for wide in (False, True):
+        monkeypatch.setattr(cuda(), "use_tcgen05_attention", wide)
+        got = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, head_mix=mix.to(DEVICE))
+        errors.append(float((got.double().cpu() - want).norm() / want.norm()))
+    assert len(calls) == 1
+    # a chain of multiply-adds rounds once per head; products of whole parts are cut once, by half a place on average
+    assert 2.0 ** -8 < errors[0] and errors[1] <= 0.5 * errors[0], errors
+
+
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 128), (3, 64, 72)])
 @pytest.mark.parametrize("lengths,slots,order", [([1, 512, 513, 1100], [3, 0, 2, 1], None), ([515, 3, 1030], [1, 2, 0], [2, 0, 1])])
 def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
