@@ -22,6 +22,12 @@
 // runs leaves its sums in float32, which a second kernel adds up in order.  (Whole entries would not balance: the last rows of a
 // prompt see all of it.)
 //
+// A run's products with the values meet in one accumulator, which is cut at every 16 keys, where the kernel before added sums of up to 384 keys in float32.  Errors
+// against 64 bits, that kernel / this one, 16 heads of 128: 2,048 rows 2.3552e-3 / 2.3556e-3, 4,000 rows 2.3645e-3 / 2.3645e-3, 4,000 rows behind 2,000
+// 2.3483e-3 / 2.3483e-3, 2,048 rows behind 30,000 2.3059e-3 / 2.3061e-3; 14 of 64: 2.2882e-3 / 2.2881e-3, 2.2787e-3 / 2.2787e-3, 2.2724e-3 / 2.2721e-3, 2.4068e-3 /
+// 2.4078e-3.  Only sums that cancel to 2^-9 and less tell them apart (by up to six times at 3,000 keys of a run).  Adding to float32 sums in device memory after every
+// three tiles took 20 us each time (4,000 rows 249 -> 408 us), after every eight 249 -> 304.
+//
 // Bound by the computing warps: a tile of 128 keys takes 11,000 cycles, of which the special-function units (an exponential and a reciprocal
 // per weight) need 4,100 and the mixing's products 2,000, two warps per scheduler hardly overlapping; then by what every piece costs whatever
 // its keys (5,000 to 12,000 cycles until its first scores, of which 3 or 4 stages' copies at a time, 4,000 for its sums).  Measured (B200), mma.sync kernel / this one, with

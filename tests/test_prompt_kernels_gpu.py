@@ -319,6 +319,29 @@ def test_heads_mixed_by_parts_lose_no_more_than_multiply_adds(heads, dim, monkey
     assert 2.0 ** -8 < errors[0] and errors[1] <= 0.5 * errors[0], errors
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim", [(16, 4, 128), (14, 2, 64)])
+def test_sigmoid_attention_of_long_contexts(heads, kv_heads, dim, monkeypatch):
+    """Thousands of keys summed in one accumulator: as near to 64 bits as sums of up to 384 keys that are added in 32 bits."""
+    rows, before, take = 2048, 6000, 128
+    (k_pool, v_pool), cpu, batch = paged([rows], [before], lambda p, j: j <= p, 16, [(kv_heads, dim, 1.0), (kv_heads, dim, 0.6)], 13)
+    q = rnd(6, rows, heads * dim).to(torch.bfloat16).to(DEVICE)
+    bias, mix = rnd(3, heads, std=0.3).to(DEVICE), (torch.eye(heads) + rnd(4, heads, heads, std=0.1)).to(DEVICE)
+    j = torch.arange(rows + before, device=DEVICE)
+    keys, values = (pool.to(DEVICE)[cpu.block_table[0].to(DEVICE).long()[j // 16], :, j % 16].double().repeat_interleave(heads // kv_heads, 1)
+                    for pool in (k_pool, v_pool))
+    scores = torch.einsum("rhd,nhd->rhn", q[-take:].view(take, heads, dim).double(), keys) * dim ** -0.5 + bias.double()[:, None]
+    seen = (j[None] <= before + rows - take + torch.arange(take, device=DEVICE)[:, None])[:, None]
+    want = torch.einsum("rhn,nhd->rhd", torch.einsum("hg,rgn->rhn", mix.double(), torch.sigmoid(scores) * seen), values).flatten(1)
+    calls, errors = on_tcgen05(monkeypatch), []
+    for wide in (False, True):
+        monkeypatch.setattr(cuda(), "use_tcgen05_attention", wide)
+        got = cuda().sigmoid_attention(q, k_pool.to(DEVICE), v_pool.to(DEVICE), batch, heads, kv_heads, dim, dim, dim ** -0.5, score_bias=bias, head_mix=mix)
+        errors.append(float((got[-take:].double() - want).norm() / want.norm()))
+    assert len(calls) == 1
+    # both are the roundings of weights and results to 8 bits, some 2^-8.8; of 200,000 numbers their means of squares differ by a few in a thousand
+    assert errors[1] <= 1.005 * errors[0], errors
+
+
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 128), (3, 64, 72)])
 @pytest.mark.parametrize("lengths,slots,order", [([1, 512, 513, 1100], [3, 0, 2, 1], None), ([515, 3, 1030], [1, 2, 0], [2, 0, 1])])
 def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
