@@ -55,7 +55,7 @@ struct MemoryArgs {
   float* ends;                          // chunks side by side: [chunks, heads, vdim + 1, dim], what a chunk's tokens leave, then the state before it
   float* spans;                         // [chunks, heads]: product of a chunk's keeps
   const int *seg_q_start, *seg_q_len, *seg_slot;
-  int segments, heads, dim, vdim;
+  int segments, least, heads, dim, vdim;      // least: rows of a segment that goes in chunks side by side; 2: single rows go as decoded ones
   float cap, guard, eps, q_scale;
 };
 
@@ -67,21 +67,24 @@ __device__ __forceinline__ float sigmoid(float z) { return 1.f / (1.f + expf(-z)
 constexpr int DECODE_THREADS = 256;
 constexpr int DECODE_WARPS = DECODE_THREADS / 32;
 
-// PIECES: 16-byte pieces of a state row per lane (dim <= 128 * PIECES, rows and pointers aligned), or 0: any
-// size, number by number.  grid: (segments, heads).
-template <typename T, int PIECES>
-__global__ void __launch_bounds__(DECODE_THREADS)
-matrix_memory_decode_kernel(MemoryArgs p, T* __restrict__ out) {
-  pdl_trigger();
-  extern __shared__ __align__(16) float shared[];      // [vdim + 1] reads
+__device__ __forceinline__ void round16(float4& x) {
+  x = make_float4(__bfloat162float(__float2bfloat16_rn(x.x)), __bfloat162float(__float2bfloat16_rn(x.y)), __bfloat162float(__float2bfloat16_rn(x.z)),
+                  __bfloat162float(__float2bfloat16_rn(x.w)));
+}
+
+// A block's row of a segment and head.  PIECES: 16-byte pieces of a state row per lane (dim <= 128 * PIECES, rows and pointers aligned), or 0: any
+// size, number by number.  shared: [vdim + 1] reads.  BESIDE: a step of longer segments, whose q, k and v enter in bfloat16; others than single rows are left to them.
+template <typename T, int PIECES, bool BESIDE>
+__device__ __forceinline__ void decode_row(const MemoryArgs& p, T* out, float* shared, int seg, int head) {
   __shared__ float scratch[32];
-  const int seg = blockIdx.x, head = blockIdx.y, D = p.dim, V = p.vdim;
+  const int D = p.dim, V = p.vdim;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t slot_head = (size_t)p.seg_slot[seg] * p.heads + head;
   const size_t row = p.seg_q_start[seg];
   float* state = p.states + slot_head * (size_t)(V + 1) * D;
   const float i_bias = p.i_bias[head], f_bias = p.f_bias[head];
   pdl_wait();
+  if (BESIDE && p.seg_q_len[seg] != 1) return;
   const float i_raw = __ldcg(p.i_raw + row * p.i_stride + head), f_raw = __ldcg(p.f_raw + row * p.f_stride + head);
   const float m_old = __ldcg(p.maxima + slot_head);
   const float* q = p.q + row * p.q_stride + (size_t)head * D;
@@ -104,6 +107,7 @@ matrix_memory_decode_kernel(MemoryArgs p, T* __restrict__ out) {
       if (d < D) {
         q4[n] = __ldcg(reinterpret_cast<const float4*>(q + d));
         k4[n] = __ldcg(reinterpret_cast<const float4*>(k + d));
+        if (BESIDE) round16(q4[n]), round16(k4[n]);
       }
     }
     bool first = true;
@@ -114,6 +118,7 @@ matrix_memory_decode_kernel(MemoryArgs p, T* __restrict__ out) {
       for (int r = 0; r < ROWS; ++r) {
         const int c = v0 + r * DECODE_WARPS;
         value[r] = c < V ? __ldcg(v + c) : 1.f;
+        if (BESIDE) value[r] = __bfloat162float(__float2bfloat16_rn(value[r]));
 #pragma unroll
         for (int n = 0; n < N; ++n) {
           const int d = (n * 32 + lane) << 2;
@@ -178,6 +183,15 @@ matrix_memory_decode_kernel(MemoryArgs p, T* __restrict__ out) {
   }
 }
 
+// grid: (segments, heads)
+template <typename T, int PIECES>
+__global__ void __launch_bounds__(DECODE_THREADS)
+matrix_memory_decode_kernel(MemoryArgs p, T* __restrict__ out) {
+  pdl_trigger();
+  extern __shared__ __align__(16) float shared[];
+  decode_row<T, PIECES, false>(p, out, shared, blockIdx.x, blockIdx.y);
+}
+
 // ------------------------------------------------------------------ gates of longer segments
 constexpr int GATE_THREADS = 1024;
 constexpr int GATE_WARPS = GATE_THREADS / 32;
@@ -196,6 +210,7 @@ matrix_memory_gates_kernel(MemoryArgs p) {
   // kernel still fills the SMs, they would land several to an SM.  So the trigger comes after the wait.
   pdl_wait();
   pdl_trigger();
+  if (q_len < p.least) return;
   float before = __ldcg(p.maxima + slot_head);       // m ahead of this turn's tokens
   float i_next = 0.f, f_next = 0.f;
   auto ask = [&](int t) {
@@ -791,18 +806,25 @@ struct SideRows {
   }
 };
 
-// A warp takes 16 key channels and its share of the column pairs.  grid: (heads, chunks)
-template <int D, int PAIRS>
+// A warp takes 16 key channels and its share of the column pairs.  SINGLES: behind the chunks' blocks come those of single rows, which keep the state in device
+// memory: as chunks of one row each of their states went through memory four times instead of two, and took a state's scratch.  (A kernel of its own: where no
+// block goes there, the branch alone cost 7 heads, 600 rows and four of 64, 42 -> 49 us.)  grid: (heads, chunks [+ segments])
+template <int D, int PAIRS, bool SINGLES>
 __global__ void __launch_bounds__(SIDE_THREADS, 2)
-memory_ends_kernel(MemoryArgs p) {
+memory_ends_kernel(MemoryArgs p, bf16* out, int chunks) {
   constexpr int PITCH = D + 8, W_APART = CHUNK * SIDE_PITCH, KEY_TILES = D / 16;
   constexpr int GROUPS = SIDE_THREADS / 32 / KEY_TILES, MOST = (PAIRS + GROUPS - 1) / GROUPS;      // of column pairs, and pairs of a group
   extern __shared__ __align__(16) uint8_t raw[];
   bf16 *k_tile = reinterpret_cast<bf16*>(raw), *w_parts = k_tile + CHUNK * PITCH;      // [64][PITCH], 3 x [64][SIDE_PITCH]
   __shared__ float keep[CHUNK], write[CHUNK], share[CHUNK], kept;
+  if (SINGLES && (int)blockIdx.y >= chunks) {
+    static_assert(SIDE_THREADS == DECODE_THREADS, "single rows");
+    decode_row<bf16, 1, true>(p, out, reinterpret_cast<float*>(raw), blockIdx.y - chunks, blockIdx.x);
+    return;
+  }
   pdl_wait();
   const int head = blockIdx.x, V = p.vdim, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, 1, blockIdx.y);
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
   if (seg < 0) return;
   const int count = min(CHUNK, length - chunk * CHUNK);
   const size_t row0 = (size_t)start + chunk * CHUNK;
@@ -906,7 +928,7 @@ memory_carry_kernel(MemoryArgs p, int cells) {
   const int seg = blockIdx.y, length = p.seg_q_len[seg], at = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (length <= CHUNK) return;
   int first = 0;
-  for (int i = threadIdx.x & 31; i < seg; i += 32) first += (max(p.seg_q_len[i], 0) + CHUNK - 1) / CHUNK;
+  for (int i = threadIdx.x & 31; i < seg; i += 32) first += p.seg_q_len[i] < p.least ? 0 : (p.seg_q_len[i] + CHUNK - 1) / CHUNK;
   first = __reduce_add_sync(0xffffffffu, first);
   if (at >= p.heads * cells) return;
   const int head = at / cells, cell = at - head * cells, chunks = (length + CHUNK - 1) / CHUNK;
@@ -984,7 +1006,7 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
   __shared__ float write[CHUNK], floor_of[CHUNK], since[CHUNK];
   pdl_wait();
   const int head = blockIdx.x, V = p.vdim, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, 1, blockIdx.y);
+  const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, blockIdx.y);
   if (seg < 0) return;
   const int count = min(CHUNK, length - chunk * CHUNK);
   const size_t row0 = (size_t)start + chunk * CHUNK;
@@ -1217,13 +1239,13 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
 }
 
 template <int D, int PAIRS>
-static int launch_side(const MemoryArgs& p, bf16* out, int rows, int segments, cudaStream_t stream) {
-  const unsigned chunks = (unsigned)long_chunks(rows, segments, 1);
+static int launch_side(const MemoryArgs& p, bf16* out, int chunks, int segments, cudaStream_t stream) {
   const int cells = (p.vdim + 1) * D;
-  cudaError_t err = cudaFuncSetAttribute(memory_ends_kernel<D, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::ENDS);
+  auto ends = p.least > 1 ? memory_ends_kernel<D, PAIRS, true> : memory_ends_kernel<D, PAIRS, false>;
+  cudaError_t err = cudaFuncSetAttribute(ends, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::ENDS);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(memory_outputs_kernel<D, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::SHARED);
   if (err != cudaSuccess) return (int)err;
-  launch_kernel(memory_ends_kernel<D, PAIRS>, dim3(p.heads, chunks), dim3(SIDE_THREADS), SideShape<D>::ENDS, stream, p);
+  launch_kernel(ends, dim3(p.heads, chunks + (p.least > 1 ? segments : 0)), dim3(SIDE_THREADS), SideShape<D>::ENDS, stream, p, out, chunks);
   int status = launch_status();
   if (status != MLR_OK) return status;
   launch_kernel(memory_carry_kernel, dim3((p.heads * cells / 4 + 255) / 256, segments), dim3(256), 0, stream, p, cells);
@@ -1304,7 +1326,7 @@ static bool side_fits(int dim, int vdim) { return (dim == 64 || dim == 128) && v
 static bool chunks_fit(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim % 8 == 0; }
 
 template <typename T>
-static int launch_memory(const MemoryArgs& p, T* out, int rows, int segments, int max_q_len, bool wide, cudaStream_t stream) {
+static int launch_memory(const MemoryArgs& p, T* out, int rows, int chunks, int segments, int max_q_len, bool wide, cudaStream_t stream) {
   const int D = p.dim;
   if (max_q_len == 1) {
     const dim3 grid(segments, p.heads);
@@ -1321,10 +1343,10 @@ static int launch_memory(const MemoryArgs& p, T* out, int rows, int segments, in
   if (status != MLR_OK) return status;
   if (p.ends != nullptr) {
     if constexpr (sizeof(T) == 2) {
-      if (!wide || !side_fits(D, p.vdim) || long_chunks(rows, segments, 1) > 65535) return MLR_BAD_SIZE;
+      if (!wide || !side_fits(D, p.vdim) || chunks <= 0 || (long long)chunks + segments > 65535) return MLR_BAD_SIZE;
       if (side_pairs(p.vdim) <= 6)
-        return D == 64 ? launch_side<64, 6>(p, out, rows, segments, stream) : launch_side<128, 6>(p, out, rows, segments, stream);
-      return D == 64 ? launch_side<64, SIDE_PAIRS>(p, out, rows, segments, stream) : launch_side<128, SIDE_PAIRS>(p, out, rows, segments, stream);
+        return D == 64 ? launch_side<64, 6>(p, out, chunks, segments, stream) : launch_side<128, 6>(p, out, chunks, segments, stream);
+      return D == 64 ? launch_side<64, SIDE_PAIRS>(p, out, chunks, segments, stream) : launch_side<128, SIDE_PAIRS>(p, out, chunks, segments, stream);
     }
     return MLR_BAD_DTYPE;
   }
@@ -1364,27 +1386,26 @@ MLR_EXPORT int mlr_matrix_memory_chunks_fit(int dim, int vdim) { return chunks_f
 // Chunks that a block walks one behind the other: 1 where a step's chunks go side by side, 0 where all of a segment's go one behind the other: where
 // no portion has more than two (one behind the other / side by side: 65 rows of 7 heads 21.5 / 24.4 us, 128 rows 22.5 / 24.4, 129 rows 24.9 / 24.8, 192 rows
 // 25.5 / 24.9, 16 heads of 129 rows 25.2 / 25.2; short portions beside a longer one take no time of their own).
-MLR_EXPORT int mlr_matrix_memory_run(int rows, int segments, int max_q_len, int heads, int vdim) {
-  return side_fits(64, vdim) && max_q_len > 2 * CHUNK && long_chunks(rows, segments, 1) <= 65535 ? 1 : 0;
+MLR_EXPORT int mlr_matrix_memory_run(int chunks, int segments, int max_q_len, int vdim) {
+  return side_fits(64, vdim) && max_q_len > 2 * CHUNK && (long long)chunks + segments <= 65535 ? 1 : 0;
 }
 // .. and the float32 numbers of scratch that side by side needs.
-MLR_EXPORT long long mlr_matrix_memory_run_scratch(int rows, int segments, int heads, int dim, int vdim) {
-  return long_chunks(rows, segments, 1) * heads * ((long long)(vdim + 1) * dim + 1);
-}
+MLR_EXPORT long long mlr_matrix_memory_run_scratch(int chunks, int heads, int dim, int vdim) { return (long long)chunks * heads * ((long long)(vdim + 1) * dim + 1); }
 
 // q, k: float32 rows of heads * dim entries; v, gate: rows of heads * vdim; i_raw, f_raw: rows of `heads` entries (each
 // with its own row stride); i_bias, f_bias: float32 [heads]; weight: float32 [heads * vdim]; coef: float32 scratch
 // [rows, heads, 4], reads: [rows, heads, vdim], norms: [rows, heads] (all three null for steps of single rows); pairs:
 // float32 scratch [rows, heads, 64 + 2] and packed: bfloat16 scratch [rows, heads, 2 dim + vdim] (both or neither: chunks
 // on the tensor cores, or the token-by-token scan; 16-byte aligned); ends: null, or the scratch of chunks side by side (as the two
-// functions above say, for bfloat16 results; reads, norms, pairs and packed are then not asked for); states:
+// functions above say, for bfloat16 results; reads, norms, pairs and packed are then not asked for) with chunks: those of all segments of `least` rows (1, or 2
+// where there may be single rows) and more, or the most there can be; states:
 // float32 [slots, heads, vdim + 1, dim], maxima: float32 [slots, heads]; out: [rows, heads * vdim] in `dtype`.
 // max_q_len: the longest segment of the step.
 MLR_EXPORT int mlr_matrix_memory(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
                                  long long v_stride, const float* i_raw, long long i_stride, const float* f_raw,
                                  long long f_stride, const float* gate, long long gate_stride, const float* i_bias,
                                  const float* f_bias, const float* weight, float* coef, float* reads, float* norms,
-                                 float* pairs, void* packed, float* ends, float* states, float* maxima, void* out, const int* seg_q_start, const int* seg_q_len,
+                                 float* pairs, void* packed, float* ends, int chunks, int least, float* states, float* maxima, void* out, const int* seg_q_start, const int* seg_q_len,
                                  const int* seg_slot, int rows, int segments, int max_q_len, int heads, int dim, int vdim,
                                  float cap, float guard, float eps, float q_scale, int dtype, cudaStream_t stream) {
   if (segments == 0 || rows == 0) return MLR_OK;
@@ -1393,18 +1414,18 @@ MLR_EXPORT int mlr_matrix_memory(const float* q, long long q_stride, const float
   bf16* q16 = (bf16*)packed;
   bf16* k16 = q16 == nullptr ? nullptr : q16 + (size_t)rows * heads * dim;
   bf16* v16 = q16 == nullptr ? nullptr : k16 + (size_t)rows * heads * dim;
-  if ((pairs == nullptr) != (packed == nullptr)) return MLR_BAD_SIZE;
+  if ((pairs == nullptr) != (packed == nullptr) || least < 1 || least > 2 || (least > 1 && ends == nullptr)) return MLR_BAD_SIZE;
   MemoryArgs p{q, k, v, i_raw, f_raw, gate, q_stride, k_stride, v_stride, i_stride, f_stride, gate_stride, i_bias, f_bias,
                weight, reinterpret_cast<float4*>(coef), reads, norms, pairs,
                pairs == nullptr ? nullptr : reinterpret_cast<float2*>(pairs + (size_t)rows * heads * CHUNK), q16, k16, v16, states, maxima, ends,
-               ends == nullptr ? nullptr : ends + (size_t)long_chunks(rows, segments, 1) * heads * (vdim + 1) * dim, seg_q_start, seg_q_len, seg_slot,
-               segments, heads, dim, vdim, cap, guard, eps, q_scale};
+               ends == nullptr ? nullptr : ends + (size_t)chunks * heads * (vdim + 1) * dim, seg_q_start, seg_q_len, seg_slot,
+               segments, least, heads, dim, vdim, cap, guard, eps, q_scale};
   auto multiple = [](long long n) { return n % 4 == 0; };
   auto aligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
   if (!aligned(coef) || !aligned(pairs) || !aligned(packed) || !aligned(ends)) return MLR_BAD_ALIGNMENT;
   const bool wide = multiple(dim) && multiple(vdim) && multiple(q_stride) && multiple(k_stride) && multiple(v_stride) &&
                     aligned(q) && aligned(k) && aligned(v) && aligned(states);
-  if (dtype == MLR_F32) return launch_memory(p, (float*)out, rows, segments, max_q_len, wide, stream);
-  if (dtype == MLR_BF16) return launch_memory(p, (bf16*)out, rows, segments, max_q_len, wide, stream);
+  if (dtype == MLR_F32) return launch_memory(p, (float*)out, rows, chunks, segments, max_q_len, wide, stream);
+  if (dtype == MLR_BF16) return launch_memory(p, (bf16*)out, rows, chunks, segments, max_q_len, wide, stream);
   return MLR_BAD_DTYPE;
 }

@@ -669,9 +669,44 @@ def test_matrix_memory_side_by_side_loses_no_bits_of_its_sums(heads, dim, vdim, 
     assert 2.0 ** -8 < errors[0] and errors[1] <= 1.03 * errors[0], errors
 
 
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 128, 128), (2, 64, 72)])
+def test_matrix_memory_of_decoded_rows_beside_a_portion(heads, dim, vdim):
+    """Decoded rows have the bits of a step of their own with q, k and v in 16 bits, and cost no chunk's scratch; a portion's bits are those of a step of its
+    own."""
+    lengths = [1, 1, 130] + [1] * 61 + [2, 200, 1]
+    count = len(lengths)
+    order = torch.randperm(count, generator=generator(1)).tolist()
+    ctx, rows = segments(lengths, torch.randperm(count, generator=generator(2)).tolist(), order), sum(lengths)
+    q, k, v, gate = rnd(1, rows, heads * dim), rnd(2, rows, heads * dim), rnd(3, rows, heads * vdim), rnd(4, rows, heads * vdim)
+    i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
+    inputs = [spaced(t, 8) for t in (q, k, v, i_raw, f_raw, gate)]
+    half = [spaced(t.to(torch.bfloat16).float(), 8) for t in (q, k, v)] + inputs[3:]
+    bias, weight = torch.zeros(heads, device=DEVICE), (1 + rnd(7, heads * vdim, std=0.1)).to(DEVICE)
+    state, maximum = rnd(8, count, heads, vdim + 1, dim, std=0.5).to(DEVICE), rnd(9, count, heads).to(DEVICE)
+
+    def call(take, ctx, inputs):
+        s, m = state.clone(), maximum.clone()
+        rows = [t[take] for t in inputs]
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        start = torch.cuda.memory_allocated()
+        out = cuda().matrix_memory(*rows[:5], bias, bias + 3, 15.0, 1e-6, rows[5], weight, 1e-6, s, m, ctx, heads, dim, vdim, torch.bfloat16)
+        return out, s, m, torch.cuda.max_memory_allocated() - start
+
+    out, s, m, extra = call(slice(None), ctx, inputs)
+    chunks = 3 + 1 + 4
+    assert extra <= chunks * heads * ((vdim + 1) * dim + 1) * 4 + rows * heads * (16 + 2 * vdim) + 4096, extra
+    for part in ctx.segments:
+        at = slice(part.row_start, part.row_start + part.length)
+        own = call(at, segments([part.length], [part.slot]), half)
+        if part.length != 2:                    # two rows alone go token by token
+            assert torch.equal(own[0], out[at]) and torch.equal(own[1][part.slot], s[part.slot]), part.length
+        assert torch.equal(own[2][part.slot], m[part.slot]), part.length
+
+
 def memory_run(ctx, rows, heads, vdim):
     from mini_llm_runtime_b200.ops import build
-    return build.load_library("matrix_memory").mlr_matrix_memory_run(rows, ctx.num_segments, int(ctx.max_q_len), heads, vdim)
+    return build.load_library("matrix_memory").mlr_matrix_memory_run(cuda()._chunks_from(ctx, rows, 1), ctx.num_segments, int(ctx.max_q_len), vdim)
 
 
 # Tiles of 128 outputs, of 16, 32, 64 and 128 rows, blocks of 64 k; 1, 2, 4 and 8 parts of the sums over k; more tiles than SMs, few rows too.
