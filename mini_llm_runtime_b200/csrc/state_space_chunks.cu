@@ -52,7 +52,8 @@ struct SpaceArgs {
   const int *seg_q_start, *seg_q_len, *seg_slot;
   int heads, groups;
   int segments, least;               // segments of `least` rows and more go in chunks
-  int scans;                         // blocks per head (and 64 state entries) that take the others token by token
+  int scans;                         // blocks per head that take the others token by token
+  bool halves;                       // .. their first rows beside the ends, the others beside the outputs
 };
 
 __device__ __forceinline__ bool partless(const float4& v) {
@@ -255,28 +256,42 @@ __device__ __noinline__ void ends_plain(const SpaceArgs& p, float* shared, const
   for (int r = 0; r < 8; ++r) store_columns<4>(to + (size_t)(j + r) * N + i, end[r]);
 }
 
+// Segments that go token by token have blocks beside the ends.  What follows waits for them, so where the chunks are a round of the outputs' blocks or less and a
+// segment is longer than those take, half of its rows go beside the outputs.  In us, all beside the ends / halves: 300, 100 and 70 rows 44 / 38 (14 heads) and
+// 60 / 56 (32 heads), 1,000 and three of 100 rows 52 / 47 (224 blocks); but 99 / 101 (512 blocks) and, of 1,531, 77, 1 and 439 rows of 32 heads, 116 / 120.
+// Staged 16 tokens at a time, their shared memory leaves the ends their four blocks per SM: 400 rows beside 64 decoded ones, 32 heads, 93 us with 32 tokens, 83 so.
+constexpr int SCAN_STAGED = 16;
+template <int N>
+struct ScanShape {
+  static constexpr int SL = N / SCAN_NPT, PARTS = VD * SL / SCAN_THREADS;      // blocks of a head
+};
+template <int N>
+__device__ __forceinline__ ScanArgs scan_args(const SpaceArgs& p) {
+  return {p.x, p.B, p.C, p.dt_raw, p.x_stride, p.b_stride, p.c_stride, p.dt_stride, p.dt_bias, p.A_log, p.D, p.states, p.y,
+          p.seg_q_start, p.seg_q_len, p.seg_slot, p.heads, VD, N, p.groups, p.least - 1};
+}
+
 constexpr size_t ENDS_SHARED = 2 * TILE_BYTES;      // inputs and B in parts
 static_assert(ENDS_SHARED >= sizeof(float) * CHUNK * (VD + HALF_N), "by multiply-adds");
 
 // A CTA takes 64 entries of the state, a warp 16 value channels of them.  grid: (heads * n / 64, scans + chunks)
-template <int N>
+template <int N, bool SCANS>
 __global__ void __launch_bounds__(SPACE_THREADS, 4)
 space_ends_kernel(const __grid_constant__ SpaceArgs p) {
   extern __shared__ __align__(16) float shared[];
   __shared__ float s_g[CHUNK], s_dt[CHUNK], s_factor[CHUNK];      // decays, step sizes, the latter times the decays' product behind a token
   const int head = blockIdx.x / (N / HALF_N), part = blockIdx.x % (N / HALF_N);
-  if ((int)blockIdx.y < p.scans) {
-    constexpr int SL = N / SCAN_NPT, PARTS = VD * SL / SCAN_THREADS, TAKEN = PARTS / (N / HALF_N);
-    const ScanArgs scan{p.x, p.B, p.C, p.dt_raw, p.x_stride, p.b_stride, p.c_stride, p.dt_stride, p.dt_bias, p.A_log, p.D, p.states, p.y,
-                        p.seg_q_start, p.seg_q_len, p.seg_slot, p.heads, VD, N, p.groups, p.least - 1};
-    scan_segment<SL, true>(scan, shared, blockIdx.y / TAKEN, head, blockIdx.y % TAKEN * (N / HALF_N) + part);
+  if (SCANS && (int)blockIdx.y < p.scans / (N / HALF_N)) {
+    constexpr int TAKEN = ScanShape<N>::PARTS / (N / HALF_N);
+    scan_segment<ScanShape<N>::SL, true, SCAN_STAGED>(scan_args<N>(p), shared, blockIdx.y / TAKEN, head, blockIdx.y % TAKEN * (N / HALF_N) + part,
+                                              p.halves ? FIRST_HALF : ALL_ROWS);
     return;
   }
   bf16 *s_x = reinterpret_cast<bf16*>(shared), *s_b = s_x + 3 * TILE_APART;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float rate = expf(p.A_log[head]), bias = p.dt_bias[head];
   pdl_wait();
-  const int index = blockIdx.y - p.scans;
+  const int index = SCANS ? (int)blockIdx.y - p.scans / (N / HALF_N) : blockIdx.y;
   const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, index);
   if (seg < 0) return;
   const int first = start + chunk * CHUNK, count = min(CHUNK, length - chunk * CHUNK), group = head / (p.heads / p.groups);
@@ -470,8 +485,8 @@ constexpr size_t WEIGHT_BYTES = CHUNK * W_PITCH * sizeof(float);
 constexpr size_t OUTPUTS_SHARED = WEIGHT_BYTES + 2 * TILE_BYTES;      // weights, inputs (then a part of the state), a part of C
 static_assert(OUTPUTS_SHARED >= sizeof(float) * (VD + CHUNK) * (128 + 4), "by multiply-adds");
 
-// A warp takes 16 rows.  grid: (heads, chunks)
-template <int N>
+// A warp takes 16 rows.  grid: (heads, scans + chunks)
+template <int N, bool SCANS>
 __global__ void __launch_bounds__(SPACE_THREADS, 3)
 space_outputs_kernel(const __grid_constant__ SpaceArgs p) {
   extern __shared__ __align__(16) float shared[];
@@ -479,7 +494,12 @@ space_outputs_kernel(const __grid_constant__ SpaceArgs p) {
   __shared__ int s_broken;                                       // the first row that goes by multiply-adds
   float* s_w = shared;                                                                                 // [CHUNK][W_PITCH]: weight of token s in row t
   bf16 *s_x = reinterpret_cast<bf16*>(s_w + CHUNK * W_PITCH), *s_c = s_x + 3 * TILE_APART;
-  const int head = blockIdx.x, index = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (SCANS && (int)blockIdx.y < (p.halves ? p.scans : 0)) {
+    constexpr int PARTS = ScanShape<N>::PARTS;
+    scan_segment<ScanShape<N>::SL, true, SCAN_STAGED>(scan_args<N>(p), shared, blockIdx.y / PARTS, blockIdx.x, blockIdx.y % PARTS, SECOND_HALF);
+    return;
+  }
+  const int head = blockIdx.x, index = SCANS && p.halves ? (int)blockIdx.y - p.scans : blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float rate = expf(p.A_log[head]), bias = p.dt_bias[head], skip = p.D[head];
   pdl_wait();
   const auto [seg, chunk, length, start, slot] = chunk_at<true>(p.seg_q_start, p.seg_q_len, p.seg_slot, p.segments, p.least, index);
@@ -633,25 +653,26 @@ space_outputs_kernel(const __grid_constant__ SpaceArgs p) {
   pdl_trigger();
 }
 
-template <int N>
+template <int N, bool SCANS>
 int launch_space(const SpaceArgs& a, int rows, cudaStream_t stream) {
   constexpr size_t pairs_shared = (N / HALF_N) * 3 * TILE_PITCH * (CHUNK + PAIRS_ROWS) * sizeof(bf16);
-  const size_t segment_shared = scan_shared(N, SCAN_THREADS / (N / SCAN_NPT));
-  const size_t ends_shared = a.scans > 0 && segment_shared > ENDS_SHARED ? segment_shared : ENDS_SHARED;
+  const size_t segment_shared = scan_shared(N, SCAN_THREADS / (N / SCAN_NPT), SCAN_STAGED);
+  const size_t ends_shared = SCANS && segment_shared > ENDS_SHARED ? segment_shared : ENDS_SHARED;
+  if (SCANS && segment_shared > OUTPUTS_SHARED) return MLR_TOO_LARGE;
   const unsigned chunks = (unsigned)long_chunks(rows, a.segments, a.least);
   cudaError_t err = cudaFuncSetAttribute(space_pairs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_shared);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(space_ends_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ends_shared);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(space_outputs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUTPUTS_SHARED);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(space_ends_kernel<N, SCANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ends_shared);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(space_outputs_kernel<N, SCANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUTPUTS_SHARED);
   if (err != cudaSuccess) return (int)err;
   launch_kernel(space_pairs_kernel<N>, dim3(chunks, a.groups * 2), dim3(PAIRS_THREADS), pairs_shared, stream, a);
   int status = launch_status();
   if (status != MLR_OK) return status;
-  launch_kernel(space_ends_kernel<N>, dim3(a.heads * (N / HALF_N), a.scans + chunks), dim3(SPACE_THREADS), ends_shared, stream, a);
+  launch_kernel(space_ends_kernel<N, SCANS>, dim3(a.heads * (N / HALF_N), a.scans / (N / HALF_N) + chunks), dim3(SPACE_THREADS), ends_shared, stream, a);
   if ((status = launch_status()) != MLR_OK) return status;
   launch_kernel(space_carry_kernel, dim3((a.heads * VD * N / 4 + 255) / 256, (unsigned)long_segments(rows, a.segments, a.least)), dim3(256), 0,
                 stream, a, VD * N);
   if ((status = launch_status()) != MLR_OK) return status;
-  launch_kernel(space_outputs_kernel<N>, dim3(a.heads, chunks), dim3(SPACE_THREADS), OUTPUTS_SHARED, stream, a);
+  launch_kernel(space_outputs_kernel<N, SCANS>, dim3(a.heads, (a.halves ? a.scans : 0) + chunks), dim3(SPACE_THREADS), OUTPUTS_SHARED, stream, a);
   return launch_status();
 }
 
@@ -670,7 +691,7 @@ MLR_EXPORT long long mlr_state_space_chunk_scratch(int rows, int segments, int l
 
 // As mlr_state_space_scan, for heads of 64 value channels with states of 64 or 128 entries and x, B, C, states, y and scratch whose
 // rows begin on 16-byte boundaries.  rows: the step's rows.  Segments of fewer than least_rows rows
-// go token by token as there; others: whether there can be any.
+// go token by token as there; others: the longest of those, or what it may be (0: there are none).
 MLR_EXPORT int mlr_state_space_chunks(const float* x, long long x_stride, const float* B, long long b_stride, const float* C,
                                       long long c_stride, const float* dt_raw, long long dt_stride, const float* dt_bias,
                                       const float* A_log, const float* D, float* states, float* y, float* scratch,
@@ -682,13 +703,15 @@ MLR_EXPORT int mlr_state_space_chunks(const float* x, long long x_stride, const 
   if (vdim != VD || (n != 64 && n != 128) || long_chunks(rows, segments, least_rows) + segments * 4ll > 65535 || groups > 65535 / 2) return MLR_TOO_LARGE;
   const uintptr_t pointers = (uintptr_t)x | (uintptr_t)B | (uintptr_t)C | (uintptr_t)states | (uintptr_t)y | (uintptr_t)scratch;
   if (pointers % 16 != 0 || (x_stride | b_stride | c_stride) % 4 != 0) return MLR_BAD_ALIGNMENT;
-  const int parts = n / HALF_N, scans = segments * (VD * (n / SCAN_NPT) / SCAN_THREADS / parts);
-  SpaceArgs a{x, B, C, dt_raw, x_stride, b_stride, c_stride, dt_stride, dt_bias, A_log, D, states, y,
-              nullptr, scratch, nullptr, nullptr, nullptr, seg_q_start, seg_q_len, seg_slot, heads, groups, segments, least_rows, others ? scans : 0};
+  const int parts = n / HALF_N, scans = others ? segments * (VD * (n / SCAN_NPT) / SCAN_THREADS) : 0;
   const size_t chunks = (size_t)long_chunks(rows, segments, least_rows);
+  SpaceArgs a{x, B, C, dt_raw, x_stride, b_stride, c_stride, dt_stride, dt_bias, A_log, D, states, y,
+              nullptr, scratch, nullptr, nullptr, nullptr, seg_q_start, seg_q_len, seg_slot, heads, groups, segments, least_rows, scans,
+              others > CHUNK && chunks * heads <= 3 * (size_t)sm_count()};
   a.parts = reinterpret_cast<bf16*>(a.ends + (size_t)chunk_places(rows) * heads * VD * n);
   a.pairs = reinterpret_cast<float*>(a.parts + chunks * groups * parts * 6 * TILE_APART);
   a.decays = a.pairs + (size_t)rows * groups * CHUNK;
   a.broken = reinterpret_cast<int*>(a.decays + (size_t)chunk_places(rows) * heads);      // an even number of them: read in pairs
-  return n == 64 ? launch_space<64>(a, rows, stream) : launch_space<128>(a, rows, stream);
+  if (others) return n == 64 ? launch_space<64, true>(a, rows, stream) : launch_space<128, true>(a, rows, stream);
+  return n == 64 ? launch_space<64, false>(a, rows, stream) : launch_space<128, false>(a, rows, stream);
 }

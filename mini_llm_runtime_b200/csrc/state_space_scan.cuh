@@ -8,7 +8,7 @@
 namespace mlr {
 
 constexpr int SCAN_NPT = 16;        // state entries of one value channel a thread holds
-constexpr int SCAN_TOKENS = 32;     // tokens staged at once
+constexpr int SCAN_TOKENS = 32;     // tokens staged at once, at most
 constexpr int SCAN_THREADS = 128;
 
 struct ScanArgs {
@@ -29,29 +29,33 @@ struct ScanArgs {
 // A block takes a segment, a head and a block of value channels.  The inputs of 32 tokens at a time are staged in shared
 // memory by asynchronous copies, the next 32 while these are walked; WIDE: in 16-byte pieces (state size,
 // channel block and all row strides multiples of four floats, pointers aligned).
-template <int SL, bool WIDE>
-__device__ __forceinline__ void scan_segment(const ScanArgs& a, float* shared, int seg, int head, int part) {
+enum ScanPart { ALL_ROWS, FIRST_HALF, SECOND_HALF };      // of a segment's rows, the second behind the first in a later kernel
+template <int SL, bool WIDE, int TOKENS = SCAN_TOKENS>
+__device__ __forceinline__ void scan_segment(const ScanArgs& a, float* shared, int seg, int head, int part, ScanPart which_rows = ALL_ROWS) {
   constexpr int P_CTA = SCAN_THREADS / SL;
   const int N = a.n, P = a.vdim;
-  const int buffer = SCAN_TOKENS * (2 * N + P_CTA + 1);      // floats of one staging buffer
-  float* decay = shared + 2 * buffer + SCAN_NPT;             // [SCAN_TOKENS]; a last piece may reach past a buffer's end
-  float* step = decay + SCAN_TOKENS;                         // [SCAN_TOKENS]
+  const int buffer = TOKENS * (2 * N + P_CTA + 1);      // floats of one staging buffer
+  float* decay = shared + 2 * buffer + SCAN_NPT;             // [TOKENS]; a last piece may reach past a buffer's end
+  float* step = decay + TOKENS;                         // [TOKENS]
   const int group = head / (a.heads / a.groups);
   const int s = threadIdx.x % SL, p_local = threadIdx.x / SL;
   const int p = part * P_CTA + p_local;
   const float rate = expf(a.A_log[head]), bias = a.dt_bias[head], skip = a.D[head];
   pdl_wait();
-  const int q_start = a.seg_q_start[seg], q_len = a.seg_q_len[seg];
-  if (q_len > a.longest) return;
+  const int q_start = a.seg_q_start[seg], all_rows = a.seg_q_len[seg];
+  if (all_rows > a.longest) return;
+  const int half = (all_rows + 2 * TOKENS - 1) / (2 * TOKENS) * TOKENS;
+  const int begin = which_rows == SECOND_HALF ? half : 0, q_len = which_rows == FIRST_HALF ? min(half, all_rows) : all_rows;
+  if (which_rows == SECOND_HALF && begin >= q_len) return;
 
   // rows [t0, t0 + 32) of the segment into buffer `which`: B and C of the head's group, the block's value
   // channels of x, the head's raw step sizes
   auto stage = [&](int t0, int which) {
     float* b_rows = shared + which * buffer;
-    float* c_rows = b_rows + SCAN_TOKENS * N;
-    float* x_rows = c_rows + SCAN_TOKENS * N;
-    float* raw = x_rows + SCAN_TOKENS * P_CTA;
-    const int tokens = min(SCAN_TOKENS, q_len - t0);
+    float* c_rows = b_rows + TOKENS * N;
+    float* x_rows = c_rows + TOKENS * N;
+    float* raw = x_rows + TOKENS * P_CTA;
+    const int tokens = min(TOKENS, q_len - t0);
     const size_t row0 = (size_t)(q_start + t0);
     if (WIDE) {
       const int per_row = N >> 2;
@@ -82,7 +86,7 @@ __device__ __forceinline__ void scan_segment(const ScanArgs& a, float* shared, i
     copy_async_commit();
   };
 
-  stage(0, 0);
+  stage(begin, 0);
   float* state = a.states + (((size_t)a.seg_slot[seg] * a.heads + head) * P + (p < P ? p : 0)) * N;
   auto entry = [&](int i) { return (((i >> 2) * SL + s) << 2) + (i & 3); };      // the state entry a thread's i-th number is
   float S[SCAN_NPT];
@@ -92,16 +96,16 @@ __device__ __forceinline__ void scan_segment(const ScanArgs& a, float* shared, i
     S[i] = (p < P && n < N) ? state[n] : 0.f;
   }
   int which = 0;
-  for (int t0 = 0; t0 < q_len; t0 += SCAN_TOKENS, which ^= 1) {
-    const int tokens = min(SCAN_TOKENS, q_len - t0);
-    const bool more = t0 + SCAN_TOKENS < q_len;
-    if (more) stage(t0 + SCAN_TOKENS, which ^ 1);
+  for (int t0 = begin; t0 < q_len; t0 += TOKENS, which ^= 1) {
+    const int tokens = min(TOKENS, q_len - t0);
+    const bool more = t0 + TOKENS < q_len;
+    if (more) stage(t0 + TOKENS, which ^ 1);
     if (more) copy_async_wait<1>(); else copy_async_wait<0>();
     __syncthreads();
     const float* b_rows = shared + which * buffer;
-    const float* c_rows = b_rows + SCAN_TOKENS * N;
-    const float* x_rows = c_rows + SCAN_TOKENS * N;
-    const float* raw = x_rows + SCAN_TOKENS * P_CTA;
+    const float* c_rows = b_rows + TOKENS * N;
+    const float* x_rows = c_rows + TOKENS * N;
+    const float* raw = x_rows + TOKENS * P_CTA;
     if (threadIdx.x < tokens) {
       const float z = raw[threadIdx.x] + bias;
       const float dt = z > 20.f ? z : log1pf(expf(z));
@@ -157,8 +161,8 @@ __device__ __forceinline__ void scan_segment(const ScanArgs& a, float* shared, i
 }
 
 // Shared memory of a block in bytes.
-inline size_t scan_shared(int n, int channels) {
-  return sizeof(float) * (2 * (size_t)SCAN_TOKENS * (2 * n + channels + 1) + SCAN_NPT + 2 * SCAN_TOKENS);
+inline size_t scan_shared(int n, int channels, int tokens = SCAN_TOKENS) {
+  return sizeof(float) * (2 * (size_t)tokens * (2 * n + channels + 1) + SCAN_NPT + 2 * tokens);
 }
 
 }  // namespace mlr

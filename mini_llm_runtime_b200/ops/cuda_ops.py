@@ -2171,7 +2171,7 @@ class CudaOps:
             _check(lib.mlr_state_space_chunks(
                 *views, _ptr(dt_bias), _ptr(A_log), _ptr(D), _ptr(state), _ptr(y), _ptr(scratch), _ptr(ctx.seg_q_start),
                 _ptr(ctx.seg_q_len), _ptr(ctx.seg_slot), ctx.num_segments, rows, int(ctx.max_q_len), least,
-                int(self._longest_below(ctx, least) > 0), heads, vdim, n, groups, _stream()), "state_space_chunks")
+                self._longest_below(ctx, least), heads, vdim, n, groups, _stream()), "state_space_chunks")
             return y
         _check(build.load_library("state_space").mlr_state_space_scan(
             *views, _ptr(dt_bias), _ptr(A_log),

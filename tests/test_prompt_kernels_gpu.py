@@ -128,6 +128,22 @@ def test_state_space_in_chunks(heads, n, groups, lengths, slots, order, monkeypa
     close(got_state.flatten(0, 1), want_state.flatten(0, 1), 200 * UNIT, "state-space state")
 
 
+@pytest.mark.parametrize("heads,n,lengths", [(6, 64, [144, 65, 96, 143, 1, 16, 17]), (4, 128, [200, 70, 97, 64, 33, 2, 128]),      # halves
+                                             (32, 128, [1000, 100, 66, 1]), (6, 64, [150, 64, 1, 33])])                          # whole
+def test_state_space_of_short_portions_beside_chunks(heads, n, lengths):
+    """Rows that go token by token beside the chunks' kernels, at once or in halves: the bits of a step of their own."""
+    count, rows, inner = len(lengths), sum(lengths), heads * 64
+    ctx = segments(lengths, list(reversed(range(count))), [*range(1, count), 0])
+    x, B, C, dt = (spaced(t) for t in (rnd(1, rows, inner), rnd(2, rows, n), rnd(3, rows, n), rnd(4, rows, heads, std=2.0)))
+    vectors, state = [rnd(i, heads).to(DEVICE) for i in (5, 6, 7)], rnd(8, count, heads, 64, n, std=0.5).to(DEVICE)
+    whole = state.clone()
+    y = cuda().state_space_scan(x, B, C, dt, *vectors, whole, ctx, heads, 64, n, 1)
+    for part in ctx.segments:
+        at, own = slice(part.row_start, part.row_start + part.length), state.clone()
+        alone = cuda().state_space_scan(x[at], B[at], C[at], dt[at], *vectors, own, segments([part.length], [part.slot]), heads, 64, n, 1)
+        assert torch.equal(alone, y[at]) and torch.equal(own[part.slot], whole[part.slot]), part.length
+
+
 @pytest.mark.parametrize("heads,n,groups", [(2, 64, 1), (4, 128, 2)])
 @pytest.mark.parametrize("where", ["x", "B", "C", "state", "before"])
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
