@@ -981,11 +981,12 @@ class CudaOps:
     # By head size: portions of fewer rows than the first number go token by token in a launch of their own, those from the second on in
     # chunks, those between token by token in the chunks' launches.  Which way a request's rows go is a matter of its own portion
     # only, as their numbers are.  Measured in us from a flushed L2, by sequence_mix.cu / walked in the chunks' launches: 14 heads of 64: 16 rows 14, 32
-    # rows 21 / 21, 64 34 / 32; 7 heads of 128, whose walk keeps a head on one CTA: 64 rows 34 / 42.  Walked (64) or by sequence_mix.cu (128) / in chunks,
-    # which pays from two chunks on: 14 heads of 64: 66 rows 32 / 34, 80 36 / 34, 100 40 / 36, 127 46 / 38, four of 100 rows 42 / 38; 32 heads 34 / 36, 36 / 36,
-    # 42 / 36, 48 / 38 and 50 / 46; 7 heads of 128: 66 rows 36 / 50, 80 42 / 50, 100 50 / 50, 128 58 / 52, four of 100 rows 50 / 55; 16 heads 38 / 50, 42 / 50,
-    # 50 / 50, 60 / 52 and 91 / 61.  Beside a long portion: 1,000, 100 and 90 rows, 7 heads of 128 100 / 59, 16 heads 131 / 109.
-    GATED_ROWS = {64: (32, 80), 128: (96, 96)}
+    # rows 21 / 21, 64 34 / 32; 7 heads of 128, whose walk keeps a head on one CTA: 64 rows 34 / 42.  By sequence_mix.cu / in chunks, heads of 128: 7 heads, 1, 2 and 4
+    # portions of 96 rows 46 / 50, 48 / 53, 48 / 55, of 112 rows 54 / 50, 54 / 50, 54 / 52, of 127 rows 58 / 52, 60 / 52, 60 / 54; 16 heads, of 96 rows 48 / 50, 48 / 55, 85 / 59, of 112
+    # rows 54 / 50, 56 / 54, 99 / 58.  Walked / in chunks, heads of 64, where few portions gain and a full step loses: 14 heads, 1, 4, 8 and 16 portions of 96 rows
+    # 40 / 34, 40 / 36, 42 / 44, 50 / 58, of 120 rows 44 / 36, 46 / 38, - , 58 / 62; 32 heads, of 96 rows 40 / 36, 48 / 44, 56 / 60, 79 / 101, of 120 rows 46 / 37, 56 / 48, - , 91 / 112;
+    # 1,000, 100 and 90 rows 77 / 81.
+    GATED_ROWS = {64: (32, 128), 128: (112, 112)}
 
     def _recurrence(self, mode, r, b, v, raw, gate, bias, aux, weight, eps, state, ctx, heads, dim, vdim, out_dtype):
         rows = r.shape[0]
