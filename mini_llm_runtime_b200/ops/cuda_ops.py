@@ -1730,6 +1730,19 @@ class CudaOps:
     SIGMOID_MMA_LONGEST = 384
     use_mma_sigmoid = True        # bfloat16 with key and value sizes of 64 or 128: the two products on the tensor cores
 
+    @staticmethod
+    def _sigmoid_few(longest: int, tiles: int, dim: int, sms: int) -> bool:
+        """Whether a step of ``tiles`` entries that see up to ``longest`` keys is less work on mma.sync.  A key tile of the tcgen05 kernel has 128 keys whatever
+        the rows see and takes longer than 64 keys there; several tiles of an entry have their sums added by a second kernel either way, and with heads of 128 take about
+        as long as CTAs of 128 keys there while those run in one round of the SMs.  From a flushed L2, mma.sync / tcgen05, 16 heads of 128: 1 to 16 decoded rows 20 keys
+        15 / 28 us, 60 keys 20 / 27, 100 keys 33 / 28, 160 keys 28 / 33, 512 keys 34 / 36, 8 rows 2,000 keys 38 / 40, 3,000 keys 63 / 42, 32 rows 512 keys 36 / 38, 700 keys
+        62 / 40, 128 rows 160 keys 46 / 35; prompts of 160 rows 32 / 37, 256 rows 38 / 36, 400 rows 40 / 38, 700 rows 54 / 46, four of 256 rows 40 / 36, eight of 192 rows 46 / 37;
+        128 rows behind 1,000 keys 38 / 42.  14 heads of 64: 20 keys 16 / 23, 8 rows 60 keys 21 / 24, 100 keys 32 / 24, 192 keys 28 / 28, 512 keys 33 / 30.
+        A captured step is planned for its context limit, 1,024 keys at least, whatever the contexts: 8 rows of 20, 200, 600 and 1,000 keys 17, 34, 36 and 36 / 30, 32, 32
+        and 36 (mma.sync), 32 rows 17, 36, 50 and 64 / 30, 32, 40 and 42 (tcgen05); heads of 64, 8 rows 17, 34, 34 and 34 / 26, 26, 26 and 30 (tcgen05)."""
+        across = -(-longest // 128)
+        return longest <= 64 or (dim == 128 and across > 1 and tiles * across <= sms)
+
     def sigmoid_attention(self, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, batch: AttentionBatch,
                           heads: int, kv_heads: int, dim: int, vdim: int, scale: float, *, distance=None,
                           score_bias: torch.Tensor | None = None, head_mix: torch.Tensor | None = None) -> torch.Tensor:
@@ -1758,12 +1771,7 @@ class CudaOps:
                 and vdim in (64, 128) and q.data_ptr() % 16 == 0):
             wide = _declared_library("attention_sigmoid_tcgen05")
             longest = int(batch.max_kv_len)
-            # A tile has 128 keys whatever the rows see, so the shortest contexts and, in a step of few rows with heads of 128, those that have half a second
-            # tile or less stay on mma.sync.  In us with mma.sync / on tcgen05, 16 heads of 128: 1 row that sees 21 keys 9 / 18, 8 rows 48 keys 15 / 18, 60 rows
-            # 17 / 20, 1 row 65 keys 20 / 18, 90 rows 23 / 20, 130 rows 25 / 24, 160 rows 25 / 28, 192 rows 25 / 28, 224 rows 31 / 28, 16 rows 192 keys 22 / 24, 224
-            # keys 28 / 24; nine portions of 160 rows (90 entries) 28 / 28, of 176 (99) 39 / 29; 14 heads of 64, 1 row 21 keys 8 / 12, 8 rows 48 keys 13 / 12, 60 rows
-            # 16 / 14, 239 keys 30 / 21.
-            few = longest <= dim // 2 or (dim == 128 and 128 < longest <= 192 and tiles <= 90)
+            few = self._sigmoid_few(longest, tiles, dim, self.sm_count(q.device))
             if (self.use_tcgen05_attention and not few and k_pool.data_ptr() % 16 == 0
                     and v_pool.data_ptr() % 16 == 0 and tiles <= wide.mlr_attention_sigmoid_tcgen05_most()
                     and wide.mlr_attention_sigmoid_tcgen05_fits(heads, kv_heads, dim, vdim, k_pool.shape[2])):

@@ -260,13 +260,23 @@ def test_sigmoid_attention_of_prompts(heads, kv_heads, dim, vdim, mixed):
     close(got, want, ATTENTION_BOUND, "sigmoid attention")
 
 
+def on_tcgen05(monkeypatch):
+    """Every sigmoid attention of sizes that fit on tcgen05, whatever it costs; how many calls went there."""
+    lib, calls = cuda_ops._declared_library("attention_sigmoid_tcgen05"), []
+    kernel = lib.mlr_attention_sigmoid_tcgen05
+    monkeypatch.setattr(cuda(), "_sigmoid_few", lambda *args: False, raising=False)
+    monkeypatch.setattr(lib, "mlr_attention_sigmoid_tcgen05", lambda *args: calls.append(1) or kernel(*args))
+    return calls
+
+
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,page_size", [(16, 4, 128, 128, 8), (14, 2, 64, 64, 16), (9, 3, 128, 64, 64), (5, 1, 64, 128, 256),
                                                                (4, 4, 64, 64, 128)])
 @pytest.mark.parametrize("lengths,before", [([129], [0]), ([16, 1, 8], [112, 640, 300]), ([1] * 7, [127, 128, 63, 64, 1000, 200, 500]), ([1] * 6, [2700, 3, 60, 127, 128, 11]),
-                                            ([70, 260, 9, 1], [250, 0, 127, 383])])
-def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, lengths, before):
+                                            ([70, 260, 9, 1], [250, 0, 127, 383]), ([1, 30, 17], [64, 70, 111]), ([40, 3, 1], [210, 250, 192]),
+                                            ([1] * 150 + [25], [40 + i % 88 for i in range(150)] + [100])])
+def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, lengths, before, monkeypatch):
     """Keys around tiles of 128 and their halves, rows around the 8 of half an entry, entries cut and whole, pages smaller and larger than a
-    tile and its halves, heads that do not fill fours; places that no row sees hold NaN.  Mixing factors large enough that what mixing in fewer
+    tile and its halves, heads that do not fill fours; steps of one and two tiles per entry, of more entries than CTAs; places that no row sees hold NaN.  Mixing factors large enough that what mixing in fewer
     than 32 bits would leave of the weights shows.  The second call finds the first one's scratch."""
     (k_pool, v_pool), cpu, batch = paged(lengths, before, lambda p, j: j <= p, page_size, [(kv_heads, dim, 1.0), (kv_heads, vdim, 0.5)], 11)
     assert cuda().use_tcgen05_attention and cuda_ops.build.load_library("attention_sigmoid_tcgen05").mlr_attention_sigmoid_tcgen05_fits(
@@ -277,10 +287,12 @@ def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, len
     args = (heads, kv_heads, dim, vdim, dim ** -0.5)
     want = FAKE.sigmoid_attention(q.float(), k_pool.float(), v_pool.float(), cpu, *args, **vectors)
     there = {k: tuple(t.to(DEVICE) for t in v) if isinstance(v, tuple) else v.to(DEVICE) for k, v in vectors.items()}
+    calls = on_tcgen05(monkeypatch)
     first = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, **there)
     got = cuda().sigmoid_attention(q.to(DEVICE), k_pool.to(DEVICE), v_pool.to(DEVICE), batch, *args, **there)
     torch.cuda.synchronize()
     cuda().raise_if_device_error()
+    assert len(calls) == 2
     # mixed weights and results are rounded to 8 bits, 2^-9 each at most; mixed with signs, weights lose size against the keys' sum of squares no
     # more than in ATTENTION_BOUND's own margin
     close(got, want, ATTENTION_BOUND, "sigmoid attention")
@@ -303,14 +315,6 @@ def test_heads_mixed_by_parts_are_mixed_in_32_bits():
     # a mixed weight is a sum of twelve products of numbers around one, each rounded to 2^-24 (the tensor cores' sums drop as much), beside a result
     # of 2^-12 / 2: below 12 * 2 * 2^-24 / 2^-13 = 2^-6.4 of it, independent from key to key
     close(got, want, ATTENTION_BOUND + 2.0 ** -6.4, "mixed weights")
-
-
-def on_tcgen05(monkeypatch):
-    """Every sigmoid attention of sizes that fit on tcgen05, whatever it costs; how many calls went there."""
-    lib, calls = cuda_ops._declared_library("attention_sigmoid_tcgen05"), []
-    kernel = lib.mlr_attention_sigmoid_tcgen05
-    monkeypatch.setattr(lib, "mlr_attention_sigmoid_tcgen05", lambda *args: calls.append(1) or kernel(*args))
-    return calls
 
 
 @pytest.mark.parametrize("heads,dim", [(12, 64), (16, 128)])

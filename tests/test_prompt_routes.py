@@ -39,6 +39,16 @@ def test_decoded_rows_contexts_do_not_move_the_borders(decoded):
         assert cuda_ops.latent_prompt_on_tcgen05(b, rows, 50) == (rows - len(ones) > 64), (lengths, before)
 
 
+@pytest.mark.parametrize("lengths,before,dim,few", [
+    ([64], [0], 128, True), ([1], [63], 64, True), ([1], [64], 64, False), ([1] * 8, [64] * 8, 128, False), ([128], [0], 128, False), ([129], [0], 128, True),
+    ([1] * 74, [255] * 74, 128, True), ([1] * 75, [255] * 75, 128, False), ([1] * 75, [127] * 75, 128, False), ([16, 1], [500, 2000], 128, True), ([512], [0], 128, True),
+    ([513], [0], 128, False), ([129], [0], 64, False)])
+def test_sigmoid_attention_of_few_keys_stays_on_mma_sync(lengths, before, dim, few):
+    """Contexts of half a key tile; with heads of 128, several tiles of an entry while all entries' tiles are a round of the SMs."""
+    b = batch(lengths, before)
+    assert cuda_ops.CudaOps._sigmoid_few(b.max_kv_len, b.counts["tiles"], dim, 148) == few
+
+
 def test_a_product_is_told_the_room_that_its_workspace_has(monkeypatch):
     """The kernel refuses plans that do not fit; what counts is the memory there is, not what a workspace made later would get."""
     asked = []
