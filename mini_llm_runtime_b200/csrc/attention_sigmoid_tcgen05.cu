@@ -633,6 +633,15 @@ sigmoid_add_runs_kernel(const SgArgs a, int vdim, int most_runs) {
   }
 }
 
+// Whether the launch takes the registers that the warps share out anew.  (Another compiler may give the kernel others; a split above the launch's waits forever.)
+template <int D, int V>
+static bool sg_registers_fit() {
+  static int registers = 0;
+  cudaFuncAttributes attributes;
+  if (registers == 0 && cudaFuncGetAttributes(&attributes, attention_sigmoid_tcgen05_kernel<D, V>) == cudaSuccess) registers = attributes.numRegs;
+  return registers == SG_LAUNCH_REGISTERS;
+}
+
 template <int D, int V>
 static int sg_launch(SgArgs a, const void* k_pool, const void* v_pool, int ctas, bool cut, cudaStream_t stream) {
   CUtensorMap k_map, v_map;
@@ -641,9 +650,7 @@ static int sg_launch(SgArgs a, const void* k_pool, const void* v_pool, int ctas,
     return MLR_BAD_SIZE;
   static bool configured = false;
   if (!configured) {
-    cudaFuncAttributes attributes;
-    if (cudaFuncGetAttributes(&attributes, attention_sigmoid_tcgen05_kernel<D, V>) != cudaSuccess || attributes.numRegs != SG_LAUNCH_REGISTERS)
-      return MLR_BAD_SIZE;      // the shares would not add up to what the launch takes
+    if (!sg_registers_fit<D, V>()) return MLR_TOO_LARGE;
     cudaError_t err = cudaFuncSetAttribute(attention_sigmoid_tcgen05_kernel<D, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg_shared<D>(SG_HEADS));
     if (err != cudaSuccess) return (int)err;
     configured = true;
@@ -663,12 +670,14 @@ using namespace mlr;
 
 MLR_DEFINE_PDL_SWITCH
 
-// 1 if the kernel takes these sizes, else 0.
+// 1 if the kernel takes these sizes as it was compiled, else 0.
 MLR_EXPORT int mlr_attention_sigmoid_tcgen05_fits(int heads, int kv_heads, int dim, int vdim, int page_size) {
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || heads > SG_HEADS) return 0;
   if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128)) return 0;
   if (kv_heads * ((heads / kv_heads + 3) / 4) * 4 > SG_SLOTS) return 0;
-  return page_size >= 8 && (page_size & (page_size - 1)) == 0 ? 1 : 0;
+  if (page_size < 8 || (page_size & (page_size - 1)) != 0) return 0;
+  if (dim == 64) return vdim == 64 ? sg_registers_fit<64, 64>() : sg_registers_fit<64, 128>();
+  return vdim == 64 ? sg_registers_fit<128, 64>() : sg_registers_fit<128, 128>();
 }
 
 // Entries of a call at most.

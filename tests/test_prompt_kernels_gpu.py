@@ -4,6 +4,8 @@ other batches."""
 
 from __future__ import annotations
 
+import ctypes
+import subprocess
 import types
 
 import pytest
@@ -297,6 +299,19 @@ def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, len
     # more than in ATTENTION_BOUND's own margin
     close(got, want, ATTENTION_BOUND, "sigmoid attention")
     assert torch.equal(first, got)
+
+
+def test_a_kernel_compiled_to_other_registers_is_not_offered(tmp_path):
+    """The shares of another launch than the compiler's: the sizes do not fit, so that calls go on to the kernel behind it."""
+    source = (cuda_ops.build.CSRC / "attention_sigmoid_tcgen05.cu").read_text()
+    shares = "SG_LAUNCH_REGISTERS = 168, SG_COMPUTE_REGISTERS = 208, SG_OTHER_REGISTERS = 88"
+    assert shares in source
+    (tmp_path / "other.cu").write_text(source.replace(shares, "SG_LAUNCH_REGISTERS = 160, SG_COMPUTE_REGISTERS = 200, SG_OTHER_REGISTERS = 80"))
+    subprocess.run([cuda_ops.build.find_nvcc(), *cuda_ops.build.ARCH_FLAGS, *cuda_ops.build.COMMON_FLAGS, f"-I{cuda_ops.build.CSRC}", "-o",
+                    str(tmp_path / "other.so"), str(tmp_path / "other.cu")], check=True)
+    other, own = ctypes.CDLL(str(tmp_path / "other.so")), cuda_ops.build.load_library("attention_sigmoid_tcgen05")
+    for dim, vdim in ((64, 64), (64, 128), (128, 64), (128, 128)):
+        assert own.mlr_attention_sigmoid_tcgen05_fits(8, 2, dim, vdim, 16) == 1 and other.mlr_attention_sigmoid_tcgen05_fits(8, 2, dim, vdim, 16) == 0
 
 
 def test_heads_mixed_by_parts_are_mixed_in_32_bits():
