@@ -9,7 +9,8 @@
 // Bound by the memory's rate for weights with few tokens per expert (a step of 40 rows reads 1.07 GB in 178 us, sorting, gathering and summing
 // included), by the round trips of four stages beside MMAs with many.  Measured (B200), whole feed-forward, tokens as the MMA's rows / so: 64 experts of
 // 2,048 -> 1,408, six per row, 2,048 rows 424 / 368 us (371 / 319 in a captured sequence, as the following), 1,000 rows 250 / 234, 300 rows 211 / 196, 40 rows 199 / 178; 16 experts of 896 -> 2,432, two per
-// row, 2,048 rows 99 / 101, 700 rows 69 / 66, 100 rows 63 / 55.  Tiles of 256 tokens with one accumulator pair and three stages: 382 us at 2,048 rows (a
+// row, 700 rows 69 / 66, 100 rows 63 / 55.  From a flushed L2, 16 experts, 2,000 rows 111 / 94, 2,048 rows, whose down product has 160 tiles, 111 / 115 and, with tiles half
+// as high, 109; 300 rows of three experts 51 / 49 / 45.  Tiles of 256 tokens with one accumulator pair and three stages: 382 us at 2,048 rows (a
 // stage's round trip and its MMAs one behind the other); four warps that write instead of eight: 323, and 122 us for the 16 experts.
 //
 // Warp 0 loads (weights in boxes of 64 rows, tokens in boxes of 32, four stages of 48 KB), warp 1 issues MMAs, warps 2 to 9 write out.
@@ -30,7 +31,7 @@ constexpr uint32_t EP_TMEM_COLS = 512;
 
 struct ExpertArgs {
   void* out;
-  const int* tiles;            // [max_tiles][3]: expert (negative: unused), first row, end row
+  const int* tiles;            // [max_tiles][3]: expert (negative: unused), first row, end row; then how many are used
   const float* row_scale;      // factor of every row's product, before the gate, or null
   int N, K;                    // rows of an expert's matrix, columns
   int entries;                 // of the list
@@ -65,7 +66,15 @@ expert_product_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
   fa_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_holder, 0);
   pdl_wait();                                // the list comes from an earlier kernel
-  const int k_blocks = (p.K + EP_K - 1) / EP_K, across = (p.N + EP_WEIGHTS - 1) / EP_WEIGHTS;
+  const int k_blocks = (p.K + EP_K - 1) / EP_K;
+  int high = EP_WEIGHTS;      // weight rows of a tile
+  if (!GATED) {
+    // Half as high, with one accumulator, where that saves so many rounds of CTAs that it pays for the smaller tiles, which take some 0.7 of the time.
+    const int used = __ldcg(p.tiles + 3 * p.entries), grid = (int)gridDim.x;
+    auto rounds = [&](int rows) { return ((p.N + rows - 1) / rows * used + grid - 1) / grid; };
+    if (rounds(EP_WEIGHTS / 2) * 7 < rounds(EP_WEIGHTS) * 10) high = EP_WEIGHTS / 2;
+  }
+  const int across = (p.N + high - 1) / high;
   const int tiles = across * p.entries;
   bool gave_up = false;
   struct Tile { int expert, row0, tokens, column; };
@@ -89,17 +98,17 @@ expert_product_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
       const Tile t = tile_at(tile);
       if (t.tokens <= 0) continue;
       const int x_boxes = (t.tokens + EP_X_BOX - 1) / EP_X_BOX;
-      const int w_row = t.expert * p.N + t.column * EP_WEIGHTS + (GATED ? (block & 1) * 128 + (block >> 1) * 64 : block * 64);
+      const int w_row = t.expert * p.N + t.column * high + (GATED ? (block & 1) * 128 + (block >> 1) * 64 : block * 64);
       const int x_row = t.row0 + (lane - 4) * EP_X_BOX;
-      const uint32_t bytes = (uint32_t)(EP_W_BYTES + x_boxes * EP_X_BOX * 128);
+      const uint32_t bytes = (uint32_t)(high * EP_K * 2 + x_boxes * EP_X_BOX * 128);
       for (int i = 0; i < k_blocks; ++i) {
         fa_wait(&empty_bar[s], phase ^ 1u, p.error_word, 0xb1, gave_up);
         gave_up = __any_sync(0xffffffffu, gave_up);
         if (!gave_up) {
           if (lane == 0) mbar_expect_tx(&full_bar[s], bytes);
           __syncwarp();
-          if (lane < 4) tma_load_2d(&w_map, &full_bar[s], own + s * EP_STAGE_BYTES, i * EP_K, w_row);
-          else if (lane - 4 < x_boxes) tma_load_2d(&x_map, &full_bar[s], own + s * EP_STAGE_BYTES, i * EP_K, x_row);
+          if (lane < high / EP_W_BOX) tma_load_2d(&w_map, &full_bar[s], own + s * EP_STAGE_BYTES, i * EP_K, w_row);
+          else if (lane >= 4 && lane - 4 < x_boxes) tma_load_2d(&x_map, &full_bar[s], own + s * EP_STAGE_BYTES, i * EP_K, x_row);
         }
         if (++s == EP_STAGES) s = 0, phase ^= 1u;
       }
@@ -123,7 +132,7 @@ expert_product_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
           for (int k = 0; k < EP_K / 16; ++k)
 #pragma unroll
             for (int half = 0; half < 2; ++half)
-              fa_mma(tmem_base + (turn & 1u) * 2 * EP_TOKENS + half * EP_TOKENS, w + half * (128 * 128 >> 4) + 2 * k, x + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+              if (half * 128 < high) fa_mma(tmem_base + (turn & 1u) * 2 * EP_TOKENS + half * EP_TOKENS, w + half * (128 * 128 >> 4) + 2 * k, x + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
           fa_commit(&empty_bar[s]);
           if (i == k_blocks - 1) fa_commit(&done_bar[turn & 1u]);
         }
@@ -181,12 +190,15 @@ expert_product_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
           asm volatile("bar.sync %0, 128;" ::"r"(1 + side) : "memory");      // staged again
         }
       } else {
-        const int n = t.column * EP_WEIGHTS + side * 128 + own;
+        const bool both = high == EP_WEIGHTS;      // accumulators; else a group of warps takes the first or the last 64 tokens of the one
+        const int n = t.column * high + (both ? side * 128 : 0) + own, from = both ? 0 : side * (EP_TOKENS / 2);
+        const int end = both ? t.tokens : min(t.tokens, from + EP_TOKENS / 2);
+        const uint32_t sums = lane_base + (both ? side * EP_TOKENS : 0);
         float* column = reinterpret_cast<float*>(p.out) + (size_t)t.row0 * p.N + n;
-        for (int c = 0; c < t.tokens; c += 32) {
+        for (int c = from; c < end; c += 32) {
           uint32_t v[32];
-          fa_tmem_load16(lane_base + side * EP_TOKENS + c, v);
-          fa_tmem_load16(lane_base + side * EP_TOKENS + c + 16, v + 16);
+          fa_tmem_load16(sums + c, v);
+          fa_tmem_load16(sums + c + 16, v + 16);
           fa_tmem_wait_ld();
           if (gave_up || n >= p.N) continue;
 #pragma unroll
@@ -221,7 +233,8 @@ static int launch_experts(const void* x, const void* w, const ExpertArgs& a, int
     if (err != cudaSuccess) return (int)err;
     configured = true;
   }
-  const long long tiles = (long long)((a.N + EP_WEIGHTS - 1) / EP_WEIGHTS) * a.entries;
+  const int least = GATED ? EP_WEIGHTS : EP_WEIGHTS / 2;      // rows of a tile
+  const long long tiles = (long long)((a.N + least - 1) / least) * a.entries;
   if (tiles > 0x3fffffff) return MLR_TOO_LARGE;
   launch_kernel(expert_product_kernel<GATED>, dim3((unsigned)(tiles < sm_count() ? tiles : sm_count())), dim3(EP_THREADS), (size_t)EP_SHARED, stream, w_map, x_map, a);
   return launch_status();
@@ -234,7 +247,7 @@ using namespace mlr;
 MLR_DEFINE_PDL_SWITCH
 
 // x: bfloat16 [rows, K], sorted by expert; w: bfloat16 [groups, N, K]; tiles: device memory, int32 [max_tiles][3] = (expert, first row, end row)
-// per tile of up to 128 rows of one expert, expert < 0 for unused entries; it may be written by the kernel just before this one.
+// per tile of up to 128 rows of one expert, expert < 0 for unused entries, and their number behind them; it may be written by the kernel just before this one.
 // gated: w holds blocks of 64 gate rows followed by the 64 up rows of the same outputs, out is act(gate) * up, bfloat16 [rows, N / 2] (act 0:
 // silu, 1: the tanh form of gelu); else out is float32 [rows, N].  row_scale: float32 [rows] or null, multiplies each row's product, before the gate.
 MLR_EXPORT int mlr_expert_product(const void* x, const void* w, void* out, const int* tiles, int max_tiles, int rows, int groups, int N, int K,

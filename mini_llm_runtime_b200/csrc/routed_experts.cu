@@ -387,7 +387,7 @@ expert_down_kernel(const T* hidden, const int* chosen, const float* weights, con
 // ---------------------------------------------------------------- sorted form for the grouped product
 // One CTA.  place[p]: where pair p lands in expert order; token_of[place]: the row it came from;
 // tiles: for every used tile of `tile_rows` rows (expert, first place, end place), then -1 entries up
-// to max_tiles.  The order inside an expert's run is not fixed (atomics); every pair's result is
+// to max_tiles, then the number of used ones.  The order inside an expert's run is not fixed (atomics); every pair's result is
 // computed from its own row alone, so the order changes no number.
 __global__ void __launch_bounds__(1024)
 sort_pairs_kernel(const int* chosen, const float* weights, int* place, int* token_of, float* sorted_weights, int* tiles,
@@ -445,7 +445,7 @@ sort_pairs_kernel(const int* chosen, const float* weights, int* place, int* toke
       at += __shfl_sync(0xffffffffu, places, 31);
       tile += __shfl_sync(0xffffffffu, tiles_to, 31);
     }
-    if (threadIdx.x == 0) used_tiles = min(tile, max_tiles);
+    if (threadIdx.x == 0) tiles[3 * max_tiles] = used_tiles = min(tile, max_tiles);
   }
   __syncthreads();
   for (int index = used_tiles + threadIdx.x; index < max_tiles; index += blockDim.x) {
@@ -632,7 +632,7 @@ MLR_EXPORT int mlr_expert_down(const void* hidden, const int* chosen, const floa
   return MLR_BAD_DTYPE;
 }
 
-// chosen: int32 [pairs]; place: int32 [pairs]; token_of: int32 [pairs]; tiles: int32 [max_tiles, 3]; weights
+// chosen: int32 [pairs]; place: int32 [pairs]; token_of: int32 [pairs]; tiles: int32 [max_tiles * 3 + 1]; weights
 // (float32 [pairs]) and sorted_weights (the same in the order of places) may both be null.
 MLR_EXPORT int mlr_sort_pairs(const int* chosen, const float* weights, int* place, int* token_of, float* sorted_weights,
                               int* tiles, int pairs, int top, int experts,

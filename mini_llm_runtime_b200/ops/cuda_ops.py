@@ -1605,7 +1605,7 @@ class CudaOps:
         max_tiles = min(pairs, -(-pairs // tile_rows) + experts)
         place = torch.empty(pairs, dtype=torch.int32, device=x.device)
         token_of = torch.empty(pairs, dtype=torch.int32, device=x.device)
-        tiles = torch.empty(max_tiles * 3, dtype=torch.int32, device=x.device)
+        tiles = torch.empty(max_tiles * 3 + 1, dtype=torch.int32, device=x.device)
         # weights of the inputs, in the order of the sorted rows: the gate/up product's epilogue applies them
         row_scale = torch.empty(pairs, dtype=torch.float32, device=x.device) if weigh_input else None
         _check(lib.mlr_sort_pairs(_ptr(chosen), _ptr(in_weights), _ptr(place), _ptr(token_of), _ptr(row_scale), _ptr(tiles),

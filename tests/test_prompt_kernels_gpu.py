@@ -561,10 +561,11 @@ def test_long_sums_of_many_rows_keep_their_scratch_bounded():
 @pytest.mark.parametrize("width,inner", [(72, 64), (200, 192), (512, 128)])
 @pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
 @pytest.mark.parametrize("weigh_input", [False, True])
-def test_experts_of_any_number_of_rows(width, inner, activation, weigh_input):
+@pytest.mark.parametrize("others", [0, 300])
+def test_experts_of_any_number_of_rows(width, inner, activation, weigh_input, others):
     """Rows of an expert around the multiples of 16 and 32 of an MMA and a copy, of the 64 and 128 of half a tile and a tile, none at all; columns
-    that fill no copy of 64, weight rows that fill no tile of 256, and so many tiles that a CTA takes several."""
-    counts = [1, 15, 0, 16, 17, 31, 33, 63, 64, 65, 96, 127, 128, 129, 255, 256, 257] + [3] * 300
+    that fill no copy of 64, weight rows that fill no tile of 256, so many tiles that a CTA takes several, and so few that the down product's are half as high."""
+    counts = [1, 15, 0, 16, 17, 31, 33, 63, 64, 65, 96, 127, 128, 129, 255, 256, 257] + [3] * others
     experts, rows = len(counts), sum(counts)
     chosen = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(rows, generator=generator(1))]
     x, weights = rnd(2, rows, width).to(torch.bfloat16), torch.rand(rows, 1, generator=generator(3)) + 0.5
