@@ -935,33 +935,31 @@ MLR_EXPORT int mlr_gemm_tcgen05(const void* x, const void* w, const void* bias, 
 
 // ---------------------------------------------------------------- grouped form
 namespace mlr {
-template <int BN, int BM = TILE_ROWS>
+template <int BN>
 static int launch_grouped(const void* x, const void* w, const GemmParams& p, int rows, int groups, int max_tiles,
                           cudaStream_t stream) {
-  const size_t shared = (size_t)p.stages * (BM * TILE_K * 2 + BN * TILE_K * 2) + 1024;
-  if (int err = allow_shared<BN, false, false, BM>(shared)) return err;
+  const size_t shared = (size_t)p.stages * (TILE_ROWS * TILE_K * 2 + BN * TILE_K * 2) + 1024;
+  if (int err = allow_shared<BN, false, false>(shared)) return err;
   CUtensorMap map_a, map_b;
   if (!cached_tile_map(&map_a, x, rows, p.K, TILE_ROWS) || !cached_tile_map(&map_b, w, groups * p.N, p.K, BN))
     return MLR_BAD_ALIGNMENT;
   if (max_tiles > 65535) return MLR_TOO_LARGE;
   dim3 grid((p.N + BN - 1) / BN, max_tiles, 1);
-  launch_kernel(gemm_tcgen05_kernel<BN, false, false, BM>, dim3(grid), dim3(GEMM_THREADS), shared, stream, map_a,
-                map_b, p);
+  launch_kernel(gemm_tcgen05_kernel<BN, false, false>, dim3(grid), dim3(GEMM_THREADS), shared, stream, map_a, map_b, p);
   return launch_status();
 }
 }  // namespace mlr
 
 // The product of rows that are sorted by group with each group's own matrix: x [rows, K], w [groups, N, K]
 // (stacked), out [rows, N].  (With the gate in the epilogue: experts_tcgen05.cu.)  `tiles` is
-// device memory, int32 [max_tiles][3] = (group, first row, end row) per tile of up to `tile_rows` (128,
-// or 256 where N is a multiple of 256: two accumulators from one load of the weight tile, one CTA
-// per SM) rows of one group, group < 0 for unused entries; it may be written by the kernel just
+// device memory, int32 [max_tiles][3] = (group, first row, end row) per tile of up to 128
+// rows of one group, group < 0 for unused entries; it may be written by the kernel just
 // before this one.  A 128-row load may run into the next group's rows (or past the last row: zeros);
 // those rows are computed and dropped.  `row_scale` (float32 [rows] or null) multiplies each row's product
 // (the same as scaling the rows of x).  A weight tile that would run into
 // the next group's rows is loaded but its columns beyond N are never written.
 MLR_EXPORT int mlr_gemm_tcgen05_grouped(const void* x, const void* w, void* out, const int* tiles, int max_tiles, int rows,
-                                        int groups, int N, int K, int out_f32, int tile_rows,
+                                        int groups, int N, int K, int out_f32,
                                         const float* row_scale, int* error_word, cudaStream_t stream) {
   if (rows == 0 || max_tiles == 0) return MLR_OK;
   if (rows < 0 || max_tiles < 0 || groups <= 0 || N <= 0 || K <= 0 || tiles == nullptr) return MLR_BAD_SIZE;
@@ -969,17 +967,15 @@ MLR_EXPORT int mlr_gemm_tcgen05_grouped(const void* x, const void* w, void* out,
   if ((long long)groups * N > 0x7fffffffll) return MLR_TOO_LARGE;
   const int total_kb = (K + TILE_K - 1) / TILE_K;
   const bool wide = N % 256 == 0 && N >= 512;
-  const bool tall = tile_rows == 2 * TILE_ROWS;
-  if ((tile_rows != TILE_ROWS && !tall) || (tall && !wide)) return MLR_BAD_SIZE;
   GemmParams p;
   p.M = rows; p.N = N; p.K = K;
   p.k_blocks_per_split = total_kb;
   p.splits = 1;
-  // tall tiles: rings of up to three 64 KB stages, one CTA per SM.  Else rings of 32 KB (128 x 128) or
+  // rings of 32 KB (128 x 128) or
   // 48 KB (128 x 256) stages, as deep as K is long, within 96 KB so that two CTAs share an SM and one's
   // epilogue runs under the other's main loop
   const int stage_bytes = TILE_ROWS * TILE_K * 2 + (wide ? 256 : 128) * TILE_K * 2;
-  int stages = tall ? 3 : 96 * 1024 / stage_bytes;
+  int stages = 96 * 1024 / stage_bytes;
   if (stages > total_kb) stages = total_kb;
   p.stages = stages < 2 ? 2 : stages;
   p.bias = nullptr;
@@ -993,6 +989,5 @@ MLR_EXPORT int mlr_gemm_tcgen05_grouped(const void* x, const void* w, void* out,
   p.error_word = error_word;
   p.group_tiles = tiles;
   p.row_scale = row_scale;
-  if (tall) return launch_grouped<256, 2 * TILE_ROWS>(x, w, p, rows, groups, max_tiles, stream);
   return wide ? launch_grouped<256>(x, w, p, rows, groups, max_tiles, stream) : launch_grouped<128>(x, w, p, rows, groups, max_tiles, stream);
 }

@@ -258,7 +258,6 @@ class CudaOps:
         self.use_tma_attention = True
         self.use_fused_rope = True
         self.use_grouped_experts = True     # routed experts of many rows: sorted pairs through the grouped tcgen05 product
-        self.use_tall_expert_tiles = False  # .. without the gate in the product: in tiles of 256 rows of an expert where experts get more than 128 (measured: no gain)
         self.use_cluster_merge = True       # chunks of a decode row merge through a cluster's shared memory
         self.split_prefill_items = True     # the tcgen05 prompt attention may cut long items into parts
         # MLR_TCGEN05_ATTENTION=0 in the environment keeps prompt attention on the mma.sync kernels
@@ -1597,11 +1596,8 @@ class CudaOps:
         # its own matrices (tiles of 128 rows of one expert), the results summed per row in the order
         # of the row's choices
         # With the gate in the epilogue an expert's weights are the rows of the MMA (experts_tcgen05.cu), else its tokens.
-        # rows of a tile there: 256 (two accumulators from one load of an expert's weight tile) when an expert
-        # gets more than 128 rows on average and both products have the columns for it, else 128
         fused = self.use_fused_swiglu and block == self.SWIGLU_BLOCK and (2 * inner) % 128 == 0
-        both_wide = all(n % 256 == 0 and n >= 512 for n in (2 * inner, N))
-        tile_rows = 256 if not fused and self.use_tall_expert_tiles and both_wide and pairs > 128 * experts else 128
+        tile_rows = 128
         max_tiles = min(pairs, -(-pairs // tile_rows) + experts)
         place = torch.empty(pairs, dtype=torch.int32, device=x.device)
         token_of = torch.empty(pairs, dtype=torch.int32, device=x.device)
@@ -1625,10 +1621,10 @@ class CudaOps:
         else:
             product = build.load_library("gemm_tcgen05").mlr_gemm_tcgen05_grouped
             both = torch.empty((pairs, 2 * inner), dtype=x.dtype, device=x.device)
-            _check(product(_ptr(sorted_x), _ptr(gate_up), _ptr(both), _ptr(tiles), max_tiles, pairs, experts, 2 * inner, K, 0, tile_rows,
+            _check(product(_ptr(sorted_x), _ptr(gate_up), _ptr(both), _ptr(tiles), max_tiles, pairs, experts, 2 * inner, K, 0,
                            _ptr(row_scale), error_word, _stream()), "grouped gate/up product")
             hidden = self.gated_activation(both, block, activation)
-            _check(product(_ptr(hidden), _ptr(down), _ptr(y), _ptr(tiles), max_tiles, pairs, experts, N, inner, 1, tile_rows, _ptr(None),
+            _check(product(_ptr(hidden), _ptr(down), _ptr(y), _ptr(tiles), max_tiles, pairs, experts, N, inner, 1, _ptr(None),
                            error_word, _stream()), "grouped down product")
         _check(lib.mlr_combine_pairs(_ptr(y), _ptr(place), _ptr(out_weights), _ptr(out), rows, N, top, _stream()),
                "combine_pairs")

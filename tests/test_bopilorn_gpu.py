@@ -72,10 +72,10 @@ def test_router_kernel_against_its_formula():
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("rows,width,inner,experts,top", [(1, 40, 24, 3, 2), (5, 72, 52, 5, 1), (150, 64, 64, 4, 3),
                                                             (300, 128, 192, 8, 2), (700, 256, 128, 16, 4), (20, 36, 20, 2, 2),
-                                                            (700, 512, 256, 4, 2), (900, 768, 384, 5, 3)])
+                                                            (700, 512, 256, 4, 2), (900, 768, 384, 5, 3), (700, 512, 200, 4, 2), (300, 256, 264, 3, 1)])
 def test_expert_kernels_against_their_formula(rows, width, inner, experts, top, dtype):
-    """Few and many rows (the sorted, grouped tensor-core product takes the latter in bfloat16: in tiles
-    of 128 rows of an expert, or of 256 where the products are wide and the experts get many rows),
+    """Few and many rows (products of sorted rows on the tensor cores take the latter in bfloat16: with weights as the MMA's rows where
+    the gate is in the product, else with tokens as its rows, in 128 or 256 columns),
     sizes with and without the interleaved gate/up blocks, experts that get no row at all."""
     from mini_llm_runtime_b200 import ops
     from mini_llm_runtime_b200.config import PartSpec
@@ -90,13 +90,8 @@ def test_expert_kernels_against_their_formula(rows, width, inner, experts, top, 
     chosen = torch.stack([torch.randperm(pool, generator=generator)[:top] for _ in range(rows)]).to(torch.int32)
     weights = torch.rand(rows, top, generator=generator)
     kernels = ops.current()
-    before = kernels.use_tall_expert_tiles
-    kernels.use_tall_expert_tiles = rows == 900          # one of the wide cases in tiles of 256 rows
-    try:
-        got = kernels.routed_experts(x.to(DEVICE).to(dtype), chosen.to(DEVICE), weights.to(DEVICE), part.w_gate_up,
-                                     part.w_down, part.block)
-    finally:
-        kernels.use_tall_expert_tiles = before
+    got = kernels.routed_experts(x.to(DEVICE).to(dtype), chosen.to(DEVICE), weights.to(DEVICE), part.w_gate_up,
+                                 part.w_down, part.block)
     want = torch.zeros(rows, width, dtype=torch.float64)
     x64 = x.double()
     for e in range(experts):
@@ -112,7 +107,7 @@ def test_expert_kernels_against_their_formula(rows, width, inner, experts, top, 
     assert error < (1e-5 if dtype == F32 else 1.5e-2), error
 
 
-def test_grouped_and_plain_products_share_a_kernel_without_harm():
+def test_grouped_and_plain_products_share_a_kernel_without_harm(monkeypatch):
     """The grouped product and the plain product of many rows are launches of one kernel with rings
     of different depths; each keeps working after the other has run."""
     from mini_llm_runtime_b200 import ops
@@ -122,14 +117,18 @@ def test_grouped_and_plain_products_share_a_kernel_without_harm():
     w = (torch.randn(1024, 1024, generator=generator) * 0.03).to(BF16).to(DEVICE)
     want = x.float() @ w.float().T
     small = torch.randn(300, 64, generator=generator).to(BF16).to(DEVICE)
-    gate_up = (torch.randn(4, 256, 64, generator=generator) * 0.1).to(BF16).to(DEVICE)
-    down = (torch.randn(4, 64, 128, generator=generator) * 0.1).to(BF16).to(DEVICE)
+    gate_up = (torch.randn(4, 208, 64, generator=generator) * 0.1).to(BF16).to(DEVICE)      # no gate in the product
+    down = (torch.randn(4, 64, 104, generator=generator) * 0.1).to(BF16).to(DEVICE)
+    launched, load = [], ops.cuda_ops.build.load_library
+    monkeypatch.setattr(ops.cuda_ops.build, "load_library", lambda name: launched.append(name) or load(name))
     chosen = torch.randint(0, 4, (300, 1), generator=generator, dtype=torch.int32).to(DEVICE)
     weights = torch.ones(300, 1, device=DEVICE)
     for _ in range(2):
         got = k.linear(x, w, out_dtype=F32)
         assert float((got - want).abs().max()) < 2e-2 * float(want.abs().max())
-        assert torch.isfinite(k.routed_experts(small, chosen, weights, gate_up, down, 64)).all()
+        launched.clear()
+        assert torch.isfinite(k.routed_experts(small, chosen, weights, gate_up, down, 104)).all()
+        assert "gemm_tcgen05" in launched and "experts_tcgen05" not in launched
     torch.cuda.synchronize()
     k.raise_if_device_error()
 
