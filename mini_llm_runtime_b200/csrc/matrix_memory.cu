@@ -1383,14 +1383,14 @@ MLR_DEFINE_PDL_SWITCH
 // Whether prompts of these head sizes can go through the tensor cores in chunks (with `pairs`).
 MLR_EXPORT int mlr_matrix_memory_chunks_fit(int dim, int vdim) { return chunks_fit(dim, vdim); }
 
-// Chunks that a block walks one behind the other: 1 where a step's chunks go side by side, 0 where all of a segment's go one behind the other: where
-// no portion has more than two (one behind the other / side by side: 65 rows of 7 heads 21.5 / 24.4 us, 128 rows 22.5 / 24.4, 129 rows 24.9 / 24.8, 192 rows
-// 25.5 / 24.9, 16 heads of 129 rows 25.2 / 25.2; short portions beside a longer one take no time of their own).
-MLR_EXPORT int mlr_matrix_memory_run(int chunks, int segments, int max_q_len, int vdim) {
+// 1 where a step's chunks go side by side, 0 where a segment's go one behind the other: where no portion has more than two.  One behind the other / side by
+// side, repeated calls: 65 rows of 7 heads 21.5 / 24.4 us, 128 rows 22.5 / 24.4, 129 rows 24.9 / 24.8, 192 rows 25.5 / 24.9, 16 heads of 129 rows 25.2 / 25.2; from a
+// flushed L2 129 rows 42 / 34, 192 rows 44 / 36, four of 129 rows 48 / 36, of 16 heads 63 / 54.
+MLR_EXPORT int mlr_matrix_memory_side_by_side(int chunks, int segments, int max_q_len, int vdim) {
   return side_fits(64, vdim) && max_q_len > 2 * CHUNK && (long long)chunks + segments <= 65535 ? 1 : 0;
 }
 // .. and the float32 numbers of scratch that side by side needs.
-MLR_EXPORT long long mlr_matrix_memory_run_scratch(int chunks, int heads, int dim, int vdim) { return (long long)chunks * heads * ((long long)(vdim + 1) * dim + 1); }
+MLR_EXPORT long long mlr_matrix_memory_side_scratch(int chunks, int heads, int dim, int vdim) { return (long long)chunks * heads * ((long long)(vdim + 1) * dim + 1); }
 
 // q, k: float32 rows of heads * dim entries; v, gate: rows of heads * vdim; i_raw, f_raw: rows of `heads` entries (each
 // with its own row stride); i_bias, f_bias: float32 [heads]; weight: float32 [heads * vdim]; coef: float32 scratch

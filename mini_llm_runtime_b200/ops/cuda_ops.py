@@ -1986,7 +1986,7 @@ class CudaOps:
     # ------------------------------------------------------------------ matrix memory
     use_memory_chunks = True      # bfloat16 prompts in chunks of 64 tokens on the tensor cores
     MEMORY_CHUNK_ROWS = 16        # longest portion of a step from which that pays
-    use_memory_runs = True        # chunks side by side
+    use_memory_side_by_side = True        # chunks side by side
 
     def _memory_chunks_fit(self, dim: int, vdim: int) -> bool:
         cache = self.__dict__.setdefault("_memory_fits", {})
@@ -2027,10 +2027,10 @@ class CudaOps:
                 # heads 167 / 81, 2,048 beside 64 118 / 76 and 236 / 151, 512 beside 8 43 / 45 and 52 / 50.
                 beside = 2 if any(s.length == 1 for s in getattr(ctx, "segments", None) or ()) else 1
                 chunks = self._chunks_from(ctx, rows, beside)
-                if self.use_memory_runs and lib.mlr_matrix_memory_run(chunks, ctx.num_segments, int(ctx.max_q_len), vdim) > 0:
+                if self.use_memory_side_by_side and lib.mlr_matrix_memory_side_by_side(chunks, ctx.num_segments, int(ctx.max_q_len), vdim) > 0:
                     least = beside
-                    lib.mlr_matrix_memory_run_scratch.restype = ctypes.c_longlong
-                    ends = torch.empty(lib.mlr_matrix_memory_run_scratch(chunks, heads, dim, vdim), dtype=torch.float32, device=q.device)
+                    lib.mlr_matrix_memory_side_scratch.restype = ctypes.c_longlong
+                    ends = torch.empty(lib.mlr_matrix_memory_side_scratch(chunks, heads, dim, vdim), dtype=torch.float32, device=q.device)
                 else:
                     pairs = torch.empty((rows, heads, 66), dtype=torch.float32, device=q.device)
                     packed = torch.empty((rows, heads, 2 * dim + vdim), dtype=torch.bfloat16, device=q.device)

@@ -379,25 +379,25 @@ def test_sigmoid_attention_of_long_contexts(heads, kv_heads, dim, monkeypatch):
 
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 128), (3, 64, 72)])
 @pytest.mark.parametrize("lengths,slots,order", [([1, 512, 513, 1100], [3, 0, 2, 1], None), ([515, 3, 1030], [1, 2, 0], [2, 0, 1])])
-def test_matrix_memory_in_runs(heads, dim, vdim, lengths, slots, order):
-    """Segments around the borders of runs of four chunks and more, rows of requests in any order, gates that forget and keep everything: as
-    without runs (which the 64-bit oracle vouches for elsewhere), whose products are the same and whose sums another order."""
+def test_matrix_memory_of_long_portions(heads, dim, vdim, lengths, slots, order):
+    """Segments of many chunks side by side, rows of requests in any order, gates that forget and keep everything: as with one chunk behind the
+    other (which the 64-bit oracle vouches for elsewhere), whose products are the same and whose sums another order."""
     ctx, rows = segments(lengths, slots, order), sum(lengths)
-    assert cuda()._memory_chunks_fit(dim, vdim) and memory_run(ctx, rows, heads, vdim) > 0
+    assert cuda()._memory_chunks_fit(dim, vdim) and beside(ctx, rows, vdim)
     q, k, v, gate = rnd(1, rows, heads * dim), rnd(2, rows, heads * dim), rnd(3, rows, heads * vdim), rnd(4, rows, heads * vdim)
     i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
     f_raw[rows // 3], f_raw[rows // 2] = -80.0, 80.0
     bias, weight = torch.zeros(heads), 1 + rnd(7, heads * vdim, std=0.1)
     state, maximum = rnd(8, len(lengths), heads, vdim + 1, dim, std=0.5), rnd(9, len(lengths), heads)
     results = []
-    for runs in (False, True):
-        cuda().use_memory_runs = runs
+    for together in (False, True):
+        cuda().use_memory_side_by_side = together
         try:
             s, m = state.to(DEVICE), maximum.to(DEVICE)
             out = cuda().matrix_memory(*(spaced(t, 8) for t in (q, k, v, i_raw, f_raw)), bias.to(DEVICE), bias.to(DEVICE) + 3, 15.0, 1e-6,
                                        spaced(gate, 8), weight.to(DEVICE), 1e-6, s, m, ctx, heads, dim, vdim, torch.bfloat16)
         finally:
-            cuda().use_memory_runs = True
+            cuda().use_memory_side_by_side = True
         results.append((out.cpu(), s.cpu(), m.cpu()))
     (out, s, m), (want, want_s, want_m) = results[1], results[0]
     assert torch.equal(m, want_m)
@@ -609,10 +609,10 @@ def test_pairs_sorted_by_expert_in_several_turns(rows, top, experts):
 
 
 @pytest.mark.parametrize("lengths,slots,order", [([1, 512, 1100], [2, 0, 1], None), ([1030, 3], [1, 0], [1, 0])])
-def test_matrix_memory_in_runs_against_64_bits(lengths, slots, order):
+def test_matrix_memory_of_long_portions_against_64_bits(lengths, slots, order):
     heads, dim, vdim = 2, 64, 64
     ctx, rows = segments(lengths, slots, order), sum(lengths)
-    assert memory_run(ctx, rows, heads, vdim) > 0
+    assert beside(ctx, rows, vdim)
     q, k, v, gate = (rnd(i, rows, heads * 64) for i in range(4))
     i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
     f_raw[rows // 3], f_raw[rows // 2] = -80.0, 80.0
@@ -637,21 +637,21 @@ def test_matrix_memory_side_by_side(heads, dim, vdim, lengths, slots, order):
     """Portions of one chunk, one row more, one less and several beside each other, few and many value channels: as one chunk behind the other.  A number
     that is none leaves the rows before it as they are."""
     ctx, rows = segments(lengths, slots, order), sum(lengths)
-    assert memory_run(ctx, rows, heads, vdim) > 0
+    assert beside(ctx, rows, vdim)
     q, k, v, gate = rnd(1, rows, heads * dim), rnd(2, rows, heads * dim), rnd(3, rows, heads * vdim), rnd(4, rows, heads * vdim)
     i_raw, f_raw = rnd(5, rows, heads), rnd(6, rows, heads, std=2.0)
     gate[5], gate[6], gate[7] = -200.0, 200.0, -87.0
     bias, weight = torch.zeros(heads), 1 + rnd(7, heads * vdim, std=0.1)
     state, maximum = rnd(8, len(lengths), heads, vdim + 1, dim, std=0.5), rnd(9, len(lengths), heads)
 
-    def call(runs, v):
-        cuda().use_memory_runs = runs
+    def call(together, v):
+        cuda().use_memory_side_by_side = together
         try:
             s, m = state.to(DEVICE), maximum.to(DEVICE)
             out = cuda().matrix_memory(*(spaced(t, 8) for t in (q, k, v, i_raw, f_raw)), bias.to(DEVICE), bias.to(DEVICE) + 3, 15.0, 1e-6,
                                        spaced(gate, 8), weight.to(DEVICE), 1e-6, s, m, ctx, heads, dim, vdim, torch.bfloat16)
         finally:
-            cuda().use_memory_runs = True
+            cuda().use_memory_side_by_side = True
         return out.cpu(), s.cpu(), m.cpu()
 
     (out, s, m), (want, want_s, want_m) = call(True, v), call(False, v)
@@ -694,12 +694,12 @@ def test_matrix_memory_side_by_side_loses_no_bits_of_its_sums(heads, dim, vdim, 
                               s64, maximum.double(), types.SimpleNamespace(**{**vars(ctx), "seg_slot": ctx.seg_slot.cpu()}), heads, dim, vdim, torch.float64)
     errors, take = [], slice(0, 64) if what == "state" else slice(63, 64)
     for together in (False, True):
-        cuda().use_memory_runs = together
+        cuda().use_memory_side_by_side = together
         try:
             got = cuda().matrix_memory(*(t.to(DEVICE) for t in (q, k, v, i_raw, f_raw, zero, zero)), 100.0, 1e-6, gate.to(DEVICE), weight.to(DEVICE),
                                        1e-30, state.to(DEVICE), maximum.to(DEVICE), ctx, heads, dim, vdim, torch.bfloat16)
         finally:
-            cuda().use_memory_runs = True
+            cuda().use_memory_side_by_side = True
         errors.append(float((got.double().cpu() - want)[take].norm() / want[take].norm()))
     # 2^-18 of a sum's 24 bits leave six.  Thousands of numbers that were lost alike: the two means of squares differ by a few in a hundred by chance
     assert 2.0 ** -8 < errors[0] and errors[1] <= 1.03 * errors[0], errors
@@ -740,9 +740,9 @@ def test_matrix_memory_of_decoded_rows_beside_a_portion(heads, dim, vdim):
         assert torch.equal(own[2][part.slot], m[part.slot]), part.length
 
 
-def memory_run(ctx, rows, heads, vdim):
+def beside(ctx, rows, vdim):
     from mini_llm_runtime_b200.ops import build
-    return build.load_library("matrix_memory").mlr_matrix_memory_run(cuda()._chunks_from(ctx, rows, 1), ctx.num_segments, int(ctx.max_q_len), vdim)
+    return build.load_library("matrix_memory").mlr_matrix_memory_side_by_side(cuda()._chunks_from(ctx, rows, 1), ctx.num_segments, int(ctx.max_q_len), vdim)
 
 
 # Tiles of 128 outputs, of 16, 32, 64 and 128 rows, blocks of 64 k; 1, 2, 4 and 8 parts of the sums over k; more tiles than SMs, few rows too.
