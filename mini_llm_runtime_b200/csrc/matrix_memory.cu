@@ -984,13 +984,6 @@ struct SideShape {
   static constexpr size_t ENDS = Q + 3 * CHUNK * SIDE_PITCH * sizeof(bf16);
 };
 
-// 1 / (1 + e^-z) without a branch: one step of Newton's on the approximate reciprocal, which leaves it within an ulp of the exact one; beyond 1e37 the
-// approximation stands (also for infinity and NaN, where the step would give NaN).
-__device__ __forceinline__ float even_sigmoid(float z) {
-  const float d = 1.f + expf(-z), r = __fdividef(1.f, d);
-  return d < 1e37f ? fmaf(r, fmaf(-d, r, 1.f), r) : r;
-}
-
 // Warps 4 i .. 4 i + 3 take 16 rows each with the i-th share of the column pairs (of the tokens for A).  grid: (heads, chunks)
 template <int D, int PAIRS>
 __global__ void __launch_bounds__(SIDE_THREADS, 2)
@@ -1231,7 +1224,7 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
     const float factor = __shfl_sync(0xffffffffu, own_factor, i);
 #pragma unroll
     for (int j = 0; j < COLUMNS; ++j) {
-      const bf16 y = __float2bfloat16(x[i][j] * factor * weight[j] * even_sigmoid(gate[i][j]));
+      const bf16 y = __float2bfloat16(x[i][j] * factor * weight[j] * sigmoid(gate[i][j]));
       if (full || (first + i < count && lane + 32 * j < V)) dst[(size_t)i * p.heads * V + 32 * j] = y;
     }
   }
