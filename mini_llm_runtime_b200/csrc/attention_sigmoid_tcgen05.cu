@@ -648,13 +648,11 @@ static int sg_launch(SgArgs a, const void* k_pool, const void* v_pool, int ctas,
   if (!cached_tile_map(&k_map, k_pool, a.pool_rows, D, a.page_size < SG_KEY_BOX ? a.page_size : SG_KEY_BOX) ||
       !cached_tile_map(&v_map, v_pool, a.pool_rows, V, a.page_size < SG_KEYS / 2 ? a.page_size : SG_KEYS / 2))
     return MLR_BAD_SIZE;
-  static bool configured = false;
-  if (!configured) {
-    if (!sg_registers_fit<D, V>()) return MLR_TOO_LARGE;
-    cudaError_t err = cudaFuncSetAttribute(attention_sigmoid_tcgen05_kernel<D, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg_shared<D>(SG_HEADS));
-    if (err != cudaSuccess) return (int)err;
-    configured = true;
-  }
+  static OncePerDevice once;
+  const cudaError_t err = once([] {
+    return cudaFuncSetAttribute(attention_sigmoid_tcgen05_kernel<D, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg_shared<D>(SG_HEADS));
+  });
+  if (err != cudaSuccess) return (int)err;
   launch_kernel(attention_sigmoid_tcgen05_kernel<D, V>, dim3(ctas), dim3(SG_THREADS), sg_shared<D>(a.heads), stream, k_map, v_map, a);
   const int status = launch_status();
   if (status != MLR_OK || !cut) return status;

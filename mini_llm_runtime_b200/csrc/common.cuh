@@ -203,6 +203,20 @@ inline void launch_kernel_clustered_balanced(void (*kernel)(KernelArgs...), dim3
 #define MLR_DEFINE_PDL_SWITCH \
   MLR_EXPORT void mlr_set_pdl(int enabled) { mlr::pdl_enabled() = enabled != 0; }
 
+// What a kernel's first launch on a device sets (its dynamic shared memory), remembered per device.
+struct OncePerDevice {
+  bool done[64] = {};
+  template <typename F>
+  cudaError_t operator()(F&& set) {
+    int device = -1;
+    const bool known = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64;
+    if (known && done[device]) return cudaSuccess;
+    const cudaError_t err = set();
+    if (known && err == cudaSuccess) done[device] = true;
+    return err;
+  }
+};
+
 // Streaming multiprocessors of the current device, asked once per process and device; planners
 // size grids and split counts from it.
 inline int sm_count() {

@@ -227,12 +227,9 @@ template <bool GATED>
 static int launch_experts(const void* x, const void* w, const ExpertArgs& a, int rows, int groups, cudaStream_t stream) {
   CUtensorMap w_map, x_map;
   if (!cached_tile_map(&w_map, w, (long long)groups * a.N, a.K, EP_W_BOX) || !cached_tile_map(&x_map, x, rows, a.K, EP_X_BOX)) return MLR_BAD_ALIGNMENT;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(expert_product_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, EP_SHARED);
-    if (err != cudaSuccess) return (int)err;
-    configured = true;
-  }
+  static OncePerDevice once;
+  const cudaError_t err = once([] { return cudaFuncSetAttribute(expert_product_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, EP_SHARED); });
+  if (err != cudaSuccess) return (int)err;
   const int least = GATED ? EP_WEIGHTS : EP_WEIGHTS / 2;      // rows of a tile
   const long long tiles = (long long)((a.N + least - 1) / least) * a.entries;
   if (tiles > 0x3fffffff) return MLR_TOO_LARGE;

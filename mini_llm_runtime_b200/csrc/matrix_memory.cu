@@ -1235,8 +1235,13 @@ template <int D, int PAIRS>
 static int launch_side(const MemoryArgs& p, bf16* out, int chunks, int segments, cudaStream_t stream) {
   const int cells = (p.vdim + 1) * D;
   auto ends = p.least > 1 ? memory_ends_kernel<D, PAIRS, true> : memory_ends_kernel<D, PAIRS, false>;
-  cudaError_t err = cudaFuncSetAttribute(ends, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::ENDS);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(memory_outputs_kernel<D, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::SHARED);
+  static OncePerDevice once;
+  const cudaError_t err = once([] {
+    cudaError_t err = cudaFuncSetAttribute(memory_outputs_kernel<D, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::SHARED);
+    for (auto kernel : {memory_ends_kernel<D, PAIRS, true>, memory_ends_kernel<D, PAIRS, false>})
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SideShape<D>::ENDS);
+    return err;
+  });
   if (err != cudaSuccess) return (int)err;
   launch_kernel(ends, dim3(p.heads, chunks + (p.least > 1 ? segments : 0)), dim3(SIDE_THREADS), SideShape<D>::ENDS, stream, p, out, chunks);
   int status = launch_status();

@@ -660,9 +660,13 @@ int launch_space(const SpaceArgs& a, int rows, cudaStream_t stream) {
   const size_t ends_shared = SCANS && segment_shared > ENDS_SHARED ? segment_shared : ENDS_SHARED;
   if (SCANS && segment_shared > OUTPUTS_SHARED) return MLR_TOO_LARGE;
   const unsigned chunks = (unsigned)long_chunks(rows, a.segments, a.least);
-  cudaError_t err = cudaFuncSetAttribute(space_pairs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_shared);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(space_ends_kernel<N, SCANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ends_shared);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(space_outputs_kernel<N, SCANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUTPUTS_SHARED);
+  static OncePerDevice once;
+  const cudaError_t err = once([&] {
+    cudaError_t err = cudaFuncSetAttribute(space_pairs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_shared);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(space_ends_kernel<N, SCANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ends_shared);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(space_outputs_kernel<N, SCANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OUTPUTS_SHARED);
+    return err;
+  });
   if (err != cudaSuccess) return (int)err;
   launch_kernel(space_pairs_kernel<N>, dim3(chunks, a.groups * 2), dim3(PAIRS_THREADS), pairs_shared, stream, a);
   int status = launch_status();
