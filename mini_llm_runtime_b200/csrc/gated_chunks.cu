@@ -15,8 +15,8 @@
 //
 // One CTA used to walk a whole segment of a head (part), 0.4 us per token on 28 of 148 SMs (2,048 tokens, 14 heads of 64 x
 // 64): bound by the latency of that chain.  Walked in chunks it is bound by instructions issued: three operations per state
-// entry and token in the walk, one in finish.  2,048 tokens of one request, B200: 761 -> 63 us (14 heads of 64), 768 -> 114
-// (32 of 64), 608 -> 88 (7 of 128), 709 -> 158 (16 of 128).
+// entry and token in the walk, one in finish.  2,048 tokens of one request, repeated calls, B200: 761 -> 53 us (14 heads of 64), 768 -> 108
+// (32 of 64), 608 -> 77 (7 of 128), 709 -> 150 (16 of 128).
 #include "chunk_places.cuh"
 #include "copy_async.cuh"
 

@@ -757,13 +757,14 @@ static int launch_chunks(const MemoryArgs& p, int segments, int max_q_len, cudaS
 }
 
 // ------------------------------------------------------------------ chunks side by side
-// Bound by the tensor cores' rate for three products of parts with a warp's instructions between them: a block of the outputs takes some 23,000
-// cycles alone on an SM, of which 8,500 are the products with the state before (loads, split and products of a part after another), 3,000 the chunk's
-// own tokens and 6,500 normaliser, norm and gate; the ends 10,000, 4,100 of them products.  The carry moves the states of all chunks through L2.
+// Bound by the tensor cores' rate for three products of parts with a warp's instructions between them: a block of the outputs took some 23,000
+// cycles alone on an SM (before the leading products had a sum of their own, 2 us of a call), of which 8,500 were the products with the state before (loads, split
+// and products of a part after another), 3,000 the chunk's own tokens and 6,500 normaliser, norm and gate; the ends 10,000, 4,100 of them products.  The carry moves
+// the states of all chunks through L2.
 // 16 warps of half the columns each were slower (splits and fragments of A twice: 56 -> 61 us at the time), a branch around a pair that a warp does not have cost
-// 10 % of the products, and rows one after the other with their divisions and roots 4,500 cycles.  Whole calls, chunks one behind the other (or in runs of
-// four and more, which these kernels replace) / side by side, 7 heads of 128 x 128: 1,300 and 748 rows 86 / 44 us, 2,048 rows 78 / 46, 4,000 rows 153 / 76,
-// 512 rows 41 / 26; 16 heads: 2,048 rows 148 / 86, 8 of 200 rows 104 / 79.
+// 10 % of the products, and rows one after the other with their divisions and roots 4,500 cycles.  Repeated calls, chunks one behind the other (2,048 and 4,000 rows
+// in parts of four and more, which these kernels replace) / side by side, 7 heads of 128 x 128: 1,300 and 748 rows 90 / 48 us, 2,048 rows 83 / 49, 4,000 rows 154 / 81,
+// 512 rows 41 / 28; 16 heads: 2,048 rows 149 / 91; from a flushed L2 8 of 200 rows 112 / 94.
 constexpr int SIDE_THREADS = 256;
 constexpr int SIDE_V = 128;               // value channels at most
 constexpr int SIDE_PAIRS = SIDE_V / 16 + 1;      // pairs of eight columns, the normaliser's among them
@@ -1028,7 +1029,7 @@ memory_outputs_kernel(MemoryArgs p, bf16* __restrict__ out) {
   };
   ask(0);
   __syncthreads();
-  {      // thread (s, eighth): token s's share at the eighth's rows
+  {      // thread (s, quarter): token s's share at the quarter's rows
     constexpr int ROWS = CHUNK * CHUNK / SIDE_THREADS;
     const int s = threadIdx.x & (CHUNK - 1), t0 = threadIdx.x / CHUNK * ROWS;
     float x = write[s], all = 1.f;

@@ -17,10 +17,10 @@
 // at a time.  A weight of zero times an infinity would reach tokens that do not see it: from the first row with a number whose parts are not
 // finite on, a chunk goes by multiply-adds (ends_plain, outputs_plain), where such weights are left out; the rows before keep their bits.
 //
-// Bound by latency and instructions, three or four CTAs of four warps per SM (1.2 of 4 instructions per cycle, tensor pipes a tenth): splitting of states
-// and inputs, decays, copies.  Measured (B200), token by token / by multiply-adds / so: 2,048 rows of 32 heads with states of 128 639 / 117 / 103 us, of 14 heads
-// with states of 64 424 / 56 / 45; 512 rows 161 / 56 / 39 and 108 / 31 / 24; 4,000 rows 216 / 188 (32 heads); portions of 1,531, 77, 1 and 439 rows 125 / 118
-// and 58 / 53.  Errors against 64 bits (means of seven lengths, outputs / states) 7.8e-8 / 7.9e-8 by multiply-adds, 7.4e-8 / 7.8e-8 so.
+// Bound by latency and instructions, three or four CTAs of four warps per SM (1.5 and 1.1 of 4 instructions per cycle in ends and outputs, tensor pipes 31 and
+// 30 %): splitting of states and inputs, decays, copies.  Measured (B200, repeated calls), token by token / by multiply-adds / so: 2,048 rows of 32 heads with states
+// of 128 639 / 120 / 100 us, of 14 heads with states of 64 424 / 56 / 45; 512 rows 161 / 56 / 35 and 108 / 40 / 24; 4,000 rows 218 / 180 (32 heads); portions of 1,531, 77, 1
+// and 439 rows 124 / 107 and 60 / 47.  Errors against 64 bits (means of seven lengths, outputs / states) 7.8e-8 / 7.9e-8 by multiply-adds, 7.4e-8 / 7.8e-8 so.
 //
 #include "chunk_places.cuh"
 #include "copy_async.cuh"
@@ -347,7 +347,7 @@ space_ends_kernel(const __grid_constant__ SpaceArgs p) {
       *reinterpret_cast<float2*>(to + (size_t)(warp * 16 + r + 8 * i) * N + j * 8 + c2) = e;
     }
   // At the end, in all of these kernels: blocks of the next that come in while these still fill some SMs land several to an SM beside empty ones.
-  // Trigger in front / at the end: 14 heads of 64, 512 rows 30.5 / 23.9 us, 2,048 rows 51 / 46, 3 times 300 rows 34 / 29; 32 heads of 128, 2,048 rows 106 / 104.
+  // Trigger in front / at the end (with arguments copied to the stack still): 14 heads of 64, 512 rows 30.5 / 23.9 us, 2,048 rows 51 / 46, 3 times 300 rows 34 / 29; 32 heads of 128, 2,048 rows 106 / 104.
   pdl_trigger();
 }
 

@@ -2144,8 +2144,8 @@ class CudaOps:
 
     use_state_space_chunks = True
     # Portions of so many rows and more go in chunks, shorter ones beside them token by token, as above.  Measured in us from a flushed L2, token by
-    # token / in chunks, 14 heads with states of 64 (32 heads, 128): 97 rows 29 / 34 (31 / 40), 112 rows 31 / 33 (33 / 39), 128 rows 35 / 34 (37 / 38), 140 rows
-    # 37 / 34 (39 / 41), 160 rows 41 / 34 (44 / 41), 512 rows 108 / 24 (161 / 39) repeated.  Three of 100 rows beside one of 1,000 would gain from chunks too (55 / 45
+    # token / in chunks, 14 heads with states of 64 (32 heads, 128): 144 rows 37 / 30 (41 / 36), 160 rows 41 / 31 (43 / 36), 512 rows 108 / 24 (161 / 35) repeated; beside
+    # 77 rows 150 39 / 36 (51 / 43), beside 100 and 90 rows 150 39 / 38 (59 / 54).  Three of 100 rows beside one of 1,000 would gain from chunks too (before: 55 / 45
     # and 108 / 97), but which way a portion goes is a matter of its own rows, as its numbers are.
     STATE_SPACE_CHUNK_ROWS = 144
 
