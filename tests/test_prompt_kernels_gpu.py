@@ -273,14 +273,17 @@ def on_tcgen05(monkeypatch):
 
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,page_size", [(16, 4, 128, 128, 8), (14, 2, 64, 64, 16), (9, 3, 128, 64, 64), (5, 1, 64, 128, 256),
                                                                (4, 4, 64, 64, 128)])
-@pytest.mark.parametrize("lengths,before", [([129], [0]), ([16, 1, 8], [112, 640, 300]), ([1] * 7, [127, 128, 63, 64, 1000, 200, 500]), ([1] * 6, [2700, 3, 60, 127, 128, 11]),
-                                            ([70, 260, 9, 1], [250, 0, 127, 383]), ([1, 30, 17], [64, 70, 111]), ([40, 3, 1], [210, 250, 192]),
-                                            ([1] * 150 + [25], [40 + i % 88 for i in range(150)] + [100])])
-def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, lengths, before, monkeypatch):
+@pytest.mark.parametrize("lengths,before,limit", [
+    ([129], [0], 0), ([16, 1, 8], [112, 640, 300], 0), ([1] * 7, [127, 128, 63, 64, 1000, 200, 500], 0), ([1] * 6, [2700, 3, 60, 127, 128, 11], 0),
+    ([70, 260, 9, 1], [250, 0, 127, 383], 0), ([1, 30, 17], [64, 70, 111], 0), ([40, 3, 1], [210, 250, 192], 0),
+    ([1] * 150 + [25], [40 + i % 88 for i in range(150)] + [100], 0), ([1] * 6, [20, 300, 64, 127, 0, 500], 1024)])
+def test_sigmoid_attention_on_tcgen05(heads, kv_heads, dim, vdim, page_size, lengths, before, limit, monkeypatch):
     """Keys around tiles of 128 and their halves, rows around the 8 of half an entry, entries cut and whole, pages smaller and larger than a
-    tile and its halves, heads that do not fill fours; steps of one and two tiles per entry, of more entries than CTAs; places that no row sees hold NaN.  Mixing factors large enough that what mixing in fewer
+    tile and its halves, heads that do not fill fours; steps of one and two tiles per entry, of more entries than CTAs, planned for a context limit as captured
+    ones are; places that no row sees hold NaN.  Mixing factors large enough that what mixing in fewer
     than 32 bits would leave of the weights shows.  The second call finds the first one's scratch."""
     (k_pool, v_pool), cpu, batch = paged(lengths, before, lambda p, j: j <= p, page_size, [(kv_heads, dim, 1.0), (kv_heads, vdim, 0.5)], 11)
+    batch.max_kv_len = max(limit, batch.max_kv_len)
     assert cuda().use_tcgen05_attention and cuda_ops.build.load_library("attention_sigmoid_tcgen05").mlr_attention_sigmoid_tcgen05_fits(
         heads, kv_heads, dim, vdim, page_size)
     q = rnd(6, sum(lengths), heads * dim).to(torch.bfloat16)
